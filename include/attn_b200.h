@@ -114,6 +114,30 @@ typedef struct AttnB200ParallelArgs {
  * and the CuTe forward (core/template/cute_template/flash_api.cpp:283-460). */
 int attn_b200_parallel_fwd(const AttnB200ParallelArgs* args, void* cuda_stream);
 
+/* Decode through the built-in softmax: a few query rows per sequence, grouped KV heads, no mask; the cache may be of
+ * different lengths and of kept blocks only.  The query rows of a KV head (heads / heads_kv * seq_q) share a tile: at most
+ * 128 of them, 64 with lengths or a block mask.  dim (= dim_qk = dim_v) is 64 or 128.  Takes the place of the reference's
+ * decode templates (core/lower/lower_decode.py:375-449, core/template/tl_template/attn/blockattn_decode_varlen_tl.py). */
+typedef struct AttnB200DecodeArgs {
+  const void* q;               /* [batch, seq_q, heads, dim] through element strides, dim contiguous */
+  const void* k;               /* [batch, seq_kv, heads_kv, dim] */
+  const void* v;
+  void* o;
+  float* lse;                  /* [batch, heads, seq_q] or NULL */
+  int32_t batch, heads, heads_kv, seq_q, seq_kv, dim, dtype;
+  float scale;
+  int64_t q_stride[3], k_stride[3], v_stride[3], o_stride[3];   /* (batch, seq, head) */
+  const uint8_t* block_mask;   /* [batch, heads_kv, n_blocks], nonzero = keep the block_size tokens of the block; or NULL */
+  const int32_t* seq_lens;     /* [batch] tokens of each sequence (clamped to 0..seq_kv), or NULL = seq_kv */
+  int32_t n_blocks, block_size;   /* block_size: 8, 16, 32, 64 or 128; n_blocks at most 4096 */
+  void* workspace;             /* attn_b200_decode_workspace_bytes() bytes of device scratch */
+  int64_t workspace_bytes;
+} AttnB200DecodeArgs;
+
+/* Scratch of a call on the current device; -1 = the call is not one that attn_b200_decode_fwd covers. */
+int64_t attn_b200_decode_workspace_bytes(const AttnB200DecodeArgs* args);
+int attn_b200_decode_fwd(const AttnB200DecodeArgs* args, void* cuda_stream);
+
 /* Bytes of scratch the forward needs for args->num_splits (0 without split-KV; -1 = bad arguments): fp32 partial
  * rows plus ATTN_B200_MAX_ROWSCALES final row scales per row and split.  Valid for *_jit libraries as well. */
 int64_t attn_b200_parallel_workspace_bytes(const AttnB200ParallelArgs* args);

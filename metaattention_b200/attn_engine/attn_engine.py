@@ -305,6 +305,9 @@ class AttentionEngine:
             # the backward of an elementwise program: source now, compiled when a gradient is first asked for
             if derivative.elementwise_program(tr) and D in (64, 128) and Dv % D == 0:
                 self._bwd_source = derivative.backward_translation_unit(derivative.emit_backward_functor(tr), D, dtype == torch.bfloat16)
+        # programs that attn_b200_decode_fwd computes (a forced split count, kv_splits, asks for the other kernel)
+        self._may_decode = (scale is not None and self.mask_kind == native.MASK_NONE and self._sparse_host is None and
+                            len(self.final_names) == 1 and D == Dv and D in (64, 128))
         self.attention = self._run_parallel
 
     def _run_parallel(self, q, k, v, *custom, block_mask=None, cache_seqlens=None):
@@ -403,6 +406,12 @@ class AttentionEngine:
         # the entry points launch on the CURRENT device and stream: make q's device current for the whole call
         with torch.cuda.device(q.device):
             sparse = None
+            if self._may_decode and self.kv_splits is None and S * H <= 128 * k.shape[2] and k.shape[1] > 128:
+                # the query rows of the heads that share a KV head fit one tile: the decode kernel, if it covers the call
+                out = native.decode_fwd(q, k, v, self._fparams[0], block_mask, cache_seqlens, self._decode_block or 0)
+                if out is not None:
+                    self.last_final_rowscales = {self.final_names[0]: out[1]}
+                    return out[0]
             if self._decode_block is not None:
                 # block-sparse, variable-length decode (examples/sparse_gqa_decode.py, blockattn_decode_varlen_tl.py):
                 # the call's block_mask [B, Hkv, blocks] and cache_seqlens [B] become, on the device, the bitmaps of

@@ -67,6 +67,17 @@ class ParallelArgs(C.Structure):
     ]
 
 
+class DecodeArgs(C.Structure):
+    _fields_ = [
+        ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("o", C.c_void_p), ("lse", C.c_void_p),
+        ("batch", C.c_int32), ("heads", C.c_int32), ("heads_kv", C.c_int32), ("seq_q", C.c_int32), ("seq_kv", C.c_int32),
+        ("dim", C.c_int32), ("dtype", C.c_int32), ("scale", C.c_float),
+        ("q_stride", C.c_int64 * 3), ("k_stride", C.c_int64 * 3), ("v_stride", C.c_int64 * 3), ("o_stride", C.c_int64 * 3),
+        ("block_mask", C.c_void_p), ("seq_lens", C.c_void_p), ("n_blocks", C.c_int32), ("block_size", C.c_int32),
+        ("workspace", C.c_void_p), ("workspace_bytes", C.c_int64),
+    ]
+
+
 class LinearArgs(C.Structure):
     _fields_ = [
         ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("log_decay", C.c_void_p), ("o", C.c_void_p),
@@ -127,6 +138,8 @@ class MlaArgs(C.Structure):
 SIGNATURES = {
     "attn_b200_parallel_fwd": (C.c_int, [C.POINTER(ParallelArgs), C.c_void_p]),
     "attn_b200_parallel_workspace_bytes": (C.c_int64, [C.POINTER(ParallelArgs)]),
+    "attn_b200_decode_workspace_bytes": (C.c_int64, [C.POINTER(DecodeArgs)]),
+    "attn_b200_decode_fwd": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     "attn_b200_decode_tiles_bytes": (C.c_int64, [C.c_int32, C.c_int32, C.c_int32]),
     "attn_b200_decode_tiles": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                          C.c_void_p, C.c_int64, C.c_void_p]),
@@ -153,7 +166,7 @@ _lib = None
 
 
 def library_sources() -> list[str]:
-    return [os.path.join(CSRC_DIR, f) for f in ("attn_b200.cu", "mla_decode.cu", "linear_fwd.cu", "softmax_bwd.cu", "row_ops.cu")]
+    return [os.path.join(CSRC_DIR, f) for f in ("attn_b200.cu", "decode_fwd.cu", "mla_decode.cu", "linear_fwd.cu", "softmax_bwd.cu", "row_ops.cu")]
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
@@ -284,6 +297,51 @@ def fill_parallel_args(q, k, v, o, *, mask_kind: int, functor: int = 0, fparams=
     return a
 
 
+def _decode_operands(block_mask, cache_seqlens, batch: int, heads_kv: int, device):
+    """The call-time block_mask / cache_seqlens of a decode as the uint8 / int32 device tensors the library reads."""
+    if block_mask is not None:
+        if block_mask.dim() != 3 or block_mask.shape[0] != batch or block_mask.shape[1] != heads_kv:
+            raise NativeError(f"block_mask must be [batch, kv heads, blocks] = [{batch}, {heads_kv}, *], got {tuple(block_mask.shape)}")
+        block_mask = block_mask.to(device=device).contiguous()
+        block_mask = block_mask.view(torch.uint8) if block_mask.dtype == torch.bool else block_mask.to(torch.uint8)
+    if cache_seqlens is not None:
+        if cache_seqlens.numel() != batch:
+            raise NativeError(f"cache_seqlens must hold one length per sequence ({batch}), got {cache_seqlens.numel()}")
+        cache_seqlens = cache_seqlens.to(device=device, dtype=torch.int32).contiguous()
+    return block_mask, cache_seqlens
+
+
+def decode_fwd(q, k, v, scale: float, block_mask=None, cache_seqlens=None, block_size: int = 0):
+    """(o, lse) of softmax(scale * q.k).v for a few query rows against a long cache through attn_b200_decode_fwd, or None if
+    the call is not one it covers (see the header: head dims, rows of a group, block sizes).  q [B, Sq, H, D],
+    k, v [B, Skv, Hkv, D] with contiguous last dim."""
+    B, Sq, H, D = q.shape
+    Skv, Hkv = k.shape[1], k.shape[2]
+    if v.shape[3] != D or D not in (64, 128) or v.shape[2] != Hkv or H % Hkv != 0:
+        return None
+    if q.dtype not in DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype or q.stride(3) != 1 or k.stride(3) != 1 or v.stride(3) != 1:
+        return None
+    block_mask, cache_seqlens = _decode_operands(block_mask, cache_seqlens, B, Hkv, q.device)
+    a = DecodeArgs()
+    a.batch, a.heads, a.heads_kv, a.seq_q, a.seq_kv, a.dim, a.dtype, a.scale = B, H, Hkv, Sq, Skv, D, DTYPE_CODES[q.dtype], scale
+    if block_mask is not None:
+        a.block_mask, a.n_blocks, a.block_size = block_mask.data_ptr(), block_mask.shape[2], block_size
+    if cache_seqlens is not None:
+        a.seq_lens = cache_seqlens.data_ptr()
+    lib = load_library()
+    need = lib.attn_b200_decode_workspace_bytes(C.byref(a))
+    if need < 0:
+        return None
+    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
+    o = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
+    lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
+    a.workspace, a.workspace_bytes = ws.data_ptr(), need
+    a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
+    a.q_stride[:], a.k_stride[:], a.v_stride[:], a.o_stride[:] = _strides_bsh(q), _strides_bsh(k), _strides_bsh(v), _strides_bsh(o)
+    check(lib.attn_b200_decode_fwd(C.byref(a), current_stream_ptr()), "attn_b200_decode_fwd")
+    return o, lse
+
+
 def decode_tiles(block_mask, cache_seqlens, batch: int, heads_kv: int, seq_kv: int, block_size: int, device) -> dict:
     """Sparse-walk description (see fill_parallel_args ``sparse``) of a block-sparse, variable-length decode, built
     on the device by attn_b200_decode_tiles.  block_mask: bool/uint8 [batch, heads_kv, blocks] or None;
@@ -293,17 +351,8 @@ def decode_tiles(block_mask, cache_seqlens, batch: int, heads_kv: int, seq_kv: i
     words = (tiles + 31) // 32
     bh = batch * heads_kv
     out = torch.empty(int(lib.attn_b200_decode_tiles_bytes(batch, heads_kv, seq_kv)) // 4, dtype=torch.int32, device=device)
-    n_blocks = 0
-    if block_mask is not None:
-        if block_mask.dim() != 3 or block_mask.shape[0] != batch or block_mask.shape[1] != heads_kv:
-            raise NativeError(f"block_mask must be [batch, kv heads, blocks] = [{batch}, {heads_kv}, *], got {tuple(block_mask.shape)}")
-        block_mask = block_mask.to(device=device).contiguous()
-        block_mask = block_mask.view(torch.uint8) if block_mask.dtype == torch.bool else block_mask.to(torch.uint8)
-        n_blocks = block_mask.shape[2]
-    if cache_seqlens is not None:
-        if cache_seqlens.numel() != batch:
-            raise NativeError(f"cache_seqlens must hold one length per sequence ({batch}), got {cache_seqlens.numel()}")
-        cache_seqlens = cache_seqlens.to(device=device, dtype=torch.int32).contiguous()
+    block_mask, cache_seqlens = _decode_operands(block_mask, cache_seqlens, batch, heads_kv, device)
+    n_blocks = block_mask.shape[2] if block_mask is not None else 0
     check(lib.attn_b200_decode_tiles(block_mask.data_ptr() if block_mask is not None else None,
                                      cache_seqlens.data_ptr() if cache_seqlens is not None else None,
                                      batch, heads_kv, n_blocks, int(block_size), seq_kv, out.data_ptr(), out.numel() * 4,

@@ -39,9 +39,9 @@ inline TensorMapEncodeTiledFn tensor_map_encoder() {
 // element strides (dim contiguous).  Dimension 0 of the map is `dim`; the
 // other three are ordered by increasing stride, and `order` tells the kernel
 // where each coordinate goes.  Box: 64 elements (128 bytes, the swizzle span)
-// of one head and one batch entry by `box_rows` sequence positions.
+// of `box_heads` heads and one batch entry by `box_rows` sequence positions.
 inline int encode_rows_map(CUtensorMap* tm, CoordOrder* order, const void* base, int dtype, int dim, int batch,
-                           int seq, int heads, const int64_t stride_bsh[3], int box_rows) {
+                           int seq, int heads, const int64_t stride_bsh[3], int box_rows, int box_heads = 1) {
   TensorMapEncodeTiledFn enc = tensor_map_encoder();
   if (enc == nullptr) return ATTN_B200_E_LAUNCH;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
@@ -70,6 +70,7 @@ inline int encode_rows_map(CUtensorMap* tm, CoordOrder* order, const void* base,
   for (int i = 0; i < 3; ++i) {
     pos[dims[i].which] = i + 1;
     if (dims[i].which == 1) box[i + 1] = (cuuint32_t)box_rows;
+    if (dims[i].which == 2) box[i + 1] = (cuuint32_t)box_heads;
   }
   order->pos_b = pos[0];
   order->pos_s = pos[1];

@@ -1,0 +1,105 @@
+"""The decode kernel (attn_b200_decode_fwd) against softmax attention in fp32: query rows packed by KV head, shares of the
+tile list that cut sequences, lengths, gathered blocks."""
+
+import pytest
+import torch
+
+from core.native import lib
+from examples_b200 import programs
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(q, k, v, scale, keep=None):
+    """q [B,Sq,H,D], k/v [B,S,Hkv,D] on the GPU, keep [B,Hkv,S] or None -> (o, lse) in fp32"""
+    g = q.shape[2] // k.shape[2]
+    kf, vf = (t.float().repeat_interleave(g, 2) for t in (k, v))
+    s = torch.einsum("bshd,bthd->bhst", q.float(), kf) * scale
+    if keep is not None:
+        s = s.masked_fill(~keep.repeat_interleave(g, 1)[:, :, None], -float("inf"))
+    return torch.einsum("bhst,bthd->bshd", s.softmax(-1), vf), s.logsumexp(-1)
+
+
+def check(got, want, dtype):
+    """o: the roundings of P (one unit of its 16-bit type, relative) and of o itself; |o| stays below ~4 here.  lse: fp32
+    sums of ex2.approx results, whose errors are below 2^-20."""
+    o, lse = got
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    ref = want[0].abs().max().item()
+    assert (o.float() - want[0]).abs().max().item() <= 2 * eps * max(1.0, ref)
+    assert (lse - want[1]).abs().max().item() <= 2e-5 * max(1.0, want[1].abs().max().item())
+
+
+def rand(gen, *shape, dtype):
+    return torch.randn(*shape, generator=gen, device="cuda").to(dtype)
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,S,D,dtype", [
+    (1, 1, 1, 1, 129, 128, torch.bfloat16),       # two tiles, the second with one row
+    (1, 4, 1, 1, 128 * 149, 128, torch.bfloat16),   # one tile more than an SM each
+    (2, 32, 8, 1, 1000, 128, torch.float16),      # shares that begin and end inside a pair
+    (3, 8, 8, 1, 257, 64, torch.bfloat16),        # fewer tiles than SMs
+    (37, 8, 4, 1, 300, 64, torch.float16),        # a whole pair per share: 148 pairs, nothing to merge
+    (40, 16, 8, 1, 130, 128, torch.bfloat16),     # shares of several pairs of two tiles
+    (2, 33, 1, 1, 700, 128, torch.bfloat16),      # two warps of a softmax group, the second with one row
+    (2, 16, 2, 8, 513, 64, torch.float16),        # 64 rows
+    (3, 32, 1, 4, 900, 128, torch.bfloat16),      # 128 rows: one query buffer
+    (5, 8, 2, 25, 2000, 64, torch.bfloat16),      # 100 rows
+])
+def test_dense(B, H, Hkv, Sq, S, D, dtype):
+    gen = torch.Generator(device="cuda").manual_seed(S + D)
+    q, k, v = rand(gen, B, Sq, H, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype)
+    k[..., S // 2:, :, :] *= 3.0   # the running maximum moves: accumulators are rescaled
+    got = lib.decode_fwd(q, k, v, D ** -0.5)
+    want = reference(q, k, v, D ** -0.5)
+    check(got, want, dtype)
+    # another order of the query rows: heads outside the sequence axis
+    qh = q.transpose(1, 2).contiguous().transpose(1, 2)
+    check(lib.decode_fwd(qh, k.transpose(1, 2).contiguous().transpose(1, 2), v, D ** -0.5), want, dtype)
+    # the engine's call
+    o = programs.gqa_engine(B, H, Hkv, Sq, S, D, D, dtype=dtype)(q, k, v)
+    assert torch.equal(o, got[0])
+    assert lib.last_device_status() == 0
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,S,D,block,masked,varlen", [
+    (3, 8, 2, 1, 1024, 128, 32, True, True),
+    (2, 8, 8, 1, 1000, 128, 8, True, True),        # 125 blocks: rows of the mask are read byte by byte
+    (5, 16, 4, 4, 777, 64, 16, True, False),       # the last block lies partly behind the sequence
+    (4, 32, 4, 1, 4096, 128, 64, True, True),
+    (70, 8, 4, 1, 640, 64, 128, True, True),       # more pairs than SMs
+    (6, 8, 2, 2, 2000, 128, 32, False, True),      # lengths only
+])
+def test_blocks_and_lengths(B, H, Hkv, Sq, S, D, block, masked, varlen):
+    dtype = torch.bfloat16
+    gen = torch.Generator(device="cuda").manual_seed(S + block)
+    q, k, v = rand(gen, B, Sq, H, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype)
+    nb = -(-S // block)
+    mask = torch.rand(B, Hkv, nb, generator=gen, device="cuda") < 0.4 if masked else None
+    lens = torch.randint(1, S + 1, (B,), generator=gen, device="cuda", dtype=torch.int32) if varlen else None
+    if varlen:
+        lens[0], lens[1] = S, 1
+    if masked:
+        mask[:, :, 0] = True
+        mask[1, 0] = False        # a pair without a kept block
+    keep = torch.ones(B, Hkv, S, dtype=torch.bool, device="cuda")
+    if masked:
+        keep &= mask.repeat_interleave(block, -1)[..., :S]
+    if varlen:
+        keep &= (torch.arange(S, device="cuda") < lens[:, None])[:, None]
+    o, lse = lib.decode_fwd(q, k, v, D ** -0.5, mask, lens, block)
+    want_o, want_lse = reference(q, k, v, D ** -0.5, keep)
+    some = keep.any(-1).repeat_interleave(H // Hkv, 1)     # [B, H]
+    assert torch.isnan(o.transpose(1, 2)[~some]).all() and (lse[~some] == -float("inf")).all()
+    check((o.transpose(1, 2)[some], lse[some]), (want_o.transpose(1, 2)[some], want_lse[some]), dtype)
+    again = lib.decode_fwd(q, k, v, D ** -0.5, mask, lens, block)
+    assert torch.equal(o.nan_to_num(7.0), again[0].nan_to_num(7.0)) and torch.equal(lse, again[1])
+    assert lib.last_device_status() == 0
+
+
+def test_calls_outside_its_range_are_left_to_the_forward_kernel():
+    q, k = torch.zeros(1, 1, 129, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 256, 1, 64, dtype=torch.bfloat16, device="cuda")
+    assert lib.decode_fwd(q, k, k, 1.0) is None                                    # 129 rows
+    mask = torch.ones(1, 1, 6, dtype=torch.bool, device="cuda")
+    assert lib.decode_fwd(q[:, :, :1], k, k, 1.0, mask, None, 48) is None           # a block that does not divide a tile
+    assert lib.decode_fwd(q[..., :48], k[..., :48], k[..., :48], 1.0) is None      # another head dim
