@@ -124,19 +124,21 @@ struct TileWalk {
 
 constexpr int kMaxTileWords = 128;   // sparse walks: at most 4096 KV tiles (512 k tokens)
 
-// NT = query tiles per CTA: 2 (K/V in two stages, shared by both tiles) or 1 (single-staged K/V; the layout that
-// fits dim_qk = 256: one 64 KB query tile, 64 KB of K, 32 KB of V)
+// NT = query tiles per CTA: 2 (K/V shared by both tiles, in two stages; with dim_qk = 192 the tiles leave room for one
+// stage of V: it is free from the second tile's P.V on and needed again behind the other tile's Q.K^T and functor stage,
+// later than its load takes) or 1 (single-staged K/V; the layout that fits dim_qk = 256: one 64 KB query tile, 64 KB
+// of K, 32 KB of V)
 template <int D, int DV, int NT = 2>
 struct ParallelSmem {
-  static constexpr int kBM = 128, kBN = 128, kStages = NT == 2 ? 2 : 1;
+  static constexpr int kBM = 128, kBN = 128, kStages = NT == 2 ? 2 : 1, kVStages = NT == 2 && D <= 128 ? 2 : 1;
   static constexpr int kQBytes = kBM * D * 2;
   static constexpr int kKBytes = kBN * D * 2;
   static constexpr int kVBytes = kBN * DV * 2;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = kOffQ + NT * kQBytes;
   static constexpr int kOffV = kOffK + kStages * kKBytes;
-  static constexpr int kOffBar = kOffV + kStages * kVBytes;
-  static constexpr int kNumBars = 2 + 4 * kStages + 6;
+  static constexpr int kOffBar = kOffV + kVStages * kVBytes;
+  static constexpr int kNumBars = 2 + 2 * kStages + 2 * kVStages + 6;
   static constexpr int kOffMisc = kOffBar + 8 * kNumBars;
   static constexpr int kOffSparse = kOffMisc + 16;     // sparse kernels: keep / partial bitmaps of the two query tiles
   static constexpr int kBytes = kOffMisc + 16 + 1024;  // + slack for manual 1024-byte alignment
@@ -148,8 +150,8 @@ __global__ void __launch_bounds__((4 * NT + 2) * 32, 1)
 parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const ParallelParams p) {
   using L = ParallelSmem<D, DV, NT>;
-  constexpr int BM = L::kBM, BN = L::kBN, ST = L::kStages;
-  static_assert(D % 64 == 0 && DV % 64 == 0 && DV <= 128 && (D <= 128 || (D <= 256 && NT == 1)), "unsupported head dims");
+  constexpr int BM = L::kBM, BN = L::kBN, ST = L::kStages, STV = L::kVStages;
+  static_assert(D % 64 == 0 && DV % 64 == 0 && DV <= 128 && (D <= 192 || (D <= 256 && NT == 1)), "unsupported head dims");
   static_assert((kSparse ? L::kBytesSparse : L::kBytes) <= 232448, "shared memory layout exceeds an SM");
   constexpr uint32_t kTmemCols = NT == 2 ? 512 : 256;
   constexpr uint32_t kColS = 0, kColO = NT * 128;
@@ -165,8 +167,8 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* k_full = bars + 2;
   uint64_t* k_empty = k_full + ST;
   uint64_t* v_full = k_empty + ST;
-  uint64_t* v_empty = v_full + ST;
-  uint64_t* s_full = v_empty + ST;   // [2] one per query tile
+  uint64_t* v_empty = v_full + STV;
+  uint64_t* s_full = v_empty + STV;   // [2] one per query tile
   uint64_t* p_ready = s_full + 2;    // [2]
   uint64_t* o_done = p_ready + 2;    // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
@@ -253,7 +255,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tma_load_rows(sK + st * L::kKBytes + c * (BN * 128), &tmK, &k_full[st], c * 64, j * BN, h / p.kv_group, b, p.ok);
   };
   auto load_v_tile = [&](int i, int j) {
-    const int st = i % ST;
+    const int st = i % STV;
     mbar_arrive_expect_tx(&v_full[st], L::kVBytes);
     for (int c = 0; c < DV / 64; ++c)
       tma_load_rows(sV + st * L::kVBytes + c * (BN * 128), &tmV, &v_full[st], c * 64, j * BN, h / p.kv_group, b, p.ov);
@@ -275,6 +277,8 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < ST; ++i) {
       mbar_init(&k_full[i], 1);
       mbar_init(&k_empty[i], 1);
+    }
+    for (int i = 0; i < STV; ++i) {
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
     }
@@ -320,7 +324,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const uint32_t ph = (i / ST) & 1;
           if (i >= ST && !mbar_wait(&k_empty[st], ph ^ 1, ab, kSiteKEmpty)) break;
           load_k_tile(i, j);
-          if (i >= ST && !mbar_wait(&v_empty[st], ph ^ 1, ab, kSiteVEmpty)) break;
+          if (i >= STV && !mbar_wait(&v_empty[i % STV], ((i / STV) & 1) ^ 1, ab, kSiteVEmpty)) break;
           load_v_tile(i, j);
         }
       }
@@ -330,7 +334,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const uint32_t ph = (i / ST) & 1;
         if (!mbar_wait(&k_empty[st], ph ^ 1, ab, kSiteKEmpty)) break;
         load_k(i);
-        if (!mbar_wait(&v_empty[st], ph ^ 1, ab, kSiteVEmpty)) break;
+        if (!mbar_wait(&v_empty[i % STV], ((i / STV) & 1) ^ 1, ab, kSiteVEmpty)) break;
         load_v(i);
       }
     }
@@ -400,9 +404,9 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         for (int i = 0; i < n_max && ok; ++i) {
           const int jn = walk.next();
-          const int st = i % ST;
+          const int st = i % STV;
           const int stn = (i + 1) % ST;
-          ok = wait(&v_full[st], (i / ST) & 1, kSiteVFull);
+          ok = wait(&v_full[st], (i / STV) & 1, kSiteVFull);
           if (ok && jn >= 0) ok = wait(&k_full[stn], ((i + 1) / ST) & 1, kSiteKFull);
           if (!ok) break;
           for (int t = 0; t < NT; ++t) {
@@ -430,9 +434,9 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         commit2(&k_empty[0], nullptr);
         for (int i = 0; i < n_max && ok; ++i) {
           const int j = j_min + i;
-          const int st = i % ST;
+          const int st = i % STV;
           const int stn = (i + 1) % ST;
-          ok = wait(&v_full[st], (i / ST) & 1, kSiteVFull);
+          ok = wait(&v_full[st], (i / STV) & 1, kSiteVFull);
           if (ok && i + 1 < n_max) ok = wait(&k_full[stn], ((i + 1) / ST) & 1, kSiteKFull);
           if (!ok) break;
           for (int t = 0; t < NT; ++t) {
