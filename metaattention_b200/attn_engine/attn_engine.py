@@ -88,63 +88,12 @@ class _ForwardOnly(torch.autograd.Function):
                                   "inputs), with no mask or a causal mask and head dims 128 / 128 or 64 / 64")
 
 
-class _SoftmaxAttention(torch.autograd.Function):
-    """Softmax attention with its native backward (attn_b200_softmax_bwd), the counterpart of the reference's
-    ``_attention`` autograd function (core/template/tl_template/attn/attn_tl.py:654-694): the forward keeps o and the
-    log-sum-exp, the backward recomputes the probabilities from them."""
-
-    @staticmethod
-    def forward(ctx, engine, q, k, v):
-        q, k, v = q.detach(), k.detach(), v.detach()
-        o = engine._run_parallel_impl(q, k, v)
-        lse = engine.last_final_rowscales[engine.final_names[0]]
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.engine = engine
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        q, k, v, o, lse = ctx.saved_tensors
-        eng = ctx.engine
-        dq, dk, dv = native.softmax_bwd(q, k, v, o, lse, d_o.to(q.dtype), eng._fparams[0], eng.mask_kind, eng.mask_band,
-                                        eng._mask_bits(q.device))
-        return None, dq, dk, dv
-
-
-class _ElementwiseAttention(torch.autograd.Function):
-    """An elementwise program (P = f(q.k): sigmoid, relu attention ...) with the backward derived from its traced
-    score_mod (core/lower/derivative.py) and compiled on first use."""
-
-    @staticmethod
-    def forward(ctx, engine, n_custom, q, k, v, *custom):
-        q, k, v = q.detach(), k.detach(), v.detach()
-        custom = tuple(t.detach() if isinstance(t, torch.Tensor) else t for t in custom)
-        o = engine._run_parallel_impl(q, k, v, *custom)
-        ctx.save_for_backward(q, k, v, *custom)
-        ctx.engine = engine
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        q, k, v, *custom = ctx.saved_tensors
-        eng = ctx.engine
-        if eng._bwd_fn is None:
-            eng._bwd_fn = native_jit.load_backward(eng._bwd_source)
-        dq, dk, dv = native.elementwise_bwd(eng._bwd_fn, q, k, v, d_o.to(q.dtype), eng.mask_kind, custom, eng.mask_band,
-                                            eng._mask_bits(q.device))
-        return (None, None, dq, dk, dv) + (None,) * len(custom)
-
-
 def plan_kv_splits(batch: int, heads: int, q_len: int, kv_len: int, device) -> int:
     """KV splits for the forward kernel: 1 unless the (query tile pair, head, batch) grid fills less than half of
     the SMs; then as many as fit, each keeping at least four 128-row KV tiles (a split re-reads Q and adds a
     combine pass)."""
-    ctas = batch * heads * ((q_len + 255) // 256)
-    sms = torch.cuda.get_device_properties(device).multi_processor_count
-    kv_tiles = (kv_len + 127) // 128
-    if 2 * ctas > sms or kv_tiles < 8:
-        return 1
-    return max(1, min(sms // ctas, kv_tiles // 4, 65535 // max(batch, 1)))
+    index = torch.device(device).index
+    return native.host().kv_splits(batch, heads, q_len, kv_len, torch.cuda.current_device() if index is None else index)
 
 
 MASK_GENERAL = -1   # classify_mask: not a band, or different per batch / head: runs as a block-sparse walk
@@ -200,7 +149,7 @@ class AttentionEngine:
         self._decode_block = None  # block size of a call-time block_mask (block-sparse, variable-length decode)
         self._sparse_host = None   # block-sparse walk of a general mask_mod (built once, on the CPU)
         self._bwd_source = None    # translation unit of the backward functor library (elementwise programs)
-        self._bwd_fn = None
+        self._plan = None          # native form of all this (csrc/host_ops.cpp), made at the first call
         self._sparse_dev = {}      # its copies by device
         self.kv_splits = None      # None = planned per call (plan_kv_splits); an int forces the split count
         self.qkv_meta = qkv_meta
@@ -292,7 +241,6 @@ class AttentionEngine:
         if scale is not None:
             self.functor_kind = "builtin_softmax"
             self._fparams = [scale]
-            self._jit_fn = None
             native.load_library() if torch.cuda.is_available() else None
         else:
             self.functor_kind = "lowered"
@@ -301,7 +249,6 @@ class AttentionEngine:
             self.functor_source = functor_lowering.translation_unit(fs, D, Dv, dtype == torch.bfloat16, sparse=self.sparse_walk)
             # compile now (works without a GPU); loading is deferred to the first call
             native_jit.build(self.functor_source)
-            self._jit_fn = None
             # the backward of an elementwise program: source now, compiled when a gradient is first asked for
             if derivative.elementwise_program(tr) and D in (64, 128) and Dv % D == 0:
                 self._bwd_source = derivative.backward_translation_unit(derivative.emit_backward_functor(tr), D, dtype == torch.bfloat16)
@@ -311,17 +258,44 @@ class AttentionEngine:
         self.attention = self._run_parallel
 
     def _run_parallel(self, q, k, v, *custom, block_mask=None, cache_seqlens=None):
-        if self._decode_block is not None:
+        if torch.is_grad_enabled() and (q.requires_grad or k.requires_grad or v.requires_grad):
+            if self._differentiates(q, v, custom):
+                return self._run_parallel_impl(q, k, v, *custom, block_mask=block_mask, cache_seqlens=cache_seqlens, grad=True)
             run = lambda *ts: self._run_parallel_impl(*ts, block_mask=block_mask, cache_seqlens=cache_seqlens)  # noqa: E731
-        else:
-            run = self._run_parallel_impl
-        if any(t.requires_grad for t in (q, k, v)) and torch.is_grad_enabled():
-            if self.has_backward(q, v) and not custom:
-                return _SoftmaxAttention.apply(self, q, k, v)
-            if self._bwd_source is not None and self._masked_for_backward():
-                return _ElementwiseAttention.apply(self, len(custom), q, k, v, *custom)
             return _ForwardOnly.apply(run, q, k, v, *custom)
-        return run(q, k, v, *custom)
+        return self._run_parallel_impl(q, k, v, *custom, block_mask=block_mask, cache_seqlens=cache_seqlens)
+
+    def _differentiates(self, q, v, custom) -> bool:
+        if self.functor_kind == "builtin_softmax":
+            return not custom and self.has_backward(q, v)
+        return self._bwd_source is not None and self._masked_for_backward()
+
+    def _make_plan(self):
+        """What was decided at construction, for the native side: constants, the address of the functor library's entry
+        point, and callbacks for what is made when a device or a gradient is first met."""
+        fn = 0
+        if self.functor_kind == "lowered":
+            fn = C.cast(native_jit.load(self.functor_source), C.c_void_p).value
+
+        def load_mask(device):
+            if device not in self._sparse_dev:
+                self._sparse_dev[device] = sparse_lowering.to_device(self._sparse_host, device)
+            return self._sparse_dev[device]
+
+        def load_backward():
+            return C.cast(native_jit.load_backward(self._bwd_source), C.c_void_p).value
+
+        def custom_spec(sym, dtype):
+            axes = custom_axes(sym)
+            literal = [int(d) if ax is None and d.isdigit() else -1 for ax, d in zip(axes, sym.shape_idx)]
+            return [-1 if ax is None else ax for ax in axes], literal, dtype == torch.float32, dtype == torch.bfloat16
+        self._plan = native.host().make_plan({
+            "builtin": self.functor_kind == "builtin_softmax", "fn": fn, "fparams": self._fparams, "n_final": len(self.final_names),
+            "mask_kind": self.mask_kind, "left": self.mask_band[0], "right": self.mask_band[1], "may_decode": self._may_decode,
+            "decode_block": self._decode_block or 0, "has_mask_walk": self._sparse_host is not None and self._decode_block is None,
+            "backward": 1 if self.functor_kind == "builtin_softmax" else 2, "load_mask": load_mask, "load_backward": load_backward,
+            "custom": [custom_spec(s, d) for s, d in zip(self._custom_syms, self._custom_dtypes)]})
+        return self._plan
 
     def _masked_for_backward(self) -> bool:
         """Masks the backward kernels take: none, causal, bands, and any other mask_mod that does not use the batch or
@@ -392,7 +366,18 @@ class AttentionEngine:
             strides.append(st)
         return tensors, strides
 
-    def _run_parallel_impl(self, q, k, v, *custom, block_mask=None, cache_seqlens=None):
+    def _run_parallel_impl(self, q, k, v, *custom, block_mask=None, cache_seqlens=None, grad=False):
+        plan = self._plan
+        out = native.host().run(plan if plan is not None else self._make_plan(), q, k, v, custom,
+                                -1 if self.kv_splits is None else self.kv_splits, block_mask, cache_seqlens, grad)
+        if out is None:
+            self._refuse(q, k, v, custom, block_mask, cache_seqlens)
+        # a lowered functor's combine gives output weights only: its splits' final row scales are not merged (none come back)
+        self.last_final_rowscales = dict(zip(self.final_names, out[1:]))
+        return out[0]
+
+    def _refuse(self, q, k, v, custom, block_mask, cache_seqlens):
+        """Raises the error of a call that the native side declined."""
         if len(custom) != len(self.custom_names):
             raise TypeError(f"expected {len(self.custom_names)} custom input tensor(s) {self.custom_names}, got {len(custom)}")
         if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
@@ -402,61 +387,11 @@ class AttentionEngine:
         if not q.is_cuda:
             raise native.NativeError("the forward kernel needs CUDA tensors: there is no CPU path")
         B, S, H, _ = q.shape
-        tensors, strides = self._custom_operands(custom, B, H, S, k.shape[1], q.device)
-        # the entry points launch on the CURRENT device and stream: make q's device current for the whole call
-        with torch.cuda.device(q.device):
-            sparse = None
-            if self._may_decode and self.kv_splits is None and S * H <= 128 * k.shape[2] and k.shape[1] > 128:
-                # the query rows of the heads that share a KV head fit one tile: the decode kernel, if it covers the call
-                out = native.decode_fwd(q, k, v, self._fparams[0], block_mask, cache_seqlens, self._decode_block or 0)
-                if out is not None:
-                    self.last_final_rowscales = {self.final_names[0]: out[1]}
-                    return out[0]
-            if self._decode_block is not None:
-                # block-sparse, variable-length decode (examples/sparse_gqa_decode.py, blockattn_decode_varlen_tl.py):
-                # the call's block_mask [B, Hkv, blocks] and cache_seqlens [B] become, on the device, the bitmaps of
-                # the KV tiles to visit and the column masks of the tiles kept in part
-                sparse = native.decode_tiles(block_mask, cache_seqlens, B, k.shape[2], k.shape[1], self._decode_block, q.device)
-            return self._launch_parallel(q, k, v, tensors, strides, sparse)
-
-    def _launch_parallel(self, q, k, v, tensors, strides, sparse=None):
-        B, S, H, _ = q.shape
-        Dv = v.shape[3]
-        o = torch.empty((B, S, H, Dv), dtype=q.dtype, device=q.device)
-        finals = [torch.empty((B, H, S), dtype=torch.float32, device=q.device) for _ in self.final_names]
-        if sparse is None and self._sparse_host is not None:
-            if q.device not in self._sparse_dev:
-                self._sparse_dev[q.device] = sparse_lowering.to_device(self._sparse_host, q.device)
-            sparse = self._sparse_dev[q.device]
-        # split-KV when the launch would leave most SMs idle (decode: few query rows and heads against a long KV): the
-        # split results are added up with the weights of the functor's combine (built-in softmax: through the
-        # log-sum-exp; lowered functors: the user's OnlineFunc.combine, which needs every split to be non-empty,
-        # i.e. no mask)
-        splits, workspace = 1, None
-        lowered_ok = self.functor_kind == "lowered" and self.mask_kind == native.MASK_NONE
-        if sparse is None and Dv <= 128 and q.shape[-1] <= 128 and (self.functor_kind == "builtin_softmax" or lowered_ok):
-            splits = self.kv_splits if self.kv_splits is not None else plan_kv_splits(B, H, S, k.shape[1], q.device)
-            if splits > 1 and self.functor_kind == "lowered":
-                kv_tiles = (k.shape[1] + 127) // 128
-                per = -(-kv_tiles // min(splits, kv_tiles))
-                splits = -(-kv_tiles // per)          # no split without KV tiles
-            if splits > 1:
-                workspace = torch.empty(B * splits * H * S * (Dv + native.MAX_ROWSCALES) * 4, dtype=torch.uint8, device=q.device)
-        args = native.fill_parallel_args(q, k, v, o, mask_kind=self.mask_kind, mask_band=self.mask_band,
-                                         num_splits=splits, workspace=workspace, functor=native.FUNCTOR_SOFTMAX,
-                                         fparams=self._fparams, final_rowscales=finals, custom=tensors,
-                                         custom_strides=strides, sparse=sparse)
-        if self.functor_kind == "builtin_softmax":
-            native.parallel_fwd(args)
-        else:
-            if self._jit_fn is None:
-                self._jit_fn = native_jit.load(self.functor_source)
-            status = native.device_status_word(q.device.index)
-            native.check(self._jit_fn(C.byref(args), native.current_stream_ptr(), status), "attn_b200_parallel_fwd_jit")
-        # a lowered functor's combine gives output weights only: its splits' final row scales are not merged
-        merged = splits == 1 or self.functor_kind == "builtin_softmax"
-        self.last_final_rowscales = dict(zip(self.final_names, finals)) if merged else {}
-        return o
+        self._custom_operands(custom, B, H, S, k.shape[1], q.device)
+        if self._decode_block is not None:
+            native.decode_operands(block_mask, cache_seqlens, B, k.shape[2], q.device)
+        native.fill_parallel_args(q, k, v, torch.empty((B, S, H, v.shape[3]), dtype=q.dtype, device=q.device), mask_kind=self.mask_kind)
+        raise native.NativeError("operands the forward kernel does not take")
 
     # ------------------------------------------------------------------
     def __call__(self, *args, **kargs):

@@ -19,6 +19,7 @@ _PKG_DIR = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__fil
 CSRC_DIR = os.path.join(_PKG_DIR, "csrc")
 INCLUDE_DIR = os.path.join(os.path.dirname(_PKG_DIR), "include")
 LIB_PATH = os.path.join(_PKG_DIR, "libattn_b200.so")
+HOST_PATH = os.path.join(_PKG_DIR, "_host_ops.so")
 
 NVCC_ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared"]
@@ -202,6 +203,28 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def build_host_ops(force: bool = False) -> str:
+    """Compile _host_ops.so (csrc/host_ops.cpp: the host side of a call against torch's C++ API) with g++."""
+    src = os.path.join(CSRC_DIR, "host_ops.cpp")
+    deps = [src, os.path.join(INCLUDE_DIR, "attn_b200.h")]
+    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(d) for d in deps):
+        return HOST_PATH
+    import sysconfig
+    torch_dir = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+            os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    tmp = HOST_PATH + f".tmp{os.getpid()}"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_host_ops",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in incs), "-I", INCLUDE_DIR, src,
+           "-o", tmp, "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise NativeError(f"g++ failed: {' '.join(cmd)}\n{r.stdout}")
+    os.replace(tmp, HOST_PATH)
+    return HOST_PATH
+
+
 def bind(lib: C.CDLL, names=None) -> C.CDLL:
     for name in (names or SIGNATURES):
         fn = getattr(lib, name)  # AttributeError if the symbol is not exported
@@ -220,6 +243,26 @@ def load_library() -> C.CDLL:
                 "from the repository root (there is no non-native fallback)")
         _lib = bind(C.CDLL(path))
     return _lib
+
+
+_host = None
+
+
+def host():
+    """Load (once) the native host side, bound to the entry points of the library and to ``check``.  Like a functor
+    library it is compiled if it is not there; there is no other way to run a call."""
+    global _host
+    if _host is None:
+        import importlib.util
+        lib = load_library()
+        if not os.path.exists(HOST_PATH):
+            build_host_ops()
+        spec = importlib.util.spec_from_file_location("_host_ops", HOST_PATH)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES}, check)
+        _host = mod
+    return _host
 
 
 def check(rc: int, what: str):
@@ -297,7 +340,7 @@ def fill_parallel_args(q, k, v, o, *, mask_kind: int, functor: int = 0, fparams=
     return a
 
 
-def _decode_operands(block_mask, cache_seqlens, batch: int, heads_kv: int, device):
+def decode_operands(block_mask, cache_seqlens, batch: int, heads_kv: int, device):
     """The call-time block_mask / cache_seqlens of a decode as the uint8 / int32 device tensors the library reads."""
     if block_mask is not None:
         if block_mask.dim() != 3 or block_mask.shape[0] != batch or block_mask.shape[1] != heads_kv:
@@ -311,37 +354,6 @@ def _decode_operands(block_mask, cache_seqlens, batch: int, heads_kv: int, devic
     return block_mask, cache_seqlens
 
 
-def decode_fwd(q, k, v, scale: float, block_mask=None, cache_seqlens=None, block_size: int = 0):
-    """(o, lse) of softmax(scale * q.k).v for a few query rows against a long cache through attn_b200_decode_fwd, or None if
-    the call is not one it covers (see the header: head dims, rows of a group, block sizes).  q [B, Sq, H, D],
-    k, v [B, Skv, Hkv, D] with contiguous last dim."""
-    B, Sq, H, D = q.shape
-    Skv, Hkv = k.shape[1], k.shape[2]
-    if v.shape[3] != D or D not in (64, 128) or v.shape[2] != Hkv or H % Hkv != 0:
-        return None
-    if q.dtype not in DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype or q.stride(3) != 1 or k.stride(3) != 1 or v.stride(3) != 1:
-        return None
-    block_mask, cache_seqlens = _decode_operands(block_mask, cache_seqlens, B, Hkv, q.device)
-    a = DecodeArgs()
-    a.batch, a.heads, a.heads_kv, a.seq_q, a.seq_kv, a.dim, a.dtype, a.scale = B, H, Hkv, Sq, Skv, D, DTYPE_CODES[q.dtype], scale
-    if block_mask is not None:
-        a.block_mask, a.n_blocks, a.block_size = block_mask.data_ptr(), block_mask.shape[2], block_size
-    if cache_seqlens is not None:
-        a.seq_lens = cache_seqlens.data_ptr()
-    lib = load_library()
-    need = lib.attn_b200_decode_workspace_bytes(C.byref(a))
-    if need < 0:
-        return None
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-    o = torch.empty((B, Sq, H, D), dtype=q.dtype, device=q.device)
-    lse = torch.empty((B, H, Sq), dtype=torch.float32, device=q.device)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    a.q, a.k, a.v, a.o, a.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
-    a.q_stride[:], a.k_stride[:], a.v_stride[:], a.o_stride[:] = _strides_bsh(q), _strides_bsh(k), _strides_bsh(v), _strides_bsh(o)
-    check(lib.attn_b200_decode_fwd(C.byref(a), current_stream_ptr()), "attn_b200_decode_fwd")
-    return o, lse
-
-
 def decode_tiles(block_mask, cache_seqlens, batch: int, heads_kv: int, seq_kv: int, block_size: int, device) -> dict:
     """Sparse-walk description (see fill_parallel_args ``sparse``) of a block-sparse, variable-length decode, built
     on the device by attn_b200_decode_tiles.  block_mask: bool/uint8 [batch, heads_kv, blocks] or None;
@@ -351,7 +363,7 @@ def decode_tiles(block_mask, cache_seqlens, batch: int, heads_kv: int, seq_kv: i
     words = (tiles + 31) // 32
     bh = batch * heads_kv
     out = torch.empty(int(lib.attn_b200_decode_tiles_bytes(batch, heads_kv, seq_kv)) // 4, dtype=torch.int32, device=device)
-    block_mask, cache_seqlens = _decode_operands(block_mask, cache_seqlens, batch, heads_kv, device)
+    block_mask, cache_seqlens = decode_operands(block_mask, cache_seqlens, batch, heads_kv, device)
     n_blocks = block_mask.shape[2] if block_mask is not None else 0
     check(lib.attn_b200_decode_tiles(block_mask.data_ptr() if block_mask is not None else None,
                                      cache_seqlens.data_ptr() if cache_seqlens is not None else None,
@@ -475,42 +487,6 @@ def _softmax_bwd_one(q, k, v, o, lse, d_o, scale: float, mask_kind: int, mask_ba
     a.workspace, a.workspace_bytes = ws.data_ptr(), need
     with torch.cuda.device(q.device):
         check(lib.attn_b200_softmax_bwd(C.byref(a), current_stream_ptr()), "attn_b200_softmax_bwd")
-    return dq, dk, dv
-
-
-def elementwise_bwd(fn, q, k, v, d_o, mask_kind: int, custom=(), mask_band=(MASK_OPEN, MASK_OPEN), mask_bits=None):
-    """(dq, dk, dv) of an elementwise program through its functor library's ``attn_b200_elementwise_bwd_jit`` (``fn``);
-    ``custom``: the program's fp32 scalar inputs, as device tensors.  dim_v may be a multiple of dim_qk."""
-    for t in (q, k, v, d_o, *custom):
-        if not t.is_cuda:
-            raise NativeError("the backward kernel needs CUDA tensors: there is no CPU path")
-    if d_o.stride(-1) != 1:
-        d_o = d_o.contiguous()
-    return _over_dim_v_slices(lambda q_, k_, v_, do_, o_: _elementwise_bwd_one(fn, q_, k_, v_, do_, mask_kind, custom, mask_band, mask_bits),
-                              q, k, v, d_o)
-
-
-def _elementwise_bwd_one(fn, q, k, v, d_o, mask_kind: int, custom, mask_band, mask_bits=None):
-    if q.dtype not in DTYPE_CODES or any(t.dtype != q.dtype for t in (k, v, d_o)):
-        raise NativeError("q, k, v, d_o must share dtype float16 or bfloat16")
-    dq, dk, dv = (torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k, v))
-    custom = [t.to(device=q.device, dtype=torch.float32).contiguous() for t in custom]
-    a = ElementwiseBwdArgs()
-    a.q, a.k, a.v, a.d_o = (t.data_ptr() for t in (q, k, v, d_o))
-    a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    B, Sq, H, D = q.shape
-    a.batch, a.heads, a.heads_kv, a.seq_q, a.seq_kv, a.dim_qk, a.dim_v = B, H, k.shape[2], Sq, k.shape[1], D, v.shape[3]
-    a.dtype, a.mask_kind = DTYPE_CODES[q.dtype], mask_kind
-    a.mask_left, a.mask_right = int(mask_band[0]), int(mask_band[1])
-    if mask_bits is not None:
-        _set_mask_bits(a, mask_bits, q, k)
-    for name, t in (("q", q), ("k", k), ("v", v), ("do", d_o), ("dq", dq), ("dk", dk), ("dv", dv)):
-        getattr(a, name + "_stride")[:] = _strides_bsh(t)
-    for i, t in enumerate(custom):
-        a.custom[i] = t.data_ptr()
-    with torch.cuda.device(q.device):
-        status = device_status_word(q.device.index)
-        check(fn(C.byref(a), current_stream_ptr(), status), "attn_b200_elementwise_bwd_jit")
     return dq, dk, dv
 
 

@@ -1,0 +1,524 @@
+// Host side of a call in native code: from tensors to the argument structs of include/attn_b200.h, outputs and scratch from
+// torch's allocator, the launch on the current stream, and the autograd functions.
+//
+// A short call's kernel runs for 5 to 20 microseconds; filling a ctypes struct field by field in Python took 35 to 50, and a
+// forward and backward through Python autograd functions 220.  Everything here works on what the engine decided once at
+// construction (`Plan`) and on the shapes and strides of this call.  Nothing is kept between calls but the plan's copies of
+// its mask on each device.
+//
+// A call whose operands are not what a kernel takes is declined (`None` / false): the Python side then raises the error
+// that names what is wrong.  Entry points of libattn_b200.so and of functor libraries come in as addresses, from the
+// libraries that Python has loaded.
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/extension.h>
+
+#include <algorithm>
+#include <cstring>
+#include <map>
+#include <memory>
+
+#include "../../include/attn_b200.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = c10::optional<Tensor>;
+
+struct Api {
+  int (*parallel_fwd)(const AttnB200ParallelArgs*, void*) = nullptr;
+  int64_t (*decode_bytes)(const AttnB200DecodeArgs*) = nullptr;
+  int (*decode_fwd)(const AttnB200DecodeArgs*, void*) = nullptr;
+  int64_t (*decode_tiles_bytes)(int32_t, int32_t, int32_t) = nullptr;
+  int (*decode_tiles)(const uint8_t*, const int32_t*, int32_t, int32_t, int32_t, int32_t, int32_t, void*, int64_t, void*) = nullptr;
+  int64_t (*softmax_bwd_bytes)(const AttnB200SoftmaxBwdArgs*) = nullptr;
+  int (*softmax_bwd)(const AttnB200SoftmaxBwdArgs*, void*) = nullptr;
+  int (*status_word)(int32_t, int32_t**) = nullptr;
+} api;
+
+template <class F>
+void take(F& slot, const py::dict& d, const char* name) {
+  slot = reinterpret_cast<F>(py::cast<uintptr_t>(d[name]));
+}
+
+PyObject* raise_status = nullptr;   // core.native.lib.check: raises NativeError for a status code; held to the end of the process
+
+void bind(const py::dict& d, py::object check) {
+  take(api.parallel_fwd, d, "attn_b200_parallel_fwd");
+  take(api.decode_bytes, d, "attn_b200_decode_workspace_bytes");
+  take(api.decode_fwd, d, "attn_b200_decode_fwd");
+  take(api.decode_tiles_bytes, d, "attn_b200_decode_tiles_bytes");
+  take(api.decode_tiles, d, "attn_b200_decode_tiles");
+  take(api.softmax_bwd_bytes, d, "attn_b200_softmax_bwd_workspace_bytes");
+  take(api.softmax_bwd, d, "attn_b200_softmax_bwd");
+  take(api.status_word, d, "attn_b200_device_status_word");
+  raise_status = check.release().ptr();
+}
+
+// Raises the Python NativeError of a status code; callable without the GIL (autograd threads).
+void check(int rc, const char* what) {
+  if (rc == ATTN_B200_OK) return;
+  py::gil_scoped_acquire gil;
+  try {
+    py::reinterpret_borrow<py::object>(raise_status)(rc, what);
+  } catch (py::error_already_set& e) {
+    e.restore();
+    python_error err;
+    err.persist();
+    throw err;
+  }
+}
+
+int dtype_code(const Tensor& t) {
+  return t.scalar_type() == at::kHalf ? ATTN_B200_DTYPE_FP16 : t.scalar_type() == at::kBFloat16 ? ATTN_B200_DTYPE_BF16 : -1;
+}
+void strides_bsh(int64_t (&dst)[3], const Tensor& t) {
+  for (int i = 0; i < 3; ++i) dst[i] = t.stride(i);
+}
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+Tensor f32(at::IntArrayRef size, const Tensor& like) { return at::empty(size, like.options().dtype(at::kFloat)); }
+Tensor bytes(int64_t n, const Tensor& like) { return at::empty({n}, like.options().dtype(at::kByte)); }
+
+// One custom input of a program: per dimension the axis it stands for (0..3 = batch, heads, seq_len, seq_len_kv; -1 = none,
+// then `literal` is its declared extent or -1), and the type the functor reads.
+struct Custom {
+  std::vector<int> axes;
+  std::vector<int64_t> literal;
+  at::ScalarType dtype;
+};
+
+// Block-sparse walk of a mask on one device (core/lower/sparse.py).
+struct Sparse {
+  Tensor keep, partial, mask_base, elem_mask, bits_q, bits_kv, tiles_q, tiles_kv;
+  int batch = 1, heads = 1, rows = 128;
+};
+
+// What an engine of the parallel pattern decided at construction.
+struct Plan {
+  bool builtin = false;        // the built-in softmax; else `fn` is attn_b200_parallel_fwd_jit of its functor library
+  uintptr_t fn = 0;
+  std::vector<float> fparams;
+  int n_final = 0;
+  int mask_kind = 0, left = 0, right = 0;
+  bool may_decode = false;     // attn_b200_decode_fwd computes this program
+  int decode_block = 0;        // > 0: block_mask / cache_seqlens arrive with the call
+  bool has_mask_walk = false;  // a general mask_mod
+  std::vector<Custom> custom;
+  int backward = 0;            // 0 none, 1 softmax, 2 elementwise
+  py::object load_mask;        // device -> dict of tensors
+  py::object load_backward;    // () -> address of attn_b200_elementwise_bwd_jit
+  uintptr_t bwd_fn = 0;
+  std::map<int, Sparse> masks;
+
+  const Sparse& mask_on(const Tensor& like) {   // with the GIL
+    const int dev = like.device().index();
+    auto it = masks.find(dev);
+    if (it != masks.end()) return it->second;
+    py::dict d = load_mask(like.device());
+    Sparse s;
+    auto get = [&](const char* k, Tensor& t) {
+      if (d.contains(k) && !d[k].is_none()) t = py::cast<Tensor>(d[k]);
+    };
+    get("keep", s.keep); get("partial", s.partial); get("mask_base", s.mask_base); get("elem_mask", s.elem_mask);
+    get("bits_q", s.bits_q); get("bits_kv", s.bits_kv); get("tiles_q", s.tiles_q); get("tiles_kv", s.tiles_kv);
+    s.batch = py::cast<int>(d["batch"]);
+    s.heads = py::cast<int>(d["heads"]);
+    s.rows = py::cast<int>(d["mask_rows"]);
+    return masks.emplace(dev, std::move(s)).first->second;
+  }
+};
+
+// The call-time masks of a decode as the types the library reads; false = not a shape it takes.
+bool decode_operands(OptTensor& block_mask, OptTensor& lens, int64_t B, int64_t Hkv, const Tensor& q) {
+  if (block_mask.has_value()) {
+    Tensor& m = *block_mask;
+    if (m.dim() != 3 || m.size(0) != B || m.size(1) != Hkv) return false;
+    if (m.device() != q.device()) m = m.to(q.device());
+    m = m.contiguous();
+    m = m.scalar_type() == at::kBool ? m.view(at::kByte) : m.to(at::kByte);
+  }
+  if (lens.has_value()) {
+    if (lens->numel() != B) return false;
+    lens = lens->to(q.device(), at::kInt).contiguous();
+  }
+  return true;
+}
+
+struct Forward {
+  bool done = false;
+  Tensor o;
+  std::vector<Tensor> finals;   // empty when split results were merged without them
+};
+
+int kv_splits_for(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int device) {
+  // 1 unless the (query tile pair, head, batch) grid fills less than half of the SMs; then as many as fit, each keeping at
+  // least four 128-row KV tiles (a split re-reads Q and adds a combine pass)
+  const int64_t ctas = B * H * ((Sq + 255) / 256), sms = at::cuda::getDeviceProperties(device)->multiProcessorCount;
+  const int64_t tiles = (Skv + 127) / 128;
+  if (2 * ctas > sms || tiles < 8) return 1;
+  return static_cast<int>(std::max<int64_t>(1, std::min({sms / ctas, tiles / 4, int64_t{65535} / std::max<int64_t>(B, 1)})));
+}
+
+// The forward of one call; `done` false = declined.  With the GIL when the plan has a mask walk that a device has not seen.
+Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
+                OptTensor block_mask, OptTensor lens) {
+  Forward r;
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
+  const int dt = dtype_code(q);
+  if (dt < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return r;
+  if (q.stride(3) != 1 || k.stride(3) != 1 || v.stride(3) != 1) return r;
+  const int64_t B = q.size(0), Sq = q.size(1), H = q.size(2), D = q.size(3), Skv = k.size(1), Hkv = k.size(2), Dv = v.size(3);
+  if (Hkv <= 0 || v.size(2) != Hkv || H % Hkv != 0 || custom.size() != plan.custom.size()) return r;
+  c10::cuda::CUDAGuard guard(q.device());
+  void* stream = stream_of(q);
+
+  if (plan.may_decode && forced_splits < 0 && Sq * H <= 128 * Hkv && Skv > 128 && D == Dv) {
+    // the query rows of the heads that share a KV head fit one tile: the decode kernel, if it covers the call
+    OptTensor bm = block_mask, ln = lens;
+    if (plan.decode_block > 0 && !decode_operands(bm, ln, B, Hkv, q)) return r;
+    AttnB200DecodeArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.batch = B; a.heads = H; a.heads_kv = Hkv; a.seq_q = Sq; a.seq_kv = Skv; a.dim = D; a.dtype = dt; a.scale = plan.fparams[0];
+    if (bm.has_value()) {
+      a.block_mask = bm->data_ptr<uint8_t>();
+      a.n_blocks = bm->size(2);
+      a.block_size = plan.decode_block;
+    }
+    if (ln.has_value()) a.seq_lens = ln->data_ptr<int32_t>();
+    const int64_t need = api.decode_bytes(&a);
+    if (need >= 0) {
+      Tensor ws = bytes(need, q), lse = f32({B, H, Sq}, q);
+      r.o = at::empty({B, Sq, H, Dv}, q.options());
+      a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = r.o.data_ptr();
+      a.lse = lse.data_ptr<float>();
+      a.workspace = ws.data_ptr();
+      a.workspace_bytes = need;
+      strides_bsh(a.q_stride, q); strides_bsh(a.k_stride, k); strides_bsh(a.v_stride, v); strides_bsh(a.o_stride, r.o);
+      check(api.decode_fwd(&a, stream), "attn_b200_decode_fwd");
+      r.finals.push_back(lse);
+      r.done = true;
+      return r;
+    }
+  }
+
+  AttnB200ParallelArgs a;
+  std::memset(&a, 0, sizeof(a));
+  // custom inputs: addressed by strides alone, so a named axis must have extent 1 (broadcast) or exactly the call's
+  const int64_t extent[4] = {B, H, Sq, Skv};
+  std::vector<Tensor> held;
+  for (size_t c = 0; c < custom.size(); ++c) {
+    const Custom& spec = plan.custom[c];
+    Tensor t = custom[c];
+    if (!t.defined() || t.dim() != static_cast<int64_t>(spec.axes.size()) || (t.is_cuda() && t.device() != q.device())) return r;
+    for (size_t d = 0; d < spec.axes.size(); ++d) {
+      const int64_t n = t.size(d);
+      if (spec.axes[d] < 0 ? (n != 1 || (spec.literal[d] >= 0 && spec.literal[d] != n)) : (n != 1 && n != extent[spec.axes[d]])) return r;
+    }
+    t = t.to(q.device(), spec.dtype);
+    for (size_t d = 0; d < spec.axes.size(); ++d)
+      if (spec.axes[d] >= 0 && t.size(d) > 1) a.custom_stride[c][spec.axes[d]] = t.stride(d);
+    a.custom[c] = t.data_ptr();
+    held.push_back(std::move(t));
+  }
+
+  Tensor tiles;   // call-time block_mask / cache_seqlens as tile bitmaps and column masks
+  if (plan.decode_block > 0) {
+    if (!decode_operands(block_mask, lens, B, Hkv, q)) return r;
+    const int64_t nt = (Skv + 127) / 128, words = (nt + 31) / 32, bh = B * Hkv;
+    const int64_t need = api.decode_tiles_bytes(B, Hkv, Skv);
+    tiles = bytes(need, q);
+    check(api.decode_tiles(block_mask.has_value() ? block_mask->data_ptr<uint8_t>() : nullptr, lens.has_value() ? lens->data_ptr<int32_t>() : nullptr, B,
+                           Hkv, block_mask.has_value() ? block_mask->size(2) : 0, plan.decode_block, Skv, tiles.data_ptr(), need, stream),
+          "attn_b200_decode_tiles");
+    uint32_t* col = static_cast<uint32_t*>(tiles.data_ptr());
+    a.elem_mask = col;
+    a.tile_keep = col + bh * nt * 4;
+    a.tile_partial = col + bh * nt * 4 + bh * words;
+    a.sparse_batch = B;
+    a.sparse_heads = Hkv;
+  } else if (plan.has_mask_walk) {
+    const Sparse& s = plan.mask_on(q);
+    a.tile_keep = static_cast<const uint32_t*>(s.keep.data_ptr());
+    a.tile_partial = static_cast<const uint32_t*>(s.partial.data_ptr());
+    a.tile_mask_base = s.mask_base.defined() ? s.mask_base.data_ptr<int32_t>() : nullptr;
+    a.elem_mask = s.elem_mask.defined() ? static_cast<const uint32_t*>(s.elem_mask.data_ptr()) : nullptr;
+    a.sparse_batch = s.batch;
+    a.sparse_heads = s.heads;
+    a.elem_mask_rows = s.rows;
+  }
+
+  r.o = at::empty({B, Sq, H, Dv}, q.options());
+  for (int i = 0; i < plan.n_final; ++i) {
+    r.finals.push_back(f32({B, H, Sq}, q));
+    a.final_rowscales[i] = r.finals.back().data_ptr<float>();
+  }
+  // split-KV when the launch would leave most SMs idle; the split results are added up with the weights of the functor's
+  // combine (lowered functors: the user's, which needs every split to be non-empty, i.e. no mask)
+  int splits = 1;
+  Tensor ws;
+  if (a.tile_keep == nullptr && Dv <= 128 && D <= 128 && (plan.builtin || plan.mask_kind == ATTN_B200_MASK_NONE)) {
+    splits = forced_splits >= 0 ? forced_splits : kv_splits_for(B, H, Sq, Skv, q.device().index());
+    if (splits > 1 && !plan.builtin) {
+      const int64_t nt = (Skv + 127) / 128, per = (nt + std::min<int64_t>(splits, nt) - 1) / std::min<int64_t>(splits, nt);
+      splits = (nt + per - 1) / per;   // no split without KV tiles
+    }
+    if (splits > 1) {
+      ws = bytes(B * splits * H * Sq * (Dv + ATTN_B200_MAX_ROWSCALES) * 4, q);
+      a.workspace = ws.data_ptr();
+      a.workspace_bytes = ws.numel();
+    }
+  }
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = r.o.data_ptr();
+  a.batch = B; a.heads = H; a.seq_q = Sq; a.seq_kv = Skv; a.dim_qk = D; a.dim_v = Dv; a.heads_kv = Hkv;
+  strides_bsh(a.q_stride, q); strides_bsh(a.k_stride, k); strides_bsh(a.v_stride, v); strides_bsh(a.o_stride, r.o);
+  a.dtype = dt;
+  a.mask_kind = plan.mask_kind;
+  a.mask_left = plan.left;
+  a.mask_right = plan.right;
+  a.functor = ATTN_B200_FUNCTOR_SOFTMAX;
+  a.num_splits = splits;
+  for (size_t i = 0; i < plan.fparams.size() && i < 8; ++i) a.fparams[i] = plan.fparams[i];
+  if (plan.builtin) {
+    check(api.parallel_fwd(&a, stream), "attn_b200_parallel_fwd");
+  } else {
+    int32_t* status = nullptr;
+    check(api.status_word(q.device().index(), &status), "attn_b200_device_status_word");
+    auto fn = reinterpret_cast<int (*)(const AttnB200ParallelArgs*, void*, int32_t*)>(plan.fn);
+    check(fn(&a, stream, status), "attn_b200_parallel_fwd_jit");
+    if (splits > 1) r.finals.clear();   // the combine gives output weights only
+  }
+  r.done = true;
+  return r;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// backward
+// ---------------------------------------------------------------------------------------------------------------
+
+Tensor grad_like(const Tensor& t) {   // the strides of t where its last dimension is contiguous and it has no holes
+  Tensor g = at::empty_like(t);
+  return g.stride(3) == 1 ? g : at::empty(t.sizes(), t.options());
+}
+
+struct Mask {
+  int kind, left, right;
+  Tensor bits_q, bits_kv, tiles_q, tiles_kv;
+};
+
+template <class Args>
+void fill_bwd(Args& a, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& d_o, const Tensor& dq, const Tensor& dk, const Tensor& dv,
+              const Mask& m) {
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.d_o = d_o.data_ptr();
+  a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr();
+  a.batch = q.size(0); a.heads = q.size(2); a.heads_kv = k.size(2); a.seq_q = q.size(1); a.seq_kv = k.size(1);
+  a.dim_qk = q.size(3); a.dim_v = v.size(3);
+  a.dtype = dtype_code(q);
+  a.mask_kind = m.kind;
+  a.mask_left = m.left;
+  a.mask_right = m.right;
+  if (m.bits_q.defined()) {
+    a.mask_kind = ATTN_B200_MASK_BITS;
+    a.mask_bits_q = m.bits_q.data_ptr();
+    a.mask_bits_kv = m.bits_kv.data_ptr();
+    if (m.tiles_q.defined()) {
+      a.mask_tiles_q = m.tiles_q.data_ptr();
+      a.mask_tiles_kv = m.tiles_kv.data_ptr();
+    }
+  }
+  strides_bsh(a.q_stride, q); strides_bsh(a.k_stride, k); strides_bsh(a.v_stride, v); strides_bsh(a.do_stride, d_o);
+  strides_bsh(a.dq_stride, dq); strides_bsh(a.dk_stride, dk); strides_bsh(a.dv_stride, dv);
+}
+
+std::vector<Tensor> softmax_bwd_one(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o,
+                                    float scale, const Mask& m) {
+  Tensor dq = grad_like(q), dk = grad_like(k), dv = grad_like(v);
+  AttnB200SoftmaxBwdArgs a;
+  std::memset(&a, 0, sizeof(a));
+  fill_bwd(a, q, k, v, d_o, dq, dk, dv, m);
+  a.o = o.data_ptr();
+  a.lse = lse.data_ptr<float>();
+  a.scale = scale;
+  strides_bsh(a.o_stride, o);
+  const int64_t need = api.softmax_bwd_bytes(&a);
+  Tensor ws = bytes(std::max<int64_t>(need, 16), q);
+  a.workspace = ws.data_ptr();
+  a.workspace_bytes = need;
+  check(api.softmax_bwd(&a, stream_of(q)), "attn_b200_softmax_bwd");
+  return {dq, dk, dv};
+}
+
+std::vector<Tensor> elementwise_bwd_one(uintptr_t fn, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& d_o,
+                                        const std::vector<Tensor>& custom, const Mask& m) {
+  Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()), dv = at::empty(v.sizes(), v.options());
+  AttnB200ElementwiseBwdArgs a;
+  std::memset(&a, 0, sizeof(a));
+  fill_bwd(a, q, k, v, d_o, dq, dk, dv, m);
+  std::vector<Tensor> held;
+  for (size_t i = 0; i < custom.size() && i < ATTN_B200_MAX_CUSTOM; ++i) {
+    held.push_back(custom[i].to(q.device(), at::kFloat).contiguous());
+    a.custom[i] = held.back().data_ptr();
+  }
+  int32_t* status = nullptr;
+  check(api.status_word(q.device().index(), &status), "attn_b200_device_status_word");
+  check(reinterpret_cast<int (*)(const AttnB200ElementwiseBwdArgs*, void*, int32_t*)>(fn)(&a, stream_of(q), status), "attn_b200_elementwise_bwd_jit");
+  return {dq, dk, dv};
+}
+
+// dim_v a multiple of dim_qk: the backward is linear in dP = dO V^T and in delta, sums over the columns of v, and dV's
+// columns are independent: one run per dim_qk-wide column slice, dQ and dK added up in fp32
+template <class Run>
+std::vector<Tensor> over_dim_v(const Tensor& q, const Tensor& v, const Run& run) {
+  const int64_t D = q.size(3), Dv = v.size(3);
+  if (Dv == D) return run(0, D);
+  Tensor dq, dk;
+  std::vector<Tensor> dvs;
+  for (int64_t c = 0; c < Dv; c += D) {
+    auto part = run(c, D);
+    dq = dq.defined() ? dq + part[0].to(at::kFloat) : part[0].to(at::kFloat);
+    dk = dk.defined() ? dk + part[1].to(at::kFloat) : part[1].to(at::kFloat);
+    dvs.push_back(part[2]);
+  }
+  return {dq.to(q.scalar_type()), dk.to(q.scalar_type()), at::cat(dvs, -1)};
+}
+
+Tensor last_contiguous(Tensor t, const Tensor& like) {
+  if (t.scalar_type() != like.scalar_type()) t = t.to(like.scalar_type());
+  return t.stride(3) == 1 ? t : t.contiguous();
+}
+
+struct PlanRef : torch::CustomClassHolder {
+  std::shared_ptr<Plan> plan;
+};
+std::shared_ptr<Plan> plan_of(torch::autograd::AutogradContext* ctx) {
+  return c10::static_intrusive_pointer_cast<PlanRef>(ctx->saved_data["plan"].toCapsule())->plan;
+}
+
+// The forward with its backward (attn_b200_softmax_bwd, attn_b200_elementwise_bwd_jit): the counterpart of the reference's
+// `_attention` autograd function (core/template/tl_template/attn/attn_tl.py:654-694).  Outputs: o, then the final row
+// scales, which carry no gradient.
+struct Attention : torch::autograd::Function<Attention> {
+  static torch::autograd::variable_list forward(torch::autograd::AutogradContext* ctx, const std::shared_ptr<Plan>& plan, const Forward& done,
+                                                const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom) {
+    auto ref = c10::make_intrusive<PlanRef>();
+    ref->plan = plan;
+    ctx->saved_data["plan"] = c10::IValue::make_capsule(ref);
+    torch::autograd::variable_list saved{q, k, v};
+    if (plan->backward == 1) {
+      saved.push_back(done.o);
+      saved.push_back(done.finals[0]);
+    } else {
+      for (const Tensor& t : custom) saved.push_back(t);
+    }
+    const size_t n_saved = saved.size();
+    if (plan->has_mask_walk) {
+      const Sparse& s = plan->masks.at(q.device().index());
+      for (const Tensor& t : {s.bits_q, s.bits_kv, s.tiles_q, s.tiles_kv}) saved.push_back(t);
+    }
+    ctx->saved_data["n_saved"] = static_cast<int64_t>(n_saved);
+    ctx->save_for_backward(saved);
+    torch::autograd::variable_list out{done.o};
+    for (const Tensor& t : done.finals) out.push_back(t);
+    ctx->mark_non_differentiable(done.finals);
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    auto plan = plan_of(ctx);
+    const auto saved = ctx->get_saved_variables();
+    const size_t n_saved = ctx->saved_data["n_saved"].toInt();
+    const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
+    c10::cuda::CUDAGuard guard(q.device());
+    Tensor g = grads[0].defined() ? grads[0] : at::zeros({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
+    const Tensor d_o = last_contiguous(g, q);
+    Mask m{plan->mask_kind, plan->left, plan->right, {}, {}, {}, {}};
+    if (saved.size() > n_saved) {
+      m.bits_q = saved[n_saved]; m.bits_kv = saved[n_saved + 1]; m.tiles_q = saved[n_saved + 2]; m.tiles_kv = saved[n_saved + 3];
+    }
+    auto cols = [](const Tensor& t, int64_t c, int64_t w) { return t.size(3) == w ? t : t.narrow(3, c, w); };
+    std::vector<Tensor> d;
+    if (plan->backward == 1) {
+      const Tensor &o = saved[3], &lse = saved[4];
+      d = over_dim_v(q, v, [&](int64_t c, int64_t w) {
+        return softmax_bwd_one(q, k, cols(v, c, w), cols(o, c, w), lse, cols(d_o, c, w), plan->fparams[0], m);
+      });
+    } else {
+      if (plan->bwd_fn == 0) {   // compiled when a gradient is first asked for
+        py::gil_scoped_acquire gil;
+        try {
+          plan->bwd_fn = py::cast<uintptr_t>(plan->load_backward());
+        } catch (py::error_already_set& e) {
+          e.restore();
+          python_error err;
+          err.persist();
+          throw err;
+        }
+      }
+      const std::vector<Tensor> custom(saved.begin() + 3, saved.begin() + n_saved);
+      d = over_dim_v(q, v, [&](int64_t c, int64_t w) {
+        return elementwise_bwd_one(plan->bwd_fn, q, k, cols(v, c, w), cols(d_o, c, w), custom, m);
+      });
+    }
+    return {Tensor(), Tensor(), d[0], d[1], d[2], Tensor()};   // one entry per argument of forward
+  }
+};
+
+// One call of an engine: None (declined) or [o, final row scales...].  `grad`: the call is recorded for the backward.
+py::object run(const std::shared_ptr<Plan>& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom,
+               int forced_splits, const OptTensor& block_mask, const OptTensor& lens, bool grad) {
+  Forward f;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;   // outputs are made, nothing is recorded
+    f = forward(*plan, q, k, v, custom, forced_splits, block_mask, lens);
+  }
+  if (!f.done) return py::none();
+  py::list out;
+  if (grad) {
+    for (Tensor& t : Attention::apply(plan, f, q, k, v, custom)) out.append(std::move(t));
+  } else {
+    out.append(f.o);
+    for (Tensor& t : f.finals) out.append(t);
+  }
+  return out;
+}
+
+std::shared_ptr<Plan> make_plan(const py::dict& d) {
+  // the last reference may be dropped by an autograd thread: Python objects go under the GIL
+  std::shared_ptr<Plan> p(new Plan, [](Plan* x) {
+    py::gil_scoped_acquire gil;
+    delete x;
+  });
+  p->builtin = py::cast<bool>(d["builtin"]);
+  p->fn = py::cast<uintptr_t>(d["fn"]);
+  p->fparams = py::cast<std::vector<float>>(d["fparams"]);
+  p->n_final = py::cast<int>(d["n_final"]);
+  p->mask_kind = py::cast<int>(d["mask_kind"]);
+  p->left = py::cast<int>(d["left"]);
+  p->right = py::cast<int>(d["right"]);
+  p->may_decode = py::cast<bool>(d["may_decode"]);
+  p->decode_block = py::cast<int>(d["decode_block"]);
+  p->has_mask_walk = py::cast<bool>(d["has_mask_walk"]);
+  p->backward = py::cast<int>(d["backward"]);
+  p->load_mask = d["load_mask"];
+  p->load_backward = d["load_backward"];
+  for (const auto& item : py::cast<py::list>(d["custom"])) {
+    const py::tuple t = py::cast<py::tuple>(item);
+    p->custom.push_back({py::cast<std::vector<int>>(t[0]), py::cast<std::vector<int64_t>>(t[1]), py::cast<bool>(t[2]) ? at::kFloat
+                                                                                                 : py::cast<bool>(t[3]) ? at::kBFloat16
+                                                                                                                        : at::kHalf});
+  }
+  return p;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  py::class_<Plan, std::shared_ptr<Plan>>(m, "Plan");
+  m.def("bind", &bind);
+  m.def("make_plan", &make_plan);
+  m.def("run", &run);
+  m.def("kv_splits", &kv_splits_for);
+}

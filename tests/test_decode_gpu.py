@@ -1,9 +1,11 @@
-"""The decode kernel (attn_b200_decode_fwd) against softmax attention in fp32: query rows packed by KV head, shares of the
-tile list that cut sequences, lengths, gathered blocks."""
+"""Decode calls of the built-in softmax (attn_b200_decode_fwd) against softmax attention in fp32: query rows packed by KV head,
+shares of the tile list that cut sequences, lengths, gathered blocks, and the calls it leaves to the forward kernel."""
 
 import pytest
 import torch
 
+from attn_engine import AttentionEngine
+from core import CustomIO, meta_tensor
 from core.native import lib
 from examples_b200 import programs
 
@@ -30,6 +32,11 @@ def check(got, want, dtype):
     assert (lse - want[1]).abs().max().item() <= 2e-5 * max(1.0, want[1].abs().max().item())
 
 
+def run(eng, *args, **kwargs):
+    o = eng(*args, **kwargs)
+    return o, eng.last_final_rowscales["lse"]
+
+
 def rand(gen, *shape, dtype):
     return torch.randn(*shape, generator=gen, device="cuda").to(dtype)
 
@@ -50,16 +57,26 @@ def test_dense(B, H, Hkv, Sq, S, D, dtype):
     gen = torch.Generator(device="cuda").manual_seed(S + D)
     q, k, v = rand(gen, B, Sq, H, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype), rand(gen, B, S, Hkv, D, dtype=dtype)
     k[..., S // 2:, :, :] *= 3.0   # the running maximum moves: accumulators are rescaled
-    got = lib.decode_fwd(q, k, v, D ** -0.5)
+    eng = programs.gqa_engine(B, H, Hkv, Sq, S, D, D, dtype=dtype)
+    got = run(eng, q, k, v)
     want = reference(q, k, v, D ** -0.5)
     check(got, want, dtype)
     # another order of the query rows: heads outside the sequence axis
     qh = q.transpose(1, 2).contiguous().transpose(1, 2)
-    check(lib.decode_fwd(qh, k.transpose(1, 2).contiguous().transpose(1, 2), v, D ** -0.5), want, dtype)
-    # the engine's call
-    o = programs.gqa_engine(B, H, Hkv, Sq, S, D, D, dtype=dtype)(q, k, v)
-    assert torch.equal(o, got[0])
+    check(run(eng, qh, k.transpose(1, 2).contiguous().transpose(1, 2), v), want, dtype)
+    eng.kv_splits = 1   # the forward kernel
+    check(run(eng, q, k, v), want, dtype)
     assert lib.last_device_status() == 0
+
+
+def decode_engine(B, H, Hkv, Sq, S, D, block):
+    scale = D ** -0.5
+
+    def score_mod(score, custom, b, h, q_idx, kv_idx):
+        return score * scale
+    meta = (meta_tensor(B, H, Sq, D, dtype=torch.bfloat16),) + (meta_tensor(B, Hkv, S, D, dtype=torch.bfloat16),) * 2
+    return AttentionEngine(meta, CustomIO({}), score_mod=score_mod, mask_mod=None, online_func=programs.NaturalSoftmax(),
+                           extern_block_mask=True, use_varlen=True, infer_mask_block_N=block)
 
 
 @pytest.mark.parametrize("B,H,Hkv,Sq,S,D,block,masked,varlen", [
@@ -69,6 +86,8 @@ def test_dense(B, H, Hkv, Sq, S, D, dtype):
     (4, 32, 4, 1, 4096, 128, 64, True, True),
     (70, 8, 4, 1, 640, 64, 128, True, True),       # more pairs than SMs
     (6, 8, 2, 2, 2000, 128, 32, False, True),      # lengths only
+    (2, 4, 2, 1, 960, 64, 48, True, True),         # a block that does not divide a tile: left to the forward kernel
+    (2, 8, 1, 9, 640, 128, 32, True, True),        # 72 rows with a block mask: left to the forward kernel
 ])
 def test_blocks_and_lengths(B, H, Hkv, Sq, S, D, block, masked, varlen):
     dtype = torch.bfloat16
@@ -87,19 +106,12 @@ def test_blocks_and_lengths(B, H, Hkv, Sq, S, D, block, masked, varlen):
         keep &= mask.repeat_interleave(block, -1)[..., :S]
     if varlen:
         keep &= (torch.arange(S, device="cuda") < lens[:, None])[:, None]
-    o, lse = lib.decode_fwd(q, k, v, D ** -0.5, mask, lens, block)
+    eng = decode_engine(B, H, Hkv, Sq, S, D, block)
+    o, lse = run(eng, q, k, v, block_mask=mask, cache_seqlens=lens)
     want_o, want_lse = reference(q, k, v, D ** -0.5, keep)
     some = keep.any(-1).repeat_interleave(H // Hkv, 1)     # [B, H]
     assert torch.isnan(o.transpose(1, 2)[~some]).all() and (lse[~some] == -float("inf")).all()
     check((o.transpose(1, 2)[some], lse[some]), (want_o.transpose(1, 2)[some], want_lse[some]), dtype)
-    again = lib.decode_fwd(q, k, v, D ** -0.5, mask, lens, block)
+    again = run(eng, q, k, v, block_mask=mask, cache_seqlens=lens)
     assert torch.equal(o.nan_to_num(7.0), again[0].nan_to_num(7.0)) and torch.equal(lse, again[1])
     assert lib.last_device_status() == 0
-
-
-def test_calls_outside_its_range_are_left_to_the_forward_kernel():
-    q, k = torch.zeros(1, 1, 129, 64, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 256, 1, 64, dtype=torch.bfloat16, device="cuda")
-    assert lib.decode_fwd(q, k, k, 1.0) is None                                    # 129 rows
-    mask = torch.ones(1, 1, 6, dtype=torch.bool, device="cuda")
-    assert lib.decode_fwd(q[:, :, :1], k, k, 1.0, mask, None, 48) is None           # a block that does not divide a tile
-    assert lib.decode_fwd(q[..., :48], k[..., :48], k[..., :48], 1.0) is None      # another head dim
