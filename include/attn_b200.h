@@ -195,6 +195,8 @@ typedef struct AttnB200LinearArgs {
                             [batch, heads_q, seq, q_ld] tensor (pointer at the range's first column, 16-byte aligned;
                             q_ld a multiple of 8) -- the backward contracts over column ranges of dO and v in place */
   int32_t k_ld;          /* the same for k */
+  int32_t segments;      /* CTAs that share the sequence of one (batch, head, dim_v slice), at most 16; 0 = planned from
+                            the shape and the SM count.  The result has the same bits for every value */
 } AttnB200LinearArgs;
 
 /* Bytes of scratch the linear forward needs: per-row (sum, sum of squares) fp32 when normalize = 1, else 0. */

@@ -115,13 +115,14 @@ def _column_range_ld(t) -> int:
 
 
 def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize: bool = False, eps: float = 1e-5,
-                             out_dtype=None, v_scale=None, precise: bool = False):
+                             out_dtype=None, v_scale=None, precise: bool = False, segments: int = 0):
     """q,k: [B,H,T,Dk]; v: [B,H,T,Dv] (fp16/bf16 CUDA); log_decay: [B,H,T] fp32, natural log of the
     per-token decay.  Returns o [B,H,T,Dv] in the input dtype, or in fp32 with ``out_dtype=torch.float32``
     (the kernel's accumulators without the output rounding).  ``normalize`` applies a per-(batch, head,
     token) normalisation over Dv (zero mean, unit variance, no affine) to the output.  ``v_scale`` [B,H,T] (fp32) is a
     per-token factor on the rows of v, applied inside the kernel.  ``precise``: the decayed scores of a block keep a
-    16-bit remainder beside their 16-bit value (a second P V pass)."""
+    16-bit remainder beside their 16-bit value (a second P V pass).  ``segments``: CTAs that share
+    a chain's sequence, 0 = planned from the shape (the result has the same bits)."""
     if out_dtype not in (None, q.dtype, torch.float32):
         raise native.NativeError("out_dtype must be the input dtype or torch.float32")
     f32_out = out_dtype == torch.float32
@@ -141,7 +142,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
             raise native.NativeError("normalize needs dim_v to be a multiple of 128")
         pad = 128 - Dv % 128
         o = linear_attention_forward(q, k, torch.nn.functional.pad(v, (0, pad)), log_decay, q_scale, False, eps, out_dtype, v_scale,
-                                     precise)
+                                     precise, segments)
         return o[..., :Dv].contiguous()
     # q and k may be column ranges of wider contiguous tensors (the backward's contractions over ranges of dim_v)
     q_ld, k_ld = _column_range_ld(q), _column_range_ld(k)
@@ -163,6 +164,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
         a.dtype = native.DTYPE_CODES[q.dtype]
         a.normalize = 1 if normalize else 0
         a.precise = 1 if precise else 0
+        a.segments = segments
         a.q_scale = float(q_scale)
         a.norm_eps = float(eps)
         lib = native.load_library()

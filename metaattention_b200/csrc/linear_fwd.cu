@@ -38,6 +38,7 @@ namespace b200 {
 constexpr int kLinT = 128;    // tokens per block
 constexpr int kLinDvs = 128;  // dim_v columns per CTA
 constexpr int kLinRowThreads = 256;              // eight warps: one TMEM lane each, two column halves
+constexpr int kLinMaxSegments = 16;                // CTAs that share a chain's sequence
 constexpr int kLinThreads = kLinRowThreads + 64;   // plus the warp that issues TMA copies and MMAs and the decay-scan warp
 
 struct LinearParams {
@@ -50,13 +51,16 @@ struct LinearParams {
   int heads, heads_q, heads_k;   // heads of v; of q and k (divisors of `heads`: consecutive v heads share a q / k head)
   float q_scale;
   int split_p;             // 1: P is written as a 16-bit high part plus a 16-bit remainder (two PV passes)
+  // blocks [cut[z], cut[z + 1]) of a chain belong to the CTA with blockIdx.z = z, which first runs the state alone over
+  // the blocks before them
+  int cut[kLinMaxSegments + 1];
   int* status;
 };
 
 __device__ __forceinline__ float clamp_h(float x) { return fminf(fmaxf(x, -65504.0f), 65504.0f); }
 
-enum LinearWaitSite { kLinQFull = 41, kLinKFull, kLinScore, kLinQh, kLinPv, kLinState, kLinPReady, kLinVReady, kLinOStaged, kLinStageFree, kLinConvDone, kLinVFull, kLinDecay, kLinHiReady };
-enum LinearBarrier { kBarQFull = 0, kBarKFull, kBarVFull, kBarScore, kBarHiReady, kBarPv, kBarState, kBarPReady, kBarVReady, kBarConvDone, kBarDecay, kNumLinBarriers };
+enum LinearWaitSite { kLinQFull = 41, kLinKFull, kLinScore, kLinQh, kLinPv, kLinState, kLinPReady, kLinVReady, kLinOStaged, kLinStageFree, kLinConvDone, kLinVFull, kLinDecay, kLinHiReady, kLinPreFull, kLinPreState, kLinPreH };
+enum LinearBarrier { kBarQFull = 0, kBarKFull, kBarVFull, kBarScore, kBarHiReady, kBarPv, kBarState, kBarPReady, kBarVReady, kBarConvDone, kBarDecay, kBarPreK, kBarPreV = kBarPreK + 2, kBarPreVReady = kBarPreV + 3, kBarPreH, kBarPreState, kNumLinBarriers };
 
 template <int DK>
 struct LinearSmem {
@@ -78,13 +82,19 @@ struct LinearSmem {
   static constexpr bool kScaledVInH = (DK == 256);
   static constexpr int kOffV2 = kScaledVInH ? kOffKh + 2 * kPairBytes + kChunkBytes : kOffStageX + kStageExtra;
   static constexpr int kV2Stride = kScaledVInH ? kPairBytes : kChunkBytes;
-  static constexpr int kOffG = kOffStageX + kStageExtra + (kScaledVInH ? 0 : kVBytes);  // float g2[2][128] + float gb[128]
+  // While only the state runs (the blocks before a CTA's own), nothing but K and V is needed: K alternates between its
+  // own place and that of the state's copy, V goes round its own place, the second buffer (dim_qk 256: the upper half
+  // of Q) and Q (dim_qk 64, whose Q is too small: a buffer of its own).
+  static constexpr int kOffG0 = kOffStageX + kStageExtra + (kScaledVInH ? 0 : kVBytes);
+  static constexpr int kOffPreV1 = kScaledVInH ? kOffQ + kVBytes : kOffV2;
+  static constexpr int kOffPreV2 = kQBytes >= kVBytes ? kOffQ : kOffG0;
+  static constexpr int kOffG = kOffG0 + (kQBytes >= kVBytes ? 0 : kVBytes);  // float g2[2][128] + float gb[128]
   static constexpr int kOffBar = kOffG + 3 * kLinT * 4 + 32;
   static constexpr int kOffMisc = kOffBar + 8 * kNumLinBarriers;
   static constexpr int kBytes = kOffMisc + 16 + 1024;
 };
 
-template <int DK, bool kBf16>
+template <int DK, bool kBf16, bool kCut>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const LinearParams p) {
@@ -118,6 +128,11 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint64_t* v_ready = bars + kBarVReady;
   uint64_t* conv_done = bars + kBarConvDone;
   uint64_t* g_ready = bars + kBarDecay;
+  uint64_t* pre_k = bars + kBarPreK;         // [2] blocks before the CTA's own: K, V (one per buffer)
+  uint64_t* pre_v = bars + kBarPreV;         // [3]
+  uint64_t* pre_vready = bars + kBarPreVReady;
+  uint64_t* pre_h = bars + kBarPreH;
+  uint64_t* pre_st = bars + kBarPreState;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);
 
@@ -127,7 +142,10 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const AbortState ab{abort_flag, p.status};
   const int slice = blockIdx.x;
   const int bh = blockIdx.y;
-  const int nblk = (p.seq + T - 1) / T;
+  // This CTA's blocks are [t0, t_end); before them it runs the state alone over blocks [0, t0).  Whole chains are an
+  // instantiation of their own: with a t0 known only at run time they ran 3 % slower (335 -> 344 us on 8 x 8 x 4096).
+  // The row threads poll on their barriers: 306 -> 300 us there.
+  const int t0 = kCut ? p.cut[blockIdx.z] : 0, t_end = kCut ? p.cut[blockIdx.z + 1] : (p.seq + T - 1) / T;
   const float* ld_row = p.log_decay + static_cast<long long>(bh) * p.seq;
   const int b_idx = bh / p.heads, h_idx = bh - b_idx * p.heads;
   const int bh_q = b_idx * p.heads_q + h_idx / (p.heads / p.heads_q), bh_k = b_idx * p.heads_k + h_idx / (p.heads / p.heads_k);
@@ -145,6 +163,11 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     mbar_init(v_ready, kLinRowThreads / 32);
     mbar_init(conv_done, kLinRowThreads / 32);
     mbar_init(g_ready, 1);
+    for (int i = 0; i < 2; ++i) mbar_init(pre_k + i, 1);
+    for (int i = 0; i < 3; ++i) mbar_init(pre_v + i, 1);
+    mbar_init(pre_vready, kLinRowThreads / 32);
+    mbar_init(pre_h, kLinRowThreads / 32);
+    mbar_init(pre_st, 1);
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
@@ -205,17 +228,72 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       // The tensor pipe executes in issue order and the issuing thread is held back while the pipe is full,
       // so the order below is the schedule.  Per block: the rest of [S | O], the state update (with mild decay its
       // operand is waiting), Q and K of the next block, P V, V of the next block, the early chunks of the next [S | O].
-      load_q(0);
-      load_k(0);
-      load_v(0);
-      for (int t = 0; t < nblk; ++t) {
-        const bool last = (t + 1 == nblk);
-        const uint32_t par = t & 1, par_prev = (t - 1) & 1;
-        if (t == 0 || KC <= kLoChunks) {
+      bool pre_ok = true;
+      if (kCut && t0 > 0) {
+        // The state alone over the blocks before this CTA's own, in the same arithmetic and order as when they are
+        // computed in full (the result does not depend on how a chain is cut).  Block t's buffers are counted back from
+        // t0, so that the K and V of t0 itself land where the loop below expects them.
+        auto pre_load_k = [&](int t) {
+          if (t > t0) return;
+          if (t == t0) return load_k(t);
+          const int b = (t0 - t) & 1;
+          mbar_arrive_expect_tx(pre_k + b, L::kQBytes);
+          for (int c = 0; c < KC; ++c)
+            tma_load_3d(sKh + c * L::kPairBytes + b * L::kChunkBytes, &tmK, pre_k + b, c * 64, t * T, bh_k);
+        };
+        auto pre_load_v = [&](int t) {
+          if (t > t0) return;
+          if (t == t0) return load_v(t);
+          const int b = (t0 - t) % 3;
+          uint8_t* dst = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
+          mbar_arrive_expect_tx(pre_v + b, L::kVBytes);
+          for (int c = 0; c < DVS / 64; ++c) tma_load_3d(dst + c * (T * 128), &tmV, pre_v + b, slice * DVS + c * 64, t * T, bh);
+        };
+        pre_load_v(0);
+        pre_load_k(0);
+        pre_load_v(1);
+        pre_load_k(1);
+        pre_load_v(2);
+        for (int t = 0; t < t0; ++t) {
+          const int kb = (t0 - t) & 1, vb = (t0 - t) % 3;
+          // the state has been decayed for this block (and so the update by the block before is done), V' is in place
+          pre_ok = mbar_wait_poll(pre_h, t & 1, ab, kLinPreH) && mbar_wait_poll(pre_k + kb, (t >> 1) & 1, ab, kLinPreFull);
+          if (!pre_ok) break;
+          tc_fence_after_sync();
+          const uint32_t va = smem_u32(vb == 0 ? sV : smem + (vb == 1 ? L::kOffPreV1 : L::kOffPreV2));
+          const uint64_t va_desc = make_smem_desc(va, T * 128, 1024);
+          const uint64_t kd_desc = k_mn_desc0 + static_cast<uint64_t>(kb) * kChunk;
+#pragma unroll
+          for (int g = 0; g < T / 64; ++g)
+            umma_ss_x4<128, 128>(tmem_base + kColH, va_desc + g * 512, kd_desc + g * 512, idesc_h, (t > 0 || g > 0) ? 1u : 0u);
+          umma_commit(pre_st);
+          if (t >= 1) {   // the buffers of block t - 1 are free
+            pre_load_k(t + 1);
+            pre_load_v(t + 2);
+          }
+        }
+        // Q's place and that of the state's copy have served as buffers
+        pre_ok = pre_ok && mbar_wait_poll(pre_st, (t0 - 1) & 1, ab, kLinPreState);
+        if (pre_ok) load_q(t0);
+      } else {
+        load_q(0);
+        load_k(0);
+        load_v(0);
+      }
+      const int conv_off = t0 > 0 ? 0 : 1;   // with blocks before, one conversion precedes the first block
+      for (int t = t0; pre_ok && t < t_end; ++t) {
+        const bool last = (t + 1 == t_end);
+        const uint32_t par = (t - t0) & 1, par_prev = (t - t0 + conv_off) & 1;
+        if (t == t0 || KC <= kLoChunks) {
           if (t > 0 && !mbar_wait_poll(conv_done, par_prev, ab, kLinConvDone)) break;
           if (!(mbar_wait_poll(q_full, par, ab, kLinQFull) && mbar_wait_poll(k_full, par, ab, kLinKFull))) break;
           tc_fence_after_sync();
-          issue_sq(t, 0, KC, true);
+          if (kCut && t > 0 && KC > kLoChunks) {   // the order of the sums is that of the blocks whose early chunks go first
+            issue_sq(t, kLoChunks, KC, true);
+            issue_sq(t, 0, kLoChunks, false);
+          } else {
+            issue_sq(t, 0, KC, true);
+          }
         } else {
           if (!mbar_wait_poll(conv_done, par_prev, ab, kLinConvDone)) break;
           tc_fence_after_sync();
@@ -272,7 +350,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     // its last entry, by those of block t - 1) and gb (read by block t's P phase only), so it may be written once the
     // row threads are through the P phase of block t - 1.
     bool ok = start_ok;
-    for (int t = 0; ok && t < nblk; ++t) {
+    for (int t = 0; ok && t < t_end; ++t) {
       float x[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -290,7 +368,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       const float pre = run - x[3];
       const float g_end = __shfl_sync(0xffffffffu, run, lane | 7);   // last token of this lane's 32-token chunk
-      if (t > 0 && lane == 0) ok = mbar_wait_poll(p_ready, (t - 1) & 1, ab, kLinDecay);
+      if (t > 0 && lane == 0)   // before the CTA's own blocks a table is read by the rescaling of V only
+        ok = t <= t0 ? mbar_wait_poll(pre_vready, (t - 1) & 1, ab, kLinDecay) : mbar_wait_poll(p_ready, (t - 1 - t0) & 1, ab, kLinDecay);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
 #pragma unroll
@@ -349,22 +428,11 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     // bytes apart).  With mild decay the result replaces V (P V then takes the same rows), which touches nothing
     // another phase of the kernel uses; else it goes to the second buffer (with 256 state columns the upper half of
     // the state copy, free once Q h has run).
-    auto rescale_v = [&](int tb, bool in_place) -> bool {
-      // a per-token factor of the caller on v (v_mod = v * t[b, h, token]) rides along: fetched before the wait for V
-      const int tok = tb * T + row;
-      const float vs = (p.v_scale != nullptr && tok < p.seq) ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
-      const bool v_ok = mbar_wait(v_full, tb & 1, ab, kLinVFull);
-      const float* g = g2 + (tb & 1) * T;
-      const float w = fast_exp2(g[T - 1] - g[row]) * vs;
-      uint4* vsrc = reinterpret_cast<uint4*>(sV + wg * (T * 128) + row * 128);
-      const uint4* vline = vsrc;
-      uint4* v2line = reinterpret_cast<uint4*>((in_place ? sV + wg * (T * 128) : sV2 + wg * L::kV2Stride) + row * 128);
-      // with strong decay P V reads V itself: the caller's factor then goes onto V in place as well
-      const bool scale_v_too = !in_place && p.v_scale != nullptr;
+    auto rescale_row = [&](uint4* vsrc, uint4* v2line, float w, float vs, bool scale_v_too) {
 #pragma unroll
       for (int q4 = 0; q4 < 8; ++q4) {
         const int piece = (q4 + lane) & 7;
-        uint4 x = vline[piece];
+        uint4 x = vsrc[piece];
         uint4 y = x;
         uint32_t* xs = reinterpret_cast<uint32_t*>(&x);
         uint32_t* ys = reinterpret_cast<uint32_t*>(&y);
@@ -386,17 +454,84 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         v2line[piece] = x;
         if (scale_v_too) vsrc[piece] = y;
       }
+    };
+    auto rescale_v = [&](int tb, bool in_place) -> bool {
+      // a per-token factor of the caller on v (v_mod = v * t[b, h, token]) rides along: fetched before the wait for V
+      const int tok = tb * T + row;
+      const float vs = (p.v_scale != nullptr && tok < p.seq) ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
+      const bool v_ok = mbar_wait(v_full, (tb - t0) & 1, ab, kLinVFull);
+      const float* g = g2 + (tb & 1) * T;
+      const float w = fast_exp2(g[T - 1] - g[row]) * vs;
+      // with strong decay P V reads V itself: the caller's factor then goes onto V in place as well
+      const bool scale_v_too = !in_place && p.v_scale != nullptr;
+      uint4* vsrc = reinterpret_cast<uint4*>(sV + wg * (T * 128) + row * 128);
+      uint4* v2line = reinterpret_cast<uint4*>((in_place ? sV + wg * (T * 128) : sV2 + wg * L::kV2Stride) + row * 128);
+      rescale_row(vsrc, v2line, w, vs, scale_v_too);
       fence_proxy_async_smem();
-      if (tb + 1 < nblk) warp_arrive(v_ready);
+      if (tb + 1 < t_end) warp_arrive(v_ready);
       return v_ok;
     };
 
-    bool ok = start_ok && mbar_wait(g_ready, 0, ab, kLinDecay);
-    if (ok && g2[T - 1] >= kMildLog2) ok = rescale_v(0, true);
-    for (int t = 0; ok && t < nblk; ++t) {
+    bool ok = start_ok;
+    // ---- the state alone, over the blocks before this CTA's own ----
+    for (int t = 0; kCut && ok && t < t0; ++t) {
+      const int b = (t0 - t) % 3;
+      uint8_t* v_buf = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
+      const int tok = t * T + row;
+      const float vs = p.v_scale != nullptr ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
+      ok = mbar_wait_poll(g_ready, t & 1, ab, kLinDecay);
+      const float* g = g2 + (t & 1) * T;
+      const float decay = fast_exp2(g[T - 1]);
+      const float w = fast_exp2(g[T - 1] - g[row]) * vs;
+      ok = mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok;
+      if (!ok) break;
+      uint4* line = reinterpret_cast<uint4*>(v_buf + wg * (T * 128) + row * 128);
+      rescale_row(line, line, w, vs, false);
+      fence_proxy_async_smem();
+      warp_arrive(pre_vready);
+      if (t > 0) {
+        ok = mbar_wait_poll(pre_st, (t - 1) & 1, ab, kLinPreState);
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < DK / 64; ++c) {
+          float hv[32];
+          tmem_ld32f(tH + wg * (DK / 2) + c * 32, hv);
+          tmem_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) hv[i] *= decay;
+          tmem_st32f(tH + wg * (DK / 2) + c * 32, hv);
+        }
+        tmem_wait_st();
+        tc_fence_before_sync();
+      }
+      warp_arrive(pre_h);
+    }
+    ok = ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay);
+    if (ok) {
+      const float g_first = g2[(t0 & 1) * T + T - 1];
+      const bool mild_first = g_first >= kMildLog2;
+      if (mild_first) ok = rescale_v(t0, true);
+      if (kCut && t0 > 0) {
+        const float decay_first = fast_exp2(g_first);
+        ok = mbar_wait(pre_st, (t0 - 1) & 1, ab, kLinPreState) && ok;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int c = 0; c < kEarlyCols / 32; ++c) convert32(128 + wg * kEarlyCols + c * 32, decay_first, mild_first);
+        if (wg * 64 < DK) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) convert32(wg * 64 + c * 32, decay_first, mild_first);
+        }
+        tmem_wait_st();
+        fence_proxy_async_smem();
+        tc_fence_before_sync();
+        warp_arrive(conv_done);
+      }
+    }
+    if (kCut && t0 > 0) ok = named_sync_and(1 + (warp & 3), 64, ok);   // the two warps of a lane quarter enter the loop together or not at all
+    for (int t = t0; ok && t < t_end; ++t) {
       const int buf = t & 1;
-      const bool last = (t + 1 == nblk);
-      const uint32_t par = t & 1;
+      const bool last = (t + 1 == t_end);
+      const uint32_t par = (t - t0) & 1;
       const float gi = g2[buf * T + row];
       const float qs = p.q_scale;
       // Mild decay (the block's total log2-decay stays inside the exponent range of the 16-bit operands with room
@@ -438,7 +573,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         // chunk: a per-row and a per-column number, both at most 1.  Chunks above the diagonal are zero and
         // are not even read.  All three cases are uniform over a warp.
         const int wq = warp & 3;
-        ok = mbar_wait(s_bar, par, ab, kLinScore) && ok;
+        ok = mbar_wait_poll(s_bar, par, ab, kLinScore) && ok;
         tc_fence_after_sync();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -512,16 +647,16 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       float decay_next = 1.0f;
       bool mild_next = false;   // the coming block multiplies Q by the state after its decay
       if (!last) {
-        ok = mbar_wait(g_ready, (t + 1) & 1, ab, kLinDecay) && ok;   // written once every warp was past the P phase
+        ok = mbar_wait_poll(g_ready, (t + 1) & 1, ab, kLinDecay) && ok;   // written once every warp was past the P phase
         const float g_next = g2[(buf ^ 1) * T + T - 1];
         decay_next = fast_exp2(g_next);
         mild_next = g_next >= kMildLog2;
-        ok = mbar_wait(st_bar, par, ab, kLinState) && ok;
+        ok = mbar_wait_poll(st_bar, par, ab, kLinState) && ok;
         tc_fence_after_sync();
 #pragma unroll
         for (int c = 0; c < kEarlyCols / 32; ++c) convert32(128 + wg * kEarlyCols + c * 32, decay_next, mild_next);
       }
-      ok = mbar_wait(pv_bar, par, ab, kLinPv) && ok;
+      ok = mbar_wait_poll(pv_bar, par, ab, kLinPv) && ok;
       tc_fence_after_sync();
       // ---- output rows to the staging buffer (while the state update runs) ----
       {
@@ -676,6 +811,54 @@ inline int encode_rows3(CUtensorMap* tm, const void* base, int dtype, uint64_t c
   return r == CUDA_SUCCESS ? ATTN_B200_OK : ATTN_B200_E_UNSUPPORTED;
 }
 
+// Cuts a chain's blocks into `segments` runs for as many CTAs.  A CTA computes its own blocks in full, but first has to
+// run the state over every block before them, each `r` as long as a full one, so the runs get shorter towards the end:
+// the smallest length L with r * start + blocks <= L for every run is looked for.  Returns L (in full blocks).
+// The share: a block of the state alone takes 1.05-1.35 us (latency of the chain update -> decay -> update), a full block
+// 3.5-4.3 us with mild and 5.1-6 us with strong decay (dim_qk 64-256), which the host does not know: 0.2-0.3.
+constexpr double kStateShare = 0.25;
+inline double cut_chain(int nblk, int segments, double r, int* cut) {
+  double lo = static_cast<double>(nblk) / segments, hi = nblk;
+  for (int it = 0; it < 24; ++it) {
+    const double mid = 0.5 * (lo + hi);
+    int at = 0;
+    for (int z = 0; z < segments; ++z) {
+      const double room = mid - r * at;
+      if (room >= 1.0) at += static_cast<int>(room);
+    }
+    (at >= nblk ? hi : lo) = mid;
+  }
+  int at = 0;
+  for (int z = 0; z < segments; ++z) {
+    cut[z] = at;
+    const double room = hi - r * at;
+    if (room >= 1.0) at += static_cast<int>(room);
+    if (at > nblk) at = nblk;
+  }
+  cut[segments] = nblk;
+  return hi;
+}
+
+// How many CTAs share a chain.  A grid that leaves SMs idle is bound by the length of one chain; cutting it shortens
+// that, at the price of repeating the state's part of the blocks.  Taken where the rounds of CTAs times the longest run
+// (a CTA's start and end cost about one block) come out at least a tenth shorter.  Measured, B x H = 4, dim_v 128, us
+// uncut -> as planned: 2000 tokens dim_qk 64 60 -> 24, 128 mild 67 -> 27, strong 85 -> 28; 4096 tokens dim_qk 256 mild
+// 144 -> 49, strong with the remainder pass 193 -> 53.  80 chains of 16 blocks: 76 uncut, 74 as three: left whole.
+// The result has the same bits either way.
+inline int plan_segments(long long chains, int nblk, int sms, double r, int* cut) {
+  int best = 1, tmp[kLinMaxSegments + 1];
+  double best_cost = 0.9 * static_cast<double>((chains + sms - 1) / sms) * (nblk + 1);
+  for (int z = 2; z <= kLinMaxSegments && z <= nblk; ++z) {
+    const double cost = static_cast<double>((chains * z + sms - 1) / sms) * (cut_chain(nblk, z, r, tmp) + 1);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = z;
+    }
+  }
+  cut_chain(nblk, best, r, cut);
+  return best;
+}
+
 template <int DK, bool kBf16>
 int launch_linear(const AttnB200LinearArgs* a, cudaStream_t stream, int* status) {
   using L = LinearSmem<DK>;
@@ -718,12 +901,23 @@ int launch_linear(const AttnB200LinearArgs* a, cudaStream_t stream, int* status)
     p.stats = static_cast<float*>(a->workspace);
     if (cudaMemsetAsync(p.stats, 0, rows * 2 * sizeof(float), stream) != cudaSuccess) return ATTN_B200_E_LAUNCH;
   }
-  auto kernel = linear_fwd_kernel<DK, kBf16>;
+  const int nblk = (a->seq + kLinT - 1) / kLinT, slices = a->dim_v / kLinDvs;
+  int segments = a->segments > nblk ? nblk : a->segments;
+  if (segments <= 0) {
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return ATTN_B200_E_LAUNCH;
+    segments = plan_segments(static_cast<long long>(bh) * slices, nblk, sms, kStateShare, p.cut);
+  } else {
+    cut_chain(nblk, segments, kStateShare, p.cut);
+  }
+  while (segments > 1 && p.cut[segments - 1] == nblk) --segments;   // more CTAs than the runs' lengths leave work for
+  auto kernel = segments > 1 ? linear_fwd_kernel<DK, kBf16, true> : linear_fwd_kernel<DK, kBf16, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes) != cudaSuccess) {
     cudaGetLastError();
     return ATTN_B200_E_LAUNCH;
   }
-  dim3 grid(a->dim_v / kLinDvs, static_cast<unsigned>(bh));
+  dim3 grid(slices, static_cast<unsigned>(bh), segments);
   kernel<<<grid, kLinThreads, L::kBytes, stream>>>(tmQ, tmK, tmV, tmO, p);
   if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
   if (a->normalize) {
@@ -753,6 +947,7 @@ int attn_b200_linear_fwd(const AttnB200LinearArgs* a, void* cuda_stream) {
   if (a->dim_v <= 0 || a->dim_v % b200::kLinDvs != 0) return ATTN_B200_E_UNSUPPORTED;
   if (a->heads_q < 0 || a->heads_k < 0 || (a->heads_q > 0 && a->heads % a->heads_q != 0) || (a->heads_k > 0 && a->heads % a->heads_k != 0))
     return ATTN_B200_E_INVALID_ARG;
+  if (a->segments < 0 || a->segments > b200::kLinMaxSegments) return ATTN_B200_E_INVALID_ARG;
   if (static_cast<long long>(a->batch) * a->heads > 65535) return ATTN_B200_E_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(a->o) & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
   if (a->normalize) {

@@ -242,3 +242,33 @@ def test_per_token_v_scale_inside_the_kernel(strong_decay):
     assert lib.last_device_status() == 0
     want = rm.decayed_linear_attention(q, k, v.float() * vs[..., None], log_decay, scale=1.0)
     check_raw(o, want)
+
+
+@pytest.mark.parametrize("Dk,S,dtype,strong,precise", [
+    (64, 1100, torch.bfloat16, True, False),     # nine blocks, the last one ragged
+    (128, 640, torch.float16, False, False),
+    (128, 2000, torch.bfloat16, True, True),
+    (256, 1000, torch.bfloat16, False, False),
+    (256, 1152, torch.float16, True, False),
+])
+def test_chains_cut_between_ctas(Dk, S, dtype, strong, precise):
+    """A chain whose blocks are shared out among CTAs (each repeats the state's part of the blocks before its own) gives
+    the bits of the uncut one, for every number of CTAs: one block in front, two, all buffers in use, more CTAs than runs
+    with a block in them."""
+    B, H, Dv = 1, 2, 256
+    g = torch.Generator().manual_seed(S + Dk)
+    q = torch.randn(B, H, S, Dk, generator=g).to(dtype)
+    k = (torch.randn(B, H, S, Dk, generator=g) * Dk ** -0.5).to(dtype)
+    v = torch.randn(B, H, S, Dv, generator=g).to(dtype)
+    vs = torch.rand(B, H, S, generator=g) + 0.5
+    ld = -torch.rand(B, H, S, generator=g) * (1.5 if strong else 0.02)
+    args = [t.cuda() for t in (q, k, v, ld)]
+    for scale in (None, vs.cuda()):
+        whole = linear_attention_forward(*args, v_scale=scale, precise=precise, segments=1)
+        check_raw(whole, rm.decayed_linear_attention(q, k, v.float() if scale is None else v.float() * vs[..., None], ld, scale=1.0))
+        for segments in (0, 2, 3, 5, 16):
+            o = linear_attention_forward(*args, v_scale=scale, precise=precise, segments=segments)
+            assert torch.equal(o, whole), segments
+    assert lib.last_device_status() == 0
+    with pytest.raises(lib.NativeError):
+        linear_attention_forward(*args, segments=17)
