@@ -197,6 +197,10 @@ typedef struct AttnB200LinearArgs {
   int32_t k_ld;          /* the same for k */
   int32_t segments;      /* CTAs that share the sequence of one (batch, head, dim_v slice), at most 16; 0 = planned from
                             the shape and the SM count.  The result has the same bits for every value */
+  int32_t reverse;       /* 1: the sums run the other way, over the tokens from a row's own to the end,
+                            o_j = sum_{i>=j} exp(G_i - G_j) (scale * q_j . k_i) v_i -- the transposed form that the gradients
+                            of k and v need (the reference's backward kernels walk the sequence backwards as well,
+                            linear_tl.py:461-975) */
 } AttnB200LinearArgs;
 
 /* Bytes of scratch the linear forward needs: per-row (sum, sum of squares) fp32 when normalize = 1, else 0. */
@@ -206,14 +210,22 @@ int64_t attn_b200_linear_workspace_bytes(const AttnB200LinearArgs* args);
  * (core/template/tl_template/linear/linear_tl.py:36-60, :146-223, :321-401, :1240-1268). */
 int attn_b200_linear_fwd(const AttnB200LinearArgs* args, void* cuda_stream);
 
-/* Row gathers of the linear-attention backward, which runs attn_b200_linear_fwd on time-reversed operands and on column
- * ranges of dim_v and adds up fp32 partial results (the reference's backward kernels walk the sequence backwards
- * themselves, linear_tl.py:461-975).  All tensors [outer, seq, cols] contiguous, pointers 16-byte aligned, column
+/* Row passes around the linear-attention backward, which runs attn_b200_linear_fwd on column ranges of dim_v and adds up
+ * fp32 partial results.  All tensors [outer, seq, cols] contiguous, pointers 16-byte aligned, column
  * counts and offsets multiples of 8.
  *   rows_copy16:   dst[o][s'][0:width] = src[o][s][col0:col0+width] for 16-bit elements, s' = reverse ? seq-1-s : s
  *   rows_sum_cast: dst[o][s'][:] = a[o][s][:] + b[o][s][:] (b may be NULL), fp32 -> `dtype` (fp16 / bf16) */
 int attn_b200_rows_copy16(const void* src, void* dst, int64_t outer, int32_t seq, int32_t src_cols, int32_t col0, int32_t width,
                           int32_t reverse, void* cuda_stream);
+/* Gradient of the log-decays and the 16-bit dq, dk in one pass over the fp32 results of the backward's runs:
+ *   dq[r][:] = dq_a[r][:] + dq_b[r][:],  dk the same (the b parts may be NULL; dq, dk in `dtype`),
+ *   row_term[r] = q[r] . (dq_a + dq_b)[r] - k[r] . (dk_a + dk_b)[r],  r = outer * seq rows of `cols` elements,
+ *   dg[o][t] = sum_{i >= t} row_term[o][i]
+ * (the dqkg kernel's row sums and compute_final_dg of the reference, linear_tl.py:63-76, 638-814).  row_term: scratch,
+ * outer * seq fp32. */
+int attn_b200_linear_decay_grad(const void* q, const void* k, const float* dq_a, const float* dq_b, const float* dk_a,
+                                const float* dk_b, void* dq, void* dk, float* row_term, float* dg, int32_t dtype, int64_t outer,
+                                int32_t seq, int32_t cols, void* cuda_stream);
 int attn_b200_rows_sum_cast(const float* a, const float* b, void* dst, int32_t dtype, int64_t outer, int32_t seq, int32_t cols,
                             int32_t reverse, void* cuda_stream);
 

@@ -115,14 +115,15 @@ def _column_range_ld(t) -> int:
 
 
 def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize: bool = False, eps: float = 1e-5,
-                             out_dtype=None, v_scale=None, precise: bool = False, segments: int = 0):
+                             out_dtype=None, v_scale=None, precise: bool = False, segments: int = 0, reverse: bool = False):
     """q,k: [B,H,T,Dk]; v: [B,H,T,Dv] (fp16/bf16 CUDA); log_decay: [B,H,T] fp32, natural log of the
     per-token decay.  Returns o [B,H,T,Dv] in the input dtype, or in fp32 with ``out_dtype=torch.float32``
     (the kernel's accumulators without the output rounding).  ``normalize`` applies a per-(batch, head,
     token) normalisation over Dv (zero mean, unit variance, no affine) to the output.  ``v_scale`` [B,H,T] (fp32) is a
     per-token factor on the rows of v, applied inside the kernel.  ``precise``: the decayed scores of a block keep a
     16-bit remainder beside their 16-bit value (a second P V pass).  ``segments``: CTAs that share
-    a chain's sequence, 0 = planned from the shape (the result has the same bits)."""
+    a chain's sequence, 0 = planned from the shape (the result has the same bits).  ``reverse``: the sums run over the
+    tokens from a row's own to the end of the sequence (see ``_reversed_forward``)."""
     if out_dtype not in (None, q.dtype, torch.float32):
         raise native.NativeError("out_dtype must be the input dtype or torch.float32")
     f32_out = out_dtype == torch.float32
@@ -142,7 +143,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
             raise native.NativeError("normalize needs dim_v to be a multiple of 128")
         pad = 128 - Dv % 128
         o = linear_attention_forward(q, k, torch.nn.functional.pad(v, (0, pad)), log_decay, q_scale, False, eps, out_dtype, v_scale,
-                                     precise, segments)
+                                     precise, segments, reverse)
         return o[..., :Dv].contiguous()
     # q and k may be column ranges of wider contiguous tensors (the backward's contractions over ranges of dim_v)
     q_ld, k_ld = _column_range_ld(q), _column_range_ld(k)
@@ -165,6 +166,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
         a.normalize = 1 if normalize else 0
         a.precise = 1 if precise else 0
         a.segments = segments
+        a.reverse = 1 if reverse else 0
         a.q_scale = float(q_scale)
         a.norm_eps = float(eps)
         lib = native.load_library()
@@ -177,85 +179,84 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
     return o
 
 
-def _rows(t, col0=0, width=None, reverse=False):
-    """Columns [col0, col0 + width) of t [B, H, T, cols], time reversed if asked, contiguous: one pass of the library's
-    row-gather kernel (torch.flip alone runs at a fifth of the copy rate)."""
-    width = t.shape[-1] - col0 if width is None else width
-    if not reverse:
-        return t[..., col0:col0 + width]    # read in place by the kernel (a pitch instead of a copy)
-    if width % 8 == 0 and col0 % 8 == 0 and t.shape[-1] % 8 == 0:
-        return native.rows_copy(t, col0, width, reverse)
-    part = t[..., col0:col0 + width]
-    return (part.flip(2) if reverse else part).contiguous()
+def _reversed_forward(q, k, v, log_decay, q_scale, out_dtype=None, precise=False):
+    """o_j = q_scale * sum_{i>=j} exp(G_i - G_j) (q_j . k_i) v_i: what ``linear_attention_forward`` gives on time-reversed
+    operands.  Position u of the reversed sequence then carries the log-decay of token T - u (0 for u = 0), so that the
+    reversed cumulative sums reproduce the same factors.  The kernel walks the sequence backwards itself."""
+    if q.is_cuda:
+        return linear_attention_forward(q, k, v, log_decay, q_scale, out_dtype=out_dtype, precise=precise, reverse=True)
+    ld_rev = torch.cat([torch.zeros_like(log_decay[..., :1]), log_decay.flip(-1)[..., :-1]], dim=-1)
+    return linear_attention_forward(q.flip(2), k.flip(2), v.flip(2), ld_rev, q_scale, out_dtype=out_dtype, precise=precise).flip(2)
 
 
-def _sum_cast(parts, dtype, reverse=False):
-    """Sum of the fp32 partial results, rounded to ``dtype``, time reversed if asked: one pass for up to two parts."""
+def _sum_cast(parts, dtype):
+    """Sum of the partial results, rounded to ``dtype``: one pass for two parts, none for one that has the dtype already."""
+    parts = _at_most_two(parts)
+    if len(parts) == 1 and parts[0].dtype == dtype:
+        return parts[0]
+    if parts[0].shape[-1] % 8 == 0:
+        return native.rows_sum_cast(parts[0], parts[1] if len(parts) > 1 else None, dtype)
+    return (parts[0] + parts[1] if len(parts) > 1 else parts[0]).to(dtype)
+
+
+def _at_most_two(parts):
     while len(parts) > 2:
         parts = [parts[0] + parts[1]] + parts[2:]
-    if parts[0].shape[-1] % 8 == 0:
-        return native.rows_sum_cast(parts[0], parts[1] if len(parts) > 1 else None, dtype, reverse)
-    out = (parts[0] + parts[1] if len(parts) > 1 else parts[0]).to(dtype)
-    return out.flip(2) if reverse else out
+    return parts
 
 
-def _retention_parts(qc, kc, vc, log_decay, q_scale, precise=False):
-    """o_i = q_scale * sum_{j<=i} exp(G_i - G_j) (qc_i . kc_j) vc_j on the forward kernel with fp32 output, for any width
-    of the contraction, as a list of partial results to be added: the sum is linear in the scores, so a contraction
-    wider than the kernel's 256 columns is the sum over column ranges it does cover (widths 256 / 128 / 64, the last one
-    zero-padded).  The kernel reads the column ranges of qc and kc in place."""
+def _retention_parts(qc, kc, vc, log_decay, q_scale, precise=False, reverse=False, fp32=True):
+    """o_i = q_scale * sum_{j<=i} exp(G_i - G_j) (qc_i . kc_j) vc_j (``reverse``: the sum over j >= i) on the forward
+    kernel, for any width of the contraction, as a list of fp32 partial results to be added: the sum is linear in the
+    scores, so a contraction wider than the kernel's 256 columns is the sum over column ranges it does cover (widths
+    256 / 128 / 64, the last one zero-padded), which the kernel reads in place.  A single result that is only to be
+    rounded (``fp32`` = False) leaves the kernel in the operands' dtype."""
+    run = _reversed_forward if reverse else linear_attention_forward
     D = qc.shape[-1]
+    out_dtype = torch.float32 if fp32 or D > 256 or D not in (64, 128, 256) else None
     parts, start = [], 0
     while start < D:
         width = next((w for w in (256, 128, 64) if D - start >= w), 64)
         have = min(width, D - start)
-        qs, ks = _rows(qc, start, have), _rows(kc, start, have)
+        qs, ks = qc[..., start:start + have], kc[..., start:start + have]
         if have < width:
             qs, ks = torch.nn.functional.pad(qs, (0, width - have)), torch.nn.functional.pad(ks, (0, width - have))
-        parts.append(linear_attention_forward(qs, ks, vc, log_decay, q_scale, out_dtype=torch.float32, precise=precise))
+        parts.append(run(qs, ks, vc, log_decay, q_scale, out_dtype=out_dtype, precise=precise))
         start += width
     return parts
 
 
 def linear_attention_backward(q, k, v, log_decay, d_o, q_scale: float = 1.0, need_dg: bool = False):
     """(dq, dk, dv[, dg]) of ``linear_attention_forward`` (no normalisation), the job of the reference's three backward
-    kernels (core/template/tl_template/linear/linear_tl.py:461-975), as five runs of the forward kernel.  With
+    kernels (core/template/tl_template/linear/linear_tl.py:461-975), as runs of the forward kernel.  With
     D_ij = exp(G_i - G_j) for j <= i:
 
         dq_i = q_scale * sum_{j<=i} D_ij (do_i . v_j) k_j      = retention(q = do, k = v, v = k)
-        dv_j = q_scale * sum_{i>=j} D_ij (q_i . k_j) do_i      = retention(q = k, k = q, v = do) with time reversed
-        dk_j = q_scale * sum_{i>=j} D_ij (do_i . v_j) q_i      = retention(q = v, k = do, v = q) with time reversed
+        dv_j = q_scale * sum_{i>=j} D_ij (q_i . k_j) do_i      = reversed retention(q = k, k = q, v = do)
+        dk_j = q_scale * sum_{i>=j} D_ij (do_i . v_j) q_i      = reversed retention(q = v, k = do, v = q)
 
-    Reversing time turns the anti-causal sums into causal ones; position u of the reversed sequence then carries the
-    log-decay of token T - u (0 for u = 0), so that the reversed cumulative sums reproduce the same D_ij.  The two
-    contractions over dim_v go through ``_retention_parts`` (dim_v may exceed the kernel's 256 columns of dim_qk).
-    Reversals, column ranges and the sums of the partial results are single passes of the library's row kernels.
+    The two contractions over dim_v go through ``_retention_parts`` (dim_v may exceed the kernel's 256 columns of dim_qk).
 
     ``need_dg``: also the gradient with respect to the per-token log-decay, fp32 [B, H, T].  A score A_ij depends on the
     log-decays of tokens j+1..i, so dg_t = sum_{i>=t, j<t} dA_ij A_ij; with dG_i = q_i . dq_i - k_i . dk_i (row sums
     minus column sums of dA o A) that is the reversed cumulative sum of dG — what the reference's dqkg kernel and its
     ``compute_final_dg`` produce per chunk (linear_tl.py:63-76, 638-814).  dg is a difference of sums over dq and dk:
-    those runs then keep the 16-bit remainder of their decayed scores."""
+    those runs then keep the 16-bit remainder of their decayed scores, and leave fp32 results for the row sums."""
     d_o = d_o.to(q.dtype)
     B, H, T, _ = q.shape
-    ld = log_decay.to(dtype=torch.float32, device=q.device).expand(B, H, T)
-    ld_rev = torch.cat([torch.zeros_like(ld[..., :1]), ld.flip(-1)[..., :-1]], dim=-1).contiguous()
-    dq_parts = _retention_parts(d_o, v, k, ld, q_scale, precise=need_dg)
-    dq = _sum_cast(dq_parts, q.dtype)
-    qr, kr, dr = _rows(q, reverse=True), _rows(k, reverse=True), _rows(d_o, reverse=True)
-    # dv: dim_qk fits the kernel, so it is one run that leaves the kernel in the operands' dtype
-    dv = _rows(linear_attention_forward(kr, qr, dr, ld_rev, q_scale), reverse=True)
-    # dk contracts over column ranges of the reversed v and dO: dO is reversed already (whole, for dv) and v is reversed
-    # once; the kernel reads the ranges in place
-    dk_parts = _retention_parts(_rows(v, reverse=True), dr, qr, ld_rev, q_scale, precise=need_dg)
-    dk = _sum_cast(dk_parts, k.dtype, reverse=True)
+    q, k, v, d_o = q.contiguous(), k.contiguous(), v.contiguous(), d_o.contiguous()
+    ld = log_decay.to(dtype=torch.float32, device=q.device).expand(B, H, T).contiguous()
+    dq_parts = _retention_parts(d_o, v, k, ld, q_scale, precise=need_dg, fp32=need_dg)
+    dv = _reversed_forward(k, q, d_o, ld, q_scale)
+    dk_parts = _retention_parts(v, d_o, q, ld, q_scale, precise=need_dg, reverse=True, fp32=need_dg)
     if not need_dg:
-        return dq, dk, dv
-    dq32 = sum(dq_parts[1:], dq_parts[0])
-    dk32_rev = sum(dk_parts[1:], dk_parts[0])
-    d_cum = (q.float() * dq32).sum(-1) - (kr.float() * dk32_rev).sum(-1).flip(-1)
-    dg = d_cum.flip(-1).cumsum(-1).flip(-1)
-    return dq, dk, dv, dg
+        return _sum_cast(dq_parts, q.dtype), _sum_cast(dk_parts, k.dtype), dv
+    dq_parts, dk_parts = _at_most_two(dq_parts), _at_most_two(dk_parts)
+    if q.is_cuda and q.shape[-1] % 8 == 0:
+        dq, dk, dg = native.linear_decay_grad(q, k, dq_parts, dk_parts)
+        return dq, dk, dv, dg
+    d_cum = (q.float() * sum(dq_parts)).sum(-1) - (k.float() * sum(dk_parts)).sum(-1)
+    return _sum_cast(dq_parts, q.dtype), _sum_cast(dk_parts, k.dtype), dv, d_cum.flip(-1).cumsum(-1).flip(-1)
 
 
 class _ForwardOnly(torch.autograd.Function):

@@ -87,7 +87,7 @@ class LinearArgs(C.Structure):
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_int64),
         ("dtype_out", C.c_int32), ("precise", C.c_int32),
         ("v_scale", C.c_void_p), ("heads_q", C.c_int32), ("heads_k", C.c_int32), ("q_ld", C.c_int32), ("k_ld", C.c_int32),
-        ("segments", C.c_int32),
+        ("segments", C.c_int32), ("reverse", C.c_int32),
     ]
 
 
@@ -148,6 +148,7 @@ SIGNATURES = {
     "attn_b200_linear_fwd": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "attn_b200_rows_copy16": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                         C.c_void_p]),
+    "attn_b200_linear_decay_grad": (C.c_int, [C.c_void_p] * 10 + [C.c_int32, C.c_int64, C.c_int32, C.c_int32, C.c_void_p]),
     "attn_b200_rows_sum_cast": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int32, C.c_int32,
                                           C.c_int32, C.c_void_p]),
     "attn_b200_linear_workspace_bytes": (C.c_int64, [C.POINTER(LinearArgs)]),
@@ -392,6 +393,27 @@ def rows_copy(src, col0: int = 0, width: int | None = None, reverse: bool = Fals
         check(load_library().attn_b200_rows_copy16(src.data_ptr(), dst.data_ptr(), src.numel() // (seq * cols), seq, cols, col0, width,
                                                    1 if reverse else 0, current_stream_ptr()), "attn_b200_rows_copy16")
     return dst
+
+
+def linear_decay_grad(q, k, dq_parts, dk_parts):
+    """dq, dk rounded to the dtype of q [B, H, T, cols] and the gradient of the log-decays [B, H, T], from one or two fp32
+    partial results each (attn_b200_linear_decay_grad)."""
+    if not q.is_cuda:
+        raise NativeError("linear_decay_grad needs CUDA tensors: there is no CPU path")
+    q, k = q.contiguous(), k.contiguous()
+    B, H, T, cols = q.shape
+    parts = [t.contiguous() for t in (*dq_parts, *dk_parts)]   # alive until the launch
+    ptrs = [t.data_ptr() for t in parts]
+    dq_a, dq_b = ptrs[0], ptrs[1] if len(dq_parts) > 1 else None
+    dk_a, dk_b = ptrs[len(dq_parts)], ptrs[len(dq_parts) + 1] if len(dk_parts) > 1 else None
+    dq, dk = torch.empty_like(q), torch.empty_like(k)
+    dg = torch.empty(B, H, T, dtype=torch.float32, device=q.device)
+    term = torch.empty_like(dg)
+    with torch.cuda.device(q.device):
+        check(load_library().attn_b200_linear_decay_grad(q.data_ptr(), k.data_ptr(), dq_a, dq_b, dk_a, dk_b, dq.data_ptr(), dk.data_ptr(),
+                                                         term.data_ptr(), dg.data_ptr(), DTYPE_CODES[q.dtype], B * H, T, cols,
+                                                         current_stream_ptr()), "attn_b200_linear_decay_grad")
+    return dq, dk, dg
 
 
 def rows_sum_cast(a, b, dtype, reverse: bool = False):

@@ -94,7 +94,7 @@ struct LinearSmem {
   static constexpr int kBytes = kOffMisc + 16 + 1024;
 };
 
-template <int DK, bool kBf16, bool kCut>
+template <int DK, bool kBf16, bool kCut, bool kRev>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const LinearParams p) {
@@ -145,7 +145,13 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   // This CTA's blocks are [t0, t_end); before them it runs the state alone over blocks [0, t0).  Whole chains are an
   // instantiation of their own: with a t0 known only at run time they ran 3 % slower (335 -> 344 us on 8 x 8 x 4096).
   // The row threads poll on their barriers: 306 -> 300 us there.
-  const int t0 = kCut ? p.cut[blockIdx.z] : 0, t_end = kCut ? p.cut[blockIdx.z + 1] : (p.seq + T - 1) / T;
+  // kRev: the sums run over the tokens from a row's own to the end of the sequence.  The blocks are walked from the last
+  // to the first; inside a block `later` tokens are those with lower rows, and a token's log-decay counts for the step to
+  // it from its successor's side, i.e. for rows below it (token tok + 1's stands between tok and tok + 1).
+  const int nblk = (p.seq + T - 1) / T;
+  auto first_token = [&](int t) { return (kRev ? nblk - 1 - t : t) * T; };   // of the t-th block walked
+  constexpr int kLast = kRev ? 0 : T - 1;                                    // the row a block's walk ends at
+  const int t0 = kCut ? p.cut[blockIdx.z] : 0, t_end = kCut ? p.cut[blockIdx.z + 1] : nblk;
   const float* ld_row = p.log_decay + static_cast<long long>(bh) * p.seq;
   const int b_idx = bh / p.heads, h_idx = bh - b_idx * p.heads;
   const int bh_q = b_idx * p.heads_q + h_idx / (p.heads / p.heads_q), bh_k = b_idx * p.heads_k + h_idx / (p.heads / p.heads_k);
@@ -189,15 +195,15 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (lane == 0 && start_ok) {
       auto load_q = [&](int t) {
         mbar_arrive_expect_tx(q_full, L::kQBytes);
-        for (int c = 0; c < KC; ++c) tma_load_3d(sQ + c * (T * 128), &tmQ, q_full, c * 64, t * T, bh_q);
+        for (int c = 0; c < KC; ++c) tma_load_3d(sQ + c * (T * 128), &tmQ, q_full, c * 64, first_token(t), bh_q);
       };
       auto load_k = [&](int t) {
         mbar_arrive_expect_tx(k_full, L::kQBytes);
-        for (int c = 0; c < KC; ++c) tma_load_3d(sKh + c * L::kPairBytes, &tmK, k_full, c * 64, t * T, bh_k);
+        for (int c = 0; c < KC; ++c) tma_load_3d(sKh + c * L::kPairBytes, &tmK, k_full, c * 64, first_token(t), bh_k);
       };
       auto load_v = [&](int t) {
         mbar_arrive_expect_tx(v_full, L::kVBytes);
-        for (int c = 0; c < DVS / 64; ++c) tma_load_3d(sV + c * (T * 128), &tmV, v_full, slice * DVS + c * 64, t * T, bh);
+        for (int c = 0; c < DVS / 64; ++c) tma_load_3d(sV + c * (T * 128), &tmV, v_full, slice * DVS + c * 64, first_token(t), bh);
       };
       // kind::f16 takes one 16-bit format for both operands: a variant with fp16 intermediates next to
       // bf16 inputs (A and B formats differing) raised a CUDA fault on B200 and is not offered.
@@ -239,7 +245,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           const int b = (t0 - t) & 1;
           mbar_arrive_expect_tx(pre_k + b, L::kQBytes);
           for (int c = 0; c < KC; ++c)
-            tma_load_3d(sKh + c * L::kPairBytes + b * L::kChunkBytes, &tmK, pre_k + b, c * 64, t * T, bh_k);
+            tma_load_3d(sKh + c * L::kPairBytes + b * L::kChunkBytes, &tmK, pre_k + b, c * 64, first_token(t), bh_k);
         };
         auto pre_load_v = [&](int t) {
           if (t > t0) return;
@@ -247,7 +253,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           const int b = (t0 - t) % 3;
           uint8_t* dst = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
           mbar_arrive_expect_tx(pre_v + b, L::kVBytes);
-          for (int c = 0; c < DVS / 64; ++c) tma_load_3d(dst + c * (T * 128), &tmV, pre_v + b, slice * DVS + c * 64, t * T, bh);
+          for (int c = 0; c < DVS / 64; ++c) tma_load_3d(dst + c * (T * 128), &tmV, pre_v + b, slice * DVS + c * 64, first_token(t), bh);
         };
         pre_load_v(0);
         pre_load_k(0);
@@ -305,7 +311,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           // in the pipe: the row threads take its completion to mean that the state's copy is no longer read.
           if (!mbar_wait_poll(v_ready, par, ab, kLinVReady)) break;
           tc_fence_after_sync();
-          const bool mild = g2[(t & 1) * T + T - 1] >= kMildLog2;
+          const bool mild = g2[(t & 1) * T + kLast] >= kMildLog2;
           const uint64_t va_desc0 = mild ? v_mn_desc0 : v2_mn_desc0;
 #pragma unroll
           for (int g = 0; g < T / 64; ++g)
@@ -354,7 +360,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       float x[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int tok = t * T + lane * 4 + k;
+        const int tok = first_token(t) + (kRev ? T - (lane * 4 + k) : lane * 4 + k);
         x[k] = tok < p.seq ? ld_row[tok] * kLog2e : 0.0f;
       }
       x[1] += x[0];
@@ -375,8 +381,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float g = pre + x[k];
-        g2[(t & 1) * T + lane * 4 + k] = g;
-        gb[lane * 4 + k] = fast_exp2(g_end - g);
+        const int i = kRev ? T - 1 - (lane * 4 + k) : lane * 4 + k;
+        g2[(t & 1) * T + i] = g;
+        gb[i] = fast_exp2(g_end - g);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(g_ready);
@@ -457,11 +464,11 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     };
     auto rescale_v = [&](int tb, bool in_place) -> bool {
       // a per-token factor of the caller on v (v_mod = v * t[b, h, token]) rides along: fetched before the wait for V
-      const int tok = tb * T + row;
+      const int tok = first_token(tb) + row;
       const float vs = (p.v_scale != nullptr && tok < p.seq) ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
       const bool v_ok = mbar_wait(v_full, (tb - t0) & 1, ab, kLinVFull);
       const float* g = g2 + (tb & 1) * T;
-      const float w = fast_exp2(g[T - 1] - g[row]) * vs;
+      const float w = fast_exp2(g[kLast] - g[row]) * vs;
       // with strong decay P V reads V itself: the caller's factor then goes onto V in place as well
       const bool scale_v_too = !in_place && p.v_scale != nullptr;
       uint4* vsrc = reinterpret_cast<uint4*>(sV + wg * (T * 128) + row * 128);
@@ -477,12 +484,12 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     for (int t = 0; kCut && ok && t < t0; ++t) {
       const int b = (t0 - t) % 3;
       uint8_t* v_buf = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
-      const int tok = t * T + row;
-      const float vs = p.v_scale != nullptr ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
+      const int tok = first_token(t) + row;
+      const float vs = p.v_scale != nullptr && tok < p.seq ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
       ok = mbar_wait_poll(g_ready, t & 1, ab, kLinDecay);
       const float* g = g2 + (t & 1) * T;
-      const float decay = fast_exp2(g[T - 1]);
-      const float w = fast_exp2(g[T - 1] - g[row]) * vs;
+      const float decay = fast_exp2(g[kLast]);
+      const float w = fast_exp2(g[kLast] - g[row]) * vs;
       ok = mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok;
       if (!ok) break;
       uint4* line = reinterpret_cast<uint4*>(v_buf + wg * (T * 128) + row * 128);
@@ -508,7 +515,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     ok = ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay);
     if (ok) {
-      const float g_first = g2[(t0 & 1) * T + T - 1];
+      const float g_first = g2[(t0 & 1) * T + kLast];
       const bool mild_first = g_first >= kMildLog2;
       if (mild_first) ok = rescale_v(t0, true);
       if (kCut && t0 > 0) {
@@ -542,7 +549,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       // P is then the masked scores themselves, O = Q h needs no pass between the two MMAs, and the rows of V are
       // rescaled a block ahead, while the output rows of the block before are being stored.  Blocks with a stronger decay (gated linear attention) keep every factor <= 1:
       // exp(g_i - g_j) in P, a rescale of Q h by exp(g_i), and the rescaled V in a buffer of its own.
-      const float g_last = g2[buf * T + T - 1];
+      const float g_last = g2[buf * T + kLast];
       const bool mild = g_last >= kMildLog2;
       if (!mild) {
         ok = mbar_wait(s_bar, par, ab, kLinQh);   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
@@ -580,7 +587,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           const int c = 2 * wg + h;  // 32-column chunk of S
           uint32_t* pkh = pk + 16 * h;
           uint32_t* plh = pl + 16 * h;
-          if (c > wq) {
+          if (kRev ? c < wq : c > wq) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) pkh[i] = plh[i] = 0u;
             continue;
@@ -594,10 +601,10 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             // the column factors are in the rows of V already: only the mask is left
             if (c == wq) {
 #pragma unroll
-              for (int i = 0; i < 32; ++i) s[i] = (i <= lane) ? s[i] : 0.0f;
+              for (int i = 0; i < 32; ++i) s[i] = (kRev ? i >= lane : i <= lane) ? s[i] : 0.0f;
             }
-          } else if (c < wq) {
-            const float a = qs * fast_exp2(fminf(gi - gcol[31], 0.0f));
+          } else if (c != wq) {
+            const float a = qs * fast_exp2(fminf(gi - gcol[kRev ? 0 : 31], 0.0f));
 #pragma unroll
             for (int i = 0; i < 32; ++i) s[i] *= a * bcol[i];
           } else {
@@ -605,7 +612,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
             for (int i = 0; i < 32; ++i) {
               // computed for every column and selected afterwards: a per-lane branch here diverges in every warp
               const float e = s[i] * qs * fast_exp2(fminf(gi - gcol[i], 0.0f));
-              s[i] = (i <= lane) ? e : 0.0f;
+              s[i] = (kRev ? i >= lane : i <= lane) ? e : 0.0f;
             }
           }
 #pragma unroll
@@ -648,7 +655,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       bool mild_next = false;   // the coming block multiplies Q by the state after its decay
       if (!last) {
         ok = mbar_wait_poll(g_ready, (t + 1) & 1, ab, kLinDecay) && ok;   // written once every warp was past the P phase
-        const float g_next = g2[(buf ^ 1) * T + T - 1];
+        const float g_next = g2[(buf ^ 1) * T + kLast];
         decay_next = fast_exp2(g_next);
         mild_next = g_next >= kMildLog2;
         ok = mbar_wait_poll(st_bar, par, ab, kLinState) && ok;
@@ -663,7 +670,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         // The rows go out through shared memory: the buffer of the state's operand copy is idle between the
         // Q.h MMA of this block and the conversion pass at its end.  Group `wg` writes the 64-column chunk
         // `wg` of its row as one swizzled 128-byte line (the layout TMA expects).
-        const int tok = t * T + row;
+        const int tok = first_token(t) + row;
         float sum = 0.f, sq = 0.f;
         uint8_t* stage = (DK == 64 && wg == 1) ? sStageX : sKh + wg * L::kPairBytes + L::kChunkBytes;
         uint8_t* line = stage + row * 128;
@@ -725,7 +732,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         fence_proxy_async_smem();   // also orders the copy's early chunks, converted above, before the arrival
         tc_fence_before_sync();
         warp_arrive(hi_ready);      // O has been read and the early chunks are in place: the next [S | O] may start
-        const int tok0 = t * T + (warp & 3) * 32;
+        const int tok0 = first_token(t) + (warp & 3) * 32;
         if (lane == 0 && p.o_f32 == nullptr && tok0 < p.seq) {
           tma_store_3d(&tmO, stage + (warp & 3) * (32 * 128), slice * DVS + wg * 64, tok0, bh);
           tma_store_commit();
@@ -912,7 +919,8 @@ int launch_linear(const AttnB200LinearArgs* a, cudaStream_t stream, int* status)
     cut_chain(nblk, segments, kStateShare, p.cut);
   }
   while (segments > 1 && p.cut[segments - 1] == nblk) --segments;   // more CTAs than the runs' lengths leave work for
-  auto kernel = segments > 1 ? linear_fwd_kernel<DK, kBf16, true> : linear_fwd_kernel<DK, kBf16, false>;
+  auto kernel = a->reverse ? (segments > 1 ? linear_fwd_kernel<DK, kBf16, true, true> : linear_fwd_kernel<DK, kBf16, false, true>)
+                           : (segments > 1 ? linear_fwd_kernel<DK, kBf16, true, false> : linear_fwd_kernel<DK, kBf16, false, false>);
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes) != cudaSuccess) {
     cudaGetLastError();
     return ATTN_B200_E_LAUNCH;

@@ -1,11 +1,8 @@
-// Row gathers around the linear-attention backward (sm_100a): the backward runs the forward kernel on time-reversed
-// operands and on column ranges of dim_v, and adds up fp32 partial results.  torch does each of these as a pass of its
-// own (flip, slice + contiguous, add, cast: ~0.2 ms apiece at the benchmark shape); here a reversed and / or
-// column-sliced copy is one pass, and sum + cast + reversal of the partial results another.
+// Row passes around the linear-attention backward (sm_100a), which adds up fp32 partial results of the forward kernel.
+// torch does each step as a pass of its own (slice + contiguous, add, cast, multiply, sum); here each is one pass.
 //   rows_copy16:    dst[o][s'][0:width] = src[o][s][col0:col0+width],  s' = reverse ? seq-1-s : s   (16-bit elements)
 //   rows_sum_cast:  dst16[o][s'][:]     = a[o][s][:] (+ b[o][s][:])                                 (fp32 -> fp16 / bf16)
-// The reference needs neither: its backward kernels walk the sequence backwards themselves
-// (core/template/tl_template/linear/linear_tl.py:461-975).
+//   decay_grad:     dq, dk as rows_sum_cast, and the gradient of the log-decays from the same reads
 #include <cstdint>
 
 #include "../../include/attn_b200.h"
@@ -58,6 +55,84 @@ __global__ void __launch_bounds__(256) rows_sum_cast_kernel(const float* __restr
   }
 }
 
+// Gradient of the log-decays (see the header).  A warp per row reads the fp32 results and the operands once, rounds the
+// gradients and leaves the row's term; torch took six passes over [rows, cols] fp32 for the same (93 us of 2 x 8 x 2000 x
+// 128, now 8).  Bound by HBM.
+template <bool kBf16>
+__global__ void __launch_bounds__(256) decay_grad_rows_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
+                                                             const float* __restrict__ dq_a, const float* __restrict__ dq_b,
+                                                             const float* __restrict__ dk_a, const float* __restrict__ dk_b,
+                                                             uint16_t* __restrict__ dq, uint16_t* __restrict__ dk,
+                                                             float* __restrict__ row_term, long long rows, int cols) {
+  const int lane = threadIdx.x & 31;
+  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  for (long long r = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
+    float term = 0.0f;
+    for (int c = lane * 4; c < cols; c += 128) {
+      const long long at = r * cols + c;
+#pragma unroll
+      for (int side = 0; side < 2; ++side) {
+        float4 x = *reinterpret_cast<const float4*>((side == 0 ? dq_a : dk_a) + at);
+        const float* second = side == 0 ? dq_b : dk_b;
+        if (second != nullptr) {
+          const float4 y = *reinterpret_cast<const float4*>(second + at);
+          x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+        }
+        const uint2 w = *reinterpret_cast<const uint2*>((side == 0 ? q : k) + at);
+        float2 w0, w1;
+        if constexpr (kBf16) {
+          w0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.x));
+          w1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w.y));
+        } else {
+          w0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
+          w1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+        }
+        const float dot = fmaf(w0.x, x.x, fmaf(w0.y, x.y, fmaf(w1.x, x.z, w1.y * x.w)));
+        term += side == 0 ? dot : -dot;
+        *reinterpret_cast<uint2*>((side == 0 ? dq : dk) + at) = make_uint2(pack2<kBf16>(x.x, x.y), pack2<kBf16>(x.z, x.w));
+      }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) term += __shfl_xor_sync(0xffffffffu, term, d);
+    if (lane == 0) row_term[r] = term;
+  }
+}
+
+// dg[t] = sum of row_term from t to the end: a CTA per sequence, from the last 1024 tokens to the first, the sum so far
+// carried along.
+__global__ void __launch_bounds__(1024) decay_grad_scan_kernel(const float* __restrict__ row_term, float* __restrict__ dg, int seq) {
+  __shared__ float warp_sum[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* in = row_term + static_cast<long long>(blockIdx.x) * seq;
+  float* out = dg + static_cast<long long>(blockIdx.x) * seq;
+  float carry = 0.0f;
+  for (int end = seq; end > 0; end -= 1024) {
+    const int t = end - 1 - static_cast<int>(threadIdx.x);
+    float x = t >= 0 ? in[t] : 0.0f;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const float y = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += y;
+    }
+    if (lane == 31) warp_sum[warp] = x;
+    __syncthreads();
+    if (warp == 0) {
+      float y = warp_sum[lane];
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const float z = __shfl_up_sync(0xffffffffu, y, d);
+        if (lane >= d) y += z;
+      }
+      warp_sum[lane] = y;
+    }
+    __syncthreads();
+    x += carry + (warp > 0 ? warp_sum[warp - 1] : 0.0f);
+    if (t >= 0) out[t] = x;
+    carry += warp_sum[31];
+    __syncthreads();
+  }
+}
+
 inline unsigned row_ops_grid(long long total_vectors) {
   const long long blocks = (total_vectors + 255) / 256;
   const long long cap = 148LL * 16;   // a multiple of the SM count; the loops stride over the rest
@@ -77,6 +152,30 @@ int attn_b200_rows_copy16(const void* src, void* dst, int64_t outer, int32_t seq
   const long long rows = static_cast<long long>(outer) * seq;
   b200::rows_copy16_kernel<<<b200::row_ops_grid(rows * (width / 8)), 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
       static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows, seq, src_cols, col0, width, reverse);
+  return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
+}
+
+int attn_b200_linear_decay_grad(const void* q, const void* k, const float* dq_a, const float* dq_b, const float* dk_a,
+                                const float* dk_b, void* dq, void* dk, float* row_term, float* dg, int32_t dtype, int64_t outer,
+                                int32_t seq, int32_t cols, void* cuda_stream) {
+  if (q == nullptr || k == nullptr || dq_a == nullptr || dk_a == nullptr || dq == nullptr || dk == nullptr || row_term == nullptr ||
+      dg == nullptr || outer <= 0 || seq <= 0 || cols <= 0)
+    return ATTN_B200_E_INVALID_ARG;
+  if (dtype != ATTN_B200_DTYPE_FP16 && dtype != ATTN_B200_DTYPE_BF16) return ATTN_B200_E_INVALID_ARG;
+  if (cols % 4 != 0 || outer > 0x7fffffff) return ATTN_B200_E_UNSUPPORTED;
+  uintptr_t bits = 0;
+  for (const void* ptr : {q, k, static_cast<const void*>(dq_a), static_cast<const void*>(dq_b), static_cast<const void*>(dk_a),
+                          static_cast<const void*>(dk_b), static_cast<const void*>(dq), static_cast<const void*>(dk)})
+    bits |= reinterpret_cast<uintptr_t>(ptr);
+  if ((bits & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
+  const long long rows = static_cast<long long>(outer) * seq;
+  cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
+  const unsigned grid = b200::row_ops_grid(rows * 32);
+  auto kernel = dtype == ATTN_B200_DTYPE_BF16 ? b200::decay_grad_rows_kernel<true> : b200::decay_grad_rows_kernel<false>;
+  kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), dq_a, dq_b, dk_a, dk_b,
+                                   static_cast<uint16_t*>(dq), static_cast<uint16_t*>(dk), row_term, rows, cols);
+  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  b200::decay_grad_scan_kernel<<<static_cast<unsigned>(outer), 1024, 0, stream>>>(row_term, dg, seq);
   return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
 }
 

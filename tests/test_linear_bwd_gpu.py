@@ -169,3 +169,44 @@ def test_row_kernels_against_torch(dtype):
         assert torch.equal(got, want.flip(2) if rev else want), (second is None, rev)
     with pytest.raises(lib.NativeError):
         lib.rows_copy(x, 4, 16, True)      # offsets and widths in units of 8 columns (16 bytes)
+
+
+@pytest.mark.parametrize("Dk,S,dtype,strong,precise", [
+    (64, 1100, torch.float16, False, False),     # ragged: the block with rows past the end is the first one walked
+    (128, 384, torch.bfloat16, True, True),
+    (128, 100, torch.bfloat16, False, False),    # one block
+    (256, 1000, torch.bfloat16, True, False),
+])
+def test_reversed_walk_against_reversed_operands(Dk, S, dtype, strong, precise):
+    """The kernel that walks the sequence from its end against the oracle on time-reversed operands, uncut and cut."""
+    from attn_engine.linear_attn_engine import linear_attention_forward
+    from core.native import lib
+    B, H, Dv = 1, 3, 128
+    g = torch.Generator().manual_seed(S + Dk)
+    q = torch.randn(B, H, S, Dk, generator=g).to(dtype)
+    k = (torch.randn(B, H, S, Dk, generator=g) * Dk ** -0.5).to(dtype)
+    v = torch.randn(B, H, S, Dv, generator=g).to(dtype)
+    ld = -torch.rand(B, H, S, generator=g) * (1.5 if strong else 0.02)
+    ld_rev = torch.cat([torch.zeros(B, H, 1), ld.flip(-1)[..., :-1]], dim=-1)
+    want = rm.decayed_linear_attention(q.flip(2), k.flip(2), v.flip(2), ld_rev, scale=0.5).flip(2)
+    args = [t.cuda() for t in (q, k, v, ld)]
+    whole = linear_attention_forward(*args, q_scale=0.5, precise=precise, segments=1, reverse=True)
+    assert ((whole.float().cpu() - want).norm() / want.norm()).item() < 1e-2
+    for segments in (0, 2, 4):
+        assert torch.equal(whole, linear_attention_forward(*args, q_scale=0.5, precise=precise, segments=segments, reverse=True))
+    assert lib.last_device_status() == 0
+
+
+@pytest.mark.parametrize("S,cols,dtype", [(301, 64, torch.float16), (1024, 128, torch.bfloat16), (2050, 256, torch.bfloat16)])
+def test_decay_gradient_kernel_against_torch(S, cols, dtype):
+    from core.native import lib
+    g = torch.Generator().manual_seed(S)
+    q, k = (torch.randn(2, 3, S, cols, generator=g).to(dtype).cuda() for _ in range(2))
+    parts = [torch.randn(2, 3, S, cols, generator=g).cuda() for _ in range(3)]
+    for dq_parts, dk_parts in ((parts[:1], parts[1:2]), (parts[:2], parts[2:]), (parts[:2], parts[1:])):
+        dq, dk, dg = lib.linear_decay_grad(q, k, dq_parts, dk_parts)
+        assert torch.equal(dq, sum(dq_parts).to(dtype)) and torch.equal(dk, sum(dk_parts).to(dtype))
+        row = (q.double() * sum(dq_parts).double()).sum(-1) - (k.double() * sum(dk_parts).double()).sum(-1)
+        want = row.flip(-1).cumsum(-1).flip(-1)
+        # fp32 sums of 2 * cols products and of S rows, pairwise or over lanes: a few units in the last place of the largest sum
+        assert (dg - want).abs().max().item() <= 2e-6 * S ** 0.5 * row.abs().max().item()
