@@ -201,6 +201,9 @@ typedef struct AttnB200LinearArgs {
                             o_j = sum_{i>=j} exp(G_i - G_j) (scale * q_j . k_i) v_i -- the transposed form that the gradients
                             of k and v need (the reference's backward kernels walk the sequence backwards as well,
                             linear_tl.py:461-975) */
+  int32_t any_dim_v;     /* 1: dim_v may be any multiple of 8 (0: of 128).  The missing columns of the last 128-column slice
+                            are read as zeros and not written; dim_v = 64 with heads / heads_q and heads / heads_k even puts
+                            two heads into one slice (Mamba2).  Not with normalize or an fp32 output */
 } AttnB200LinearArgs;
 
 /* Bytes of scratch the linear forward needs: per-row (sum, sum of squares) fp32 when normalize = 1, else 0. */

@@ -136,11 +136,12 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
     if H % q.shape[1] != 0 or H % k.shape[1] != 0:
         raise native.NativeError("the heads of v must be a multiple of the heads of q and of k")
     Dv = v.shape[-1]
-    if Dv % 128 != 0:
-        # the kernel works on 128-column slices of dim_v: a narrower v (Mamba2's head dim 64) is padded with
-        # zero columns, which stay zero in the output and are cut off again
-        if normalize:
-            raise native.NativeError("normalize needs dim_v to be a multiple of 128")
+    if Dv % 128 != 0 and normalize:
+        raise native.NativeError("normalize needs dim_v to be a multiple of 128")
+    if Dv % 8 != 0 or (f32_out and Dv % 128 != 0):
+        # rows of v that are not whole 16-byte pieces, or fp32 rows that are not whole slices: padded with zero columns,
+        # which stay zero in the output and are cut off again (otherwise the kernel reads the columns that a slice of 128
+        # is short of as zeros)
         pad = 128 - Dv % 128
         o = linear_attention_forward(q, k, torch.nn.functional.pad(v, (0, pad)), log_decay, q_scale, False, eps, out_dtype, v_scale,
                                      precise, segments, reverse)
@@ -167,6 +168,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
         a.precise = 1 if precise else 0
         a.segments = segments
         a.reverse = 1 if reverse else 0
+        a.any_dim_v = 1
         a.q_scale = float(q_scale)
         a.norm_eps = float(eps)
         lib = native.load_library()

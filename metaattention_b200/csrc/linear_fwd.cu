@@ -89,12 +89,13 @@ struct LinearSmem {
   static constexpr int kOffPreV1 = kScaledVInH ? kOffQ + kVBytes : kOffV2;
   static constexpr int kOffPreV2 = kQBytes >= kVBytes ? kOffQ : kOffG0;
   static constexpr int kOffG = kOffG0 + (kQBytes >= kVBytes ? 0 : kVBytes);  // float g2[2][128] + float gb[128]
-  static constexpr int kOffBar = kOffG + 3 * kLinT * 4 + 32;
+  static constexpr int kTables = DK == 256 ? 3 : 6;   // decay tables: two per head and one more (two heads: dim_qk <= 128)
+  static constexpr int kOffBar = kOffG + kTables * kLinT * 4 + 32;
   static constexpr int kOffMisc = kOffBar + 8 * kNumLinBarriers;
   static constexpr int kBytes = kOffMisc + 16 + 1024;
 };
 
-template <int DK, bool kBf16, bool kCut, bool kRev>
+template <int DK, bool kBf16, bool kCut, bool kRev, bool kPair>
 __global__ void __launch_bounds__(kLinThreads, 1)
 linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, const LinearParams p) {
@@ -107,6 +108,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   // (never with the remainder pass of P, which exists for the accuracy the rounded rows of V would give away)
   const float kMildLog2 = p.split_p ? 1.0f : (kBf16 ? -100.0f : -8.0f);
 
+  // kPair: dim_v is 64 and two consecutive heads that share their q and k heads make up the 128 columns, one V chunk,
+  // one half of the state's rows and one half of O's columns each.  S is then computed once for both.
+  constexpr int NH = kPair ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem + L::kOffQ;
@@ -114,8 +118,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint8_t* sV = smem + L::kOffV;
   uint8_t* sStageX = smem + L::kOffStageX;
   uint8_t* sV2 = smem + L::kOffV2;
-  float* g2 = reinterpret_cast<float*>(smem + L::kOffG);  // [2][T] cumulative log2-decay inside a block
-  float* gb = g2 + 2 * T;   // [T] exp2(g at the end of the column's 32-token chunk - g of the column), current block
+  float* g2 = reinterpret_cast<float*>(smem + L::kOffG);  // [heads][2][T] cumulative log2-decay inside a block
+  float* gb = g2 + 2 * NH * T;   // [T] exp2(g at the end of the column's 32-token chunk - g of the column), current block
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kOffBar);
   uint64_t* q_full = bars + kBarQFull;
   uint64_t* k_full = bars + kBarKFull;
@@ -141,7 +145,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int row = (warp & 3) * 32 + lane;   // TMEM lane owned by a row thread
   const AbortState ab{abort_flag, p.status};
   const int slice = blockIdx.x;
-  const int bh = blockIdx.y;
+  const int bh = blockIdx.y * NH;
   // This CTA's blocks are [t0, t_end); before them it runs the state alone over blocks [0, t0).  Whole chains are an
   // instantiation of their own: with a t0 known only at run time they ran 3 % slower (335 -> 344 us on 8 x 8 x 4096).
   // The row threads poll on their barriers: 306 -> 300 us there.
@@ -151,6 +155,12 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int nblk = (p.seq + T - 1) / T;
   auto first_token = [&](int t) { return (kRev ? nblk - 1 - t : t) * T; };   // of the t-th block walked
   constexpr int kLast = kRev ? 0 : T - 1;                                    // the row a block's walk ends at
+  auto block_mild = [&](int t) {   // of every head of the CTA
+    const float* g = g2 + (t & 1) * T + kLast;
+    return kPair ? fminf(g[0], g[2 * T]) >= kMildLog2 : g[0] >= kMildLog2;
+  };
+  auto v_col = [&](int c) { return kPair ? 0 : slice * DVS + c * 64; };   // column and (batch, head) of a CTA's 64-column chunk
+  auto v_bh = [&](int c) { return kPair ? bh + c : bh; };
   const int t0 = kCut ? p.cut[blockIdx.z] : 0, t_end = kCut ? p.cut[blockIdx.z + 1] : nblk;
   const float* ld_row = p.log_decay + static_cast<long long>(bh) * p.seq;
   const int b_idx = bh / p.heads, h_idx = bh - b_idx * p.heads;
@@ -203,27 +213,28 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       };
       auto load_v = [&](int t) {
         mbar_arrive_expect_tx(v_full, L::kVBytes);
-        for (int c = 0; c < DVS / 64; ++c) tma_load_3d(sV + c * (T * 128), &tmV, v_full, slice * DVS + c * 64, first_token(t), bh);
+        for (int c = 0; c < DVS / 64; ++c) tma_load_3d(sV + c * (T * 128), &tmV, v_full, v_col(c), first_token(t), v_bh(c));
       };
       // kind::f16 takes one 16-bit format for both operands: a variant with fp16 intermediates next to
       // bf16 inputs (A and B formats differing) raised a CUDA fault on B200 and is not offered.
       constexpr uint32_t idesc_s = make_idesc_f16(T, T, kBf16, false, false);          // S = Q K^T (first block)
       constexpr uint32_t idesc_sq = make_idesc_f16(T, T + DVS, kBf16, false, false);   // [S | O] = Q [K^T | hT^T]
       constexpr uint32_t idesc_pv = make_idesc_f16(T, DVS, kBf16, false, true);        // O += P V   (B = V, MN-major)
+      constexpr uint32_t idesc_pv64 = make_idesc_f16(T, 64, kBf16, false, true);       // one head's columns of it
       constexpr uint32_t idesc_h = make_idesc_f16(DVS, DK, kBf16, true, true);         // hT += V'^T K (A M-major, B MN-major)
       // descriptors are built once; the issue loops only move the start-address field (units of 16 bytes)
       const uint64_t q_desc0 = make_smem_desc(smem_u32(sQ), 16, 1024), kh_desc0 = make_smem_desc(smem_u32(sKh), 16, 1024);
       const uint64_t v_mn_desc0 = make_smem_desc(smem_u32(sV), T * 128, 1024);
       const uint64_t k_mn_desc0 = make_smem_desc(smem_u32(sKh), L::kPairBytes, 1024);
       const uint64_t v2_mn_desc0 = make_smem_desc(smem_u32(sV2), L::kV2Stride, 1024);
-      constexpr uint64_t kChunk = (T * 128) >> 4, kPair = L::kPairBytes >> 4;
+      constexpr uint64_t kChunk = (T * 128) >> 4, kKhPair = L::kPairBytes >> 4;
       static_assert(kColO == kColS + T, "S and O are the two halves of one accumulator");
       // Chunks [c0, c1) of dim_qk of [S | O] = Q [K^T | hT^T]: the K rows and the rows of the state's copy of a chunk
       // lie one after the other, so both products share the reads of Q.  In the first block there is no state yet
       // and only S is computed (P V then starts O afresh).
       auto issue_sq = [&](int t, int c0, int c1, bool fresh) {
         for (int ch = c0; ch < c1; ++ch)
-          umma_ss_x4<2, 2>(tmem_base + kColS, q_desc0 + ch * kChunk, kh_desc0 + ch * kPair, t == 0 ? idesc_s : idesc_sq,
+          umma_ss_x4<2, 2>(tmem_base + kColS, q_desc0 + ch * kChunk, kh_desc0 + ch * kKhPair, t == 0 ? idesc_s : idesc_sq,
                            (fresh && ch == c0) ? 0u : 1u);
       };
       // The copy's columns [0, 128) (chunks 0 and 1) are converted last, because their place stages the output rows;
@@ -253,7 +264,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           const int b = (t0 - t) % 3;
           uint8_t* dst = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
           mbar_arrive_expect_tx(pre_v + b, L::kVBytes);
-          for (int c = 0; c < DVS / 64; ++c) tma_load_3d(dst + c * (T * 128), &tmV, pre_v + b, slice * DVS + c * 64, first_token(t), bh);
+          for (int c = 0; c < DVS / 64; ++c) tma_load_3d(dst + c * (T * 128), &tmV, pre_v + b, v_col(c), first_token(t), v_bh(c));
         };
         pre_load_v(0);
         pre_load_k(0);
@@ -311,7 +322,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           // in the pipe: the row threads take its completion to mean that the state's copy is no longer read.
           if (!mbar_wait_poll(v_ready, par, ab, kLinVReady)) break;
           tc_fence_after_sync();
-          const bool mild = g2[(t & 1) * T + kLast] >= kMildLog2;
+          const bool mild = block_mild(t);
           const uint64_t va_desc0 = mild ? v_mn_desc0 : v2_mn_desc0;
 #pragma unroll
           for (int g = 0; g < T / 64; ++g)
@@ -328,10 +339,19 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         // O (+)= P V
         if (!(mbar_wait_poll(p_ready, par, ab, kLinPReady) && mbar_wait_poll(v_full, par, ab, kLinVFull))) break;
         tc_fence_after_sync();
+        if (kPair && !block_mild(t)) {   // a P of its own for each head
 #pragma unroll
-        for (int g = 0; g < T / 64; ++g)
-          umma_ts_x4<8, 128>(tmem_base + kColO, tmem_base + kColS + g * 32, v_mn_desc0 + g * 512, idesc_pv, (t > 0 || g > 0) ? 1u : 0u);
-        if (p.split_p) {
+          for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int g = 0; g < T / 64; ++g)
+              umma_ts_x4<8, 128>(tmem_base + kColO + n * 64, tmem_base + kColS + n * 64 + g * 32, v_mn_desc0 + n * kChunk + g * 512,
+                                 idesc_pv64, (t > 0 || g > 0) ? 1u : 0u);
+        } else {
+#pragma unroll
+          for (int g = 0; g < T / 64; ++g)
+            umma_ts_x4<8, 128>(tmem_base + kColO, tmem_base + kColS + g * 32, v_mn_desc0 + g * 512, idesc_pv, (t > 0 || g > 0) ? 1u : 0u);
+        }
+        if (!kPair && p.split_p) {
 #pragma unroll
           for (int g = 0; g < T / 64; ++g)
             umma_ts_x4<8, 128>(tmem_base + kColO, tmem_base + kColS + 64 + g * 32, v_mn_desc0 + g * 512, idesc_pv, 1u);
@@ -357,33 +377,39 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     // row threads are through the P phase of block t - 1.
     bool ok = start_ok;
     for (int t = 0; ok && t < t_end; ++t) {
-      float x[4];
+      float x[NH][4], pre[NH], g_end[NH];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int tok = first_token(t) + (kRev ? T - (lane * 4 + k) : lane * 4 + k);
-        x[k] = tok < p.seq ? ld_row[tok] * kLog2e : 0.0f;
-      }
-      x[1] += x[0];
-      x[2] += x[1];
-      x[3] += x[2];
-      float run = x[3];
+      for (int n = 0; n < NH; ++n) {
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const float y = __shfl_up_sync(0xffffffffu, run, d);
-        if (lane >= d) run += y;
+        for (int k = 0; k < 4; ++k) {
+          const int tok = first_token(t) + (kRev ? T - (lane * 4 + k) : lane * 4 + k);
+          x[n][k] = tok < p.seq ? ld_row[n * p.seq + tok] * kLog2e : 0.0f;
+        }
+        x[n][1] += x[n][0];
+        x[n][2] += x[n][1];
+        x[n][3] += x[n][2];
+        float run = x[n][3];
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const float y = __shfl_up_sync(0xffffffffu, run, d);
+          if (lane >= d) run += y;
+        }
+        pre[n] = run - x[n][3];
+        g_end[n] = __shfl_sync(0xffffffffu, run, lane | 7);   // last token of this lane's 32-token chunk
       }
-      const float pre = run - x[3];
-      const float g_end = __shfl_sync(0xffffffffu, run, lane | 7);   // last token of this lane's 32-token chunk
       if (t > 0 && lane == 0)   // before the CTA's own blocks a table is read by the rescaling of V only
         ok = t <= t0 ? mbar_wait_poll(pre_vready, (t - 1) & 1, ab, kLinDecay) : mbar_wait_poll(p_ready, (t - 1 - t0) & 1, ab, kLinDecay);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const float g = pre + x[k];
-        const int i = kRev ? T - 1 - (lane * 4 + k) : lane * 4 + k;
-        g2[(t & 1) * T + i] = g;
-        gb[i] = fast_exp2(g_end - g);
+      for (int n = 0; n < NH; ++n) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float g = pre[n] + x[n][k];
+          const int i = kRev ? T - 1 - (lane * 4 + k) : lane * 4 + k;
+          g2[(2 * n + (t & 1)) * T + i] = g;
+          gb[n * T + i] = fast_exp2(g_end[n] - g);
+        }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(g_ready);
@@ -391,6 +417,10 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   } else {
     // ======================= row threads: one TMEM lane (token / state row) each =======================
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    // the head of this thread's V chunk and O columns, and of its row of the state: their tables of block t
+    const int hv = kPair ? wg : 0, hs = kPair ? (warp & 3) >> 1 : 0;
+    auto g_v = [&](int t) -> const float* { return g2 + (2 * hv + (t & 1)) * T; };
+    auto g_s = [&](int t) -> const float* { return g2 + (2 * hs + (t & 1)) * T; };
     const uint32_t tH = tmem_base + lane_base + kColH;
     const uint32_t tS = tmem_base + lane_base + kColS;
     const uint32_t tO = tmem_base + lane_base + kColO;
@@ -465,9 +495,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     auto rescale_v = [&](int tb, bool in_place) -> bool {
       // a per-token factor of the caller on v (v_mod = v * t[b, h, token]) rides along: fetched before the wait for V
       const int tok = first_token(tb) + row;
-      const float vs = (p.v_scale != nullptr && tok < p.seq) ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
-      const bool v_ok = mbar_wait(v_full, (tb - t0) & 1, ab, kLinVFull);
-      const float* g = g2 + (tb & 1) * T;
+      const float vs = (p.v_scale != nullptr && tok < p.seq) ? p.v_scale[static_cast<long long>(bh + hv) * p.seq + tok] : 1.0f;
+      const bool v_ok = mbar_wait_poll(v_full, (tb - t0) & 1, ab, kLinVFull);
+      const float* g = g_v(tb);
       const float w = fast_exp2(g[kLast] - g[row]) * vs;
       // with strong decay P V reads V itself: the caller's factor then goes onto V in place as well
       const bool scale_v_too = !in_place && p.v_scale != nullptr;
@@ -485,10 +515,10 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const int b = (t0 - t) % 3;
       uint8_t* v_buf = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
       const int tok = first_token(t) + row;
-      const float vs = p.v_scale != nullptr && tok < p.seq ? p.v_scale[static_cast<long long>(bh) * p.seq + tok] : 1.0f;
+      const float vs = p.v_scale != nullptr && tok < p.seq ? p.v_scale[static_cast<long long>(bh + hv) * p.seq + tok] : 1.0f;
       ok = mbar_wait_poll(g_ready, t & 1, ab, kLinDecay);
-      const float* g = g2 + (t & 1) * T;
-      const float decay = fast_exp2(g[kLast]);
+      const float* g = g_v(t);
+      const float decay = fast_exp2(g_s(t)[kLast]);
       const float w = fast_exp2(g[kLast] - g[row]) * vs;
       ok = mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok;
       if (!ok) break;
@@ -515,11 +545,10 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     ok = ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay);
     if (ok) {
-      const float g_first = g2[(t0 & 1) * T + kLast];
-      const bool mild_first = g_first >= kMildLog2;
+      const bool mild_first = block_mild(t0);
       if (mild_first) ok = rescale_v(t0, true);
       if (kCut && t0 > 0) {
-        const float decay_first = fast_exp2(g_first);
+        const float decay_first = fast_exp2(g_s(t0)[kLast]);
         ok = mbar_wait(pre_st, (t0 - 1) & 1, ab, kLinPreState) && ok;
         tc_fence_after_sync();
 #pragma unroll
@@ -536,10 +565,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     if (kCut && t0 > 0) ok = named_sync_and(1 + (warp & 3), 64, ok);   // the two warps of a lane quarter enter the loop together or not at all
     for (int t = t0; ok && t < t_end; ++t) {
-      const int buf = t & 1;
       const bool last = (t + 1 == t_end);
       const uint32_t par = (t - t0) & 1;
-      const float gi = g2[buf * T + row];
+      const float gi = g_v(t)[row];
       const float qs = p.q_scale;
       // Mild decay (the block's total log2-decay stays inside the exponent range of the 16-bit operands with room
       // to spare): exp(g_i - g_j) is split as exp(g_i - g_last) * exp(g_last - g_j).  The second factor is the one
@@ -549,8 +577,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       // P is then the masked scores themselves, O = Q h needs no pass between the two MMAs, and the rows of V are
       // rescaled a block ahead, while the output rows of the block before are being stored.  Blocks with a stronger decay (gated linear attention) keep every factor <= 1:
       // exp(g_i - g_j) in P, a rescale of Q h by exp(g_i), and the rescaled V in a buffer of its own.
-      const float g_last = g2[buf * T + kLast];
-      const bool mild = g_last >= kMildLog2;
+      const float g_last = g_v(t)[kLast];
+      const bool mild = kPair ? block_mild(t) : g_last >= kMildLog2;
       if (!mild) {
         ok = mbar_wait(s_bar, par, ab, kLinQh);   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
         tc_fence_after_sync();
@@ -582,21 +610,18 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const int wq = warp & 3;
         ok = mbar_wait_poll(s_bar, par, ab, kLinScore) && ok;
         tc_fence_after_sync();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int c = 2 * wg + h;  // 32-column chunk of S
-          uint32_t* pkh = pk + 16 * h;
-          uint32_t* plh = pl + 16 * h;
+        // 32-column chunk c of the row: P into pkh, with split_p its 16-bit remainder into plh
+        auto make_p = [&](int c, uint32_t* pkh, uint32_t* plh) {
           if (kRev ? c < wq : c > wq) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) pkh[i] = plh[i] = 0u;
-            continue;
+            return;
           }
           float s[32];
           tmem_ld32f(tS + c * 32, s);
           tmem_wait_ld();
-          const float* gcol = g2 + buf * T + c * 32;
-          const float* bcol = gb + c * 32;
+          const float* gcol = g_v(t) + c * 32;
+          const float* bcol = gb + hv * T + c * 32;
           if (mild) {
             // the column factors are in the rows of V already: only the mask is left
             if (c == wq) {
@@ -617,7 +642,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           }
 #pragma unroll
           for (int i = 0; i < 16; ++i) pkh[i] = pack2<kBf16>(s[2 * i], s[2 * i + 1]);
-          if (p.split_p) {
+          if (!kPair && p.split_p) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
               float h0, h1;
@@ -633,6 +658,19 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
               plh[i] = pack2<kBf16>(s[2 * i] - h0, s[2 * i + 1] - h1);
             }
           }
+        };
+        // Two heads with strong decay: each warp group makes its own head's P, all four chunks of it (in pk and pl; the
+        // remainder pass does not come with two heads), and writes it to columns [64 wg, 64 wg + 64).
+        const bool two_p = kPair && !mild;
+        if (two_p) {
+          uint32_t none[16];
+          make_p(0, pk, none);
+          make_p(1, pk + 16, none);
+          make_p(2, pl, none);
+          make_p(3, pl + 16, none);
+        } else {
+          make_p(2 * wg, pk, pl);
+          make_p(2 * wg + 1, pk + 16, pl + 16);
         }
         // P overwrites S: 16-bit pairs in columns [0, 64), and with split_p the 16-bit remainder P - round(P) in
         // columns [64, 128) for a second PV pass.  Those columns belong to the other group's half of the same rows
@@ -641,8 +679,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         ok = named_sync_and(1 + (warp & 3), 64, ok);
         if (!ok) break;
         tc_fence_after_sync();
-        tmem_st32(tS + wg * 32, pk);
-        if (p.split_p) tmem_st32(tS + 64 + wg * 32, pl);
+        tmem_st32(tS + wg * (two_p ? 64 : 32), pk);
+        if (two_p) tmem_st32(tS + wg * 64 + 32, pl);
+        if (!kPair && p.split_p) tmem_st32(tS + 64 + wg * 32, pl);
       }
       tmem_wait_st();
       tc_fence_before_sync();
@@ -655,9 +694,9 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       bool mild_next = false;   // the coming block multiplies Q by the state after its decay
       if (!last) {
         ok = mbar_wait_poll(g_ready, (t + 1) & 1, ab, kLinDecay) && ok;   // written once every warp was past the P phase
-        const float g_next = g2[(buf ^ 1) * T + kLast];
+        const float g_next = g_s(t + 1)[kLast];
         decay_next = fast_exp2(g_next);
-        mild_next = g_next >= kMildLog2;
+        mild_next = kPair ? block_mild(t + 1) : g_next >= kMildLog2;
         ok = mbar_wait_poll(st_bar, par, ab, kLinState) && ok;
         tc_fence_after_sync();
 #pragma unroll
@@ -685,8 +724,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           if (p.o_f32 != nullptr) {
             // fp32 output: this thread's 32 columns of its token row, 128 contiguous bytes
             if (tok < p.seq) {
-              float4* dst = reinterpret_cast<float4*>(p.o_f32 + (static_cast<long long>(bh) * p.seq + tok) * p.dim_v +
-                                                      slice * DVS + wg * 64 + c * 32);
+              const int col0 = v_col(wg) + c * 32;
+              float4* dst = reinterpret_cast<float4*>(p.o_f32 + (static_cast<long long>(v_bh(wg)) * p.seq + tok) * p.dim_v + col0);
 #pragma unroll
               for (int v = 0; v < 8; ++v) dst[v] = make_float4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
             }
@@ -733,8 +772,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         tc_fence_before_sync();
         warp_arrive(hi_ready);      // O has been read and the early chunks are in place: the next [S | O] may start
         const int tok0 = first_token(t) + (warp & 3) * 32;
-        if (lane == 0 && p.o_f32 == nullptr && tok0 < p.seq) {
-          tma_store_3d(&tmO, stage + (warp & 3) * (32 * 128), slice * DVS + wg * 64, tok0, bh);
+        if (lane == 0 && p.o_f32 == nullptr && tok0 < p.seq && v_col(wg) < p.dim_v) {
+          tma_store_3d(&tmO, stage + (warp & 3) * (32 * 128), v_col(wg), tok0, v_bh(wg));
           tma_store_commit();
         }
       }
@@ -908,24 +947,30 @@ int launch_linear(const AttnB200LinearArgs* a, cudaStream_t stream, int* status)
     p.stats = static_cast<float*>(a->workspace);
     if (cudaMemsetAsync(p.stats, 0, rows * 2 * sizeof(float), stream) != cudaSuccess) return ATTN_B200_E_LAUNCH;
   }
-  const int nblk = (a->seq + kLinT - 1) / kLinT, slices = a->dim_v / kLinDvs;
+  // Heads of 64 columns that share q and k (Mamba2) go two to a CTA (1 x 80 x 2048 x 128 / 64: 79 -> 45 us) instead of one head
+  // per CTA with half of its columns zero.
+  const bool pair = DK <= 128 && a->dim_v == 64 && (a->heads / heads_q) % 2 == 0 && (a->heads / heads_k) % 2 == 0 && !p.split_p && !a->reverse;
+  const int nblk = (a->seq + kLinT - 1) / kLinT, slices = (a->dim_v + kLinDvs - 1) / kLinDvs;
   int segments = a->segments > nblk ? nblk : a->segments;
   if (segments <= 0) {
     int sms = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return ATTN_B200_E_LAUNCH;
-    segments = plan_segments(static_cast<long long>(bh) * slices, nblk, sms, kStateShare, p.cut);
+    segments = plan_segments(static_cast<long long>(pair ? bh / 2 : bh) * slices, nblk, sms, kStateShare, p.cut);
   } else {
     cut_chain(nblk, segments, kStateShare, p.cut);
   }
   while (segments > 1 && p.cut[segments - 1] == nblk) --segments;   // more CTAs than the runs' lengths leave work for
-  auto kernel = a->reverse ? (segments > 1 ? linear_fwd_kernel<DK, kBf16, true, true> : linear_fwd_kernel<DK, kBf16, false, true>)
-                           : (segments > 1 ? linear_fwd_kernel<DK, kBf16, true, false> : linear_fwd_kernel<DK, kBf16, false, false>);
+  const bool cut = segments > 1;
+  auto kernel = a->reverse ? (cut ? linear_fwd_kernel<DK, kBf16, true, true, false> : linear_fwd_kernel<DK, kBf16, false, true, false>)
+                           : (cut ? linear_fwd_kernel<DK, kBf16, true, false, false> : linear_fwd_kernel<DK, kBf16, false, false, false>);
+  if constexpr (DK <= 128)
+    if (pair) kernel = cut ? linear_fwd_kernel<DK, kBf16, true, false, true> : linear_fwd_kernel<DK, kBf16, false, false, true>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes) != cudaSuccess) {
     cudaGetLastError();
     return ATTN_B200_E_LAUNCH;
   }
-  dim3 grid(slices, static_cast<unsigned>(bh), segments);
+  dim3 grid(slices, static_cast<unsigned>(pair ? bh / 2 : bh), segments);
   kernel<<<grid, kLinThreads, L::kBytes, stream>>>(tmQ, tmK, tmV, tmO, p);
   if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
   if (a->normalize) {
@@ -952,7 +997,9 @@ int attn_b200_linear_fwd(const AttnB200LinearArgs* a, void* cuda_stream) {
   if (a->batch <= 0 || a->heads <= 0 || a->seq <= 0) return ATTN_B200_E_INVALID_ARG;
   if (a->dtype != ATTN_B200_DTYPE_FP16 && a->dtype != ATTN_B200_DTYPE_BF16) return ATTN_B200_E_INVALID_ARG;
   if (a->dtype_out != ATTN_B200_DTYPE_SAME && a->dtype_out != ATTN_B200_DTYPE_FP32) return ATTN_B200_E_INVALID_ARG;
-  if (a->dim_v <= 0 || a->dim_v % b200::kLinDvs != 0) return ATTN_B200_E_UNSUPPORTED;
+  if (a->dim_v <= 0 || a->dim_v % (a->any_dim_v ? 8 : b200::kLinDvs) != 0) return ATTN_B200_E_UNSUPPORTED;
+  // an fp32 output leaves the kernel as whole 128-column rows: a bound on the columns there cost every other call 1.5 %
+  if ((a->normalize || a->dtype_out == ATTN_B200_DTYPE_FP32) && a->dim_v % b200::kLinDvs != 0) return ATTN_B200_E_UNSUPPORTED;
   if (a->heads_q < 0 || a->heads_k < 0 || (a->heads_q > 0 && a->heads % a->heads_q != 0) || (a->heads_k > 0 && a->heads % a->heads_k != 0))
     return ATTN_B200_E_INVALID_ARG;
   if (a->segments < 0 || a->segments > b200::kLinMaxSegments) return ATTN_B200_E_INVALID_ARG;

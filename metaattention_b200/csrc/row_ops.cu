@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(256) rows_sum_cast_kernel(const float* __restr
 
 // Gradient of the log-decays (see the header).  A warp per row reads the fp32 results and the operands once, rounds the
 // gradients and leaves the row's term; torch took six passes over [rows, cols] fp32 for the same (93 us of 2 x 8 x 2000 x
-// 128, now 8).  Bound by HBM.
+// 128, now 16 with the scan below).  Bound by HBM.
 template <bool kBf16>
 __global__ void __launch_bounds__(256) decay_grad_rows_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
                                                              const float* __restrict__ dq_a, const float* __restrict__ dq_b,

@@ -33,7 +33,7 @@ def test_struct_layouts_match_header(tmp_path):
     import subprocess
     probes = {
         "AttnB200ParallelArgs": (lib.ParallelArgs, ["o", "seq_kv", "o_stride", "heads_kv", "fparams", "custom_stride", "mask_left", "mask_right", "num_splits", "workspace", "workspace_bytes"]),
-        "AttnB200LinearArgs": (lib.LinearArgs, ["log_decay", "dim_v", "normalize", "q_scale", "workspace", "workspace_bytes", "precise", "v_scale", "heads_k", "q_ld", "k_ld", "segments", "reverse"]),
+        "AttnB200LinearArgs": (lib.LinearArgs, ["log_decay", "dim_v", "normalize", "q_scale", "workspace", "workspace_bytes", "precise", "v_scale", "heads_k", "q_ld", "k_ld", "segments", "reverse", "any_dim_v"]),
         "AttnB200DecodeArgs": (lib.DecodeArgs, ["lse", "dim", "scale", "q_stride", "block_mask", "block_size", "workspace_bytes"]),
         "AttnB200MlaShape": (lib.MlaShape, ["dim_v"]),
         "AttnB200SoftmaxBwdArgs": (lib.SoftmaxBwdArgs, ["lse", "dv", "dim_v", "scale", "q_stride", "dv_stride", "workspace_bytes",

@@ -272,3 +272,37 @@ def test_chains_cut_between_ctas(Dk, S, dtype, strong, precise):
     assert lib.last_device_status() == 0
     with pytest.raises(lib.NativeError):
         linear_attention_forward(*args, segments=17)
+
+
+@pytest.mark.parametrize("B,H,Hq,S,Dk,Dv,dtype", [
+    (1, 6, 1, 700, 128, 64, torch.bfloat16),    # two heads of 64 columns to a CTA, ragged
+    (2, 4, 2, 300, 64, 64, torch.float16),      # pairs inside the groups of two q / k heads
+    (1, 2, 1, 100, 64, 64, torch.bfloat16),     # one block
+    (1, 3, 1, 400, 128, 64, torch.bfloat16),    # an odd number of heads: half of a slice's columns missing
+    (1, 2, 1, 400, 256, 64, torch.float16),
+    (1, 2, 2, 260, 64, 192, torch.bfloat16),    # a slice and a half
+    (1, 2, 1, 260, 128, 40, torch.float16),     # columns that end inside a 64-column chunk
+])
+def test_dim_v_that_is_not_a_whole_slice(B, H, Hq, S, Dk, Dv, dtype):
+    """dim_v other than multiples of 128, against the oracle: heads with mild and with strong decay side by side (the two
+    heads of a CTA in either form, and one in each), with and without a factor on v, 16-bit and fp32 results, cut and
+    uncut."""
+    g = torch.Generator().manual_seed(S + Dv)
+    q = torch.randn(B, Hq, S, Dk, generator=g).to(dtype)
+    k = (torch.randn(B, Hq, S, Dk, generator=g) * Dk ** -0.5).to(dtype)
+    v = torch.randn(B, H, S, Dv, generator=g).to(dtype)
+    vs = torch.rand(B, H, S, generator=g) + 0.5
+    qe, ke = (t.repeat_interleave(H // Hq, dim=1) for t in (q, k))
+    for rates in ([0.02], [1.5], [0.02, 1.5]):
+        ld = -torch.rand(B, H, S, generator=g) * torch.tensor([rates[h % len(rates)] for h in range(H)]).view(1, H, 1)
+        for scale in (None, vs):
+            want = rm.decayed_linear_attention(qe, ke, v.float() if scale is None else v.float() * scale[..., None], ld, scale=0.7)
+            args, kw = (q.cuda(), k.cuda(), v.cuda(), ld.cuda()), dict(q_scale=0.7, v_scale=None if scale is None else scale.cuda())
+            o = linear_attention_forward(*args, segments=1, **kw)
+            assert o.shape == (B, H, S, Dv) and o.is_contiguous()
+            check_raw(o, want)
+            for segments in (0, 3):
+                assert torch.equal(o, linear_attention_forward(*args, segments=segments, **kw))
+            o32 = linear_attention_forward(*args, out_dtype=torch.float32, **kw)
+            assert ((o32.cpu() - want).norm() / want.norm()).item() < 1e-2
+    assert lib.last_device_status() == 0
