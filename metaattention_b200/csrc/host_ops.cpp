@@ -423,6 +423,7 @@ struct Attention : torch::autograd::Function<Attention> {
     torch::autograd::variable_list out{done.o};
     for (const Tensor& t : done.finals) out.push_back(t);
     ctx->mark_non_differentiable(done.finals);
+    ctx->set_materialize_grads(false);   // nobody reads the zeros that would be made for them
     return out;
   }
 
