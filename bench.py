@@ -573,7 +573,7 @@ def extras_retention(sampler, peaks, launches):
         eng = programs.mamba2_engine(B, HQ, S, D, Dv, HK=HK, HV=HV)
         dtb = dt.to(torch.bfloat16)
         ms = statistics.median(time_launches(lambda: eng(q, k, v, dt, A, dtb), 20, 3))
-        out["mamba2_1x80x2048_128_64"] = {"ms": ms, "note": "v_mod = v * dt and the shared q / k heads are handled inside the kernel; includes the whole-tensor decay_mod statement and the padding of dim_v 64 to 128"}
+        out["mamba2_1x80x2048_128_64"] = {"ms": ms, "note": "v_mod = v * dt and the shared q / k heads are handled inside the kernel; two 64-column heads share a 128-column slice; includes the whole-tensor decay_mod statement"}
     except Exception as exc:
         out["retention_error"] = repr(exc)[:300]
     torch.cuda.empty_cache()
