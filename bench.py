@@ -438,8 +438,8 @@ def extras_backward(peaks, launches=10):
         out["softmax_backward_document_mask_1024"] = {"ms": ms, "kept_tiles": doc._sparse_host["kept_tiles"],
                                                       "all_tiles": doc._sparse_host["all_tiles"]}
         del q, k, v, o, d_o, o_doc
-        # RetNet retention backward on the benchmark shape: five runs of the forward kernel plus the time reversals
-        # and fp32 sums around them (torch), timed as one call
+        # RetNet retention backward on the benchmark shape: five runs of the forward kernel (dk, dv on its reversed walk)
+        # and fp32 sums around them, timed as one call
         from attn_engine.linear_attn_engine import linear_attention_backward
         qr, kr, vr, decay = [t.cuda() for t in oracle_inputs.retention_bhsd(C4["B"], C4["H"], C4["S"], C4["D"], C4["Dv"], C4["seed"])]
         ld = decay.log()
