@@ -382,6 +382,9 @@ class AttentionEngine:
             raise TypeError(f"expected {len(self.custom_names)} custom input tensor(s) {self.custom_names}, got {len(custom)}")
         if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
             raise ValueError("q, k, v must be [batch, seq, heads, dim]")
+        fault = native.host().fault(q, k, v)
+        if fault is not None:
+            raise ValueError(f"{fault}: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
         if k.device != q.device or v.device != q.device:
             raise ValueError(f"q, k, v must be on one device (got {q.device}, {k.device}, {v.device})")
         if not q.is_cuda:

@@ -154,20 +154,29 @@ struct Forward {
   std::vector<Tensor> finals;   // empty when split results were merged without them
 };
 
-int kv_splits_for(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int device) {
+int splits_on(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int64_t sms) {
   // 1 unless the (query tile pair, head, batch) grid fills less than half of the SMs; then as many as fit, each keeping at
   // least four 128-row KV tiles (a split re-reads Q and adds a combine pass)
-  const int64_t ctas = B * H * ((Sq + 255) / 256), sms = at::cuda::getDeviceProperties(device)->multiProcessorCount;
+  const int64_t ctas = B * H * ((Sq + 255) / 256);
   const int64_t tiles = (Skv + 127) / 128;
-  if (2 * ctas > sms || tiles < 8) return 1;
+  if (ctas <= 0 || 2 * ctas > sms || tiles < 8) return 1;   // nothing to compute: nothing to split
   return static_cast<int>(std::max<int64_t>(1, std::min({sms / ctas, tiles / 4, int64_t{65535} / std::max<int64_t>(B, 1)})));
+}
+int kv_splits_for(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int device) {
+  return splits_on(B, H, Sq, Skv, at::cuda::getDeviceProperties(device)->multiProcessorCount);
+}
+
+// What is wrong with the extents of a call's 4-dimensional operands, or null.
+const char* fault(const Tensor& q, const Tensor& k, const Tensor& v) {
+  if (q.numel() == 0 || k.numel() == 0 || v.numel() == 0) return "q, k and v must not be empty";
+  return nullptr;
 }
 
 // The forward of one call; `done` false = declined.  With the GIL when the plan has a mask walk that a device has not seen.
 Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
                 OptTensor block_mask, OptTensor lens) {
   Forward r;
-  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(q, k, v) != nullptr || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
   const int dt = dtype_code(q);
   if (dt < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return r;
   if (q.stride(3) != 1 || k.stride(3) != 1 || v.stride(3) != 1) return r;
@@ -522,4 +531,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("make_plan", &make_plan);
   m.def("run", &run);
   m.def("kv_splits", &kv_splits_for);
+  m.def("splits_on", &splits_on);
+  m.def("fault", &fault);
 }
