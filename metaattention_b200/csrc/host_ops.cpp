@@ -166,9 +166,14 @@ int kv_splits_for(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int device) {
   return splits_on(B, H, Sq, Skv, at::cuda::getDeviceProperties(device)->multiProcessorCount);
 }
 
-// What is wrong with the extents of a call's 4-dimensional operands, or null.
+// What is wrong with the extents of a call's 4-dimensional operands, or null.  The kernels walk k and v with the batch and
+// head dim of q and the length of k: an operand that has less would be read past its end.  One that has more is read in
+// part (caches laid out for more sequences).
 const char* fault(const Tensor& q, const Tensor& k, const Tensor& v) {
   if (q.numel() == 0 || k.numel() == 0 || v.numel() == 0) return "q, k and v must not be empty";
+  if (k.size(0) < q.size(0) || v.size(0) < q.size(0)) return "k and v hold fewer sequences than q";
+  if (k.size(3) < q.size(3)) return "k has a smaller head dim than q";
+  if (v.size(1) < k.size(1)) return "v is shorter than k";
   return nullptr;
 }
 
@@ -441,6 +446,9 @@ struct Attention : torch::autograd::Function<Attention> {
     const auto saved = ctx->get_saved_variables();
     const size_t n_saved = ctx->saved_data["n_saved"].toInt();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
+    // the gradients of what the forward left unread would not be written
+    if (k.size(0) != q.size(0) || v.size(0) != q.size(0) || k.size(3) != q.size(3) || v.size(1) != k.size(1))
+      check(ATTN_B200_E_INVALID_ARG, "backward with k or v larger than the call's batch, length or head dim");
     c10::cuda::CUDAGuard guard(q.device());
     Tensor g = grads[0].defined() ? grads[0] : at::zeros({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
     const Tensor d_o = last_contiguous(g, q);

@@ -31,3 +31,20 @@ def test_split_plan(host):
     assert host.splits_on(1, 32, 1, 32768, 148) == 4      # 32 CTAs of 148 SMs
     assert host.splits_on(1, 1, 1, 2048, 148) == 4        # four tiles to a split
     assert host.splits_on(8, 32, 1, 32768, 148) == 1
+
+
+@pytest.mark.parametrize("q,k,v,what", [
+    ((2, 1, 8, 128), (1, 2048, 2, 128), (2, 2048, 2, 128), "fewer sequences"),
+    ((2, 1, 8, 128), (2, 2048, 2, 128), (1, 2048, 2, 128), "fewer sequences"),
+    ((2, 1, 8, 128), (2, 2048, 2, 64), (2, 2048, 2, 128), "smaller head dim"),
+    ((2, 1, 8, 128), (2, 2048, 2, 128), (2, 2047, 2, 128), "shorter"),
+    ((2, 300, 8, 128), (2, 300, 8, 128), (2, 172, 8, 128), "shorter"),
+])
+def test_operands_that_would_be_read_past_their_end_are_refused(host, q, k, v, what):
+    with pytest.raises(ValueError, match=what):
+        programs.gqa_engine(2, 8, 2, q[1], k[1], 128, 128)(*operands(q, k, v))
+
+
+def test_larger_caches_are_read_in_part(host):
+    """a batch of three out of caches laid out for eight, and rows of v past the last of k"""
+    assert host.fault(*operands((3, 1, 8, 128), (8, 512, 8, 128), (8, 600, 8, 128))) is None
