@@ -220,6 +220,7 @@ class AttentionEngine:
             # the reference's choice for anything that is not causal (core/lower/lower.py:723-738): block sparsity.
             # KV tiles without a kept position are skipped, partially kept ones carry their element mask.
             self._sparse_host = sparse_lowering.build_block_sparse(mask_mod, B, H, S, Skv)
+            self._mask_lengths = (S, Skv)
             self.mask_kind = native.MASK_NONE
         self.sparse_walk = self._sparse_host is not None or self._decode_block is not None
         neg_inf_mask = str(mask_value).strip() in ("-inf", "-float('inf')")
@@ -289,10 +290,12 @@ class AttentionEngine:
             axes = custom_axes(sym)
             literal = [int(d) if ax is None and d.isdigit() else -1 for ax, d in zip(axes, sym.shape_idx)]
             return [-1 if ax is None else ax for ax in axes], literal, dtype == torch.float32, dtype == torch.bfloat16
+        walk = self._sparse_host is not None and self._decode_block is None
         self._plan = native.host().make_plan({
             "builtin": self.functor_kind == "builtin_softmax", "fn": fn, "fparams": self._fparams, "n_final": len(self.final_names),
             "mask_kind": self.mask_kind, "left": self.mask_band[0], "right": self.mask_band[1], "may_decode": self._may_decode,
-            "decode_block": self._decode_block or 0, "has_mask_walk": self._sparse_host is not None and self._decode_block is None,
+            "decode_block": self._decode_block or 0, "has_mask_walk": walk,
+            "mask_extents": (*self._mask_lengths, self._sparse_host["batch"] * self._sparse_host["heads"]) if walk else (0, 0, 1),
             "backward": 1 if self.functor_kind == "builtin_softmax" else 2, "load_mask": load_mask, "load_backward": load_backward,
             "custom": [custom_spec(s, d) for s, d in zip(self._custom_syms, self._custom_dtypes)]})
         return self._plan
@@ -382,9 +385,10 @@ class AttentionEngine:
             raise TypeError(f"expected {len(self.custom_names)} custom input tensor(s) {self.custom_names}, got {len(custom)}")
         if q.dim() != 4 or k.dim() != 4 or v.dim() != 4:
             raise ValueError("q, k, v must be [batch, seq, heads, dim]")
-        fault = native.host().fault(q, k, v)
+        fault = native.host().fault(self._plan, q, k, v)
         if fault is not None:
-            raise ValueError(f"{fault}: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
+            raise ValueError(f"{fault}: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}" +
+                             (f", mask {self._mask_lengths}" if self._sparse_host is not None else ""))
         if k.device != q.device or v.device != q.device:
             raise ValueError(f"q, k, v must be on one device (got {q.device}, {k.device}, {v.device})")
         if not q.is_cuda:

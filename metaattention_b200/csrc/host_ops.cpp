@@ -20,6 +20,7 @@
 #include <cstring>
 #include <map>
 #include <memory>
+#include <tuple>
 
 #include "../../include/attn_b200.h"
 
@@ -106,7 +107,8 @@ struct Plan {
   int mask_kind = 0, left = 0, right = 0;
   bool may_decode = false;     // attn_b200_decode_fwd computes this program
   int decode_block = 0;        // > 0: block_mask / cache_seqlens arrive with the call
-  bool has_mask_walk = false;  // a general mask_mod
+  bool has_mask_walk = false;  // a general mask_mod, evaluated for mask_q x mask_kv positions of mask_bh (batch, head) pairs
+  int64_t mask_q = 0, mask_kv = 0, mask_bh = 1;
   std::vector<Custom> custom;
   int backward = 0;            // 0 none, 1 softmax, 2 elementwise
   py::object load_mask;        // device -> dict of tensors
@@ -169,11 +171,21 @@ int kv_splits_for(int64_t B, int64_t H, int64_t Sq, int64_t Skv, int device) {
 // What is wrong with the extents of a call's 4-dimensional operands, or null.  The kernels walk k and v with the batch and
 // head dim of q and the length of k: an operand that has less would be read past its end.  One that has more is read in
 // part (caches laid out for more sequences).
-const char* fault(const Tensor& q, const Tensor& k, const Tensor& v) {
+const char* fault(const Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v) {
   if (q.numel() == 0 || k.numel() == 0 || v.numel() == 0) return "q, k and v must not be empty";
   if (k.size(0) < q.size(0) || v.size(0) < q.size(0)) return "k and v hold fewer sequences than q";
   if (k.size(3) < q.size(3)) return "k has a smaller head dim than q";
   if (v.size(1) < k.size(1)) return "v is shorter than k";
+  if (plan.has_mask_walk) {
+    // The bitmaps have a row of `words` words per query tile, the rows of the (batch, head) pairs one after the other: a
+    // call may be shorter than what the mask was evaluated for where that leaves the rows in their places.
+    const int64_t Sq = q.size(1), Skv = k.size(1);
+    auto tiles = [](int64_t n) { return (n + 127) / 128; };
+    auto words = [&](int64_t n) { return (tiles(n) + 31) / 32; };
+    if (Sq > plan.mask_q || Skv > plan.mask_kv) return "longer than the lengths that mask_mod was evaluated for";
+    if ((plan.mask_bh > 1 && tiles(Sq) != tiles(plan.mask_q)) || (words(Skv) != words(plan.mask_kv) && (plan.mask_bh > 1 || tiles(Sq) > 1)))
+      return "too much shorter than the lengths that mask_mod was evaluated for";
+  }
   return nullptr;
 }
 
@@ -181,7 +193,7 @@ const char* fault(const Tensor& q, const Tensor& k, const Tensor& v) {
 Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
                 OptTensor block_mask, OptTensor lens) {
   Forward r;
-  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(q, k, v) != nullptr || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(plan, q, k, v) != nullptr || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
   const int dt = dtype_code(q);
   if (dt < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return r;
   if (q.stride(3) != 1 || k.stride(3) != 1 || v.stride(3) != 1) return r;
@@ -335,6 +347,9 @@ void fill_bwd(Args& a, const Tensor& q, const Tensor& k, const Tensor& v, const 
   a.mask_left = m.left;
   a.mask_right = m.right;
   if (m.bits_q.defined()) {
+    const int64_t nq = (q.size(1) + 127) / 128, nk = (k.size(1) + 127) / 128;
+    if (m.bits_q.size(0) != nq * 128 || m.bits_q.size(1) != nk || m.bits_kv.size(0) != nk * 128 || m.bits_kv.size(1) != nq)
+      check(ATTN_B200_E_INVALID_ARG, "backward at other lengths than mask_mod was evaluated for");
     a.mask_kind = ATTN_B200_MASK_BITS;
     a.mask_bits_q = m.bits_q.data_ptr();
     a.mask_bits_kv = m.bits_kv.data_ptr();
@@ -519,6 +534,7 @@ std::shared_ptr<Plan> make_plan(const py::dict& d) {
   p->may_decode = py::cast<bool>(d["may_decode"]);
   p->decode_block = py::cast<int>(d["decode_block"]);
   p->has_mask_walk = py::cast<bool>(d["has_mask_walk"]);
+  std::tie(p->mask_q, p->mask_kv, p->mask_bh) = py::cast<std::tuple<int64_t, int64_t, int64_t>>(d["mask_extents"]);
   p->backward = py::cast<int>(d["backward"]);
   p->load_mask = d["load_mask"];
   p->load_backward = d["load_backward"];

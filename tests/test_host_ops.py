@@ -47,4 +47,60 @@ def test_operands_that_would_be_read_past_their_end_are_refused(host, q, k, v, w
 
 def test_larger_caches_are_read_in_part(host):
     """a batch of three out of caches laid out for eight, and rows of v past the last of k"""
-    assert host.fault(*operands((3, 1, 8, 128), (8, 512, 8, 128), (8, 600, 8, 128))) is None
+    eng = programs.gqa_engine(3, 8, 8, 1, 512, 128, 128)
+    assert host.fault(eng._make_plan(), *operands((3, 1, 8, 128), (8, 512, 8, 128), (8, 600, 8, 128))) is None
+
+
+def document(b, h, q_idx, kv_idx):
+    return (q_idx // 200 == kv_idx // 200) & (q_idx >= kv_idx)
+
+
+def document_of_head(b, h, q_idx, kv_idx):
+    return (q_idx // (200 + h) == kv_idx // (200 + h)) & (q_idx >= kv_idx)
+
+
+@pytest.mark.parametrize("mask,built,call,refused", [
+    (document, 500, 500, None),
+    (document, 500, 505, "longer"),              # the same tiles, but rows the mask was not evaluated for
+    (document, 500, 700, "longer"),              # bitmaps and element masks would be read past their end
+    (document, 500, 400, None),                  # the same tiles
+    (document, 500, 130, None),                  # fewer tiles of the same rows
+    (document, 4200, 4200, None),
+    (document, 4200, 4000, "too much shorter"),  # rows of one word instead of two
+    (document, 4200, 100, None),                 # one row
+    (document_of_head, 500, 390, None),
+    (document_of_head, 500, 380, "too much shorter"),   # rows of the second head further in front
+    (document_of_head, 4200, 100, "too much shorter"),
+])
+def test_lengths_that_a_mask_was_not_evaluated_for(host, mask, built, call, refused):
+    eng = programs.masked_softmax_engine(1, 2, built, 64, 64, mask)
+    q, k, v = operands(*[(1, call, 2, 64)] * 3)
+    got = host.fault(eng._make_plan(), q, k, v)
+    assert got is None if refused is None else refused in got
+    with pytest.raises(lib.NativeError if refused is None else ValueError, match=refused or "CUDA"):
+        eng(q, k, v)
+
+
+def test_reading_of_a_mask_at_the_lengths_of_a_call(host):
+    """The lengths that are accepted are those at which the bitmaps, read as the kernel does with the rows and words of the
+    call, are the ones that the mask gives when it is evaluated for the call."""
+    from core.lower import sparse
+    for mask in (document, document_of_head):
+        for built in (300, 4200):
+            eng = programs.masked_softmax_engine(1, 2, built, 64, 64, mask)
+            plan, was = eng._make_plan(), eng._sparse_host
+            for sq in {100, 128, 129, 256, 300, 4100} & set(range(built + 1)):
+                for skv in {100, 128, 300, 4096, 4097} & set(range(built + 1)):
+                    q, k = torch.zeros(1, sq, 2, 64), torch.zeros(1, skv, 2, 64)
+                    now = sparse.build_block_sparse(mask, 1, 2, sq, skv)
+                    rows, words = now["keep"].shape[1] * now["keep"].shape[2], now["keep"].shape[3]
+                    flat = was["keep"].flatten()
+                    same = rows * words <= flat.numel() and now["heads"] == was["heads"]
+                    if same:   # tiles past the call's last are loaded as zeros and masked
+                        live = torch.tensor([(1 << min(32, max(0, -(-skv // 128) - 32 * w))) - 1 for w in range(words)])
+                        read = flat[:rows * words].view(rows, words).long() & live
+                        want = now["keep"].view(rows, words).long() & live
+                        base = was["mask_base"].flatten()[:rows]
+                        same = torch.equal(read, want) and torch.equal(base, was["mask_base"].reshape(
+                            was["mask_base"].shape[1], -1)[:, :now["keep"].shape[2]].reshape(-1)[:rows])
+                    assert (host.fault(plan, q, k, k) is None) == same, (mask.__name__, built, sq, skv)
