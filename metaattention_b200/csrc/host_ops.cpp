@@ -114,9 +114,9 @@ struct Plan {
   py::object load_mask;        // device -> dict of tensors
   py::object load_backward;    // () -> address of attn_b200_elementwise_bwd_jit
   uintptr_t bwd_fn = 0;
-  std::map<int, Sparse> masks;
+  std::map<int, std::shared_ptr<const Sparse>> masks;
 
-  const Sparse& mask_on(const Tensor& like) {   // with the GIL
+  std::shared_ptr<const Sparse> mask_on(const Tensor& like) {   // with the GIL
     const int dev = like.device().index();
     auto it = masks.find(dev);
     if (it != masks.end()) return it->second;
@@ -130,7 +130,7 @@ struct Plan {
     s.batch = py::cast<int>(d["batch"]);
     s.heads = py::cast<int>(d["heads"]);
     s.rows = py::cast<int>(d["mask_rows"]);
-    return masks.emplace(dev, std::move(s)).first->second;
+    return masks.emplace(dev, std::make_shared<const Sparse>(std::move(s))).first->second;
   }
 };
 
@@ -152,6 +152,7 @@ bool decode_operands(OptTensor& block_mask, OptTensor& lens, int64_t B, int64_t 
 
 struct Forward {
   bool done = false;
+  std::shared_ptr<const Sparse> mask;   // the general mask it ran under, kept for the backward
   Tensor o;
   std::vector<Tensor> finals;   // empty when split results were merged without them
 };
@@ -267,7 +268,8 @@ Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, c
     a.sparse_batch = B;
     a.sparse_heads = Hkv;
   } else if (plan.has_mask_walk) {
-    const Sparse& s = plan.mask_on(q);
+    r.mask = plan.mask_on(q);
+    const Sparse& s = *r.mask;
     a.tile_keep = static_cast<const uint32_t*>(s.keep.data_ptr());
     a.tile_partial = static_cast<const uint32_t*>(s.partial.data_ptr());
     a.tile_mask_base = s.mask_base.defined() ? s.mask_base.data_ptr<int32_t>() : nullptr;
@@ -419,12 +421,12 @@ Tensor last_contiguous(Tensor t, const Tensor& like) {
   return t.stride(3) == 1 ? t : t.contiguous();
 }
 
+// What a backward needs beside the saved tensors.  The mask's tensors belong to the plan: they are no variables of the
+// graph (saved ones would go through the user's saved-tensor hooks, and may not have been made in inference mode).
 struct PlanRef : torch::CustomClassHolder {
   std::shared_ptr<Plan> plan;
+  std::shared_ptr<const Sparse> mask;
 };
-std::shared_ptr<Plan> plan_of(torch::autograd::AutogradContext* ctx) {
-  return c10::static_intrusive_pointer_cast<PlanRef>(ctx->saved_data["plan"].toCapsule())->plan;
-}
 
 // The forward with its backward (attn_b200_softmax_bwd, attn_b200_elementwise_bwd_jit): the counterpart of the reference's
 // `_attention` autograd function (core/template/tl_template/attn/attn_tl.py:654-694).  Outputs: o, then the final row
@@ -434,6 +436,7 @@ struct Attention : torch::autograd::Function<Attention> {
                                                 const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom) {
     auto ref = c10::make_intrusive<PlanRef>();
     ref->plan = plan;
+    ref->mask = done.mask;
     ctx->saved_data["plan"] = c10::IValue::make_capsule(ref);
     torch::autograd::variable_list saved{q, k, v};
     if (plan->backward == 1) {
@@ -442,12 +445,6 @@ struct Attention : torch::autograd::Function<Attention> {
     } else {
       for (const Tensor& t : custom) saved.push_back(t);
     }
-    const size_t n_saved = saved.size();
-    if (plan->has_mask_walk) {
-      const Sparse& s = plan->masks.at(q.device().index());
-      for (const Tensor& t : {s.bits_q, s.bits_kv, s.tiles_q, s.tiles_kv}) saved.push_back(t);
-    }
-    ctx->saved_data["n_saved"] = static_cast<int64_t>(n_saved);
     ctx->save_for_backward(saved);
     torch::autograd::variable_list out{done.o};
     for (const Tensor& t : done.finals) out.push_back(t);
@@ -457,9 +454,9 @@ struct Attention : torch::autograd::Function<Attention> {
   }
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
-    auto plan = plan_of(ctx);
+    const auto ref = c10::static_intrusive_pointer_cast<PlanRef>(ctx->saved_data["plan"].toCapsule());
+    const std::shared_ptr<Plan>& plan = ref->plan;
     const auto saved = ctx->get_saved_variables();
-    const size_t n_saved = ctx->saved_data["n_saved"].toInt();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
     // the gradients of what the forward left unread would not be written
     if (k.size(0) != q.size(0) || v.size(0) != q.size(0) || k.size(3) != q.size(3) || v.size(1) != k.size(1))
@@ -468,8 +465,8 @@ struct Attention : torch::autograd::Function<Attention> {
     Tensor g = grads[0].defined() ? grads[0] : at::zeros({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
     const Tensor d_o = last_contiguous(g, q);
     Mask m{plan->mask_kind, plan->left, plan->right, {}, {}, {}, {}};
-    if (saved.size() > n_saved) {
-      m.bits_q = saved[n_saved]; m.bits_kv = saved[n_saved + 1]; m.tiles_q = saved[n_saved + 2]; m.tiles_kv = saved[n_saved + 3];
+    if (ref->mask != nullptr) {
+      m.bits_q = ref->mask->bits_q; m.bits_kv = ref->mask->bits_kv; m.tiles_q = ref->mask->tiles_q; m.tiles_kv = ref->mask->tiles_kv;
     }
     auto cols = [](const Tensor& t, int64_t c, int64_t w) { return t.size(3) == w ? t : t.narrow(3, c, w); };
     std::vector<Tensor> d;
@@ -490,7 +487,7 @@ struct Attention : torch::autograd::Function<Attention> {
           throw err;
         }
       }
-      const std::vector<Tensor> custom(saved.begin() + 3, saved.begin() + n_saved);
+      const std::vector<Tensor> custom(saved.begin() + 3, saved.end());
       d = over_dim_v(q, v, [&](int64_t c, int64_t w) {
         return elementwise_bwd_one(plan->bwd_fn, q, k, cols(v, c, w), cols(d_o, c, w), custom, m);
       });

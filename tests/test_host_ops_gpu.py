@@ -1,0 +1,44 @@
+"""The native host side of a call (csrc/host_ops.cpp) on the GPU: what surrounds the launches."""
+
+import pytest
+import torch
+
+from core.native import lib
+from examples_b200 import programs
+
+pytestmark = pytest.mark.gpu
+
+
+def document(b, h, q_idx, kv_idx):
+    return (q_idx // 200 == kv_idx // 200) & (q_idx >= kv_idx)
+
+
+def rand(*shape):
+    return torch.randn(*shape, generator=torch.Generator(device="cuda").manual_seed(len(shape) + shape[1]), device="cuda").to(torch.bfloat16)
+
+
+def test_training_after_a_first_call_in_inference_mode():
+    """the mask's device copies are made by the first call: here as inference tensors, which autograd does not save"""
+    grads = []
+    for first in (False, True):
+        eng = programs.masked_softmax_engine(1, 2, 512, 64, 64, document)
+        q, k, v = (rand(1, 512, 2, 64).mul_(s) for s in (1.0, 0.5, 2.0))
+        if first:
+            with torch.inference_mode():
+                eng(q, k, v)
+        for t in (q, k, v):
+            t.requires_grad_()
+        grads.append(torch.autograd.grad(eng(q, k, v), (q, k, v), rand(1, 512, 2, 64)))
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
+    assert lib.last_device_status() == 0
+
+
+def test_saved_tensor_hooks_see_the_call_s_tensors_only():
+    eng = programs.masked_softmax_engine(1, 2, 512, 64, 64, document)
+    q, k, v = (rand(1, 512, 2, 64).requires_grad_() for _ in range(3))
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.dtype) or t, lambda t: t):
+        o = eng(q, k, v)
+    assert sorted(map(str, seen)) == ["torch.bfloat16"] * 4 + ["torch.float32"]     # q, k, v, o and lse
+    o.sum().backward()
+    assert q.grad is not None and lib.last_device_status() == 0
