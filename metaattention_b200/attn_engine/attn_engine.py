@@ -273,18 +273,20 @@ class AttentionEngine:
 
     def _make_plan(self):
         """What was decided at construction, for the native side: constants, the address of the functor library's entry
-        point, and callbacks for what is made when a device or a gradient is first met."""
+        point, and callbacks for what is made when a device or a gradient is first met.  The callbacks do not refer to the
+        engine: the garbage collector does not see what a plan holds, and the engine holds the plan."""
         fn = 0
         if self.functor_kind == "lowered":
             fn = C.cast(native_jit.load(self.functor_source), C.c_void_p).value
+        sparse_host, sparse_dev, bwd_source = self._sparse_host, self._sparse_dev, self._bwd_source
 
         def load_mask(device):
-            if device not in self._sparse_dev:
-                self._sparse_dev[device] = sparse_lowering.to_device(self._sparse_host, device)
-            return self._sparse_dev[device]
+            if device not in sparse_dev:
+                sparse_dev[device] = sparse_lowering.to_device(sparse_host, device)
+            return sparse_dev[device]
 
         def load_backward():
-            return C.cast(native_jit.load_backward(self._bwd_source), C.c_void_p).value
+            return C.cast(native_jit.load_backward(bwd_source), C.c_void_p).value
 
         def custom_spec(sym, dtype):
             axes = custom_axes(sym)

@@ -9,6 +9,7 @@
 // A call whose operands are not what a kernel takes is declined (`None` / false): the Python side then raises the error
 // that names what is wrong.  Entry points of libattn_b200.so and of functor libraries come in as addresses, from the
 // libraries that Python has loaded.
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -96,6 +97,15 @@ struct Custom {
 struct Sparse {
   Tensor keep, partial, mask_base, elem_mask, bits_q, bits_kv, tiles_q, tiles_kv;
   int batch = 1, heads = 1, rows = 128;
+
+  // Around a launch on the current stream: the tensors go when the engine does, perhaps with that launch still to run.
+  static void used(const Tensor& q, std::initializer_list<const Tensor*> by_it) {
+    const auto now = c10::cuda::getCurrentCUDAStream(q.device().index());
+    for (const Tensor* t : by_it)
+      if (t->defined()) c10::cuda::CUDACachingAllocator::recordStream(t->storage().data_ptr(), now);
+  }
+  void used_by_forward(const Tensor& q) const { used(q, {&keep, &partial, &mask_base, &elem_mask}); }
+  void used_by_backward(const Tensor& q) const { used(q, {&bits_q, &bits_kv, &tiles_q, &tiles_kv}); }
 };
 
 // What an engine of the parallel pattern decided at construction.
@@ -270,6 +280,7 @@ Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, c
   } else if (plan.has_mask_walk) {
     r.mask = plan.mask_on(q);
     const Sparse& s = *r.mask;
+    s.used_by_forward(q);
     a.tile_keep = static_cast<const uint32_t*>(s.keep.data_ptr());
     a.tile_partial = static_cast<const uint32_t*>(s.partial.data_ptr());
     a.tile_mask_base = s.mask_base.defined() ? s.mask_base.data_ptr<int32_t>() : nullptr;
@@ -466,6 +477,7 @@ struct Attention : torch::autograd::Function<Attention> {
     const Tensor d_o = last_contiguous(g, q);
     Mask m{plan->mask_kind, plan->left, plan->right, {}, {}, {}, {}};
     if (ref->mask != nullptr) {
+      ref->mask->used_by_backward(q);
       m.bits_q = ref->mask->bits_q; m.bits_kv = ref->mask->bits_kv; m.tiles_q = ref->mask->tiles_q; m.tiles_kv = ref->mask->tiles_kv;
     }
     auto cols = [](const Tensor& t, int64_t c, int64_t w) { return t.size(3) == w ? t : t.narrow(3, c, w); };

@@ -1,6 +1,9 @@
 """The native host side of a call (csrc/host_ops.cpp) without a GPU: the calls it refuses before anything is launched, and
 the life of the plans that engines give it."""
 
+import gc
+import weakref
+
 import pytest
 import torch
 
@@ -104,3 +107,17 @@ def test_reading_of_a_mask_at_the_lengths_of_a_call(host):
                         same = torch.equal(read, want) and torch.equal(base, was["mask_base"].reshape(
                             was["mask_base"].shape[1], -1)[:, :now["keep"].shape[2]].reshape(-1)[:rows])
                     assert (host.fault(plan, q, k, k) is None) == same, (mask.__name__, built, sq, skv)
+
+
+@pytest.mark.parametrize("make", [
+    lambda: programs.gqa_engine(1, 8, 2, 256, 256, 128, 128, is_causal=True),
+    lambda: programs.masked_softmax_engine(1, 2, 500, 64, 64, document),
+])
+def test_an_engine_goes_when_its_last_user_does(host, make):
+    """with its plan, and so with the device copies of its mask"""
+    eng = make()
+    plan = eng._make_plan()
+    left = weakref.ref(eng)
+    del eng
+    gc.collect()
+    assert left() is None and plan is not None

@@ -1,5 +1,7 @@
 """The native host side of a call (csrc/host_ops.cpp) on the GPU: what surrounds the launches."""
 
+import gc
+
 import pytest
 import torch
 
@@ -42,3 +44,26 @@ def test_saved_tensor_hooks_see_the_call_s_tensors_only():
     assert sorted(map(str, seen)) == ["torch.bfloat16"] * 4 + ["torch.float32"]     # q, k, v, o and lse
     o.sum().backward()
     assert q.grad is not None and lib.last_device_status() == 0
+
+
+def test_masks_of_engines_that_are_gone_give_their_memory_back():
+    """each engine's mask takes 4 MB of bits twice; used on another stream as well as on the one it was made on"""
+    q, k, v = (rand(1, 6000, 2, 64) for _ in range(3))
+    other = torch.cuda.Stream()
+    want, held = None, []
+    for _ in range(3):
+        eng = programs.masked_softmax_engine(1, 2, 6000, 64, 64, document)
+        o = eng(q, k, v)
+        other.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(other):
+            o2 = eng(q, k, v)
+        del eng
+        gc.collect()
+        torch.cuda.synchronize()
+        assert torch.equal(o, o2) and (want is None or torch.equal(o, want))
+        want = o
+        del o, o2
+        torch.cuda.empty_cache()
+        held.append(torch.cuda.memory_allocated())
+    assert held[2] - held[0] < 1 << 20
+    assert lib.last_device_status() == 0
