@@ -302,6 +302,10 @@ class AttentionEngine:
             "custom": [custom_spec(s, d) for s, d in zip(self._custom_syms, self._custom_dtypes)]})
         return self._plan
 
+    def __getstate__(self):
+        """Copies and pickles come without the native plan: they make their own at their first call."""
+        return {**self.__dict__, "_plan": None}
+
     def _masked_for_backward(self) -> bool:
         """Masks the backward kernels take: none, causal, bands, and any other mask_mod that does not use the batch or
         head index (as keep bits)."""

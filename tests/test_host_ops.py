@@ -1,7 +1,9 @@
 """The native host side of a call (csrc/host_ops.cpp) without a GPU: the calls it refuses before anything is launched, and
 the life of the plans that engines give it."""
 
+import copy
 import gc
+import pickle
 import weakref
 
 import pytest
@@ -121,3 +123,12 @@ def test_an_engine_goes_when_its_last_user_does(host, make):
     del eng
     gc.collect()
     assert left() is None and plan is not None
+
+
+@pytest.mark.parametrize("duplicate", [copy.copy, copy.deepcopy, lambda eng: pickle.loads(pickle.dumps(eng))])
+def test_engines_that_have_been_called_are_copied_and_pickled(host, duplicate):
+    eng = programs.masked_softmax_engine(1, 2, 500, 64, 64, document)
+    plan = eng._make_plan()
+    twin = duplicate(eng)
+    assert twin._plan is None and eng._plan is plan
+    assert host.fault(twin._make_plan(), *operands(*[(1, 700, 2, 64)] * 3)) is not None
