@@ -212,6 +212,10 @@ Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, c
   if (Hkv <= 0 || v.size(2) != Hkv || H % Hkv != 0 || custom.size() != plan.custom.size()) return r;
   c10::cuda::CUDAGuard guard(q.device());
   void* stream = stream_of(q);
+  if (plan.decode_block == 0) {   // nothing is made of them: they are not in a form a kernel takes
+    block_mask.reset();
+    lens.reset();
+  }
 
   if (plan.may_decode && forced_splits < 0 && Sq * H <= 128 * Hkv && Skv > 128 && D == Dv) {
     // the query rows of the heads that share a KV head fit one tile: the decode kernel, if it covers the call

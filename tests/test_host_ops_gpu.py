@@ -67,3 +67,12 @@ def test_masks_of_engines_that_are_gone_give_their_memory_back():
         held.append(torch.cuda.memory_allocated())
     assert held[2] - held[0] < 1 << 20
     assert lib.last_device_status() == 0
+
+
+def test_decode_arguments_of_an_engine_without_them_are_left_alone():
+    eng = programs.gqa_engine(2, 8, 2, 1, 1024, 128, 128)
+    q, k, v = rand(2, 1, 8, 128), rand(2, 1024, 2, 128), rand(2, 1024, 2, 128)
+    want = eng(q, k, v)
+    mask = torch.zeros(2, 2, 8, dtype=torch.bool, device="cuda")
+    assert torch.equal(eng.attention(q, k, v, block_mask=mask, cache_seqlens=torch.tensor([3, 5])), want)
+    assert lib.last_device_status() == 0
