@@ -276,12 +276,6 @@ def current_stream_ptr() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-def device_status_word(device: int) -> int:
-    out = C.c_void_p()
-    check(load_library().attn_b200_device_status_word(device, C.byref(out)), "attn_b200_device_status_word")
-    return out.value
-
-
 def last_device_status(device: int | None = None) -> int:
     """Synchronise and return (then clear) the device status word: 0, or
     100 + id of the device-side wait that gave up."""
@@ -432,25 +426,6 @@ def rows_sum_cast(a, b, dtype, reverse: bool = False):
     return dst
 
 
-def _over_dim_v_slices(run, q, k, v, d_o, o=None):
-    """dim_v a multiple of dim_qk (the 128 / 256 of the reference's suite, testing/test.py:55): the backward is linear in
-    dP = dO V^T and in delta = rowsum(dO o O), both sums over the columns of v, and dV's columns are independent, so it
-    is one kernel run per dim_qk-wide column slice of (v, o, dO) — each recomputing P — with dQ and dK added up in fp32."""
-    D, Dv = q.shape[-1], v.shape[-1]
-    if Dv == D:
-        return run(q, k, v, d_o, o)
-    if Dv % D != 0:
-        raise NativeError(f"the backward covers dim_v = a multiple of dim_qk (got {D} / {Dv})")
-    dq = dk = None
-    dvs = []
-    for c in range(0, Dv, D):
-        part = run(q, k, v[..., c:c + D], d_o[..., c:c + D], None if o is None else o[..., c:c + D])
-        dq = part[0].float() if dq is None else dq + part[0].float()
-        dk = part[1].float() if dk is None else dk + part[1].float()
-        dvs.append(part[2])
-    return dq.to(q.dtype), dk.to(k.dtype), torch.cat(dvs, dim=-1)
-
-
 def softmax_bwd(q, k, v, o, lse, d_o, scale: float, mask_kind: int, mask_band=(MASK_OPEN, MASK_OPEN), mask_bits=None):
     """(dq, dk, dv) of softmax attention from the forward's o and lse [B, H, Sq] and the gradient of o
     (attn_b200_softmax_bwd: mask NONE, CAUSAL or BAND with ``mask_band`` = (left, right); head dims 128 / 128 and
@@ -460,57 +435,20 @@ def softmax_bwd(q, k, v, o, lse, d_o, scale: float, mask_kind: int, mask_band=(M
     for t in (q, k, v, o, d_o, lse):
         if not t.is_cuda:
             raise NativeError("the backward kernel needs CUDA tensors: there is no CPU path")
-    if d_o.stride(-1) != 1:
-        d_o = d_o.contiguous()
-    return _over_dim_v_slices(lambda q_, k_, v_, do_, o_: _softmax_bwd_one(q_, k_, v_, o_, lse, do_, scale, mask_kind, mask_band, mask_bits),
-                              q, k, v, d_o, o)
-
-
-def _set_mask_bits(a, mask_bits, q, k):
-    """Fills mask_kind / mask_bits_* of a backward argument struct from (bits_q, bits_kv) after checking their shapes."""
-    bq, bk = mask_bits[:2]
-    nq, nk = -(-q.shape[1] // 128), -(-k.shape[1] // 128)
-    want = [(bq, (nq * 128, nk, 4)), (bk, (nk * 128, nq, 4))]
-    if len(mask_bits) == 4:   # + bitmaps of the tiles that keep anything
-        want += [(mask_bits[2], (nq, -(-nk // 32))), (mask_bits[3], (nk, -(-nq // 32)))]
-    for t, shape in want:
-        if not (t.is_cuda and t.dtype == torch.int32 and t.is_contiguous() and tuple(t.shape) == shape):
-            raise NativeError(f"mask bits: expected a contiguous CUDA int32 tensor of shape {shape}, got {tuple(t.shape)}")
-    a.mask_kind, a.mask_bits_q, a.mask_bits_kv = MASK_BITS, bq.data_ptr(), bk.data_ptr()
-    if len(mask_bits) == 4:
-        a.mask_tiles_q, a.mask_tiles_kv = mask_bits[2].data_ptr(), mask_bits[3].data_ptr()
-
-
-def _softmax_bwd_one(q, k, v, o, lse, d_o, scale: float, mask_kind: int, mask_band, mask_bits=None):
     for t in (q, k, v, o):
         if t.stride(-1) != 1:
             raise NativeError("last dimension must be contiguous")
     if q.dtype not in DTYPE_CODES or any(t.dtype != q.dtype for t in (k, v, o, d_o)):
         raise NativeError("q, k, v, o, d_o must share dtype float16 or bfloat16")
-    lse = lse.contiguous().float()
-    dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    if dq.stride(-1) != 1 or dk.stride(-1) != 1 or dv.stride(-1) != 1:
-        dq, dk, dv = (torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in (q, k, v))
-    a = SoftmaxBwdArgs()
-    a.q, a.k, a.v, a.o, a.d_o, a.lse = (t.data_ptr() for t in (q, k, v, o, d_o, lse))
-    a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    B, Sq, H, D = q.shape
-    a.batch, a.heads, a.heads_kv, a.seq_q, a.seq_kv, a.dim_qk, a.dim_v = B, H, k.shape[2], Sq, k.shape[1], D, v.shape[3]
-    a.dtype, a.mask_kind, a.scale = DTYPE_CODES[q.dtype], mask_kind, float(scale)
-    a.mask_left, a.mask_right = int(mask_band[0]), int(mask_band[1])
-    if mask_bits is not None:
-        _set_mask_bits(a, mask_bits, q, k)
-    for name, t in (("q", q), ("k", k), ("v", v), ("o", o), ("do", d_o), ("dq", dq), ("dk", dk), ("dv", dv)):
-        getattr(a, name + "_stride")[:] = _strides_bsh(t)
-    lib = load_library()
-    need = lib.attn_b200_softmax_bwd_workspace_bytes(C.byref(a))
-    if need < 0:
-        raise NativeError("attn_b200_softmax_bwd_workspace_bytes: bad arguments")
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-    a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    with torch.cuda.device(q.device):
-        check(lib.attn_b200_softmax_bwd(C.byref(a), current_stream_ptr()), "attn_b200_softmax_bwd")
-    return dq, dk, dv
+    if v.shape[-1] % q.shape[-1] != 0:
+        raise NativeError(f"the backward covers dim_v = a multiple of dim_qk (got {q.shape[-1]} / {v.shape[-1]})")
+    for t in mask_bits or ():
+        if not (t.is_cuda and t.dtype == torch.int32 and t.is_contiguous()):
+            raise NativeError(f"mask bits: expected contiguous CUDA int32 tensors, got {t.dtype} on {t.device}")
+    if d_o.stride(-1) != 1:
+        d_o = d_o.contiguous()
+    return tuple(host().softmax_bwd(q, k, v, o, lse.contiguous().float(), d_o, float(scale), int(mask_kind), int(mask_band[0]),
+                                    int(mask_band[1]), mask_bits or ()))
 
 
 def parallel_fwd(args: ParallelArgs):

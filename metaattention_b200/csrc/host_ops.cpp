@@ -371,6 +371,8 @@ void fill_bwd(Args& a, const Tensor& q, const Tensor& k, const Tensor& v, const 
     a.mask_bits_q = m.bits_q.data_ptr();
     a.mask_bits_kv = m.bits_kv.data_ptr();
     if (m.tiles_q.defined()) {
+      if (m.tiles_q.numel() != nq * ((nk + 31) / 32) || m.tiles_kv.numel() != nk * ((nq + 31) / 32))
+        check(ATTN_B200_E_INVALID_ARG, "backward with bitmaps of other lengths than the call's");
       a.mask_tiles_q = m.tiles_q.data_ptr();
       a.mask_tiles_kv = m.tiles_kv.data_ptr();
     }
@@ -431,6 +433,21 @@ std::vector<Tensor> over_dim_v(const Tensor& q, const Tensor& v, const Run& run)
   return {dq.to(q.scalar_type()), dk.to(q.scalar_type()), at::cat(dvs, -1)};
 }
 
+Tensor cols(const Tensor& t, int64_t c, int64_t w) { return t.size(3) == w ? t : t.narrow(3, c, w); }
+
+std::vector<Tensor> softmax_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o, float scale,
+                                const Mask& m) {
+  return over_dim_v(q, v, [&](int64_t c, int64_t w) {
+    return softmax_bwd_one(q, k, cols(v, c, w), cols(o, c, w), lse, cols(d_o, c, w), scale, m);
+  });
+}
+
+// Of a k or v larger than the call, gradients of what the forward left unread would not be written.
+void whole(const Tensor& q, const Tensor& k, const Tensor& v) {
+  if (k.size(0) != q.size(0) || v.size(0) != q.size(0) || k.size(3) != q.size(3) || v.size(1) != k.size(1) || v.size(2) != k.size(2))
+    check(ATTN_B200_E_INVALID_ARG, "backward with k or v of another batch, length or head dim than the call");
+}
+
 Tensor last_contiguous(Tensor t, const Tensor& like) {
   if (t.scalar_type() != like.scalar_type()) t = t.to(like.scalar_type());
   return t.stride(3) == 1 ? t : t.contiguous();
@@ -473,9 +490,7 @@ struct Attention : torch::autograd::Function<Attention> {
     const std::shared_ptr<Plan>& plan = ref->plan;
     const auto saved = ctx->get_saved_variables();
     const Tensor &q = saved[0], &k = saved[1], &v = saved[2];
-    // the gradients of what the forward left unread would not be written
-    if (k.size(0) != q.size(0) || v.size(0) != q.size(0) || k.size(3) != q.size(3) || v.size(1) != k.size(1))
-      check(ATTN_B200_E_INVALID_ARG, "backward with k or v larger than the call's batch, length or head dim");
+    whole(q, k, v);
     c10::cuda::CUDAGuard guard(q.device());
     Tensor g = grads[0].defined() ? grads[0] : at::zeros({q.size(0), q.size(1), q.size(2), v.size(3)}, q.options());
     const Tensor d_o = last_contiguous(g, q);
@@ -484,13 +499,9 @@ struct Attention : torch::autograd::Function<Attention> {
       ref->mask->used_by_backward(q);
       m.bits_q = ref->mask->bits_q; m.bits_kv = ref->mask->bits_kv; m.tiles_q = ref->mask->tiles_q; m.tiles_kv = ref->mask->tiles_kv;
     }
-    auto cols = [](const Tensor& t, int64_t c, int64_t w) { return t.size(3) == w ? t : t.narrow(3, c, w); };
     std::vector<Tensor> d;
     if (plan->backward == 1) {
-      const Tensor &o = saved[3], &lse = saved[4];
-      d = over_dim_v(q, v, [&](int64_t c, int64_t w) {
-        return softmax_bwd_one(q, k, cols(v, c, w), cols(o, c, w), lse, cols(d_o, c, w), plan->fparams[0], m);
-      });
+      d = softmax_bwd(q, k, v, saved[3], saved[4], d_o, plan->fparams[0], m);
     } else {
       if (plan->bwd_fn == 0) {   // compiled when a gradient is first asked for
         py::gil_scoped_acquire gil;
@@ -531,6 +542,28 @@ py::object run(const std::shared_ptr<Plan>& plan, const Tensor& q, const Tensor&
   return out;
 }
 
+// The softmax backward by itself (core.native.lib.softmax_bwd, which has looked at types, devices and strides).  `bits`:
+// empty, or bits_q, bits_kv and optionally tiles_q, tiles_kv of a general mask.
+std::vector<Tensor> softmax_bwd_call(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& d_o,
+                                     float scale, int kind, int left, int right, const std::vector<Tensor>& bits) {
+  whole(q, k, v);
+  if (o.size(0) != q.size(0) || o.size(1) != q.size(1) || o.size(2) != q.size(2) || o.size(3) != v.size(3) || d_o.sizes() != o.sizes() ||
+      lse.numel() != q.size(0) * q.size(1) * q.size(2))
+    check(ATTN_B200_E_INVALID_ARG, "backward with o, lse or a gradient of another shape than the output");
+  c10::cuda::CUDAGuard guard(q.device());
+  Mask m{kind, left, right, {}, {}, {}, {}};
+  if (bits.size() >= 2) {
+    m.bits_q = bits[0];
+    m.bits_kv = bits[1];
+  }
+  if (bits.size() == 4) {
+    m.tiles_q = bits[2];
+    m.tiles_kv = bits[3];
+  }
+  at::AutoDispatchBelowADInplaceOrView below;
+  return softmax_bwd(q, k, v, o, lse, d_o, scale, m);
+}
+
 std::shared_ptr<Plan> make_plan(const py::dict& d) {
   // the last reference may be dropped by an autograd thread: Python objects go under the GIL
   std::shared_ptr<Plan> p(new Plan, [](Plan* x) {
@@ -567,6 +600,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("bind", &bind);
   m.def("make_plan", &make_plan);
   m.def("run", &run);
+  m.def("softmax_bwd", &softmax_bwd_call);
   m.def("kv_splits", &kv_splits_for);
   m.def("splits_on", &splits_on);
   m.def("fault", &fault);

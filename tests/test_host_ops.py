@@ -132,3 +132,13 @@ def test_engines_that_have_been_called_are_copied_and_pickled(host, duplicate):
     twin = duplicate(eng)
     assert twin._plan is None and eng._plan is plan
     assert host.fault(twin._make_plan(), *operands(*[(1, 700, 2, 64)] * 3)) is not None
+
+
+def test_backward_refuses_what_it_would_leave_unwritten(host):
+    """a status of the library, raised from native code, arrives as the library's error"""
+    q, k, v, o = operands((2, 256, 8, 64), (3, 256, 8, 64), (3, 256, 8, 64), (2, 256, 8, 64))
+    lse = torch.zeros(2, 8, 256)
+    with pytest.raises(lib.NativeError, match="invalid argument"):
+        host.softmax_bwd(q, k, v, o, lse, o, 0.125, lib.MASK_CAUSAL, 0, 0, ())
+    with pytest.raises(lib.NativeError, match="invalid argument"):
+        host.softmax_bwd(q, k[:2], v[:2], o, lse[:1], o, 0.125, lib.MASK_CAUSAL, 0, 0, ())
