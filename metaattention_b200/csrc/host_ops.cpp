@@ -18,6 +18,7 @@
 #include <torch/extension.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -123,7 +124,7 @@ struct Plan {
   int backward = 0;            // 0 none, 1 softmax, 2 elementwise
   py::object load_mask;        // device -> dict of tensors
   py::object load_backward;    // () -> address of attn_b200_elementwise_bwd_jit
-  uintptr_t bwd_fn = 0;
+  std::atomic<uintptr_t> bwd_fn{0};   // loaded by the first backward; autograd runs one thread per device
   std::map<int, std::shared_ptr<const Sparse>> masks;
 
   std::shared_ptr<const Sparse> mask_on(const Tensor& like) {   // with the GIL
@@ -200,8 +201,8 @@ const char* fault(const Plan& plan, const Tensor& q, const Tensor& k, const Tens
   return nullptr;
 }
 
-// The forward of one call; `done` false = declined.  With the GIL when the plan has a mask walk that a device has not seen.
-Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
+// The forward of one call; `done` false = declined.  `mask`: the plan's on q's device, if it has one.
+Forward forward(const Plan& plan, const std::shared_ptr<const Sparse>& mask, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
                 OptTensor block_mask, OptTensor lens) {
   Forward r;
   if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(plan, q, k, v) != nullptr || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
@@ -282,8 +283,8 @@ Forward forward(Plan& plan, const Tensor& q, const Tensor& k, const Tensor& v, c
     a.sparse_batch = B;
     a.sparse_heads = Hkv;
   } else if (plan.has_mask_walk) {
-    r.mask = plan.mask_on(q);
-    const Sparse& s = *r.mask;
+    r.mask = mask;
+    const Sparse& s = *mask;
     s.used_by_forward(q);
     a.tile_keep = static_cast<const uint32_t*>(s.keep.data_ptr());
     a.tile_partial = static_cast<const uint32_t*>(s.partial.data_ptr());
@@ -526,19 +527,30 @@ struct Attention : torch::autograd::Function<Attention> {
 // One call of an engine: None (declined) or [o, final row scales...].  `grad`: the call is recorded for the backward.
 py::object run(const std::shared_ptr<Plan>& plan, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom,
                int forced_splits, const OptTensor& block_mask, const OptTensor& lens, bool grad) {
-  Forward f;
+  std::shared_ptr<const Sparse> mask;
+  if (plan->has_mask_walk && q.is_cuda()) {
+    c10::cuda::CUDAGuard guard(q.device());
+    at::AutoDispatchBelowADInplaceOrView below;
+    mask = plan->mask_on(q);   // calls Python the first time
+  }
+  std::vector<Tensor> results;
   {
-    at::AutoDispatchBelowADInplaceOrView below;   // outputs are made, nothing is recorded
-    f = forward(*plan, q, k, v, custom, forced_splits, block_mask, lens);
+    py::gil_scoped_release others_run;   // a launch waits while the stream's queue is full
+    Forward f;
+    {
+      at::AutoDispatchBelowADInplaceOrView below;   // outputs are made, nothing is recorded
+      f = forward(*plan, mask, q, k, v, custom, forced_splits, block_mask, lens);
+    }
+    if (f.done && grad) {
+      results = Attention::apply(plan, f, q, k, v, custom);
+    } else if (f.done) {
+      results.push_back(std::move(f.o));
+      for (Tensor& t : f.finals) results.push_back(std::move(t));
+    }
   }
-  if (!f.done) return py::none();
+  if (results.empty()) return py::none();
   py::list out;
-  if (grad) {
-    for (Tensor& t : Attention::apply(plan, f, q, k, v, custom)) out.append(std::move(t));
-  } else {
-    out.append(f.o);
-    for (Tensor& t : f.finals) out.append(t);
-  }
+  for (Tensor& t : results) out.append(std::move(t));
   return out;
 }
 
@@ -560,6 +572,7 @@ std::vector<Tensor> softmax_bwd_call(const Tensor& q, const Tensor& k, const Ten
     m.tiles_q = bits[2];
     m.tiles_kv = bits[3];
   }
+  py::gil_scoped_release others_run;
   at::AutoDispatchBelowADInplaceOrView below;
   return softmax_bwd(q, k, v, o, lse, d_o, scale, m);
 }

@@ -1,6 +1,8 @@
 """The native host side of a call (csrc/host_ops.cpp) on the GPU: what surrounds the launches."""
 
 import gc
+import threading
+import time
 
 import pytest
 import torch
@@ -76,3 +78,33 @@ def test_decode_arguments_of_an_engine_without_them_are_left_alone():
     mask = torch.zeros(2, 2, 8, dtype=torch.bool, device="cuda")
     assert torch.equal(eng.attention(q, k, v, block_mask=mask, cache_seqlens=torch.tensor([3, 5])), want)
     assert lib.last_device_status() == 0
+
+
+def test_other_threads_run_while_a_call_waits_for_the_stream():
+    """Behind 0.7 s of work on the stream, calls fill its queue (about a thousand launches) and the next one waits."""
+    eng = programs.gqa_engine(1, 2, 2, 128, 128, 64, 64, is_causal=True)
+    q, k, v = (rand(1, 128, 2, 64) for _ in range(3))
+    eng(q, k, v)
+    torch.cuda.synchronize()
+    longest, stop = [0.0], threading.Event()
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            longest[0], last = max(longest[0], now - last), now
+
+    ticker = threading.Thread(target=tick)
+    ticker.start()
+    time.sleep(0.05)
+    torch.cuda._sleep(int(0.7 * 1.9e9))
+    start = time.perf_counter()
+    for _ in range(3000):
+        eng(q, k, v)
+    waited = time.perf_counter() - start
+    stop.set()
+    ticker.join()
+    torch.cuda.synchronize()
+    assert waited > 0.4, "the queue was never full"
+    assert longest[0] < 0.2, longest[0]
