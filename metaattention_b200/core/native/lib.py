@@ -9,7 +9,9 @@ entry points do (core/template/cute_template_kvshared/flash_api.cpp:46-47,133,18
 
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
+import hashlib
 import os
 import subprocess
 
@@ -19,9 +21,9 @@ _PKG_DIR = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(__fil
 CSRC_DIR = os.path.join(_PKG_DIR, "csrc")
 INCLUDE_DIR = os.path.join(os.path.dirname(_PKG_DIR), "include")
 LIB_PATH = os.path.join(_PKG_DIR, "libattn_b200.so")
-HOST_PATH = os.path.join(_PKG_DIR, "_host_ops.so")
 
 NVCC_ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_host_ops"]
 NVCC_COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-shared"]
 
 MAX_CUSTOM = 4
@@ -205,26 +207,39 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def host_path() -> str:
+    """Where the native host side lies that belongs to these sources and this torch: it fills the structs of the header by
+    their compiled-in layout and calls torch's C++ API, so one built from others is never loaded."""
+    key = hashlib.sha256(" ".join([torch.__version__, *HOST_FLAGS]).encode())
+    for path in (os.path.join(CSRC_DIR, "host_ops.cpp"), os.path.join(INCLUDE_DIR, "attn_b200.h")):
+        with open(path, "rb") as f:
+            key.update(f.read())
+    return os.path.join(_PKG_DIR, f"_host_ops_{key.hexdigest()[:16]}.so")
+
+
 def build_host_ops(force: bool = False) -> str:
-    """Compile _host_ops.so (csrc/host_ops.cpp: the host side of a call against torch's C++ API) with g++."""
-    src = os.path.join(CSRC_DIR, "host_ops.cpp")
-    deps = [src, os.path.join(INCLUDE_DIR, "attn_b200.h")]
-    if not force and os.path.exists(HOST_PATH) and os.path.getmtime(HOST_PATH) >= max(os.path.getmtime(d) for d in deps):
-        return HOST_PATH
+    """Compile the native host side (csrc/host_ops.cpp: the host side of a call against torch's C++ API) with g++; those of
+    other sources are removed."""
+    path = host_path()
+    if not force and os.path.exists(path):
+        return path
     import sysconfig
     torch_dir = os.path.dirname(torch.__file__)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
             os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
-    tmp = HOST_PATH + f".tmp{os.getpid()}"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_host_ops",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in incs), "-I", INCLUDE_DIR, src,
-           "-o", tmp, "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    tmp = path + f".tmp{os.getpid()}"
+    cmd = ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in incs), "-I", INCLUDE_DIR,
+           os.path.join(CSRC_DIR, "host_ops.cpp"), "-o", tmp, "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise NativeError(f"g++ failed: {' '.join(cmd)}\n{r.stdout}")
-    os.replace(tmp, HOST_PATH)
-    return HOST_PATH
+    os.replace(tmp, path)
+    for name in os.listdir(_PKG_DIR):
+        if name.startswith("_host_ops") and name.endswith(".so") and name != os.path.basename(path):
+            with contextlib.suppress(FileNotFoundError):   # another process that builds the same
+                os.remove(os.path.join(_PKG_DIR, name))
+    return path
 
 
 def bind(lib: C.CDLL, names=None) -> C.CDLL:
@@ -252,14 +267,12 @@ _host = None
 
 def host():
     """Load (once) the native host side, bound to the entry points of the library and to ``check``.  Like a functor
-    library it is compiled if it is not there; there is no other way to run a call."""
+    library it is compiled if the one of these sources is not there; there is no other way to run a call."""
     global _host
     if _host is None:
         import importlib.util
         lib = load_library()
-        if not os.path.exists(HOST_PATH):
-            build_host_ops()
-        spec = importlib.util.spec_from_file_location("_host_ops", HOST_PATH)
+        spec = importlib.util.spec_from_file_location("_host_ops", build_host_ops())
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
         mod.bind({name: C.cast(getattr(lib, name), C.c_void_p).value for name in SIGNATURES}, check)

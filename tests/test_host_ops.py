@@ -3,7 +3,9 @@ the life of the plans that engines give it."""
 
 import copy
 import gc
+import os
 import pickle
+import shutil
 import weakref
 
 import pytest
@@ -142,3 +144,18 @@ def test_backward_refuses_what_it_would_leave_unwritten(host):
         host.softmax_bwd(q, k, v, o, lse, o, 0.125, lib.MASK_CAUSAL, 0, 0, ())
     with pytest.raises(lib.NativeError, match="invalid argument"):
         host.softmax_bwd(q, k[:2], v[:2], o, lse[:1], o, 0.125, lib.MASK_CAUSAL, 0, 0, ())
+
+
+def test_a_host_side_of_other_sources_is_not_loaded(host, monkeypatch, tmp_path):
+    """the header gives the layout of the structs that it fills"""
+    assert host.__file__ == lib.host_path() == lib.build_host_ops()
+    shutil.copy(os.path.join(lib.INCLUDE_DIR, "attn_b200.h"), tmp_path)
+    with monkeypatch.context() as m:
+        m.setattr(lib, "INCLUDE_DIR", str(tmp_path))
+        assert lib.host_path() == host.__file__
+        with open(tmp_path / "attn_b200.h", "a") as f:
+            f.write("/* a field more */")
+        assert lib.host_path() != host.__file__
+    with monkeypatch.context() as m:
+        m.setattr(torch, "__version__", "0.0")
+        assert lib.host_path() != host.__file__
