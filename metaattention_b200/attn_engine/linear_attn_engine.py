@@ -182,9 +182,9 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
 
 
 def _reversed_forward(q, k, v, log_decay, q_scale, out_dtype=None, precise=False):
-    """o_j = q_scale * sum_{i>=j} exp(G_i - G_j) (q_j . k_i) v_i: what ``linear_attention_forward`` gives on time-reversed
-    operands.  Position u of the reversed sequence then carries the log-decay of token T - u (0 for u = 0), so that the
-    reversed cumulative sums reproduce the same factors.  The kernel walks the sequence backwards itself."""
+    """o_j = q_scale * sum_{i>=j} exp(G_i - G_j) (q_j . k_i) v_i, G the inclusive cumulative sum of log_decay: the kernel
+    walks the sequence from its end.  The same on time-reversed operands, where position u carries the log-decay of token
+    T - u (0 for u = 0), is how the composition is followed without a GPU, the oracle in the kernel's place."""
     if q.is_cuda:
         return linear_attention_forward(q, k, v, log_decay, q_scale, out_dtype=out_dtype, precise=precise, reverse=True)
     ld_rev = torch.cat([torch.zeros_like(log_decay[..., :1]), log_decay.flip(-1)[..., :-1]], dim=-1)

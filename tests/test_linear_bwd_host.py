@@ -106,3 +106,21 @@ def test_engine_differentiates_through_its_mods(oracle_kernel):
         assert got.grad is not None, what
         err = (got.grad.double() - want.grad).abs().max().item()
         assert err <= 2e-3 * max(1.0, want.grad.abs().max().item()), (what, err)
+
+
+@pytest.mark.parametrize("S,Dk,Dv", [(1, 64, 64), (50, 64, 128), (97, 128, 64)])
+def test_reversed_operands_are_the_sums_to_the_end_of_the_sequence(oracle_kernel, S, Dk, Dv):
+    """The composition above takes its reversed runs through time-reversed operands; on the GPU they are the kernel's walk
+    from the end (tests/test_linear_bwd_gpu.py compares that with reversed operands).  Both stand for the same sums:
+    o_j = sum_{i>=j} exp(G_i - G_j) (scale q_j . k_i) v_i, here as a matrix."""
+    B, H = 2, 3
+    g = torch.Generator().manual_seed(S)
+    q, k = (torch.randn(B, H, S, Dk, generator=g) for _ in range(2))
+    v = torch.randn(B, H, S, Dv, generator=g)
+    log_decay = -torch.rand(B, H, S, generator=g)
+    G = log_decay.double().cumsum(-1)
+    decay = torch.exp((G.unsqueeze(-2) - G.unsqueeze(-1)).masked_fill(torch.ones(S, S).triu() == 0, float("-inf")))
+    want = (0.3 * q.double() @ k.double().transpose(-1, -2) * decay) @ v.double()
+    got = oracle_kernel._reversed_forward(q, k, v, log_decay, 0.3)
+    # one rounding of the oracle's 64-bit sums to fp32
+    assert (got.double() - want).abs().max().item() <= 2.0 ** -23 * want.abs().max().item()
