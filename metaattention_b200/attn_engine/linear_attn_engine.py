@@ -127,6 +127,9 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
     if out_dtype not in (None, q.dtype, torch.float32):
         raise native.NativeError("out_dtype must be the input dtype or torch.float32")
     f32_out = out_dtype == torch.float32
+    # the kernel walks k and v with the extents of q: what has others would be read askew or past its end
+    if k.shape[3] != q.shape[3] or k.shape[2] != q.shape[2] or v.shape[2] != q.shape[2] or min(k.shape[0], v.shape[0]) < q.shape[0]:
+        raise native.NativeError(f"q, k, v do not fit together: {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
     if not q.is_cuda:
         raise native.NativeError("linear attention needs CUDA tensors")
     if q.dtype not in native.DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype:

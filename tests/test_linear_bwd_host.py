@@ -124,3 +124,12 @@ def test_reversed_operands_are_the_sums_to_the_end_of_the_sequence(oracle_kernel
     got = oracle_kernel._reversed_forward(q, k, v, log_decay, 0.3)
     # one rounding of the oracle's 64-bit sums to fp32
     assert (got.double() - want).abs().max().item() <= 2.0 ** -23 * want.abs().max().item()
+
+
+@pytest.mark.parametrize("k,v", [((2, 1, 96, 64), (2, 4, 100, 128)), ((2, 1, 100, 128), (2, 4, 100, 128)), ((1, 1, 100, 64), (2, 4, 100, 128)),
+                                 ((2, 1, 100, 64), (2, 4, 104, 128)), ((2, 1, 100, 64), (1, 4, 100, 128))])
+def test_operands_that_do_not_fit_together_are_refused(k, v):
+    from attn_engine.linear_attn_engine import linear_attention_forward
+    from core.native import lib
+    with pytest.raises(lib.NativeError, match="do not fit together"):
+        linear_attention_forward(torch.zeros(2, 2, 100, 64), torch.zeros(*k), torch.zeros(*v), torch.zeros(2, 4, 100))
