@@ -127,18 +127,16 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
     if out_dtype not in (None, q.dtype, torch.float32):
         raise native.NativeError("out_dtype must be the input dtype or torch.float32")
     f32_out = out_dtype == torch.float32
+    (B, HQ, T, Dk), (Bk, HK, Tk, Dkk), (Bv, H, Tv, Dv) = q.shape, k.shape, v.shape
     # the kernel walks k and v with the extents of q: what has others would be read askew or past its end
-    if k.shape[3] != q.shape[3] or k.shape[2] != q.shape[2] or v.shape[2] != q.shape[2] or min(k.shape[0], v.shape[0]) < q.shape[0]:
+    if Dkk != Dk or Tk != T or Tv != T or Bk < B or Bv < B:
         raise native.NativeError(f"q, k, v do not fit together: {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
     if not q.is_cuda:
         raise native.NativeError("linear attention needs CUDA tensors")
     if q.dtype not in native.DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype:
         raise native.NativeError("q, k, v must share dtype float16 or bfloat16")
-    B, _, T, Dk = q.shape
-    H = v.shape[1]
-    if H % q.shape[1] != 0 or H % k.shape[1] != 0:
+    if H % HQ != 0 or H % HK != 0:
         raise native.NativeError("the heads of v must be a multiple of the heads of q and of k")
-    Dv = v.shape[-1]
     if Dv % 128 != 0 and normalize:
         raise native.NativeError("normalize needs dim_v to be a multiple of 128")
     if Dv % 8 != 0 or (f32_out and Dv % 128 != 0):
@@ -164,7 +162,7 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
         a.q, a.k, a.v, a.log_decay, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), log_decay.data_ptr(), o.data_ptr()
         a.v_scale = v_scale.data_ptr() if v_scale is not None else None
         a.batch, a.heads, a.seq, a.dim_qk, a.dim_v = B, H, T, Dk, Dv
-        a.heads_q, a.heads_k = q.shape[1], k.shape[1]
+        a.heads_q, a.heads_k = HQ, HK
         a.q_ld, a.k_ld = q_ld, k_ld
         a.dtype = native.DTYPE_CODES[q.dtype]
         a.normalize = 1 if normalize else 0
