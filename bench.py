@@ -418,7 +418,7 @@ def extras_backward(peaks, launches=10):
         fl = 2.5 * attention_flops(B, H, S, D, D, True)
         rec["tflops"] = fl / rec["ms"] / 1e9
         rec["roofline"] = tensor_roofline(fl, rec["ms"], peaks, sustained=False)
-        rec["note"] = "FLOPs of five tile products per (query tile, KV tile); the two kernels execute seven"
+        rec["note"] = "FLOPs of five tile products per (query tile, KV tile); its two roles execute seven"
         out["softmax_backward_causal_8x32x4096x128"] = rec
         # the same shape under masks that skip tiles: a sliding window and causal documents of 1024 tokens (a general
         # mask_mod: keep bits and tile bitmaps from the front-end)

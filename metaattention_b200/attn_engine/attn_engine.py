@@ -172,7 +172,8 @@ class AttentionEngine:
         elif self.pattern in ("gqa", "gqa_decode"):
             # grouped KV heads (the reference's lower_gqa.py / attn_gqa_tl.py and the dense case of its GQA decode):
             # the same forward kernel, query head h reading KV head h / (H / Hkv); K/V of a group are fetched
-            # once per query head and mostly hit L2.  With extern_block_mask / use_varlen (examples/sparse_gqa_decode.py)
+            # once per query head and mostly hit L2 (decode through the built-in softmax: once per KV head,
+            # csrc/decode_fwd.cu).  With extern_block_mask / use_varlen (examples/sparse_gqa_decode.py)
             # the kept blocks and cache lengths of each call select the KV tiles that are visited.
             if H % Hkv != 0:
                 raise NotImplementedError(f"query heads ({H}) must be a multiple of KV heads ({Hkv})")
@@ -181,9 +182,9 @@ class AttentionEngine:
             self._build_parallel(B, H, Sq, D, Dv, dtype, score_mod, mask_mod, online_func, mask_value, kv_len=Skv)
         elif self.pattern == "mha_decode":
             # A few query rows against a long KV (examples/mha_decode.py; the reference lowers it to a split-KV
-            # kernel plus OnlineFunc.combine, lower_decode.py:375-449).  The forward kernel takes any
-            # q_len != kv_len, streams K/V once per (batch, head) and needs no combine step; with few
-            # (batch, head) pairs it leaves SMs idle.
+            # kernel plus OnlineFunc.combine, lower_decode.py:375-449).  The built-in softmax has a decode kernel
+            # (csrc/decode_fwd.cu); other programs run on the forward kernel, which takes any q_len != kv_len and
+            # splits the KV with few (batch, head) pairs, through the program's combine.
             if use_varlen or extern_block_mask:
                 self._decode_block = int(infer_mask_block_N)
             self._build_parallel(B, H, Sq, D, Dv, dtype, score_mod, mask_mod, online_func, mask_value, kv_len=Skv)

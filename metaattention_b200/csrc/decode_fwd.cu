@@ -17,9 +17,9 @@
 //     unit through tensor memory (both accumulators of a row are in the lane of its thread).  With one group the warp that
 //     holds the only used rows is the bound: ~1600 cycles a tile, against 1480 for the bytes of a 64-wide tile;
 //   * K and V each have a ring of 96 KB: ~190 KB in flight per SM, three times what latency times bandwidth asks for.
-// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 120 -> 92 us = 5.8 TB/s of K and V;
-// 8 sequences x 32 heads on 8 KV heads, up to 8192 tokens, 30 % of the 32-token blocks kept 208 -> 40 us; 16 sequences, the
-// same heads, 2500 tokens, the kernel alone 153 -> 32 us.
+// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 127 -> 95-102 us = 5.3-5.6 TB/s of K
+// and V; 8 sequences x 32 heads on 8 KV heads, up to 8192 tokens, 30 % of the 32-token blocks kept 212 -> 39 us.  8 such
+// sequences of 16384 tokens: dense 5.8 TB/s, every block kept (the gather) 3.9; of 32768, 30 % kept: 2.7.
 // A unit that is a whole (sequence, KV head) pair writes its output; the others leave fp32 partial rows that a second
 // small kernel adds up, launched early (programmatic dependent launch) so that only its own microseconds show.
 #include <cstring>

@@ -18,7 +18,9 @@
 // are 128 tokens (the MMA M) instead of the reference's default 64; the result does not depend on
 // the block size.
 //
-// One CTA per (128-column slice of dim_v, batch*head), walking the sequence in 128-token blocks.
+// One CTA per (128-column slice of dim_v, batch*head), walking the sequence in 128-token blocks (from its end for the
+// gradients of k and v); where that leaves SMs idle several CTAs share a chain's blocks (plan_segments), and two heads of 64
+// columns that share q and k go to one CTA (kPair).
 // The state is held transposed, hT[dv_slice=128][dim_qk], so that its MMAs have M = 128 for any
 // dim_qk: TMEM columns [0, DK) = hT, [256, 384) = S / P, [384, 512) = O.
 // Shared memory: Q, K (DK/64 chunks of 128 rows x 128 B each), V (2 chunks), bf16 hT (DK/64 chunks;
