@@ -229,8 +229,9 @@ def build_host_ops(force: bool = False) -> str:
     incs = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
             os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
     tmp = path + f".tmp{os.getpid()}"
-    cmd = ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in incs), "-I", INCLUDE_DIR,
-           os.path.join(CSRC_DIR, "host_ops.cpp"), "-o", tmp, "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
+    cmd = ["g++", *HOST_FLAGS, f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-isystem{i}" for i in incs),
+           "-I", INCLUDE_DIR, os.path.join(CSRC_DIR, "host_ops.cpp"), "-o", tmp,
+           "-L", os.path.join(torch_dir, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if r.returncode != 0:
         raise NativeError(f"g++ failed: {' '.join(cmd)}\n{r.stdout}")

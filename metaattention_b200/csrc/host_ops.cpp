@@ -202,10 +202,11 @@ const char* fault(const Plan& plan, const Tensor& q, const Tensor& k, const Tens
 }
 
 // The forward of one call; `done` false = declined.  `mask`: the plan's on q's device, if it has one.
-Forward forward(const Plan& plan, const std::shared_ptr<const Sparse>& mask, const Tensor& q, const Tensor& k, const Tensor& v, const std::vector<Tensor>& custom, int forced_splits,
-                OptTensor block_mask, OptTensor lens) {
+Forward forward(const Plan& plan, const std::shared_ptr<const Sparse>& mask, const Tensor& q, const Tensor& k, const Tensor& v,
+                const std::vector<Tensor>& custom, int forced_splits, OptTensor block_mask, OptTensor lens) {
   Forward r;
-  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(plan, q, k, v) != nullptr || !q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4 || fault(plan, q, k, v) != nullptr) return r;
+  if (!q.is_cuda() || k.device() != q.device() || v.device() != q.device()) return r;
   const int dt = dtype_code(q);
   if (dt < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return r;
   if (q.stride(3) != 1 || k.stride(3) != 1 || v.stride(3) != 1) return r;
@@ -366,7 +367,8 @@ void fill_bwd(Args& a, const Tensor& q, const Tensor& k, const Tensor& v, const 
   a.mask_right = m.right;
   if (m.bits_q.defined()) {
     const int64_t nq = (q.size(1) + 127) / 128, nk = (k.size(1) + 127) / 128;
-    if (m.bits_q.size(0) != nq * 128 || m.bits_q.size(1) != nk || m.bits_kv.size(0) != nk * 128 || m.bits_kv.size(1) != nq)
+    const std::vector<int64_t> want_q{nq * 128, nk, 4}, want_kv{nk * 128, nq, 4};
+    if (m.bits_q.sizes() != want_q || m.bits_kv.sizes() != want_kv)
       check(ATTN_B200_E_INVALID_ARG, "backward at other lengths than mask_mod was evaluated for");
     a.mask_kind = ATTN_B200_MASK_BITS;
     a.mask_bits_q = m.bits_q.data_ptr();

@@ -122,4 +122,10 @@ def test_refusals_of_the_library_arrive_as_its_error():
     assert torch.equal(o, eng(q, k[:1].detach(), v[:1].detach()))
     with pytest.raises(lib.NativeError, match="invalid argument"):
         o.sum().backward()
+    # keep bits of another extent than the call's, in each of their dimensions
+    q, k, v, o = (t.detach() for t in (q, k[:1], v[:1], o))
+    for shape in ((384, 2, 4), (256, 3, 4), (256, 2, 2)):
+        bits = [torch.zeros(*shape, dtype=torch.int32, device="cuda")] * 2
+        with pytest.raises(lib.NativeError, match="invalid argument"):
+            lib.softmax_bwd(q, k, v, o, torch.zeros(1, 2, 256, device="cuda"), o, 0.125, lib.MASK_NONE, mask_bits=bits)
     assert lib.last_device_status() == 0
