@@ -408,8 +408,8 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
           for (int i = 0; i < N; ++i) s[i] = i < left ? s[i] : -INFINITY;
         }
-        const float o_scale = F::template tile_pieces<N>(s, rs, ctx, [&](int c) {
-          constexpr int W = N / F::kPieces / 2;
+        const float o_scale = F::template tile_pieces<N, 4>(s, rs, ctx, [](float mx) { return mx; }, [&](int c) {
+          constexpr int W = N / 4 / 2;
           uint32_t pk[W];
 #pragma unroll
           for (int i = 0; i < W; ++i) pk[i] = pack2<kBf16>(s[c * 2 * W + 2 * i], s[c * 2 * W + 2 * i + 1]);

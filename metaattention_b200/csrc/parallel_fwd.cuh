@@ -9,16 +9,22 @@
 // (attention_engine/core/template/tl_template/attn/attn_tl.py:93-190) and its
 // CuTe warp-specialised forward (core/template/cute_template/flash_fwd_kernel.h:28-199).
 //
-// One CTA owns two 128-row query tiles of one (batch, head) and walks the KV
-// sequence in 128-row tiles:
-//   warp 8      TMA producer: Q once, then K and V tiles into 2-stage rings
-//   warp 9      tcgen05.mma issuer (one thread): S_t = Q_t.K^T into TMEM,
-//               O_t += P_t.V with P_t read from TMEM (aliasing S_t)
-//   warps 0-3   row-per-thread functor stage for query tile 0
-//   warps 4-7   same for query tile 1
-// The two query tiles ping-pong: while the functor stage of one tile runs on
-// the CUDA cores, the tensor pipe works on the other tile.
-// TMEM columns: S0 [0,128) S1 [128,256) O0 [256,256+DV) O1 [256+DV,256+2DV).
+// One CTA owns two 128-row query tiles (NT; one for the widest heads) of one (batch, head) and walks the KV
+// sequence in 128-row tiles.  Warps, with RT threads to a query row (two where the functor allows it):
+//   4 RT per query tile   functor stage: scores from tensor memory to registers, P back to tensor memory
+//   1                     loads of Q and K (TMA rings), 1 loads of V
+//   1                     issues S = Q_t.K^T (tcgen05.mma), 1 issues O_t += P_t.V with P_t read from tensor memory
+// What bounds it is the functor stage: 128 x 128 exponentials are 1024 cycles of the special-function unit, and both
+// tiles' together equal the 2048 cycles of their MMAs.  So the functor warps never wait for each other's tile or for the
+// pipe: P has columns of its own, and a score tile leaves its buffer for registers as soon as it is there, so the
+// next one (the other tile's, where there is one buffer) is computed under the exponentials; the four service warps wait
+// for nothing but their own operands (one warp that issued both products in turn: 4950 cycles for a step of both tiles
+// against 3300, its barriers and bookkeeping of 400-600 cycles a product standing in front of an idle pipe).  With P
+// written over its own scores (so that a tile's chain functor -> P.V -> Q.K^T was serial), 192 / 128 causal
+// 2 x 16 x 3000 took 154 us, now 124; sigmoid 2 x 32 x 4096 523, now 488; causal 8 x 32 x 4096 1216, now 1157 (at its power cap).
+// Two threads to a row (16 functor warps, four to a scheduler) against one: causal 6 x 8 x 965 33 us against 34-37, long
+// calls 2 % slower for softmax and sigmoid alike.
+// Tensor memory: O0 O1 (DV columns each), P0 P1 (64 each), then one or two score buffers (128 each).
 // Masks are bands kv_idx in [q_idx - left, q_idx + right] (none / causal / explicit bounds): a query tile
 // walks only the KV tiles its band touches, the CTA loads the union of its two tiles' ranges, and tiles
 // that cross an edge of the band are masked element by element.  K/V heads may be shared by groups of
@@ -44,13 +50,16 @@ struct FunctorArgs {
   long long cstride[kMaxCustom][4];  // element strides of (batch, heads, seq_len, seq_len_kv)
 };
 
-// What a functor knows about the row it is working on.
-// A functor may offer tile_halves<N>() (see SoftmaxFunctor) beside tile<N>().
+// Threads that share a row: two where the functor allows it (it keeps nothing per row, or its row values are a maximum
+// that the threads exchange and a sum that is added up at the end), so that four functor warps run on each scheduler.
 template <class F, class = void>
-struct functor_half_store : std::false_type {};
+struct functor_split_sum : std::false_type {};
 template <class F>
-struct functor_half_store<F, std::void_t<decltype(F::kHalfStore)>> : std::integral_constant<bool, F::kHalfStore> {};
+struct functor_split_sum<F, std::void_t<decltype(F::kSplitSum)>> : std::true_type {};
+template <class F>
+constexpr int kRowThreads = functor_split_sum<F>::value || (F::kRowScales == 0 && F::kUnitOScale) ? 2 : 1;
 
+// What a functor knows about the row it is working on.
 struct RowCtx {
   int b, h, q_idx;   // batch, head, query position of this thread's row
   int kv0;           // first KV position of the current tile
@@ -101,7 +110,7 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const CUtensorMap* tm, 
 
 // wait-site ids reported through the device status word
 enum ParallelWaitSite {
-  kSiteQFull = 1, kSiteKFull, kSiteVFull, kSiteKEmpty, kSiteVEmpty, kSiteSFull, kSitePReady, kSiteODone, kSiteOFinal
+  kSiteQFull = 1, kSiteKFull, kSiteVFull, kSiteKEmpty, kSiteVEmpty, kSiteSFull, kSitePReady, kSiteODone, kSiteOFinal, kSiteSFree, kSiteSmemAlign
 };
 
 // Walks the set bits of one bitmap, or of the union of two, in increasing order (KV tile indices of a sparse walk).
@@ -122,6 +131,10 @@ struct TileWalk {
   }
 };
 
+// four functor warps per query tile and thread of a row, two loading and two issuing warps
+template <int NT, int RT>
+constexpr int kParallelThreads = (4 * NT * RT + 4) * 32;
+
 constexpr int kMaxTileWords = 128;   // sparse walks: at most 4096 KV tiles (512 k tokens)
 
 // NT = query tiles per CTA: 2 (K/V shared by both tiles, in two stages; with dim_qk = 192 the tiles leave room for one
@@ -138,27 +151,34 @@ struct ParallelSmem {
   static constexpr int kOffK = kOffQ + NT * kQBytes;
   static constexpr int kOffV = kOffK + kStages * kKBytes;
   static constexpr int kOffBar = kOffV + kVStages * kVBytes;
-  static constexpr int kNumBars = 2 + 2 * kStages + 2 * kVStages + 6;
+  static constexpr int kNumBars = 2 + 2 * kStages + 2 * kVStages + 8;
   static constexpr int kOffMisc = kOffBar + 8 * kNumBars;
-  static constexpr int kOffSparse = kOffMisc + 16;     // sparse kernels: keep / partial bitmaps of the two query tiles
-  static constexpr int kBytes = kOffMisc + 16 + 1024;  // + slack for manual 1024-byte alignment
+  static constexpr int kOffExchange = kOffMisc + 16;   // row maxima of the two threads of a row: [steps][NT][2][128]
+  // one step's only where the tiles leave no room for two: a second barrier then keeps the next step's write off
+  static constexpr int kExchangeSteps = NT == 2 && D > 128 ? 1 : 2;
+  static constexpr int kOffSparse = kOffExchange + kExchangeSteps * NT * 2 * kBM * 4;     // sparse kernels: keep / partial bitmaps of the two query tiles
+  static constexpr int kBytes = kOffSparse;            // the dynamic shared memory is declared 1024-byte aligned
   static constexpr int kBytesSparse = kBytes + 4 * kMaxTileWords * 4;
 };
 
 template <class F, int D, int DV, bool kBf16, int NT = 2, bool kSparse = false>
-__global__ void __launch_bounds__((4 * NT + 2) * 32, 1)
+__global__ void __launch_bounds__(kParallelThreads<NT, kRowThreads<F>>, 1)
 parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const ParallelParams p) {
   using L = ParallelSmem<D, DV, NT>;
   constexpr int BM = L::kBM, BN = L::kBN, ST = L::kStages, STV = L::kVStages;
   static_assert(D % 64 == 0 && DV % 64 == 0 && DV <= 128 && (D <= 192 || (D <= 256 && NT == 1)), "unsupported head dims");
   static_assert((kSparse ? L::kBytesSparse : L::kBytes) <= 232448, "shared memory layout exceeds an SM");
-  constexpr uint32_t kTmemCols = NT == 2 ? 512 : 256;
-  constexpr uint32_t kColS = 0, kColO = NT * 128;
-  constexpr int kTmaWarp = 4 * NT, kMmaWarp = 4 * NT + 1;
+  // score buffers: one that both query tiles take in turn where the accumulators leave room for no more (dim_v 128),
+  // else one per query tile; a CTA with a single query tile takes two in turn
+  constexpr int NSB = NT == 2 && DV > 64 ? 1 : 2;
+  constexpr uint32_t kTmemCols = 512;
+  constexpr uint32_t kColO = 0, kColP = NT * DV, kColS = 512 - NSB * BN;
+  static_assert(kColP + NT * (BN / 2) <= kColS, "tensor memory layout");
+  constexpr int RT = kRowThreads<F>, TC = BN / RT;   // threads per query row, score columns per thread
+  constexpr int kKWarp = 4 * NT * RT, kVWarp = kKWarp + 1, kQkWarp = kKWarp + 2, kPvWarp = kKWarp + 3;
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem + L::kOffQ;
   uint8_t* sK = smem + L::kOffK;
   uint8_t* sV = smem + L::kOffV;
@@ -168,9 +188,10 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint64_t* k_empty = k_full + ST;
   uint64_t* v_full = k_empty + ST;
   uint64_t* v_empty = v_full + STV;
-  uint64_t* s_full = v_empty + STV;   // [2] one per query tile
-  uint64_t* p_ready = s_full + 2;    // [2]
-  uint64_t* o_done = p_ready + 2;    // [2]
+  uint64_t* s_full = v_empty + STV;   // [2] one per query tile; with one query tile one per score buffer
+  uint64_t* s_free = s_full + 2;      // [2] one per score buffer: its scores are in registers
+  uint64_t* p_ready = s_free + 2;     // [2] one per query tile
+  uint64_t* o_done = p_ready + 2;     // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);
 
@@ -242,7 +263,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
   auto active = [&](int t, int j) {
     if constexpr (kSparse) return j >= 0 && ((sp_keep[t * kMaxTileWords + (j >> 5)] >> (j & 31)) & 1u) != 0;
-    else return j >= j_lo[t] && j < j_hi[t];
+    else return t == 0 ? (j >= j_lo[0] && j < j_hi[0]) : (j >= j_lo[1] && j < j_hi[1]);
   };
 
   // ---------------- setup ----------------
@@ -260,15 +281,12 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int c = 0; c < DV / 64; ++c)
       tma_load_rows(sV + st * L::kVBytes + c * (BN * 128), &tmV, &v_full[st], c * 64, j * BN, h / p.kv_group, b, p.ov);
   };
-  auto load_k = [&](int i) { load_k_tile(i, j_min + i); };
-  auto load_v = [&](int i) { load_v_tile(i, j_min + i); };
   auto load_q = [&](int t) {
     mbar_arrive_expect_tx(&q_full[t], L::kQBytes);
     for (int c = 0; c < D / 64; ++c)
       tma_load_rows(sQ + t * L::kQBytes + c * (BM * 128), &tmQ, &q_full[t], c * 64, m0 + t * BM, h, b, p.oq);
   };
-  bool early_loads = false;
-  if (warp == kTmaWarp && lane == 0) {
+  if (warp == kKWarp && lane == 0) {
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
@@ -284,25 +302,31 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     for (int t = 0; t < 2; ++t) {
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_ready[t], 128);
+      mbar_init(&s_free[t], 4 * RT);
+      mbar_init(&p_ready[t], 4 * RT);
       mbar_init(&o_done[t], 1);
     }
     fence_barrier_init();
     if (n_max > 0 && !kSparse) {
       // in the order of first use: query tile 0 and K so that its scores can start, then query tile 1, then V
-      const int nq = act1 ? 2 : 1;
-      load_q(0);
-      load_k(0);
-      if (nq > 1) load_q(1);
-      load_v(0);
-      early_loads = true;
+      if (act0) load_q(0);
+      load_k_tile(0, j_min);
+      if (act1) load_q(1);
+      load_v_tile(0, j_min);
     }
   }
   // The device status word (set by a CTA whose wait ran out) is read by another thread meanwhile: a global-memory
   // round trip that the first loads do not wait for.  If it is set, nobody consumes those loads and the teardown
   // below gives them time to land.
-  if (threadIdx.x == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
-  if (warp == kMmaWarp) {
+  if (threadIdx.x == 0) {
+    *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    // the operand tiles use the 128-byte swizzle, whose pattern repeats every 1024 bytes of the shared window
+    if ((smem_u32(smem) & 1023u) != 0) {
+      *abort_flag = 1;
+      atomicCAS(p.status, 0, kStatusTimeoutBase + kSiteSmemAlign);
+    }
+  }
+  if (warp == kQkWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
@@ -311,158 +335,132 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  if (warp == kTmaWarp) {
-    // =============== TMA producer ===============
+  // the steps of the walk: `body(i, j)` for the i-th KV tile j of the union, until it returns false
+  auto for_steps = [&](auto&& body) {
     if constexpr (kSparse) {
-      if (lane == 0 && n_max > 0 && !*abort_flag) {
-        TileWalk walk(sp_keep, sp_keep + kMaxTileWords, p.tile_words);
-        load_q(0);
-        if (NT > 1 && act1) load_q(1);
-        for (int i = 0; i < n_max; ++i) {
-          const int j = walk.next();
-          const int st = i % ST;
-          const uint32_t ph = (i / ST) & 1;
-          if (i >= ST && !mbar_wait(&k_empty[st], ph ^ 1, ab, kSiteKEmpty)) break;
-          load_k_tile(i, j);
-          if (i >= STV && !mbar_wait(&v_empty[i % STV], ((i / STV) & 1) ^ 1, ab, kSiteVEmpty)) break;
-          load_v_tile(i, j);
-        }
-      }
-    } else if (lane == 0 && early_loads && !*abort_flag) {
-      for (int i = 1; i < n_max; ++i) {
-        const int st = i % ST;
-        const uint32_t ph = (i / ST) & 1;
-        if (!mbar_wait(&k_empty[st], ph ^ 1, ab, kSiteKEmpty)) break;
-        load_k(i);
-        if (!mbar_wait(&v_empty[i % STV], ((i / STV) & 1) ^ 1, ab, kSiteVEmpty)) break;
-        load_v(i);
-      }
+      TileWalk walk(sp_keep, sp_keep + kMaxTileWords, p.tile_words);
+      for (int i = 0; i < n_max; ++i)
+        if (!body(i, walk.next())) break;
+    } else {
+      for (int i = 0; i < n_max; ++i)
+        if (!body(i, j_min + i)) break;
     }
-  } else if (warp == kMmaWarp) {
-    // =============== MMA issuer ===============
-    // The whole warp runs this code converged; one elected lane issues each batch of MMAs with its commit.  The
+  };
+  if (warp == kKWarp) {
+    // =============== loads of Q and K ===============
+    if (lane == 0 && n_max > 0 && !*abort_flag) {
+      for_steps([&](int i, int j) {
+        if (i == 0) {
+          if constexpr (kSparse) {
+            if (act0) load_q(0);
+            load_k_tile(0, j);
+            if (act1) load_q(1);
+          }
+          return true;   // otherwise on their way since before the CTA-wide sync
+        }
+        if (i >= ST && !mbar_wait(&k_empty[i % ST], ((i / ST) & 1) ^ 1, ab, kSiteKEmpty)) return false;
+        load_k_tile(i, j);
+        return true;
+      });
+    }
+  } else if (warp == kVWarp) {
+    // =============== loads of V ===============
+    if (lane == 0 && n_max > 0 && !*abort_flag) {
+      for_steps([&](int i, int j) {
+        if (i == 0 && !kSparse) return true;
+        if (i >= STV && !mbar_wait(&v_empty[i % STV], ((i / STV) & 1) ^ 1, ab, kSiteVEmpty)) return false;
+        load_v_tile(i, j);
+        return true;
+      });
+    }
+  } else if (warp == kQkWarp || warp == kPvWarp) {
+    // =============== MMA issuers: one warp for Q.K^T, one for P.V ===============
+    // Each warp runs its loop converged; one elected lane issues each batch of MMAs with its commits.  The
     // descriptors then live in uniform registers and a batch leaves at the tensor pipe's rate whatever the functor
     // warps do: issued from inside an `if (lane == 0)` region an MMA with N = 128 took ~90 cycles beside busy warps,
-    // against the 64 the pipe needs for it.
+    // against the 64 the pipe needs for it.  A batch occupies its warp until the pipe has nearly done with it, so what
+    // a warp does between two batches (barriers, tile bookkeeping: 400-600 cycles beside the functor warps) is time
+    // without MMAs unless the other warp's are queued: one warp for both products took 4950 cycles a pair-step.
     if (n_max > 0 && __all_sync(0xffffffffu, !*abort_flag)) {
       auto wait = [&](uint64_t* bar, uint32_t parity, int site) -> bool {
         return __all_sync(0xffffffffu, mbar_wait(bar, parity, ab, site));
       };
-      auto wait_poll = [&](uint64_t* bar, uint32_t parity, int site) -> bool {
-        return __all_sync(0xffffffffu, mbar_wait_poll(bar, parity, ab, site));
-      };
-      auto commit2 = [&](uint64_t* c1, uint64_t* c2) {
-        if (elect_one()) {
-          umma_commit(c1);
-          if (c2 != nullptr) umma_commit(c2);
-        }
-      };
-      constexpr uint32_t idesc_qk = make_idesc_f16(BM, BN, kBf16, false, false);
-      constexpr uint32_t idesc_pv = make_idesc_f16(BM, DV, kBf16, false, true);
       // Descriptors are built once; per MMA only the start-address field moves (units of 16 bytes), and four
-      // K steps go out per asm block: the issuing lane's instruction count is latency in front of the tensor pipe.
-      const uint64_t q_desc0 = make_smem_desc(smem_u32(sQ), 16, 1024);
-      const uint64_t k_desc0 = make_smem_desc(smem_u32(sK), 16, 1024);
-      const uint64_t v_desc0 = make_smem_desc(smem_u32(sV), BN * 128, 1024);
-      auto issue_qk = [&](int t, int st) {
-        const uint64_t a = q_desc0 + static_cast<uint64_t>(t * (L::kQBytes >> 4));
-        const uint64_t bq = k_desc0 + static_cast<uint64_t>(st * (L::kKBytes >> 4));
-        if (elect_one()) {
+      // K steps go out per asm block.
+      if (warp == kQkWarp) {
+        constexpr uint32_t idesc_qk = make_idesc_f16(BM, BN, kBf16, false, false);
+        const uint64_t q_desc0 = make_smem_desc(smem_u32(sQ), 16, 1024);
+        const uint64_t k_desc0 = make_smem_desc(smem_u32(sK), 16, 1024);
+        int n = 0, own[2] = {0, 0};   // score tiles issued: all, and per query tile
+        for_steps([&](int i, int j) {
+          const int st = i % ST;
+          if (!wait(&k_full[st], (i / ST) & 1, kSiteKFull)) return false;
 #pragma unroll
-          for (int ch = 0; ch < D / 64; ++ch)
-            umma_ss_x4<2, 2>(tmem_base + kColS + t * BN, a + ch * ((BM * 128) >> 4), bq + ch * ((BN * 128) >> 4), idesc_qk, ch > 0 ? 1u : 0u);
-          umma_commit(&s_full[t]);
-        }
-      };
-      auto issue_pv = [&](int t, int st, bool first) {
-        const uint64_t bv = v_desc0 + static_cast<uint64_t>(st * (L::kVBytes >> 4));
-        if (elect_one()) {
-#pragma unroll
-          for (int g = 0; g < BN / 64; ++g)   // 16 KV rows (2048 B) per K step, P advances 8 TMEM columns
-            umma_ts_x4<8, 128>(tmem_base + kColO + t * DV, tmem_base + kColS + t * BN + g * 32, bv + g * 512, idesc_pv,
-                               (!first || g > 0) ? 1u : 0u);
-          umma_commit(&o_done[t]);
-        }
-      };
-      bool ok = wait(&q_full[0], 0, kSiteQFull);
-      ok = ok && wait(&k_full[0], 0, kSiteKFull);
-      if constexpr (kSparse) {
-        // the same schedule over the union of the two tiles' KV tile sets; a tile takes part in a step when the
-        // step's KV tile is in its own set, and its barrier phases count its own tiles
-        TileWalk walk(sp_keep, sp_keep + kMaxTileWords, p.tile_words);
-        int j = walk.next();
-        int done[2] = {0, 0};
-        if (ok) {
-          tc_fence_after_sync();
-          if (active(0, j)) issue_qk(0, 0);
-          if (NT > 1 && act1) {
-            ok = wait(&q_full[1], 0, kSiteQFull);
+          for (int t = 0; t < NT; ++t) {
+            if (!active(t, j)) continue;
+            if (own[t] == 0 && !wait(&q_full[t], 0, kSiteQFull)) return false;
+            // the scores that were in this buffer before have left it for registers
+            const int buf = NSB == 1 ? 0 : (NT == 1 ? n & 1 : t);
+            const int use = NSB == 1 ? n : (NT == 1 ? n >> 1 : own[t]);
+            if (use > 0 && !wait(&s_free[buf], (use - 1) & 1, kSiteSFree)) return false;
             tc_fence_after_sync();
-            if (ok && active(1, j)) issue_qk(1, 0);
-          }
-          commit2(&k_empty[0], nullptr);
-        }
-        for (int i = 0; i < n_max && ok; ++i) {
-          const int jn = walk.next();
-          const int st = i % STV;
-          const int stn = (i + 1) % ST;
-          ok = wait(&v_full[st], (i / STV) & 1, kSiteVFull);
-          if (ok && jn >= 0) ok = wait(&k_full[stn], ((i + 1) / ST) & 1, kSiteKFull);
-          if (!ok) break;
-          for (int t = 0; t < NT; ++t) {
-            if (active(t, j)) {
-              ok = wait_poll(&p_ready[t], done[t] & 1, kSitePReady);
-              if (!ok) break;
-              tc_fence_after_sync();
-              issue_pv(t, st, done[t] == 0);
-              ++done[t];
+            const uint64_t a = q_desc0 + static_cast<uint64_t>(t * (L::kQBytes >> 4));
+            const uint64_t bq = k_desc0 + static_cast<uint64_t>(st * (L::kKBytes >> 4));
+            const bool last = t == NT - 1 || !active(1, j);
+            if (elect_one()) {
+#pragma unroll
+              for (int ch = 0; ch < D / 64; ++ch)
+                umma_ss_x4<2, 2>(tmem_base + kColS + buf * BN, a + ch * ((BM * 128) >> 4), bq + ch * ((BN * 128) >> 4), idesc_qk,
+                                 ch > 0 ? 1u : 0u);
+              umma_commit(&s_full[NT == 1 ? n & 1 : t]);
+              if (last) umma_commit(&k_empty[st]);   // the step's last scores: its K tile may be overwritten behind them
             }
-            if (active(t, jn)) issue_qk(t, stn);
+            ++n;
+            ++own[t];
           }
-          if (!ok) break;
-          commit2(&v_empty[st], jn >= 0 ? &k_empty[stn] : nullptr);
-          j = jn;
-        }
-      } else if (ok) {
-        tc_fence_after_sync();
-        if (active(0, j_min)) issue_qk(0, 0);
-        if (NT > 1 && act1) {
-          ok = wait(&q_full[1], 0, kSiteQFull);
-          tc_fence_after_sync();
-          if (ok && active(1, j_min)) issue_qk(1, 0);
-        }
-        commit2(&k_empty[0], nullptr);
-        for (int i = 0; i < n_max && ok; ++i) {
-          const int j = j_min + i;
+          return true;
+        });
+      } else {
+        constexpr uint32_t idesc_pv = make_idesc_f16(BM, DV, kBf16, false, true);
+        const uint64_t v_desc0 = make_smem_desc(smem_u32(sV), BN * 128, 1024);
+        int own[2] = {0, 0};
+        for_steps([&](int i, int j) {
           const int st = i % STV;
-          const int stn = (i + 1) % ST;
-          ok = wait(&v_full[st], (i / STV) & 1, kSiteVFull);
-          if (ok && i + 1 < n_max) ok = wait(&k_full[stn], ((i + 1) / ST) & 1, kSiteKFull);
-          if (!ok) break;
+          if (!wait(&v_full[st], (i / STV) & 1, kSiteVFull)) return false;
+          const uint64_t bv = v_desc0 + static_cast<uint64_t>(st * (L::kVBytes >> 4));
+#pragma unroll
           for (int t = 0; t < NT; ++t) {
-            if (active(t, j)) {
-              // on the serial chain of the tile: polled, a suspended wait wakes up ~150 cycles late
-              ok = wait_poll(&p_ready[t], (j - j_lo[t]) & 1, kSitePReady);
-              if (!ok) break;
-              tc_fence_after_sync();
-              issue_pv(t, st, j == j_lo[t]);
+            if (!active(t, j)) continue;
+            if (!wait(&p_ready[t], own[t] & 1, kSitePReady)) return false;
+            tc_fence_after_sync();
+            const bool last = t == NT - 1 || !active(1, j);
+            if (elect_one()) {
+#pragma unroll
+              for (int g = 0; g < BN / 64; ++g)   // 16 KV rows (2048 B) per K step, P advances 8 TMEM columns
+                umma_ts_x4<8, 128>(tmem_base + kColO + t * DV, tmem_base + kColP + t * (BN / 2) + g * 32, bv + g * 512, idesc_pv,
+                                   (own[t] > 0 || g > 0) ? 1u : 0u);
+              umma_commit(&o_done[t]);
+              if (last) umma_commit(&v_empty[st]);
             }
-            // the tile's next scores; also its first ones when its KV range starts later than the other tile's
-            if (active(t, j + 1)) issue_qk(t, stn);
+            ++own[t];
           }
-          if (!ok) break;
-          commit2(&v_empty[st], i + 1 < n_max ? &k_empty[stn] : nullptr);
-        }
+          return true;
+        });
       }
     }
   } else {
-    // =============== functor stage: one query row per thread ===============
-    const int t = warp >> 2;
+    // =============== functor stage: RT threads per query row, TC of its columns each ===============
+    const int t = warp / (4 * RT);
+    const int half = RT == 1 ? 0 : (warp >> 2) & 1;
     const int row = (warp & 3) * 32 + lane;
     const int q_idx = m0 + t * BM + row;
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem_base + lane_base + kColS + t * BN;
-    const uint32_t tO = tmem_base + lane_base + kColO + t * DV;
+    const uint32_t tS = tmem_base + lane_base + kColS + (NSB == 2 && NT == 2 ? t * BN : 0) + half * TC;
+    const uint32_t tP = tmem_base + lane_base + kColP + t * (BN / 2) + half * (TC / 2);
+    constexpr int OC = DV / RT;   // output columns per thread
+    const uint32_t tO = tmem_base + lane_base + kColO + t * DV + half * OC;
+    const int pair_bar = 1 + t * 4 + (warp & 3);   // named barrier of the two warps that share rows
+    float* xch = reinterpret_cast<float*>(smem + L::kOffExchange) + t * 2 * BM + row;
     const int n = kSparse ? n_tiles[t] : j_hi[t] - j_lo[t];
     const int row0 = m0 + t * BM;
     TileWalk walk(sp_keep + t * kMaxTileWords, nullptr, kSparse ? p.tile_words : 0);
@@ -470,18 +468,33 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     float rs[F::kRowScales > 0 ? F::kRowScales : 1];
     RowCtx ctx{b, h, q_idx, 0, p.seq_q, p.seq_kv, &p.fa};
     F::init(rs, ctx);
-    bool ok = (n > 0) && !*abort_flag;
-    for (int j = 0; j < n && ok; ++j) {   // j counts this query tile's own KV tiles
-      ok = mbar_wait(&s_full[t], j & 1, ab, kSiteSFull);
-      if (!ok) break;
+    // Where two warps share rows they leave this loop together: each passes what it knows through the exchange of the
+    // row maxima, and one that has given up a wait goes on to the next exchange, so that its partner never waits there alone.
+    constexpr bool kPairs = functor_split_sum<F>::value;
+    bool ok = !*abort_flag;
+    for (int j = 0; j < n && (kPairs || ok); ++j) {   // j counts this query tile's own KV tiles
+      const int buf = NSB == 1 ? 0 : (NT == 1 ? j & 1 : t);
+      ok = ok && (NT == 1 ? mbar_wait(&s_full[buf], (j >> 1) & 1, ab, kSiteSFull) : mbar_wait(&s_full[t], j & 1, ab, kSiteSFull));
+      if (!kPairs && !ok) break;
       tc_fence_after_sync();
-      float s[BN];
+      float s[TC];
 #pragma unroll
-      for (int c = 0; c < BN / 32; ++c) tmem_ld32f(tS + c * 32, &s[c * 32]);
+      for (int c = 0; c < TC / 32; ++c) tmem_ld32f(tS + (NT == 1 ? buf * BN : 0) + c * 32, &s[c * 32]);
       tmem_wait_ld();
+      // the scores are in registers: their buffer may take the next ones
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s_free[buf]);
+      // before P is written: the P.V that reads this tile's previous P (and whose sum a rescale would touch) is done
+      auto p_free = [&]() {
+        if (j > 0) {
+          ok = ok && mbar_wait(&o_done[t], (j - 1) & 1, ab, kSiteODone);
+          tc_fence_after_sync();
+        }
+      };
       const int jt = kSparse ? walk.next() : j_lo[t] + j;   // KV tile of this step
       const int kv0 = jt * BN;
-      ctx.kv0 = kv0;
+      ctx.kv0 = kv0 + half * TC;
       if constexpr (kSparse) {
         // element mask of a partial tile: 128 keep bits for this thread's row (or one column mask for all rows)
         if (F::kNegInfMask && ((sp_part[t * kMaxTileWords + (jt >> 5)] >> (jt & 31)) & 1u) != 0) {
@@ -493,10 +506,15 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const int n_kv = (p.seq_kv + BN - 1) / BN;
             mrow = p.elem_mask + ((static_cast<long long>(sp_row[t]) / ((p.seq_q + BM - 1) / BM)) * n_kv + jt) * 4;
           }
-          const uint4 mw = *reinterpret_cast<const uint4*>(mrow);
-          const uint32_t words[4] = {mw.x, mw.y, mw.z, mw.w};
+          uint32_t words[TC / 32];
 #pragma unroll
-          for (int i = 0; i < BN; ++i) s[i] = ((words[i >> 5] >> (i & 31)) & 1u) ? s[i] : -INFINITY;
+          for (int i = 0; i < TC / 32; i += 2) {
+            const uint2 mw = *reinterpret_cast<const uint2*>(mrow + half * (TC / 32) + i);
+            words[i] = mw.x;
+            words[i + 1] = mw.y;
+          }
+#pragma unroll
+          for (int i = 0; i < TC; ++i) s[i] = ((words[i >> 5] >> (i & 31)) & 1u) ? s[i] : -INFINITY;
         }
       }
       // a tile needs element masking when it crosses an edge of the mask band or the end of the KV sequence
@@ -507,100 +525,113 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int kv_first = left < kNoBound ? q_idx - left : -kNoBound;
           const int kv_last = right < kNoBound ? min(q_idx + right, p.seq_kv - 1) : p.seq_kv - 1;
 #pragma unroll
-          for (int i = 0; i < BN; ++i) {
-            const int kv = kv0 + i;
+          for (int i = 0; i < TC; ++i) {
+            const int kv = kv0 + half * TC + i;
             const bool keep = (kv >= kv_first) && (kv <= kv_last);
             s[i] = keep ? s[i] : -INFINITY;
           }
         }
       }
-      // P (16-bit, two per column) overwrites the first BN/2 columns of S
+      // P: 16-bit, two per column, in columns of its own
       auto store_half = [&](int c) {
         uint32_t pk[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) pk[i] = pack2<kBf16>(s[c * 64 + 2 * i], s[c * 64 + 2 * i + 1]);
-        tmem_st32(tS + c * 32, pk);
+        tmem_st32(tP + c * 32, pk);
       };
       float o_scale;
-      if constexpr (functor_half_store<F>::value && BN == 128) {
-        // the functor hands over a piece of the row (BN / kPieces columns) as soon as its probabilities are final: the
-        // piece is on its way to tensor memory while the exponentials of the next one run
-        o_scale = F::template tile_pieces<BN>(s, rs, ctx, [&](int c) {
-          constexpr int W = BN / F::kPieces / 2;   // packed columns per piece
-          uint32_t pk[W];
+      bool both_ok = true;
+      if constexpr (kPairs) {
+        // the functor hands over a piece of the row (32 columns) as soon as its probabilities are final: the piece is on
+        // its way to tensor memory while the exponentials of the next one run
+        auto row_max = [&](float mx) {   // two buffers in turn: the partner may still read the last step's
+          float* x = xch + (L::kExchangeSteps == 2 ? (j & 1) * (NT * 2 * BM) : 0);
+          x[half * BM] = mx;
+          ok = named_sync_and(pair_bar, 64, ok);
+          both_ok = ok;
+          mx = fmaxf(mx, x[(half ^ 1) * BM]);
+          if constexpr (L::kExchangeSteps == 1) named_sync(pair_bar, 64);
+          return mx;
+        };
+        o_scale = F::template tile_pieces<TC, TC / 32>(s, rs, ctx, row_max, [&](int c) {
+          if (c == 0) p_free();
+          uint32_t pk[16];
 #pragma unroll
-          for (int i = 0; i < W; ++i) pk[i] = pack2<kBf16>(s[c * 2 * W + 2 * i], s[c * 2 * W + 2 * i + 1]);
-          if constexpr (W == 32) tmem_st32(tS + c * W, reinterpret_cast<const uint32_t(&)[32]>(pk));
-          else if constexpr (W == 16) tmem_st16(tS + c * W, pk);
-          else tmem_st8(tS + c * W, pk);
+          for (int i = 0; i < 16; ++i) pk[i] = pack2<kBf16>(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]);
+          tmem_st16(tP + c * 16, pk);
         });
-      } else if constexpr (F::kUnitOScale && BN == 128) {
-        // no rescale: the row can be handed to the functor as four narrower tiles, each stored as soon as it is done
+      } else if constexpr (F::kUnitOScale) {
+        // no rescale: the row can be handed to the functor as narrower tiles, each stored as soon as it is done
         o_scale = 1.0f;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          ctx.kv0 = kv0 + c * 32;
+        for (int c = 0; c < TC / 32; ++c) {
+          ctx.kv0 = kv0 + half * TC + c * 32;
           F::template tile<32>(reinterpret_cast<float(&)[32]>(s[c * 32]), rs, ctx);
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = pack2<kBf16>(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]);
-          tmem_st16(tS + c * 16, pk);
+          if (c == 0) p_free();
+          tmem_st16(tP + c * 16, pk);
         }
-        ctx.kv0 = kv0;
       } else {
-        o_scale = F::template tile<BN>(s, rs, ctx);
+        o_scale = F::template tile<TC>(s, rs, ctx);
+        p_free();
 #pragma unroll
-        for (int c = 0; c < BN / 64; ++c) store_half(c);
+        for (int c = 0; c < TC / 64; ++c) store_half(c);
       }
+      if (kPairs && !both_ok) break;
       if (!F::kUnitOScale && j > 0) {
         const bool need = (o_scale != 1.0f);
         if (__any_sync(0xffffffffu, need)) {
-          ok = mbar_wait(&o_done[t], (j - 1) & 1, ab, kSiteODone);
-          if (ok) {
-            tc_fence_after_sync();
 #pragma unroll
-            for (int c = 0; c < DV / 32; ++c) {
-              float o[32];
-              tmem_ld32f(tO + c * 32, o);
-              tmem_wait_ld();
+          for (int c = 0; c < OC / 32; ++c) {
+            float o[32];
+            tmem_ld32f(tO + c * 32, o);
+            tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] *= o_scale;
-              tmem_st32f(tO + c * 32, o);
-            }
+            for (int i = 0; i < 32; ++i) o[i] *= o_scale;
+            tmem_st32f(tO + c * 32, o);
           }
         }
       }
       tmem_wait_st();
       tc_fence_before_sync();
-      mbar_arrive(&p_ready[t]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&p_ready[t]);
     }
     // a query tile of a sparse walk that visits no KV tile at all still owes its output rows: the epilogue of an
     // empty accumulator (what the reference's kernel leaves there as well)
-    const bool empty_tile = kSparse && n == 0 && t < NT && row0 < p.seq_q && !*abort_flag;
-    if ((ok && n > 0) || empty_tile) {
-      ok = n > 0 ? mbar_wait(&o_done[t], (n - 1) & 1, ab, kSiteOFinal) : true;
+    const bool empty_tile = kSparse && n == 0 && row0 < p.seq_q;
+    if (n > 0 || empty_tile) {
+      if (n > 0) ok = ok && mbar_wait(&o_done[t], (n - 1) & 1, ab, kSiteOFinal);
+      if constexpr (kPairs) {   // the row's sum from its two threads' parts
+        float* x = xch + (L::kExchangeSteps == 2 ? (n & 1) * (NT * 2 * BM) : 0);   // not the buffer of the last exchange
+        x[half * BM] = rs[F::kSplitSum];
+        ok = named_sync_and(pair_bar, 64, ok);
+        rs[F::kSplitSum] += x[(half ^ 1) * BM];
+      }
       if (ok) {
         tc_fence_after_sync();
         const bool in_range = q_idx < p.seq_q;
-        float o[DV];
+        float o[OC];
         if (n > 0) {
 #pragma unroll
-          for (int c = 0; c < DV / 32; ++c) tmem_ld32f(tO + c * 32, &o[c * 32]);
+          for (int c = 0; c < OC / 32; ++c) tmem_ld32f(tO + c * 32, &o[c * 32]);
           tmem_wait_ld();
         } else {
 #pragma unroll
-          for (int i = 0; i < DV; ++i) o[i] = 0.0f;
+          for (int i = 0; i < OC; ++i) o[i] = 0.0f;
         }
-        F::template epilogue<DV>(o, rs, ctx);
+        F::template epilogue<OC>(o, rs, ctx);
         if (p.kv_splits > 1) {
           // split-KV: the normalised rows and their log-sum-exp go to the scratch the combine kernel reads
           if (in_range) {
             const long long prow = ((static_cast<long long>(b) * p.kv_splits + split) * p.heads + h) * p.seq_q + q_idx;
-            float4* dst = reinterpret_cast<float4*>(p.part_o + prow * DV);
+            float4* dst = reinterpret_cast<float4*>(p.part_o + prow * DV + half * OC);
 #pragma unroll
-            for (int v = 0; v < DV / 4; ++v) dst[v] = make_float4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
+            for (int v = 0; v < OC / 4; ++v) dst[v] = make_float4(o[4 * v], o[4 * v + 1], o[4 * v + 2], o[4 * v + 3]);
 #pragma unroll
-            for (int i = 0; i < F::kFinal; ++i) p.part_final[i * p.part_final_stride + prow] = F::final_rowscale(i, rs, ctx);
+            for (int i = 0; i < (half == 0 ? F::kFinal : 0); ++i) p.part_final[i * p.part_final_stride + prow] = F::final_rowscale(i, rs, ctx);
           }
         } else {
           // Output rows leave through the tile's own Q buffer (free: its last Q.K^T ran before the P.V that o_done
@@ -609,10 +640,10 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           // contiguous bytes per row and 512 bytes per instruction.  A thread storing its own row put 32 pieces
           // into 32 different rows with every instruction, and the tile's last output took ~3100 cycles.
           static_assert(DV <= D, "the output tile is staged in the query tile's buffer");
-          constexpr int PR = DV / 8;     // 16-byte pieces per row
+          constexpr int PR = OC / 8;     // 16-byte pieces of a row's columns
           constexpr int RPI = 32 / PR;   // rows per warp instruction
-          const uint32_t stage = smem_u32(sQ + t * L::kQBytes) + (warp & 3) * (32 * DV * 2);
-          const uint32_t mine = stage + lane * (DV * 2);
+          const uint32_t stage = smem_u32(sQ + t * L::kQBytes) + ((warp & 3) * RT + half) * (32 * OC * 2);
+          const uint32_t mine = stage + lane * (OC * 2);
 #pragma unroll
           for (int v = 0; v < PR; ++v) {
             uint4 pk;
@@ -626,12 +657,12 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int c = lane & (PR - 1), rsub = lane / PR;
           const int row_first = row0 + (warp & 3) * 32;
           uint8_t* obase = reinterpret_cast<uint8_t*>(p.o) +
-                           2 * (static_cast<long long>(b) * p.o_sb + static_cast<long long>(h) * p.o_sh) + c * 16;
+                           2 * (static_cast<long long>(b) * p.o_sb + static_cast<long long>(h) * p.o_sh + half * OC) + c * 16;
           uint4 val[PR];   // all loads first, then all stores: one after the other each pair costs a shared-memory round trip
 #pragma unroll
           for (int i = 0; i < PR; ++i) {
             const int r = i * RPI + rsub;
-            val[i] = ld_shared_v4(stage + r * (DV * 2) + ((c ^ (r & (PR - 1))) << 4));
+            val[i] = ld_shared_v4(stage + r * (OC * 2) + ((c ^ (r & (PR - 1))) << 4));
           }
 #pragma unroll
           for (int i = 0; i < PR; ++i) {
@@ -640,7 +671,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               *reinterpret_cast<uint4*>(obase + 2 * static_cast<long long>(row_first + r) * p.o_ss) = val[i];
           }
         }
-        if (in_range && p.kv_splits <= 1) {
+        if (in_range && half == 0 && p.kv_splits <= 1) {
 #pragma unroll
           for (int i = 0; i < F::kFinal; ++i) {
             if (p.final_out[i] != nullptr) {
@@ -653,8 +684,8 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   }
 
   // a split whose share of the KV tiles is empty for a query tile contributes nothing
-  if (p.kv_splits > 1 && warp < 4 * NT) {
-    const int t = warp >> 2;
+  if (p.kv_splits > 1 && warp < 4 * NT * RT) {
+    const int t = warp / (4 * RT);
     const int q_idx = m0 + t * BM + (warp & 3) * 32 + lane;
     if (j_hi[t] <= j_lo[t] && q_idx < p.seq_q)
       p.part_final[((static_cast<long long>(b) * p.kv_splits + split) * p.heads + h) * p.seq_q + q_idx] = -INFINITY;
@@ -669,7 +700,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < 200; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == kMmaWarp) {
+  if (warp == kQkWarp) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_base, kTmemCols);
   }

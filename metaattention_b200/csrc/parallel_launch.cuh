@@ -181,7 +181,7 @@ int launch_parallel(const AttnB200ParallelArgs* a, cudaStream_t stream, int* dev
     return ATTN_B200_E_LAUNCH;
   }
   dim3 grid((a->seq_q + NT * L::kBM - 1) / (NT * L::kBM), a->heads, a->batch * splits);
-  kernel<<<grid, (4 * NT + 2) * 32, kSmem, stream>>>(tmQ, tmK, tmV, p);
+  kernel<<<grid, kParallelThreads<NT, kRowThreads<F>>, kSmem, stream>>>(tmQ, tmK, tmV, p);
   if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
   if (splits > 1) {
     const long long rows = static_cast<long long>(a->batch) * a->heads * a->seq_q;

@@ -598,3 +598,45 @@ def test_decode_tiles_entry_point():
         for h in range(Hkv):
             assert [(int(kept_words[b, h]) >> j) & 1 for j in range(8)] == [int(x) for x in any_[b, h]]
             assert [(int(part_words[b, h]) >> j) & 1 for j in range(8)] == [int(x and not y) for x, y in zip(any_[b, h], all_[b, h])]
+
+
+@pytest.mark.parametrize("B,H,Hkv,Sq,Skv,D,Dv,causal", [
+    (1, 2, 1, 640, 640, 64, 64, True),      # a score buffer per query tile
+    (1, 2, 2, 1030, 1030, 128, 128, False), # one score buffer for both; ragged, nine KV tiles
+    (1, 1, 1, 1, 900, 192, 128, False),     # one row, second query tile absent
+    (1, 2, 2, 700, 700, 192, 128, True),    # one exchange buffer
+    (1, 1, 1, 700, 700, 256, 256, True),    # one query tile to a CTA, two score buffers in turn
+])
+def test_row_maxima_that_move_between_the_threads_of_a_row(B, H, Hkv, Sq, Skv, D, Dv, causal):
+    """The largest score of a row grows from KV tile to KV tile and sits in the lower or the upper 64 columns of a tile in
+    turn: the two threads of a row exchange it, and accumulator and sums are rescaled on almost every tile.  Logits reach
+    +-60, where bf16 operands leave the fp32 reference's own products exact; the tolerance is that of P's rounding."""
+    gen = torch.Generator().manual_seed(Sq + Skv + D)
+    q = torch.randn(B, Sq, H, D, generator=gen) * 0.05
+    q[..., 0] = 8.0
+    k = torch.randn(B, Skv, Hkv, D, generator=gen) * 0.05
+    pos = torch.arange(Skv)
+    peak = torch.where(pos // 128 % 2 == 0, 3, 100)                 # lower half in even tiles, upper half in odd ones
+    k[:, :, :, 0] = (torch.where(pos % 128 == peak, 6.0 * (pos // 128 + 1), -4.0) * D ** 0.5 / 8.0)[None, :, None]
+    v = torch.randn(B, Skv, Hkv, Dv, generator=gen)
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    e = _engine(B, H, Hkv, Sq, Skv, D, Dv, causal)
+    o = e(*cuda(q, k, v))
+    kk, vv = (t.repeat_interleave(H // Hkv, dim=2) for t in (k, v))
+    s = torch.einsum("bqhd,bkhd->bhqk", q.float(), kk.float()) * D ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(Sq, Skv).tril() == 0, -math.inf)
+    check(o, torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), vv.float()))
+    assert (e.last_final_rowscales["lse"].cpu() - s.logsumexp(-1)).abs().max().item() < 1e-3
+
+
+def _engine(B, H, Hkv, Sq, Skv, D, Dv, causal):
+    from attn_engine import AttentionEngine
+    from core import CustomIO, meta_tensor
+
+    def score_mod(score, custom, b, h, q_idx, kv_idx):
+        return score * D ** -0.5
+    metas = (meta_tensor(B, H, Sq, D, dtype=torch.bfloat16), meta_tensor(B, Hkv, Skv, D, dtype=torch.bfloat16),
+             meta_tensor(B, Hkv, Skv, Dv, dtype=torch.bfloat16))
+    return AttentionEngine(metas, CustomIO({}), score_mod=score_mod, mask_mod=programs.causal if causal else None,
+                           online_func=programs.NaturalSoftmax())
