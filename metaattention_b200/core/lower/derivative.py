@@ -150,7 +150,7 @@ def emit_backward_functor(tr: TracedParallel, struct_name: str = "UserBwdFunctor
     p_out = {v};
     g_out = {d if d is not None else '0.0f'};
   }}
-  __device__ static float grad(float g, float dp, float, const Ctx&) {{ return dp * g; }}
+  __device__ static float grad(float g, float dp, const Ctx&) {{ return dp * g; }}
   __device__ static float out_scale(const Ctx&) {{ return 1.0f; }}
 }};
 """

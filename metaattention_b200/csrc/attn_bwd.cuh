@@ -15,18 +15,24 @@
 //   F::kNegInfMask           P and dS vanish at a score of -inf: masked pairs are given that score
 //   F::Ctx F::make(params)   per-thread constants
 //   F::score(s, lse2, ctx, b, h, q_idx, kv_idx, p_out, g_out)   P, and the factor g that turns dP into dS
-//   F::grad(g, dp, delta, ctx)                                   dS without its constant factor
+//   F::grad(g, dp, ctx)                                          dS without its constant factor; with statistics instead
+//   F::score_row, F::grad_row                                    score() for a row of an unmasked tile, and dS of a row
 //   F::out_scale(ctx)                                            the constant factor, applied to the finished dK, dQ rows
 // softmax_bwd.cu instantiates it for the built-in softmax; lowered score_mod functors (elementwise programs: no row
 // scales) get a library of their own, compiled from the forward-mode derivative of the traced expression.
 //
-// The tensor pipe executes in issue order, and both roles lean on that to keep it and the row threads busy at once:
-//   KV role   ... dV(i) | S(i+1) | dK(i) | dP(i+1) ...   row threads: P(i) from S(i), then dS(i) from dP(i)
-//             S(i+1) overwrites P(i) behind dV(i), dP(i+1) overwrites dS(i) behind dK(i); while the rows turn dP(i)
-//             into dS(i) the pipe computes dV(i) and S(i+1), while they turn S(i+1) into P(i+1) it computes dK(i)
-//             and dP(i+1).
-//   Q role    ... S(i+1), dP(i+1) | dQ(i) ...            dS sits in two buffers of its own (the role has no second
-//             accumulator), so S, dP of the next tile are issued once the rows hold this tile's in registers.
+// What bounds it: the row threads, whose phases for a tile follow one another (take S, exponentials, hand over P, take dP, dS,
+// hand over), and in long calls the power that the seven products draw.  So a tile's S and dP leave their buffers for
+// registers at once and the next ones are computed under the row threads' work, P and dS have columns of their own (over
+// S and dP each product waited for the one that read them: 3330 and 2550 cycles a tile for the KV and the query
+// role), S and dP are issued by one warp and the accumulators by another, and four threads share a row, four row warps
+// to a scheduler.  Now 3000 and 2400 cycles with D = 128 (1 x 32 x 4096 non-causal forward and backward; products alone 2048 and
+// 1536), 2400 and 1960 with D = 64; training step of 4 x 32 x 4096 x 128 causal 2775 -> 2610 us (at its power cap), of
+// 4 x 8 / 2 x 2118 x 128 237 -> 215.  In the KV role the statistics of a tile's columns come through shared memory, 256
+// sixteen-byte broadcasts a tile of ~3 cycles each beside the operands of the products (2048 cycles of its bandwidth).
+//   KV role, D = 128  S and dP take one buffer in turn: S(i+1) is issued once dP(i) is in registers, dV(i) and dK(i) behind it.
+//   Otherwise         a buffer each: S(i+1) and dP(i+1) are issued once S(i) and dP(i) are in registers.
+//   Q role            dS sits in two buffers (the role has no second accumulator).
 #pragma once
 
 #include <cstring>
@@ -40,8 +46,9 @@
 namespace b200 {
 
 constexpr int kBwdT = 128;                // rows of a tile, both ways
-constexpr int kBwdRowThreads = 256;       // eight warps: one TMEM lane each, two column halves
-constexpr int kBwdThreads = kBwdRowThreads + 64;   // plus the loading warp and the MMA-issuing warp
+constexpr int kBwdRowGroups = 4;                                // threads that share a row of a tile
+constexpr int kBwdRowWarps = kBwdRowGroups * kBwdT / 32;        // row warps: one TMEM lane and a part of the columns per thread
+constexpr int kBwdThreads = kBwdRowWarps * 32 + 96;             // plus the loading warp and two that issue MMAs
 constexpr int kBwdStages1 = 3;            // ring of Y1 (read by the first and by the last MMA of its tile)
 constexpr int kBwdStages2 = 2;            // ring of Y2
 
@@ -70,19 +77,23 @@ struct BwdParams {
   int* status;
 };
 
-enum BwdWaitSite { kBwdXFull = 61, kBwdYFull, kBwdYEmpty, kBwdSDone, kBwdPReady, kBwdAccDone, kBwdSdpFree, kBwdDpDone, kBwdDsReady, kBwdSmemAlign };
+enum BwdWaitSite { kBwdXFull = 61, kBwdYFull, kBwdYEmpty, kBwdSFull, kBwdPReady, kBwdAccDone, kBwdSFree, kBwdDpFull, kBwdDsReady, kBwdSmemAlign, kBwdDpFree, kBwdPFree, kBwdDsFree, kBwdSIssued };
 enum BwdBarrier {
   kBarXFull = 0,
   kBarY1Full,                               // kBwdStages1 of them
   kBarY1Empty = kBarY1Full + kBwdStages1,
   kBarY2Full = kBarY1Empty + kBwdStages1,   // kBwdStages2 of them
   kBarY2Empty = kBarY2Full + kBwdStages2,
-  kBarSDone = kBarY2Empty + kBwdStages2,
-  kBarDpDone,
-  kBarPReadyB,
-  kBarDsReady,
+  kBarSFull = kBarY2Empty + kBwdStages2,    // scores / dP of a tile in tensor memory, and in the row threads' registers
+  kBarSFree,
+  kBarDpFull,
+  kBarDpFree,
+  kBarPReady,                               // P of a tile in tensor memory, and read by its product (KV role)
+  kBarPFree,
+  kBarDsReady,                              // the same of dS, one per buffer of the query role
+  kBarDsFree = kBarDsReady + 2,
+  kBarSIssued = kBarDsFree + 2,             // the next tile's S is in the pipe (KV role with a shared buffer)
   kBarAccDone,
-  kBarSdpFree,
   kNumBwdBarriers
 };
 
@@ -135,16 +146,19 @@ struct KeptTiles {
 
 // kRoleQ = false: CTA = (KV tile, KV head, batch), streams the query tiles (of every query head of its group) and
 // writes dK, dV.  kRoleQ = true: CTA = (query tile, query head, batch), streams the KV tiles and writes dQ.
-// Tensor memory: S [0,128), dP [128,256), accumulator 1 [256,384) (dV or dQ), accumulator 2 [384,512) (dK; the
-// query role's two dS buffers).  KV role: P is written over S, dS over dP.
+// Tensor memory.  KV role: accumulators dV, dK (D columns each), P and dS (64 each, 16-bit pairs), then S and dP: with D = 128
+// one buffer that they take in turn, with D = 64 one each.  Query role: accumulator dQ, two dS buffers, S, dP.
 template <class F, bool kRoleQ, bool kBf16, int D, bool kBits>
 __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUtensorMap& tmK, const CUtensorMap& tmV, const CUtensorMap& tmDO,
                                              const BwdParams& p, const int tile, const int hx, const int b) {
   using L = BwdSmem<D>;
-  constexpr int T = kBwdT, KC = D / 64, HALF = D / 2;   // chunks of a tile; columns of an accumulator row per warp group
+  constexpr int T = kBwdT, KC = D / 64;   // chunks of a tile
+  constexpr int C = T / kBwdRowGroups, AC = D / kBwdRowGroups, kRowWarps = kBwdRowWarps;   // columns per thread: of a tile, of an accumulator
   constexpr int N1 = kBwdStages1, N2 = kBwdStages2;
   static_assert(D == 64 || D == 128, "head dims 64 and 128");
-  constexpr uint32_t kTmemCols = 512, kColS = 0, kColDP = 128, kColA = 256, kColB = 384, kColDS = 384;
+  constexpr bool kShared = !kRoleQ && D == 128;   // S and dP share a buffer
+  constexpr uint32_t kTmemCols = 512, kColA = 0, kColB = D, kColP = 2 * D, kColDS = kRoleQ ? 128 : 2 * D + 64, kColDP = 384,
+                     kColS = kShared ? 384 : 256;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sX1 = smem + L::kOffX1;
@@ -159,12 +173,16 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   uint64_t* y1_empty = bars + kBarY1Empty;
   uint64_t* y2_full = bars + kBarY2Full;
   uint64_t* y2_empty = bars + kBarY2Empty;
-  uint64_t* s_done = bars + kBarSDone;
-  uint64_t* dp_done = bars + kBarDpDone;
-  uint64_t* p_ready = bars + kBarPReadyB;
+  uint64_t* s_full = bars + kBarSFull;
+  uint64_t* s_free = bars + kBarSFree;
+  uint64_t* dp_full = bars + kBarDpFull;
+  uint64_t* dp_free = bars + kBarDpFree;
+  uint64_t* p_ready = bars + kBarPReady;
+  uint64_t* p_free = bars + kBarPFree;
   uint64_t* ds_ready = bars + kBarDsReady;
+  uint64_t* ds_free = bars + kBarDsFree;
+  uint64_t* s_issued = bars + kBarSIssued;
   uint64_t* acc_done = bars + kBarAccDone;
-  uint64_t* sdp_free = bars + kBarSdpFree;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kOffMisc + 8);
 
@@ -205,12 +223,18 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       mbar_init(y2_full + i, 1);
       mbar_init(y2_empty + i, 1);
     }
-    mbar_init(s_done, 1);
-    mbar_init(dp_done, 1);
-    mbar_init(p_ready, kBwdRowThreads / 32);
-    mbar_init(ds_ready, kBwdRowThreads / 32);
+    mbar_init(s_full, 1);
+    mbar_init(s_free, kRowWarps);
+    mbar_init(dp_full, 1);
+    mbar_init(dp_free, kRowWarps);
+    mbar_init(p_ready, kRowWarps);
+    mbar_init(p_free, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(ds_ready + i, kRowWarps);
+      mbar_init(ds_free + i, 1);
+    }
+    mbar_init(s_issued, 1);
     mbar_init(acc_done, 1);
-    mbar_init(sdp_free, kBwdRowThreads / 32);
     fence_barrier_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
@@ -227,7 +251,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   const uint32_t tmem_base = *tmem_slot;
   const bool start_ok = !*abort_flag;
 
-  if (warp == kBwdRowThreads / 32) {
+  if (warp == kRowWarps) {
     // ======================= loading warp =======================
     if (lane == 0 && start_ok && n_iter > 0) {
       mbar_arrive_expect_tx(x_full, 2 * L::kTileBytes);
@@ -272,90 +296,97 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         if constexpr (!kRoleQ && F::kUsesStats) bulk_load(sDelta + s2 * T, p.delta + stat_off, L::kStatBytes, y2_full + s2);
       }
     }
-  } else if (warp == kBwdRowThreads / 32 + 1) {
-    // ======================= issuing warp: every MMA =======================
-    // The whole warp runs this code converged and one elected lane issues each batch of MMAs with its commits: the
-    // descriptors then live in uniform registers, and a batch leaves at the pipe's rate whatever the row warps do
-    // (issued from inside an `if (lane == 0)` region an MMA with N = 128 took ~90 cycles under load, against the 64
-    // the pipe needs for it).
+  } else if (warp > kRowWarps) {
+    // ======================= issuing warps: one for S and dP, one for the accumulators =======================
+    // Each runs its loop converged and one elected lane issues a batch of MMAs with its commits: the descriptors then live
+    // in uniform registers, and a batch leaves at the pipe's rate whatever the row warps do (issued from inside an
+    // `if (lane == 0)` region an MMA with N = 128 took ~90 cycles under load, against the 64 the pipe needs for it).  Two
+    // warps, because a batch occupies its warp until the pipe has nearly done with it: what one warp does between its
+    // batches is covered by the other's.
     if (__all_sync(0xffffffffu, start_ok) && n_iter > 0) {
-      constexpr uint32_t idesc_kk = make_idesc_f16(T, T, kBf16, false, false);      // S, dP: both operands K-major
-      constexpr uint32_t idesc_mn = make_idesc_f16(T, D, kBf16, false, true);       // accumulators: B = streamed tile, MN-major
       constexpr uint64_t kChunk = L::kChunkBytes >> 4;
-      const uint64_t x1_desc = make_smem_desc(smem_u32(sX1), 16, 1024), x2_desc = make_smem_desc(smem_u32(sX2), 16, 1024);
       auto wait = [&](uint64_t* bar, uint32_t parity, int site) -> bool {
         return __all_sync(0xffffffffu, mbar_wait_poll(bar, parity, ab, site));
       };
-      // out = X Y^T behind the arrival of the streamed tile, then up to two commits
-      auto issue_xy = [&](uint32_t out_col, uint64_t x_desc, const uint8_t* y_tile, uint64_t* full, uint32_t parity, uint64_t* c1,
-                          uint64_t* c2) -> bool {
-        if (!wait(full, parity, kBwdYFull)) return false;
-        tc_fence_after_sync();
-        const uint64_t y_desc = make_smem_desc(smem_u32(y_tile), 16, 1024);
-        if (elect_one()) {
-#pragma unroll
-          for (int ch = 0; ch < KC; ++ch)
-            umma_ss_x4<2, 2>(tmem_base + out_col, x_desc + ch * kChunk, y_desc + ch * kChunk, idesc_kk, ch > 0 ? 1u : 0u);
-          if (c1 != nullptr) umma_commit(c1);
-          if (c2 != nullptr) umma_commit(c2);
-        }
-        return true;
-      };
-      auto issue_s = [&](int it, uint64_t* c1) -> bool {
-        return issue_xy(kColS, x1_desc, sY1 + (it % N1) * L::kTileBytes, y1_full + it % N1, (it / N1) & 1, c1, nullptr);
-      };
-      auto issue_dp = [&](int it, uint64_t* c1, uint64_t* c2) -> bool {
-        return issue_xy(kColDP, x2_desc, sY2 + (it % N2) * L::kTileBytes, y2_full + it % N2, (it / N2) & 1, c1, c2);
-      };
-      // acc += A (16-bit, tensor memory columns a_col...) x streamed tile (MN-major), then up to three commits
-      auto issue_acc = [&](uint32_t acc_col, uint32_t a_col, const uint8_t* y_tile, bool accumulate, uint64_t* c0, uint64_t* c1, uint64_t* c2) {
-        const uint64_t y_mn = make_smem_desc(smem_u32(y_tile), L::kChunkBytes, 1024);
-        if (elect_one()) {
-          if (c0 != nullptr) umma_commit(c0);   // for what was issued before this batch
-#pragma unroll
-          for (int g = 0; g < T / 64; ++g)
-            umma_ts_x4<8, 128>(tmem_base + acc_col, tmem_base + a_col + g * 32, y_mn + g * 512, idesc_mn, (accumulate || g > 0) ? 1u : 0u);
-          if (c1 != nullptr) umma_commit(c1);
-          if (c2 != nullptr) umma_commit(c2);
-        }
-      };
-      bool ok = wait(x_full, 0, kBwdXFull);
-      if constexpr (kRoleQ) {
-        ok = ok && issue_s(0, nullptr) && issue_dp(0, y2_empty, s_done);
-        for (int it = 0; ok && it < n_iter; ++it) {
-          if (it + 1 < n_iter) {
-            // the row threads hold S, dP of tile it in registers: those of tile it + 1 go ahead of tile it's dQ
-            if (!wait(sdp_free, it & 1, kBwdSdpFree)) break;
-            if (!(issue_s(it + 1, nullptr) && issue_dp(it + 1, y2_empty + (it + 1) % N2, s_done))) break;   // V is read by dP only
-          }
-          if (!wait(p_ready, it & 1, kBwdPReady)) break;
+      if (warp == kRowWarps + 1) {
+        constexpr uint32_t idesc_kk = make_idesc_f16(T, T, kBf16, false, false);      // both operands K-major
+        const uint64_t x1_desc = make_smem_desc(smem_u32(sX1), 16, 1024), x2_desc = make_smem_desc(smem_u32(sX2), 16, 1024);
+        // out = X Y^T, then up to two commits
+        auto issue_xy = [&](uint32_t out_col, uint64_t x_desc, const uint8_t* y_tile, uint64_t* c1, uint64_t* c2) {
           tc_fence_after_sync();
-          issue_acc(kColA, kColDS + (it & 1) * 64, sY1 + (it % N1) * L::kTileBytes, it > 0, nullptr, y1_empty + it % N1,
-                    it + 1 == n_iter ? acc_done : nullptr);
+          const uint64_t y_desc = make_smem_desc(smem_u32(y_tile), 16, 1024);
+          if (elect_one()) {
+#pragma unroll
+            for (int ch = 0; ch < KC; ++ch)
+              umma_ss_x4<2, 2>(tmem_base + out_col, x_desc + ch * kChunk, y_desc + ch * kChunk, idesc_kk, ch > 0 ? 1u : 0u);
+            umma_commit(c1);
+            if (c2 != nullptr) umma_commit(c2);
+          }
+        };
+        bool ok = wait(x_full, 0, kBwdXFull);
+        for (int it = 0; ok && it < n_iter; ++it) {
+          const int s1 = it % N1, s2 = it % N2;
+          if (!wait(y1_full + s1, (it / N1) & 1, kBwdYFull)) break;
+          // the buffer's last contents are in the row threads' registers.  The row threads learn from s_full and dp_full
+          // what else they need for a tile (every barrier that they look at costs them 50-200 cycles behind their
+          // exponentials): the statistics came with the tiles waited for here; query role: dS's buffer has been read
+          if (it > 0 && !(kShared ? wait(dp_free, (it - 1) & 1, kBwdDpFree) : wait(s_free, (it - 1) & 1, kBwdSFree))) break;
+          issue_xy(kColS, x1_desc, sY1 + s1 * L::kTileBytes, s_full, nullptr);
+          if (kShared && it > 0 && lane == 0) mbar_arrive(s_issued);
+          if (!wait(y2_full + s2, (it / N2) & 1, kBwdYFull)) break;
+          if constexpr (kShared) ok = wait(s_free, it & 1, kBwdSFree);
+          else ok = it == 0 || wait(dp_free, (it - 1) & 1, kBwdDpFree);
+          if (kRoleQ && ok && it >= 2) ok = wait(ds_free + (it & 1), ((it >> 1) - 1) & 1, kBwdDsFree);
+          if (!ok) break;
+          issue_xy(kColDP, x2_desc, sY2 + s2 * L::kTileBytes, dp_full, kRoleQ ? y2_empty + s2 : nullptr);   // V is read by dP only
         }
       } else {
-        ok = ok && issue_s(0, s_done) && issue_dp(0, dp_done, nullptr);
-        for (int it = 0; ok && it < n_iter; ++it) {
-          const bool more = it + 1 < n_iter;
-          if (!wait(p_ready, it & 1, kBwdPReady)) break;
+        constexpr uint32_t idesc_mn = make_idesc_f16(T, D, kBf16, false, true);       // B = streamed tile, MN-major
+        // acc += A (16-bit, tensor memory columns a_col...) x streamed tile (MN-major), then up to three commits; c0 is
+        // for what was issued before this batch
+        auto issue_acc = [&](uint32_t acc_col, uint32_t a_col, const uint8_t* y_tile, bool accumulate, uint64_t* c0, uint64_t* c1, uint64_t* c2,
+                             uint64_t* c3) {
           tc_fence_after_sync();
-          issue_acc(kColA, kColS, sY2 + (it % N2) * L::kTileBytes, it > 0, nullptr, nullptr, nullptr);    // dV += P^T dO
-          if (more && !issue_s(it + 1, s_done)) break;     // over P(it), behind dV(it) in the pipe
-          if (!wait(ds_ready, it & 1, kBwdDsReady)) break;
-          tc_fence_after_sync();
-          // dO(it) has been read by dV(it); its stage also holds delta(it), which the row threads have now used
-          issue_acc(kColB, kColDP, sY1 + (it % N1) * L::kTileBytes, it > 0, y2_empty + it % N2, y1_empty + it % N1,
-                    more ? nullptr : acc_done);   // dK += dS^T Q
-          if (more && !issue_dp(it + 1, dp_done, nullptr)) break;    // over dS(it), behind dK(it)
+          const uint64_t y_mn = make_smem_desc(smem_u32(y_tile), L::kChunkBytes, 1024);
+          if (elect_one()) {
+            if (c0 != nullptr) umma_commit(c0);
+#pragma unroll
+            for (int g = 0; g < T / 64; ++g)
+              umma_ts_x4<8, 128>(tmem_base + acc_col, tmem_base + a_col + g * 32, y_mn + g * 512, idesc_mn, (accumulate || g > 0) ? 1u : 0u);
+            umma_commit(c1);
+            if (c2 != nullptr) umma_commit(c2);
+            if (c3 != nullptr) umma_commit(c3);
+          }
+        };
+        for (int it = 0; it < n_iter; ++it) {
+          const int s1 = it % N1, s2 = it % N2;
+          uint64_t* last = it + 1 == n_iter ? acc_done : nullptr;
+          if (!wait(y1_full + s1, (it / N1) & 1, kBwdYFull)) break;
+          if constexpr (kRoleQ) {
+            if (!wait(ds_ready + (it & 1), (it >> 1) & 1, kBwdDsReady)) break;
+            issue_acc(kColA, kColDS + (it & 1) * 64, sY1 + s1 * L::kTileBytes, it > 0, nullptr, ds_free + (it & 1), y1_empty + s1, last);   // dQ += dS K
+          } else {
+            if (!wait(y2_full + s2, (it / N2) & 1, kBwdYFull)) break;
+            if (!wait(p_ready, it & 1, kBwdPReady)) break;
+            // Where S waits for the buffer that dP was taken from, the row threads wait for S while dV would do a tile later
+            // as well: it queues up behind S (in front of it: 3300 cycles a tile)
+            if (kShared && it + 1 < n_iter && !wait(s_issued, it & 1, kBwdSIssued)) break;
+            issue_acc(kColA, kColP, sY2 + s2 * L::kTileBytes, it > 0, nullptr, p_free, nullptr, nullptr);    // dV += P^T dO
+            if (!wait(ds_ready, it & 1, kBwdDsReady)) break;
+            // dO(it) has been read by dP(it) and, behind this commit, by dV(it); its stage also holds delta(it), which
+            // the row threads have now used
+            issue_acc(kColB, kColDS, sY1 + s1 * L::kTileBytes, it > 0, y2_empty + s2, ds_free, y1_empty + s1, last);   // dK += dS^T Q
+          }
         }
       }
     }
   } else {
-    // ======================= row threads: one TMEM lane each, 64 columns =======================
+    // ======================= row threads: one TMEM lane each, C columns =======================
     const int wq = warp & 3, wg = warp >> 2;
     const int row = wq * 32 + lane;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + kColS, tDP = tmem_base + lane_base + kColDP;
+    const uint32_t tP = tmem_base + lane_base + kColP, tDS = tmem_base + lane_base + kColDS;
     const typename F::Ctx fctx = F::make(p);
     float lse2_r = 0.0f, delta_r = 0.0f;
     if constexpr (kRoleQ && F::kUsesStats) {
@@ -367,17 +398,17 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
     // band keeps, for this thread's row, the columns [col_lo, col_hi] of the tile (set per streamed tile; everything
     // when no edge of the band crosses the pair); a functor whose P vanishes at a score of -inf (softmax) gets the mask
     // through the score
-    int col_lo = 0, col_hi = T;
-    uint4 keep_bits = make_uint4(0, 0, 0, 0);   // kBits: this thread's row of the streamed tile
-    auto score_of = [&](auto edge_tile, float s, float l2, int ys, int hq, int col, float& pr, float& g) {
+    int col_lo = 0, col_hi = T;   // counted from this thread's first column
+    uint32_t keep_bits = 0;       // kBits: this thread's part of its row of the streamed tile
+    auto score_of = [&](auto edge_tile, float s, float l2, int ys, int hq, int k, float& pr, float& g) {
+      const int col = wg * C + k;
       const int q_idx = kRoleQ ? tile * T + row : ys * T + col;
       const int kv_idx = kRoleQ ? ys * T + col : tile * T + row;
       bool masked;
       if constexpr (kBits) {
-        const uint32_t w = (col >> 5) == 0 ? keep_bits.x : (col >> 5) == 1 ? keep_bits.y : (col >> 5) == 2 ? keep_bits.z : keep_bits.w;
-        masked = ((w >> (col & 31)) & 1u) == 0u;
+        masked = ((keep_bits >> k) & 1u) == 0u;
       } else {
-        masked = decltype(edge_tile)::value && (col < col_lo || col > col_hi);
+        masked = decltype(edge_tile)::value && (k < col_lo || k > col_hi);
       }
       F::score((F::kNegInfMask && masked) ? -INFINITY : s, l2, fctx, b, hq, q_idx, kv_idx, pr, g);
       if (!F::kNegInfMask && masked) pr = g = 0.0f;
@@ -389,127 +420,97 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
     };
     bool ok = start_ok;
     KeptTiles kept(tiles_row, tiles_words);
+    int next_i = 0, next_hq = kRoleQ ? hx : hx * p.kv_group;   // without a division per tile: rows are the serial chain
     for (int it = 0; ok && it < n_iter; ++it) {
       // the streamed tile index, its query head, and whether an edge of the band crosses this pair of tiles
-      const int ys = walk_tiles ? kept.next() : (kRoleQ ? j0 + it : i0 + it % max(per_head, 1));
-      const int hq = kRoleQ ? hx : hx * p.kv_group + it / max(per_head, 1);
+      const int ys = walk_tiles ? kept.next() : (kRoleQ ? j0 : i0) + next_i;
+      const int hq = next_hq;
+      if (++next_i == per_head && !kRoleQ) {
+        next_i = 0;
+        ++next_hq;
+      }
       // Pairs of tiles that an edge of the band crosses take a second copy of the row loops, with the mask: the row
       // phases sit on the kernel's serial chain, and two compares per element on every tile cost 15 %
-      const long long q0 = static_cast<long long>(kRoleQ ? tile : ys) * T, k0 = static_cast<long long>(kRoleQ ? ys : tile) * T;
-      const bool edge = kBits || (k0 + T - 1 > q0 + p.mask_right) || (k0 + p.mask_left < q0 + T - 1);
+      const int kv_minus_q = (kRoleQ ? ys - tile : tile - ys) * T;   // of the tiles' first rows
+      const bool edge = kBits || kv_minus_q + T - 1 > p.mask_right || kv_minus_q - (T - 1) < -p.mask_left;
       if constexpr (kBits) {
         const uint32_t* bits = kRoleQ ? p.bits_q : p.bits_kv;
         const long long pitch = 4LL * (kRoleQ ? nk : nq);   // words per row: four per streamed tile
-        keep_bits = *reinterpret_cast<const uint4*>(bits + (static_cast<long long>(tile) * T + row) * pitch + 4LL * ys);
+        keep_bits = bits[(static_cast<long long>(tile) * T + row) * pitch + 4LL * ys + wg];
       } else if (edge) {
         // kv - q of (row, col) is base + col (query role) or base - col (KV role); kept where -left <= kv - q <= right
-        const long long base = kRoleQ ? k0 - q0 - row : k0 - q0 + row;
+        const long long base = kRoleQ ? kv_minus_q - row : kv_minus_q + row;
         const long long lo = kRoleQ ? -static_cast<long long>(p.mask_left) - base : base - p.mask_right;
         const long long hi = kRoleQ ? static_cast<long long>(p.mask_right) - base : base + p.mask_left;
-        col_lo = static_cast<int>(max(lo, 0LL));
-        col_hi = static_cast<int>(min(hi, static_cast<long long>(T)));
+        col_lo = static_cast<int>(max(lo, 0LL)) - wg * C;
+        col_hi = static_cast<int>(min(hi, static_cast<long long>(T))) - wg * C;
       }
-      if constexpr (kRoleQ) {
-        ok = mbar_wait(s_done, it & 1, ab, kBwdSDone);
-        if (!ok) break;
+      // this thread's columns of S or dP to registers, their buffer free behind them
+      auto take = [&](uint32_t taddr, uint64_t* free_bar, float (&x)[C]) {
         tc_fence_after_sync();
-        uint32_t pds[32];
-        auto rows_q = [&](auto edge_tile) {
+        tmem_ld32f(taddr + wg * C, x);
+        tmem_wait_ld();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(free_bar);
+      };
+      auto hand_over = [&](uint32_t taddr, const float (&x)[C], uint64_t* ready_bar) {   // as 16-bit pairs
+        uint32_t pk[C / 2];
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int c0 = wg * 64 + u * 32;
-            float s[32], dp[32];
-            tmem_ld32f(tS + c0, s);
-            tmem_ld32f(tDP + c0, dp);
-            tmem_wait_ld();
-            if (u == 1) {   // this tile's S and dP are in registers: the next tile's may be computed
-              tc_fence_before_sync();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(sdp_free);
-            }
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              float pr, g;
-              score_of(edge_tile, s[k], lse2_r, ys, hq, c0 + k, pr, g);
-              dp[k] = F::grad(g, dp[k], delta_r, fctx);
-            }
-#pragma unroll
-            for (int k = 0; k < 16; ++k) pds[u * 16 + k] = pack2<kBf16>(dp[2 * k], dp[2 * k + 1]);
-          }
-        };
-        if (edge) rows_q(std::true_type{});
-        else rows_q(std::false_type{});
-        tmem_st32(tmem_base + lane_base + kColDS + (it & 1) * 64 + wg * 32, pds);
+        for (int k = 0; k < C / 2; ++k) pk[k] = pack2<kBf16>(x[2 * k], x[2 * k + 1]);
+        tmem_st16(taddr + wg * (C / 2), pk);
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready);
-      } else {
-        // ---- S -> P (and g, kept in registers for the second half) ----
-        if constexpr (F::kUsesStats) ok = mbar_wait(y1_full + it % N1, (it / N1) & 1, ab, kBwdYFull);   // lse came with the tile
-        ok = mbar_wait_poll(s_done, it & 1, ab, kBwdSDone) && ok;
-        if (!ok) break;
-        tc_fence_after_sync();
-        const float* st_lse = sLse + (it % N1) * T;
-        const float* st_delta = sDelta + (it % N2) * T;
-        float g[64];
-        uint32_t pk[32];
-        auto rows_p = [&](auto edge_tile) {
+        if (lane == 0) mbar_arrive(ready_bar);
+      };
+      static_assert(C == 32, "one tensor-memory load and one store of a row's part, one word of its keep bits");
+      ok = mbar_wait(s_full, it & 1, ab, kBwdSFull);
+      if (!ok) break;
+      // the statistics of the query rows: this thread's own (query role) or those of its columns, which came with the tiles
+      const float* st_lse = sLse + (it % N1) * T + wg * C;
+      const float* st_delta = sDelta + (it % N2) * T + wg * C;
+      float s[C], g[C];
+      take(tS, s_free, s);
+      auto probabilities = [&](auto edge_tile) {
 #pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const int c0 = wg * 64 + u * 32;
-            float s[32];
-            tmem_ld32f(tS + c0, s);
-            tmem_wait_ld();
-#pragma unroll
-            for (int k = 0; k < 32; ++k) {
-              float pr;
-              score_of(edge_tile, s[k], F::kUsesStats ? stat_of(st_lse + c0, k) : 0.0f, ys, hq, c0 + k, pr, g[u * 32 + k]);
-              s[k] = pr;
-            }
-#pragma unroll
-            for (int k = 0; k < 16; ++k) pk[u * 16 + k] = pack2<kBf16>(s[2 * k], s[2 * k + 1]);
-          }
-        };
-        if (edge) rows_p(std::true_type{});
-        else rows_p(std::false_type{});
-        // the 16-bit pairs of columns [64 wg, 64 wg + 64) go to 32-bit columns [32 wg, 32 wg + 32), which the other warp
-        // of this lane quarter reads as fp32: both must have their values in registers first
-        tc_fence_before_sync();
-        ok = named_sync_and(1 + wq, 64, ok);
-        if (!ok) break;
-        tc_fence_after_sync();
-        tmem_st32(tS + wg * 32, pk);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready);
-        // ---- dP -> dS, beside the pipe's dV(it) and S(it + 1) ----
-        if constexpr (F::kUsesStats) ok = mbar_wait(y2_full + it % N2, (it / N2) & 1, ab, kBwdYFull);   // delta came with the tile
-        ok = mbar_wait(dp_done, it & 1, ab, kBwdDpDone) && ok;
-        if (!ok) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int c0 = wg * 64 + u * 32;
-          float dp[32];
-          tmem_ld32f(tDP + c0, dp);
-          tmem_wait_ld();
-#pragma unroll
-          for (int k = 0; k < 32; ++k) dp[k] = F::grad(g[u * 32 + k], dp[k], F::kUsesStats ? stat_of(st_delta + c0, k) : 0.0f, fctx);
-#pragma unroll
-          for (int k = 0; k < 16; ++k) pk[u * 16 + k] = pack2<kBf16>(dp[2 * k], dp[2 * k + 1]);
+        for (int k = 0; k < C; ++k) {
+          float pr;
+          score_of(edge_tile, s[k], kRoleQ ? lse2_r : F::kUsesStats ? stat_of(st_lse, k) : 0.0f, ys, hq, k, pr, g[k]);
+          s[k] = pr;
         }
-        tc_fence_before_sync();
-        ok = named_sync_and(1 + wq, 64, ok);
+      };
+      if (edge) {
+        probabilities(std::true_type{});
+      } else {
+        if constexpr (F::kUsesStats) F::template score_row<C, !kRoleQ>(s, g, kRoleQ ? &lse2_r : st_lse, fctx);
+        else probabilities(std::false_type{});
+      }
+      if constexpr (!kRoleQ) {
+        if (it > 0) {   // dV of the last tile has read its P
+          ok = mbar_wait(p_free, (it - 1) & 1, ab, kBwdPFree);
+          if (!ok) break;
+          tc_fence_after_sync();
+        }
+        hand_over(tP, s, p_ready);
+      }
+      // ---- dP -> dS ----
+      ok = mbar_wait(dp_full, it & 1, ab, kBwdDpFull);
+      if (!ok) break;
+      take(tDP, dp_free, s);
+      if constexpr (F::kUsesStats) {
+        F::template grad_row<C, !kRoleQ>(g, s, kRoleQ ? &delta_r : st_delta);
+      } else {
+#pragma unroll
+        for (int k = 0; k < C; ++k) s[k] = F::grad(g[k], s[k], fctx);
+      }
+      if (!kRoleQ && it > 0) {   // dK of the last tile has read its dS
+        ok = mbar_wait(ds_free, (it - 1) & 1, ab, kBwdDsFree);
         if (!ok) break;
         tc_fence_after_sync();
-        tmem_st32(tDP + wg * 32, pk);
-        tmem_wait_st();
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(ds_ready);
       }
+      const int ds_buf = kRoleQ ? it & 1 : 0;
+      hand_over(tDS + ds_buf * 64, s, ds_ready + ds_buf);
     }
     // ---- epilogue: the accumulators as 16-bit rows (dK and dQ times the functor's constant factor) ----
     if (ok && n_iter > 0) {
@@ -531,20 +532,20 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         const float f = (kRoleQ || a == 1) ? F::out_scale(fctx) : 1.0f;
         const bool in_range = r < (kRoleQ ? p.seq_q : p.seq_kv);
 #pragma unroll
-        for (int u = 0; u < HALF / 32; ++u) {
-          const int c0 = wg * HALF + u * 32;
-          float v[32];
+        for (int u = 0; u < AC / 16; ++u) {
+          const int c0 = wg * AC + u * 16;
+          float v[16];
           if (n_iter > 0) {
-            tmem_ld32f(tmem_base + lane_base + (a == 0 ? kColA : kColB) + c0, v);
+            tmem_ld16f(tmem_base + lane_base + (a == 0 ? kColA : kColB) + c0, v);
             tmem_wait_ld();
           } else {
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = 0.0f;
+            for (int k = 0; k < 16; ++k) v[k] = 0.0f;
           }
           if (in_range) {
             uint4* dst = reinterpret_cast<uint4*>(base + c0);
 #pragma unroll
-            for (int q4 = 0; q4 < 4; ++q4) {
+            for (int q4 = 0; q4 < 2; ++q4) {
               uint4 pk;
               pk.x = pack2<kBf16>(v[8 * q4 + 0] * f, v[8 * q4 + 1] * f);
               pk.y = pack2<kBf16>(v[8 * q4 + 2] * f, v[8 * q4 + 3] * f);

@@ -81,8 +81,8 @@ struct SoftmaxFunctor {
     for (int hf = 0; hf < kPieces; ++hf) {
 #pragma unroll
       for (int i = hf * (N / kPieces); i < (hf + 1) * (N / kPieces); i += 4) {
-        fma_x2(s[i], s[i + 1], c2, neg);
-        fma_x2(s[i + 2], s[i + 3], c2, neg);
+        fma_x2(s[i], s[i + 1], c2, c2, neg, neg);
+        fma_x2(s[i + 2], s[i + 3], c2, c2, neg, neg);
         s[i] = fast_exp2(s[i]);
         s[i + 1] = fast_exp2(s[i + 1]);
         s[i + 2] = fast_exp2(s[i + 2]);

@@ -533,15 +533,20 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return r;
 }
 
-// two fp32 operations to an instruction: (x0, x1) * m + a, and (x0, x1) += (y0, y1)
-__device__ __forceinline__ void fma_x2(float& x0, float& x1, float m, float a) {
-  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %2};\n\tmov.b64 a, {%3, %3};\n\t"
+// two fp32 operations to an instruction: x = x * m + a, x += y, x *= y
+__device__ __forceinline__ void fma_x2(float& x0, float& x1, float m0, float m1, float a0, float a1) {
+  asm("{\n\t.reg .b64 x, m, a;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 m, {%2, %3};\n\tmov.b64 a, {%4, %5};\n\t"
       "fma.rn.f32x2 x, x, m, a;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(x0), "+f"(x1)
-      : "f"(m), "f"(a));
+      : "f"(m0), "f"(m1), "f"(a0), "f"(a1));
 }
 __device__ __forceinline__ void add_x2(float& x0, float& x1, float y0, float y1) {
   asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "+f"(x0), "+f"(x1)
+      : "f"(y0), "f"(y1));
+}
+__device__ __forceinline__ void mul_x2(float& x0, float& x1, float y0, float y1) {
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
       : "+f"(x0), "+f"(x1)
       : "f"(y0), "f"(y1));
 }

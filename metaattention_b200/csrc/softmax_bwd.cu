@@ -10,16 +10,8 @@
 // :246-275 = dQ to 16 bits; autograd wrapper :669-694), for the built-in softmax.  Differences: three launches
 // without atomics or an fp32 dQ buffer -- (1) delta and log2-domain lse into a padded scratch, (2) one CTA per KV tile
 // accumulating dK and dV over the query tiles, (3) one CTA per query tile accumulating dQ over the KV tiles (S and dP
-// are computed a second time there: 7 tile products instead of 5 for no read-modify-write traffic on dQ).
-//
-// Both main launches are one kernel template (attn_bwd.cuh, shared with the lowered functors).  A CTA keeps one 128-row tile pair resident (X: K_j, V_j or Q_i, dO_i)
-// and streams the other (Y: Q_i, dO_i or K_j, V_j) through a two-stage TMA ring.  Per streamed tile:
-//   S  = X1 Y1^T, dP = X2 Y2^T           tcgen05 SS, fp32 in tensor memory (columns [0,128) and [128,256))
-//   row threads (thread = TMEM lane x column half): P and dS as 16-bit pairs written over S and dP
-//   acc1 += P  Y2   (dV; KV role only)    tcgen05 TS, A from tensor memory, B = the streamed tile MN-major
-//   acc2 += dS Y1   (dK or dQ)
-// With the KV role the lanes are KV rows and the columns query rows (S^T, dP^T), so that P^T and dS^T are the A
-// operands as they stand; the statistics (lse, delta) then belong to columns and come with the streamed tile.
+// are computed a second time there: 7 tile products instead of 5 for no read-modify-write traffic on dQ; (2) and (3) are
+// one launch).  Their kernel template is attn_bwd.cuh, shared with the lowered functors.
 #include "attn_bwd.cuh"
 
 namespace b200 {
@@ -36,7 +28,29 @@ struct SoftmaxBwdFunctor {
   __device__ static void score(float s, float lse2, const Ctx& c, int, int, int, int, float& p_out, float& g_out) {
     p_out = g_out = fast_exp2(fmaf(s, c.c2, -lse2));
   }
-  __device__ static float grad(float g, float dp, float delta, const Ctx&) { return g * (dp - delta); }
+  // For the N columns of a row, two to an instruction; kColumns: one statistic per column, else one for the row.
+  template <int N, bool kColumns>
+  __device__ static void score_row(float (&s)[N], float (&g)[N], const float* lse2, const Ctx& c) {
+#pragma unroll
+    for (int k = 0; k < N; k += 4) {
+      const float4 l = kColumns ? *reinterpret_cast<const float4*>(lse2 + k) : make_float4(*lse2, *lse2, *lse2, *lse2);
+      fma_x2(s[k], s[k + 1], c.c2, c.c2, -l.x, -l.y);
+      fma_x2(s[k + 2], s[k + 3], c.c2, c.c2, -l.z, -l.w);
+#pragma unroll
+      for (int i = k; i < k + 4; ++i) s[i] = g[i] = fast_exp2(s[i]);
+    }
+  }
+  template <int N, bool kColumns>
+  __device__ static void grad_row(const float (&g)[N], float (&dp)[N], const float* delta) {
+#pragma unroll
+    for (int k = 0; k < N; k += 4) {
+      const float4 d = kColumns ? *reinterpret_cast<const float4*>(delta + k) : make_float4(*delta, *delta, *delta, *delta);
+      add_x2(dp[k], dp[k + 1], -d.x, -d.y);
+      add_x2(dp[k + 2], dp[k + 3], -d.z, -d.w);
+      mul_x2(dp[k], dp[k + 1], g[k], g[k + 1]);
+      mul_x2(dp[k + 2], dp[k + 3], g[k + 2], g[k + 3]);
+    }
+  }
   __device__ static float out_scale(const Ctx& c) { return c.scale; }
 };
 
