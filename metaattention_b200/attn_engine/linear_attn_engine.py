@@ -17,8 +17,6 @@ and ignored.
 
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from core.native import lib as native
@@ -103,17 +101,6 @@ def _constant_multiple(out: SymbolScalar, leaf: SymbolScalar):
     return None
 
 
-def _column_range_ld(t) -> int:
-    """The row pitch of t [B, H, T, w] if it is a column range of a contiguous [B, H, T, ld] tensor that the kernel can
-    read in place (16-byte aligned start, ld a multiple of 8), else 0."""
-    B, H, T, w = t.shape
-    ld = t.stride(2)
-    if (t.stride(3) == 1 and ld > w and ld % 8 == 0 and t.stride(1) == T * ld and t.stride(0) == H * T * ld
-            and t.data_ptr() % 16 == 0):
-        return ld
-    return 0
-
-
 def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize: bool = False, eps: float = 1e-5,
                              out_dtype=None, v_scale=None, precise: bool = False, segments: int = 0, reverse: bool = False):
     """q,k: [B,H,T,Dk]; v: [B,H,T,Dv] (fp16/bf16 CUDA); log_decay: [B,H,T] fp32, natural log of the
@@ -126,60 +113,22 @@ def linear_attention_forward(q, k, v, log_decay, q_scale: float = 1.0, normalize
     tokens from a row's own to the end of the sequence (see ``_reversed_forward``)."""
     if out_dtype not in (None, q.dtype, torch.float32):
         raise native.NativeError("out_dtype must be the input dtype or torch.float32")
-    f32_out = out_dtype == torch.float32
-    (B, HQ, T, Dk), (Bk, HK, Tk, Dkk), (Bv, H, Tv, Dv) = q.shape, k.shape, v.shape
-    # the kernel walks k and v with the extents of q: what has others would be read askew or past its end
-    if Dkk != Dk or Tk != T or Tv != T or Bk < B or Bv < B:
-        raise native.NativeError(f"q, k, v do not fit together: {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}")
-    if not q.is_cuda:
-        raise native.NativeError("linear attention needs CUDA tensors")
-    if q.dtype not in native.DTYPE_CODES or k.dtype != q.dtype or v.dtype != q.dtype:
-        raise native.NativeError("q, k, v must share dtype float16 or bfloat16")
-    if H % HQ != 0 or H % HK != 0:
-        raise native.NativeError("the heads of v must be a multiple of the heads of q and of k")
-    if Dv % 128 != 0 and normalize:
-        raise native.NativeError("normalize needs dim_v to be a multiple of 128")
-    if Dv % 8 != 0 or (f32_out and Dv % 128 != 0):
-        # rows of v that are not whole 16-byte pieces, or fp32 rows that are not whole slices: padded with zero columns,
-        # which stay zero in the output and are cut off again (otherwise the kernel reads the columns that a slice of 128
-        # is short of as zeros)
-        pad = 128 - Dv % 128
-        o = linear_attention_forward(q, k, torch.nn.functional.pad(v, (0, pad)), log_decay, q_scale, False, eps, out_dtype, v_scale,
-                                     precise, segments, reverse)
-        return o[..., :Dv].contiguous()
-    # q and k may be column ranges of wider contiguous tensors (the backward's contractions over ranges of dim_v)
-    q_ld, k_ld = _column_range_ld(q), _column_range_ld(k)
-    q = q if q_ld else q.contiguous()
-    k = k if k_ld else k.contiguous()
-    v = v.contiguous()
-    log_decay = log_decay.to(dtype=torch.float32, device=q.device).expand(B, H, T).contiguous()
-    if v_scale is not None:
-        v_scale = v_scale.to(dtype=torch.float32, device=q.device).expand(B, H, T).contiguous()
-    with torch.cuda.device(q.device):
-        o = torch.empty((B, H, T, Dv), dtype=torch.float32 if f32_out else q.dtype, device=q.device)
-        a = native.LinearArgs()
-        a.dtype_out = native.DTYPE_OUT_FP32 if f32_out else native.DTYPE_OUT_SAME
-        a.q, a.k, a.v, a.log_decay, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), log_decay.data_ptr(), o.data_ptr()
-        a.v_scale = v_scale.data_ptr() if v_scale is not None else None
-        a.batch, a.heads, a.seq, a.dim_qk, a.dim_v = B, H, T, Dk, Dv
-        a.heads_q, a.heads_k = HQ, HK
-        a.q_ld, a.k_ld = q_ld, k_ld
-        a.dtype = native.DTYPE_CODES[q.dtype]
-        a.normalize = 1 if normalize else 0
-        a.precise = 1 if precise else 0
-        a.segments = segments
-        a.reverse = 1 if reverse else 0
-        a.any_dim_v = 1
-        a.q_scale = float(q_scale)
-        a.norm_eps = float(eps)
-        lib = native.load_library()
-        need = int(lib.attn_b200_linear_workspace_bytes(C.byref(a)))
-        ws = None
-        if need > 0:
-            ws = torch.empty(need, dtype=torch.uint8, device=q.device)
-            a.workspace, a.workspace_bytes = ws.data_ptr(), need
-        native.check(lib.attn_b200_linear_fwd(C.byref(a), native.current_stream_ptr()), "attn_b200_linear_fwd")
+    o = native.host().linear_forward(q, k, v, log_decay, q_scale, normalize, eps, out_dtype == torch.float32, v_scale, precise, segments,
+                                     reverse)
+    if not isinstance(o, torch.Tensor):
+        _refuse(o, q, k, v)
     return o
+
+
+def _refuse(why: int, q, k, v):
+    """The error of a call that the native host side refuses (LinearRefusal in csrc/host_ops.cpp)."""
+    (_, _, _, _), (_, _, _, _), (_, _, _, _) = q.shape, k.shape, v.shape
+    raise native.NativeError({
+        2: f"q, k, v do not fit together: {tuple(q.shape)}, {tuple(k.shape)}, {tuple(v.shape)}",
+        3: "linear attention needs CUDA tensors",
+        4: "q, k, v must share dtype float16 or bfloat16",
+        5: "the heads of v must be a multiple of the heads of q and of k",
+        6: "normalize needs dim_v to be a multiple of 128"}[why])
 
 
 def _reversed_forward(q, k, v, log_decay, q_scale, out_dtype=None, precise=False):

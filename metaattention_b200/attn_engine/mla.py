@@ -98,79 +98,34 @@ def mla_decode_forward(q, kv, dim_v: int, scale: float, q_rope=None, kv_rope=Non
     to be faster for equal lengths.
     Returns (o [B,H,dim_v] in the input dtype, lse [B,H] fp32)."""
     global last_plan
-    q3, kv3 = _rows(q, "q"), _rows(kv, "kv")
-    if not q3.is_cuda:
-        raise native.NativeError("MLA decode needs CUDA tensors")
-    B, H, dq = q3.shape
-    S = kv3.shape[1]
-    page_size = num_pages = 0
-    if block_table is not None:
-        if block_table.dtype != torch.int32 or not block_table.is_cuda or block_table.dim() != 2 or block_table.shape[0] != B:
-            raise ValueError("block_table must be a CUDA int32 tensor [batch, max_blocks]")
-        if block_table.stride(1) != 1:
-            block_table = block_table.contiguous()
-        num_pages, page_size = kv3.shape[0], kv3.shape[1]
-        S = block_table.shape[1] * page_size if max_seqlen is None else int(max_seqlen)
-        if S > block_table.shape[1] * page_size:
-            raise ValueError("max_seqlen exceeds the block table")
-    if cache_seqlens is not None:
-        if cache_seqlens.dtype != torch.int32 or not cache_seqlens.is_cuda or cache_seqlens.numel() != B:
-            raise ValueError("cache_seqlens must be a CUDA int32 tensor [batch]")
-        cache_seqlens = cache_seqlens.contiguous()
-    rope_dim = 0
-    qr3 = kr3 = None
-    if (q_rope is None) != (kv_rope is None):
-        raise ValueError("q_rope and kv_rope must be given together")
-    if q_rope is not None:
-        qr3, kr3 = _rows(q_rope, "q_rope"), _rows(kv_rope, "kv_rope")
-        rope_dim = qr3.shape[2]
-    dim_qk = dq + rope_dim
-    if q3.dtype not in native.DTYPE_CODES or kv3.dtype != q3.dtype:
-        raise native.NativeError("q and kv must share dtype float16 or bfloat16")
-    with torch.cuda.device(q3.device):
-        if num_splits is None:
-            # ragged lengths: scheduled; equal lengths: whichever the plan estimates faster (0 = scheduled)
-            num_splits = 0 if (cache_seqlens is not None or tile_scheduler_metadata is not None) else \
-                plan_splits(B, H, S, dim_qk, dim_v, _sm_count(q3.device))
-        need = workspace_bytes(B, H, S, dim_qk, dim_v, num_splits)
-        last_plan = {"mode": "scheduled", "parts": num_parts(H, q3.device)} if num_splits == 0 else {"mode": "uniform", "num_splits": num_splits}
-        if need < 0:
-            raise native.NativeError(f"MLA decode does not support dims qk={dim_qk} v={dim_v}")
-        if need > 0 and (workspace is None or workspace.numel() * workspace.element_size() < need):
-            workspace = torch.empty(need, dtype=torch.uint8, device=q3.device)
-        o = torch.empty((B, H, dim_v), dtype=q3.dtype, device=q3.device)
-        lse = torch.empty((B, H), dtype=torch.float32, device=q3.device)
-        a = native.MlaArgs()
-        a.q, a.kv = q3.data_ptr(), kv3.data_ptr()
-        a.q_stride[:] = (q3.stride(0), q3.stride(1))
-        a.kv_stride[:] = (kv3.stride(0), kv3.stride(1))
-        if qr3 is not None:
-            a.q_rope, a.kv_rope = qr3.data_ptr(), kr3.data_ptr()
-            a.q_rope_stride[:] = (qr3.stride(0), qr3.stride(1))
-            a.kv_rope_stride[:] = (kr3.stride(0), kr3.stride(1))
-        a.o, a.lse = o.data_ptr(), lse.data_ptr()
-        a.workspace = workspace.data_ptr() if need > 0 else None
-        a.workspace_bytes = need
-        a.shape = native.MlaShape(B, H, S, dim_qk, dim_v)
-        a.num_splits = num_splits
-        a.dtype = native.DTYPE_CODES[q3.dtype]
-        a.scale = float(scale)
-        if cache_seqlens is not None:
-            a.seq_lens = cache_seqlens.data_ptr()
-        if num_splits == 0 and tile_scheduler_metadata is not None:
-            if num_splits_cum is None or tile_scheduler_metadata.dtype != torch.int32 or num_splits_cum.dtype != torch.int32:
-                raise ValueError("tile_scheduler_metadata and num_splits_cum must be the int32 tensors of mla_schedule")
-            if tile_scheduler_metadata.shape[0] != num_parts(H, q3.device) or num_splits_cum.numel() != B + 1:
-                raise ValueError("the schedule was made for another batch or device")
-            a.sched_meta, a.sched_num_splits = tile_scheduler_metadata.data_ptr(), num_splits_cum.data_ptr()
-            a.sched_parts = tile_scheduler_metadata.shape[0]
-        if block_table is not None:
-            a.block_table = block_table.data_ptr()
-            a.block_table_stride = block_table.stride(0)
-            a.page_size, a.num_pages = page_size, num_pages
-        native.check(native.load_library().attn_b200_mla_decode(C.byref(a), native.current_stream_ptr()),
-                     "attn_b200_mla_decode")
+    r = native.host().mla_decode(q, kv, dim_v, scale, q_rope, kv_rope, num_splits, workspace, cache_seqlens, block_table, max_seqlen,
+                                 tile_scheduler_metadata, num_splits_cum)
+    if isinstance(r, int):
+        _refuse(r, q, kv, q_rope, kv_rope, dim_v)
+    o, lse, splits, parts = r
+    last_plan = {"mode": "scheduled", "parts": parts} if splits == 0 else {"mode": "uniform", "num_splits": splits}
     return o, lse
+
+
+def _refuse(why: int, q, kv, q_rope, kv_rope, dim_v):
+    """The error of a call that the native host side refuses (MlaRefusal in csrc/host_ops.cpp)."""
+    if why == 1:
+        for t, what in ((q, "q"), (kv, "kv"), (q_rope, "q_rope"), (kv_rope, "kv_rope")):
+            if t is not None:
+                _rows(t, what)
+    if why == 2:
+        raise native.NativeError("MLA decode needs CUDA tensors")
+    if why == 7:
+        raise native.NativeError("q and kv must share dtype float16 or bfloat16")
+    if why == 8:
+        raise native.NativeError(f"MLA decode does not support dims qk={q.shape[-1] + (q_rope.shape[-1] if q_rope is not None else 0)} v={dim_v}")
+    raise ValueError({
+        3: "block_table must be a CUDA int32 tensor [batch, max_blocks]",
+        4: "max_seqlen exceeds the block table",
+        5: "cache_seqlens must be a CUDA int32 tensor [batch]",
+        6: "q_rope and kv_rope must be given together",
+        9: "tile_scheduler_metadata and num_splits_cum must be the int32 tensors of mla_schedule",
+        10: "the schedule was made for another batch or device"}[why])
 
 
 def build_mla_decode(engine, B, H, Hkv, Skv, D, Dv, dtype, backend):

@@ -408,20 +408,7 @@ def linear_decay_grad(q, k, dq_parts, dk_parts):
     partial results each (attn_b200_linear_decay_grad)."""
     if not q.is_cuda:
         raise NativeError("linear_decay_grad needs CUDA tensors: there is no CPU path")
-    q, k = q.contiguous(), k.contiguous()
-    B, H, T, cols = q.shape
-    parts = [t.contiguous() for t in (*dq_parts, *dk_parts)]   # alive until the launch
-    ptrs = [t.data_ptr() for t in parts]
-    dq_a, dq_b = ptrs[0], ptrs[1] if len(dq_parts) > 1 else None
-    dk_a, dk_b = ptrs[len(dq_parts)], ptrs[len(dq_parts) + 1] if len(dk_parts) > 1 else None
-    dq, dk = torch.empty_like(q), torch.empty_like(k)
-    dg = torch.empty(B, H, T, dtype=torch.float32, device=q.device)
-    term = torch.empty_like(dg)
-    with torch.cuda.device(q.device):
-        check(load_library().attn_b200_linear_decay_grad(q.data_ptr(), k.data_ptr(), dq_a, dq_b, dk_a, dk_b, dq.data_ptr(), dk.data_ptr(),
-                                                         term.data_ptr(), dg.data_ptr(), DTYPE_CODES[q.dtype], B * H, T, cols,
-                                                         current_stream_ptr()), "attn_b200_linear_decay_grad")
-    return dq, dk, dg
+    return tuple(host().linear_decay_grad(q, k, list(dq_parts), list(dk_parts)))
 
 
 def rows_sum_cast(a, b, dtype, reverse: bool = False):
@@ -429,15 +416,7 @@ def rows_sum_cast(a, b, dtype, reverse: bool = False):
     (attn_b200_rows_sum_cast)."""
     if not a.is_cuda:
         raise NativeError("rows_sum_cast needs CUDA tensors: there is no CPU path")
-    a = a.contiguous()
-    b = None if b is None else b.contiguous()
-    cols, seq = a.shape[-1], a.shape[-2]
-    dst = torch.empty(a.shape, dtype=dtype, device=a.device)
-    with torch.cuda.device(a.device):
-        check(load_library().attn_b200_rows_sum_cast(a.data_ptr(), None if b is None else b.data_ptr(), dst.data_ptr(),
-                                                     DTYPE_CODES[dtype], a.numel() // (seq * cols), seq, cols, 1 if reverse else 0,
-                                                     current_stream_ptr()), "attn_b200_rows_sum_cast")
-    return dst
+    return host().rows_sum_cast(a, b, DTYPE_CODES[dtype] == DTYPE_CODES[torch.bfloat16], reverse)
 
 
 def softmax_bwd(q, k, v, o, lse, d_o, scale: float, mask_kind: int, mask_band=(MASK_OPEN, MASK_OPEN), mask_bits=None):

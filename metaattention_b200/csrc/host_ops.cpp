@@ -1,7 +1,7 @@
 // Host side of a call in native code: from tensors to the argument structs of include/attn_b200.h, outputs and scratch from
 // torch's allocator, the launch on the current stream, and the autograd functions.
 //
-// A short call's kernel runs for 5 to 20 microseconds; filling a ctypes struct field by field in Python took 35 to 50, and a
+// A short call's kernel runs for 5 to 30 microseconds; filling a ctypes struct field by field in Python took 35 to 50, and a
 // forward and backward through Python autograd functions 220.  Everything here works on what the engine decided once at
 // construction (`Plan`) and on the shapes and strides of this call.  Nothing is kept between calls but the plan's copies of
 // its mask on each device.
@@ -41,6 +41,14 @@ struct Api {
   int64_t (*softmax_bwd_bytes)(const AttnB200SoftmaxBwdArgs*) = nullptr;
   int (*softmax_bwd)(const AttnB200SoftmaxBwdArgs*, void*) = nullptr;
   int (*status_word)(int32_t, int32_t**) = nullptr;
+  int64_t (*linear_bytes)(const AttnB200LinearArgs*) = nullptr;
+  int (*linear_fwd)(const AttnB200LinearArgs*, void*) = nullptr;
+  decltype(&attn_b200_linear_decay_grad) linear_decay_grad = nullptr;
+  decltype(&attn_b200_rows_sum_cast) rows_sum_cast = nullptr;
+  int (*mla_plan)(const AttnB200MlaShape*, int32_t, int32_t*) = nullptr;
+  int64_t (*mla_bytes)(const AttnB200MlaShape*, int32_t) = nullptr;
+  int32_t (*mla_num_parts)(int32_t, int32_t) = nullptr;
+  int (*mla_decode)(const AttnB200MlaArgs*, void*) = nullptr;
 } api;
 
 template <class F>
@@ -59,6 +67,14 @@ void bind(const py::dict& d, py::object check) {
   take(api.softmax_bwd_bytes, d, "attn_b200_softmax_bwd_workspace_bytes");
   take(api.softmax_bwd, d, "attn_b200_softmax_bwd");
   take(api.status_word, d, "attn_b200_device_status_word");
+  take(api.linear_bytes, d, "attn_b200_linear_workspace_bytes");
+  take(api.linear_fwd, d, "attn_b200_linear_fwd");
+  take(api.linear_decay_grad, d, "attn_b200_linear_decay_grad");
+  take(api.rows_sum_cast, d, "attn_b200_rows_sum_cast");
+  take(api.mla_plan, d, "attn_b200_mla_plan");
+  take(api.mla_bytes, d, "attn_b200_mla_workspace_bytes");
+  take(api.mla_num_parts, d, "attn_b200_mla_num_parts");
+  take(api.mla_decode, d, "attn_b200_mla_decode");
   raise_status = check.release().ptr();
 }
 
@@ -608,6 +624,258 @@ std::shared_ptr<Plan> make_plan(const py::dict& d) {
   return p;
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// chunked linear attention
+// ---------------------------------------------------------------------------------------------------------------
+
+// The row pitch of t [B, H, T, w] if it is a column range of a contiguous [B, H, T, ld] tensor that the kernel can read in
+// place (16-byte aligned start, ld a multiple of 8), else 0.
+int64_t column_range_ld(const Tensor& t) {
+  const int64_t ld = t.stride(2), T = t.size(2);
+  return t.stride(3) == 1 && ld > t.size(3) && ld % 8 == 0 && t.stride(1) == T * ld && t.stride(0) == t.size(1) * T * ld &&
+                 (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0
+             ? ld
+             : 0;
+}
+
+// Why attn_engine/linear_attn_engine.py refuses a call (it words the errors).
+enum LinearRefusal { kLinearOk = 0, kLinearShapes, kLinearFit, kLinearDevice, kLinearType, kLinearHeads, kLinearNormalize };
+
+LinearRefusal linear_refusal(const Tensor& q, const Tensor& k, const Tensor& v, bool normalize) {
+  if (q.dim() != 4 || k.dim() != 4 || v.dim() != 4) return kLinearShapes;
+  // the kernel walks k and v with the extents of q: what has others would be read askew or past its end
+  if (k.size(3) != q.size(3) || k.size(2) != q.size(2) || v.size(2) != q.size(2) || k.size(0) < q.size(0) || v.size(0) < q.size(0)) return kLinearFit;
+  if (!q.is_cuda() || !k.is_cuda() || !v.is_cuda()) return kLinearDevice;
+  if (dtype_code(q) < 0 || k.scalar_type() != q.scalar_type() || v.scalar_type() != q.scalar_type()) return kLinearType;
+  if (q.size(1) <= 0 || k.size(1) <= 0 || v.size(1) % q.size(1) != 0 || v.size(1) % k.size(1) != 0) return kLinearHeads;
+  if (normalize && v.size(3) % 128 != 0) return kLinearNormalize;
+  return kLinearOk;
+}
+
+struct LinearCall {
+  double q_scale, eps;
+  bool normalize, f32_out, precise, reverse;
+  int segments;
+};
+
+Tensor linear_forward(Tensor q, Tensor k, Tensor v, Tensor log_decay, OptTensor v_scale, const LinearCall& c) {
+  const int64_t B = q.size(0), T = q.size(2), Dk = q.size(3), H = v.size(1), Dv = v.size(3);
+  if (Dv % 8 != 0 || (c.f32_out && Dv % 128 != 0)) {
+    // rows of v that are not whole 16-byte pieces, or fp32 rows that are not whole slices: padded with zero columns,
+    // which stay zero in the output and are cut off again (otherwise the kernel reads the columns that a slice of 128
+    // is short of as zeros)
+    Tensor o = linear_forward(q, k, at::constant_pad_nd(v, {0, 128 - Dv % 128}), log_decay, v_scale, c);
+    return o.narrow(3, 0, Dv).contiguous();
+  }
+  // q and k may be column ranges of wider contiguous tensors (the backward's contractions over ranges of dim_v)
+  const int64_t q_ld = column_range_ld(q), k_ld = column_range_ld(k);
+  if (q_ld == 0) q = q.contiguous();
+  if (k_ld == 0) k = k.contiguous();
+  v = v.contiguous();
+  log_decay = log_decay.to(q.device(), at::kFloat).expand({B, H, T}).contiguous();
+  if (v_scale.has_value()) v_scale = v_scale->to(q.device(), at::kFloat).expand({B, H, T}).contiguous();
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor o = at::empty({B, H, T, Dv}, c.f32_out ? q.options().dtype(at::kFloat) : q.options());
+  AttnB200LinearArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.dtype_out = c.f32_out ? ATTN_B200_DTYPE_FP32 : ATTN_B200_DTYPE_SAME;
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr();
+  a.log_decay = log_decay.data_ptr<float>();
+  a.v_scale = v_scale.has_value() ? v_scale->data_ptr<float>() : nullptr;
+  a.batch = B; a.heads = H; a.seq = T; a.dim_qk = Dk; a.dim_v = Dv;
+  a.heads_q = q.size(1); a.heads_k = k.size(1);
+  a.q_ld = q_ld; a.k_ld = k_ld;
+  a.dtype = dtype_code(q);
+  a.normalize = c.normalize; a.precise = c.precise; a.segments = c.segments; a.reverse = c.reverse; a.any_dim_v = 1;
+  a.q_scale = c.q_scale; a.norm_eps = c.eps;
+  const int64_t need = api.linear_bytes(&a);
+  Tensor ws;
+  if (need > 0) {
+    ws = bytes(need, q);
+    a.workspace = ws.data_ptr();
+    a.workspace_bytes = need;
+  }
+  check(api.linear_fwd(&a, stream_of(q)), "attn_b200_linear_fwd");
+  return o;
+}
+
+// The output, or the number of a refusal.
+py::object linear_forward_call(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& log_decay, double q_scale, bool normalize, double eps,
+                               bool f32_out, const OptTensor& v_scale, bool precise, int segments, bool reverse) {
+  const LinearRefusal why = linear_refusal(q, k, v, normalize);
+  if (why != kLinearOk) return py::int_(static_cast<int>(why));
+  Tensor o;
+  {
+    py::gil_scoped_release others_run;
+    at::AutoDispatchBelowADInplaceOrView below;
+    o = linear_forward(q, k, v, log_decay, v_scale, {q_scale, eps, normalize, f32_out, precise, reverse, segments});
+  }
+  return py::cast(o);
+}
+
+// dq, dk rounded to the dtype of q [B, H, T, cols] and the gradient of the log-decays [B, H, T], from one or two fp32
+// partial results each (attn_b200_linear_decay_grad).
+std::vector<Tensor> linear_decay_grad(const Tensor& q_in, const Tensor& k_in, const std::vector<Tensor>& dq_in, const std::vector<Tensor>& dk_in) {
+  py::gil_scoped_release others_run;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const Tensor q = q_in.contiguous(), k = k_in.contiguous();
+  std::vector<Tensor> parts;   // alive until the launch
+  auto part = [&](const std::vector<Tensor>& from, size_t i) -> const float* {
+    if (i >= from.size()) return nullptr;
+    parts.push_back(from[i].contiguous());
+    return parts.back().data_ptr<float>();
+  };
+  const float *dq_a = part(dq_in, 0), *dq_b = part(dq_in, 1), *dk_a = part(dk_in, 0), *dk_b = part(dk_in, 1);
+  c10::cuda::CUDAGuard guard(q.device());
+  Tensor dq = at::empty_like(q), dk = at::empty_like(k), dg = f32({q.size(0), q.size(1), q.size(2)}, q), term = at::empty_like(dg);
+  check(api.linear_decay_grad(q.data_ptr(), k.data_ptr(), dq_a, dq_b, dk_a, dk_b, dq.data_ptr(), dk.data_ptr(), term.data_ptr<float>(),
+                              dg.data_ptr<float>(), dtype_code(q), q.size(0) * q.size(1), static_cast<int32_t>(q.size(2)),
+                              static_cast<int32_t>(q.size(3)), stream_of(q)),
+        "attn_b200_linear_decay_grad");
+  return {dq, dk, dg};
+}
+
+// a (+ b), fp32 [..., seq, cols], rounded to fp16 or bf16, the rows of every sequence reversed if asked.
+Tensor rows_sum_cast(const Tensor& a_in, const OptTensor& b_in, bool bf16, bool reverse) {
+  py::gil_scoped_release others_run;
+  at::AutoDispatchBelowADInplaceOrView below;
+  const Tensor a = a_in.contiguous();
+  Tensor b;
+  if (b_in.has_value()) b = b_in->contiguous();
+  const int64_t cols = a.size(-1), seq = a.size(-2);
+  c10::cuda::CUDAGuard guard(a.device());
+  Tensor dst = at::empty(a.sizes(), a.options().dtype(bf16 ? at::kBFloat16 : at::kHalf));
+  check(api.rows_sum_cast(a.data_ptr<float>(), b.defined() ? b.data_ptr<float>() : nullptr, dst.data_ptr(),
+                          bf16 ? ATTN_B200_DTYPE_BF16 : ATTN_B200_DTYPE_FP16, seq * cols > 0 ? a.numel() / (seq * cols) : 0,
+                          static_cast<int32_t>(seq), static_cast<int32_t>(cols), reverse ? 1 : 0, stream_of(a)),
+        "attn_b200_rows_sum_cast");
+  return dst;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// MLA decode
+// ---------------------------------------------------------------------------------------------------------------
+
+// [B, R, C] view of a [B, R, C], [B, 1, R, C] or [B, R, 1, C] tensor with contiguous columns.
+bool rows_of(const Tensor& t, Tensor& out) {
+  out = t;
+  if (t.dim() == 4) {
+    if (t.size(1) == 1) out = t.select(1, 0);
+    else if (t.size(2) == 1) out = t.select(2, 0);
+    else return false;
+  }
+  return out.dim() == 3 && out.stride(2) == 1;
+}
+
+// Why attn_engine/mla.py refuses a call (it words the errors).
+enum MlaRefusal { kMlaRows = 1, kMlaDevice, kMlaTable, kMlaMaxLen, kMlaLens, kMlaRope, kMlaType, kMlaDims, kMlaSchedule, kMlaOtherSchedule };
+
+struct MlaResult {
+  int refusal = 0, num_splits = 0, parts = 0;
+  Tensor o, lse;
+};
+
+MlaResult mla_decode(const Tensor& q_in, const Tensor& kv_in, int64_t dim_v, double scale, const OptTensor& q_rope, const OptTensor& kv_rope,
+                     c10::optional<int64_t> num_splits, const OptTensor& workspace, const OptTensor& lens_in, const OptTensor& table_in,
+                     c10::optional<int64_t> max_seqlen, const OptTensor& sched, const OptTensor& sched_cum) {
+  MlaResult r;
+  auto refuse = [&](int why) {
+    r.refusal = why;
+    return r;
+  };
+  Tensor q, kv, qr, kr, table, lens;
+  if (!rows_of(q_in, q) || !rows_of(kv_in, kv)) return refuse(kMlaRows);
+  if (!q.is_cuda() || !kv.is_cuda()) return refuse(kMlaDevice);
+  const int64_t B = q.size(0), H = q.size(1);
+  int64_t S = kv.size(1);
+  if (table_in.has_value()) {
+    table = *table_in;
+    if (table.scalar_type() != at::kInt || !table.is_cuda() || table.dim() != 2 || table.size(0) != B) return refuse(kMlaTable);
+    if (table.stride(1) != 1) table = table.contiguous();
+    const int64_t most = table.size(1) * kv.size(1);
+    S = max_seqlen.value_or(most);
+    if (S > most) return refuse(kMlaMaxLen);
+  }
+  if (lens_in.has_value()) {
+    if (lens_in->scalar_type() != at::kInt || !lens_in->is_cuda() || lens_in->numel() != B) return refuse(kMlaLens);
+    lens = lens_in->contiguous();
+  }
+  if (q_rope.has_value() != kv_rope.has_value()) return refuse(kMlaRope);
+  int64_t rope = 0;
+  if (q_rope.has_value()) {
+    if (!rows_of(*q_rope, qr) || !rows_of(*kv_rope, kr)) return refuse(kMlaRows);
+    rope = qr.size(2);
+  }
+  if (dtype_code(q) < 0 || kv.scalar_type() != q.scalar_type()) return refuse(kMlaType);
+  c10::cuda::CUDAGuard guard(q.device());
+  const int sms = at::cuda::getDeviceProperties(q.device().index())->multiProcessorCount;
+  AttnB200MlaArgs a;
+  std::memset(&a, 0, sizeof(a));
+  a.shape.batch = B; a.shape.heads_q = H; a.shape.seq_kv = S; a.shape.dim_qk = q.size(2) + rope; a.shape.dim_v = dim_v;
+  int32_t splits = 0;
+  if (num_splits.has_value()) splits = static_cast<int32_t>(*num_splits);
+  else if (!lens.defined() && !sched.has_value()) check(api.mla_plan(&a.shape, sms, &splits), "attn_b200_mla_plan");
+  r.num_splits = splits;
+  r.parts = api.mla_num_parts(H, sms);
+  const int64_t need = api.mla_bytes(&a.shape, splits);
+  if (need < 0) return refuse(kMlaDims);
+  Tensor ws;
+  if (need > 0) {
+    ws = workspace.has_value() && static_cast<int64_t>(workspace->nbytes()) >= need ? *workspace : bytes(need, q);
+    a.workspace = ws.data_ptr();
+  }
+  a.workspace_bytes = need;
+  r.o = at::empty({B, H, dim_v}, q.options());
+  r.lse = f32({B, H}, q);
+  a.q = q.data_ptr(); a.kv = kv.data_ptr(); a.o = r.o.data_ptr();
+  a.lse = r.lse.data_ptr<float>();
+  for (int i = 0; i < 2; ++i) {
+    a.q_stride[i] = q.stride(i);
+    a.kv_stride[i] = kv.stride(i);
+    if (rope > 0 || qr.defined()) {
+      a.q_rope_stride[i] = qr.stride(i);
+      a.kv_rope_stride[i] = kr.stride(i);
+    }
+  }
+  if (qr.defined()) {
+    a.q_rope = qr.data_ptr();
+    a.kv_rope = kr.data_ptr();
+  }
+  a.num_splits = splits;
+  a.dtype = dtype_code(q);
+  a.scale = scale;
+  if (lens.defined()) a.seq_lens = lens.data_ptr<int32_t>();
+  if (splits == 0 && sched.has_value()) {
+    if (!sched_cum.has_value() || sched->scalar_type() != at::kInt || sched_cum->scalar_type() != at::kInt) return refuse(kMlaSchedule);
+    if (sched->size(0) != r.parts || sched_cum->numel() != B + 1) return refuse(kMlaOtherSchedule);
+    a.sched_meta = sched->data_ptr<int32_t>();
+    a.sched_num_splits = sched_cum->data_ptr<int32_t>();
+    a.sched_parts = r.parts;
+  }
+  if (table.defined()) {
+    a.block_table = table.data_ptr<int32_t>();
+    a.block_table_stride = table.stride(0);
+    a.page_size = kv.size(1);
+    a.num_pages = kv.size(0);
+  }
+  check(api.mla_decode(&a, stream_of(q)), "attn_b200_mla_decode");
+  return r;
+}
+
+// (o, lse, splits, parts), or the number of a refusal.
+py::object mla_decode_call(const Tensor& q, const Tensor& kv, int64_t dim_v, double scale, const OptTensor& q_rope, const OptTensor& kv_rope,
+                           c10::optional<int64_t> num_splits, const OptTensor& workspace, const OptTensor& lens, const OptTensor& table,
+                           c10::optional<int64_t> max_seqlen, const OptTensor& sched, const OptTensor& sched_cum) {
+  MlaResult r;
+  {
+    py::gil_scoped_release others_run;
+    at::AutoDispatchBelowADInplaceOrView below;
+    r = mla_decode(q, kv, dim_v, scale, q_rope, kv_rope, num_splits, workspace, lens, table, max_seqlen, sched, sched_cum);
+  }
+  if (r.refusal != 0) return py::int_(r.refusal);
+  return py::make_tuple(r.o, r.lse, r.num_splits, r.parts);
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -619,4 +887,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("kv_splits", &kv_splits_for);
   m.def("splits_on", &splits_on);
   m.def("fault", &fault);
+  m.def("linear_forward", &linear_forward_call);
+  m.def("linear_decay_grad", &linear_decay_grad);
+  m.def("rows_sum_cast", &rows_sum_cast);
+  m.def("mla_decode", &mla_decode_call);
 }

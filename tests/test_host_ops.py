@@ -159,3 +159,25 @@ def test_a_host_side_of_other_sources_is_not_loaded(host, monkeypatch, tmp_path)
     with monkeypatch.context() as m:
         m.setattr(torch, "__version__", "0.0")
         assert lib.host_path() != host.__file__
+
+
+def test_refusals_of_linear_and_mla_calls_keep_their_errors():
+    """Shapes, types and devices that the native host side refuses, before anything is launched."""
+    from attn_engine.linear_attn_engine import linear_attention_forward
+    from attn_engine.mla import mla_decode_forward
+    from core.native.lib import NativeError
+    q, k, v, g = torch.zeros(2, 2, 64, 64), torch.zeros(2, 2, 64, 64), torch.zeros(2, 4, 64, 128), torch.zeros(2, 4, 64)
+    with pytest.raises(NativeError, match="needs CUDA tensors"):
+        linear_attention_forward(q, k, v, g)
+    with pytest.raises(NativeError, match="do not fit together"):
+        linear_attention_forward(q, k[:1], v, g)
+    with pytest.raises(ValueError):
+        linear_attention_forward(q[0], k, v, g)
+    with pytest.raises(NativeError, match="out_dtype"):
+        linear_attention_forward(q, k, v, g, out_dtype=torch.float64)
+    with pytest.raises(NativeError, match="needs CUDA tensors"):
+        mla_decode_forward(torch.zeros(2, 128, 576), torch.zeros(2, 64, 576), 512, 1.0)
+    with pytest.raises(ValueError, match="q: expected a singleton axis"):
+        mla_decode_forward(torch.zeros(2, 2, 128, 576), torch.zeros(2, 64, 576), 512, 1.0)
+    with pytest.raises(ValueError, match="kv: expected .batch, rows, cols. with contiguous columns"):
+        mla_decode_forward(torch.zeros(2, 128, 576), torch.zeros(2, 576, 64).transpose(1, 2), 512, 1.0)
