@@ -17,9 +17,11 @@
 //     unit through tensor memory (both accumulators of a row are in the lane of its thread).  With one group the warp that
 //     holds the only used rows is the bound: ~1600 cycles a tile, against 1480 for the bytes of a 64-wide tile;
 //   * K and V each have a ring of 96 KB: ~190 KB in flight per SM, three times what latency times bandwidth asks for.
-// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 127 -> 95-102 us = 5.3-5.6 TB/s of K
-// and V; 8 sequences x 32 heads on 8 KV heads, up to 8192 tokens, 30 % of the 32-token blocks kept 212 -> 39 us.  8 such
-// sequences of 16384 tokens: dense 5.8 TB/s, every block kept (the gather) 3.9; of 32768, 30 % kept: 2.7.
+// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 94 us = 5.7 TB/s of K and V, x 4312
+// tokens 23.7 (25.2 before the first loads went ahead of the CTA's set-up and the merge kernel fetched its code early); 8
+// sequences x 32 heads on 8 KV heads, up to 8192 tokens, 30 % of the 32-token blocks kept 38 -> 30: of its 26 us in the
+// kernel 8 went to counting the mask at four flags a load, 2 to a list of kept blocks made the same way, 2 to boxes issued
+// by one lane.  8 such sequences of 16384 tokens, dense: 5.8 TB/s.
 // A unit that is a whole (sequence, KV head) pair writes its output; the others leave fp32 partial rows that a second
 // small kernel adds up, launched early (programmatic dependent launch) so that only its own microseconds show.
 #include <cstring>
@@ -119,6 +121,25 @@ struct DecodeWalk {
   }
 };
 
+// Flags [i, i + 16) of a mask row as bits, those from `n` on as zeros; `wide`: the row may be read sixteen flags at a time.
+__device__ __forceinline__ uint32_t dec_flags16(const uint8_t* row, int i, int n, bool wide) {
+  uint32_t m = 0;
+  if (wide) {
+    if (i < n) {   // rows are whole pieces of sixteen
+      const uint4 v = *reinterpret_cast<const uint4*>(row + i);
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) m |= ((__vsetne4(w[k], 0u) * 0x10204080u) >> 28) << (4 * k);   // four bytes of 0 / 1 to four bits
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+      if (i + k < n && row[i + k] != 0) m |= 1u << k;
+  }
+  const int in = min(max(n - i, 0), 16);
+  return m & ((1u << in) - 1u);
+}
+
 template <int D, bool kBf16, bool kCounted>
 __global__ void __launch_bounds__(kDecThreads, 1)
 decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
@@ -149,8 +170,19 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge kernel may be made ready
 
-  if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+  const int per_pair = (p.seq_kv + N - 1) / N;
+  const int cta = static_cast<int>(blockIdx.x);
+  // The loading lane sets the barriers up; without counts to wait for it sends the first loads off at once, under the
+  // tensor-memory allocation and the CTA-wide sync.  (If the status word turns out set nobody takes them, and the teardown
+  // below gives them time to land.)
+  auto load_q = [&](int buf, int pair) {
+    const int b = pair / p.heads_kv, hk = pair - b * p.heads_kv;
+    mbar_arrive_expect_tx(bars + L::kQFull + buf, KC * p.rows * 128);
+    for (int c = 0; c < KC; ++c)
+      tma_load_rows(sQ + buf * p.q_bytes + c * (p.rows_pad * 128), &tmQ, bars + L::kQFull + buf, c * 64, 0, hk * p.group, b, p.oq);
+  };
+  int early = 0;   // tiles of the first unit on their way
+  if (warp == 8 && lane == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(bars + L::kQFull + i, 1);
       mbar_init(bars + L::kQEmpty + i, 1);
@@ -167,42 +199,54 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       mbar_init(bars + L::kVEmpty + i, 1);
     }
     fence_barrier_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
+    if constexpr (!kCounted) {
+      const int total = pairs * per_pair, shares = min(static_cast<int>(gridDim.x), total);
+      if (cta < shares) {
+        DecodeWalk u(nullptr, nullptr, pairs, per_pair, p.seq_kv, dec_share(total, cta, shares), dec_share(total, cta + 1, shares));
+        u.next();
+        load_q(0, u.pair);
+        const int b = u.pair / p.heads_kv, hk = u.pair - b * p.heads_kv;
+        early = min(u.n, ST);
+#pragma unroll 1
+        for (int i = 0; i < early; ++i) {
+          mbar_arrive_expect_tx(bars + L::kKFull + i, L::kTileBytes);
+          mbar_arrive_expect_tx(bars + L::kVFull + i, L::kTileBytes);
+          for (int c = 0; c < KC; ++c)
+            tma_load_rows(sK + i * L::kTileBytes + c * kChunk, &tmK, bars + L::kKFull + i, c * 64, (u.t0 + i) * N, hk, b, p.ok);
+          for (int c = 0; c < KC; ++c)
+            tma_load_rows(sV + i * L::kTileBytes + c * kChunk, &tmV, bars + L::kVFull + i, c * 64, (u.t0 + i) * N, hk, b, p.ov);
+        }
+      }
+    } else {
+      tma_prefetch_desc(&tmQ);
+      tma_prefetch_desc(&tmK);
+      tma_prefetch_desc(&tmV);
+    }
   }
+  if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
   // ---- how many KV rows of every pair take part, and the tiles in front of it ----
+  const bool wide = sparse && (p.n_blocks & 15) == 0 && (reinterpret_cast<uintptr_t>(p.block_mask) & 15) == 0;
   if constexpr (kCounted) {
     auto len_of = [&](int b) { return p.seq_lens != nullptr ? min(max(p.seq_lens[b], 0), p.seq_kv) : p.seq_kv; };
     if (sparse) {
       for (int i = tid; i < pairs; i += kDecThreads) s_valid[i] = 0;
       __syncthreads();
-      // Four flags per item (the mask row is read as words where it is a multiple of four); the items of a thread are
-      // independent loads.
-      const int wpr = (p.n_blocks + 3) / 4;
-      const bool words = (p.n_blocks & 3) == 0 && (reinterpret_cast<uintptr_t>(p.block_mask) & 3) == 0;
+      // Sixteen flags per item; the items of a thread are independent loads, all of them in flight at once where there
+      // are no more than four (64 rows of 256 flags: 5.4 k cycles, 12.4 k at four flags an item)
+      const int ipr = (p.n_blocks + 15) / 16;
 #pragma unroll 4
-      for (int i = tid; i < pairs * wpr; i += kDecThreads) {
-        const int pair = i / wpr, w = i - pair * wpr;
+      for (int i = tid; i < pairs * ipr; i += kDecThreads) {
+        const int pair = i / ipr, at = 16 * (i - pair * ipr);
+        const uint32_t m = dec_flags16(p.block_mask + static_cast<long long>(pair) * p.n_blocks, at, p.n_blocks, wide);
         const int len = len_of(pair / p.heads_kv);
         const int nb = min(p.n_blocks, (len + p.block - 1) / p.block);   // blocks that begin inside the sequence
-        const uint8_t* row = p.block_mask + static_cast<long long>(pair) * p.n_blocks;
-        uint32_t f = 0;
-        if (words) {
-          f = __vsetne4(*reinterpret_cast<const uint32_t*>(row + 4 * w), 0u);
-        } else {
-          for (int k = 0; k < 4; ++k)
-            if (4 * w + k < p.n_blocks) f |= static_cast<uint32_t>(row[4 * w + k] != 0) << (8 * k);
-        }
-        const int in = min(max(nb - 4 * w, 0), 4);
-        f = in == 4 ? f : f & ((1u << (8 * in)) - 1u);
-        const int last = nb - 1 - 4 * w;   // the sequence's last block, which may be cut by its end
-        int r = __popc(f) * p.block;
-        if (last >= 0 && last < 4 && ((f >> (8 * last)) & 1u)) r -= max(nb * p.block - len, 0);
+        const int in = min(max(nb - at, 0), 16), last = nb - 1 - at;     // the sequence's last block may be cut by its end
+        int r = __popc(m & ((1u << in) - 1u)) * p.block;
+        if (last >= 0 && last < 16 && ((m >> last) & 1u)) r -= max(nb * p.block - len, 0);
         if (r > 0) atomicAdd(&s_valid[pair], r);
       }
       __syncthreads();
@@ -230,10 +274,8 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const int per_pair = (p.seq_kv + N - 1) / N;
   const int total = kCounted ? s_cum[pairs] : pairs * per_pair;
   const int shares = min(static_cast<int>(gridDim.x), total);   // none is empty
-  const int cta = static_cast<int>(blockIdx.x);
   const int T0 = cta < shares ? dec_share(total, cta, shares) : 0, T1 = cta < shares ? dec_share(total, cta + 1, shares) : 0;
   if (kCounted && blockIdx.x == 0)
     for (int i = tid; i <= pairs; i += kDecThreads) p.cum[i] = s_cum[i];
@@ -242,8 +284,9 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   if (warp == 8) {
     // ======================= loading warp =======================
-    if (run_cta) {
+    if (__all_sync(0xffffffffu, run_cta)) {
       DecodeWalk u = make_walk();
+      const int n_early = __shfl_sync(0xffffffffu, early, 0);
       bool ok = true;
       int J = 0;
       for (int ui = 0; ok && u.next(); ++ui) {
@@ -251,19 +294,17 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         const int bpt = sparse ? N / p.block : 1;
         int kept_here = 0;
         if (sparse) {
-          // ranks [t0 * bpt, (t0 + n) * bpt) of the row's kept blocks, four flags per lane and step
+          // ranks [t0 * bpt, (t0 + n) * bpt) of the row's kept blocks, sixteen flags per lane and step
           const uint8_t* row = p.block_mask + static_cast<long long>(u.pair) * p.n_blocks;
           const int len = p.seq_lens != nullptr ? min(max(p.seq_lens[b], 0), p.seq_kv) : p.seq_kv;
           const int nb = min(p.n_blocks, (len + p.block - 1) / p.block);
           const int r0 = u.t0 * bpt, r1 = r0 + u.n * bpt;
-          __syncwarp();   // lane 0 has read the previous unit's list
+          __syncwarp();   // the previous unit's list has been read
           int rank = 0;
-          for (int base = 0; base < nb && rank < r1; base += 128) {
-            const int i0 = base + 4 * lane;
-            uint32_t flags = 0;
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (i0 + k < nb && row[i0 + k] != 0) flags |= 1u << k;
+          for (int base = 0; base < p.n_blocks && rank < r1; base += 512) {
+            const int i0 = base + 16 * lane;
+            uint32_t flags = dec_flags16(row, i0, p.n_blocks, wide);   // does not wait for the length
+            flags &= (1u << min(max(nb - i0, 0), 16)) - 1u;
             const int mine = __popc(flags);
             int x = mine;
 #pragma unroll
@@ -272,51 +313,41 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
               if (lane >= d) x += y;
             }
             int r = rank + x - mine;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              if ((flags >> k) & 1u) {
-                if (r >= r0 && r < r1) s_list[r - r0] = static_cast<uint16_t>(i0 + k);
-                ++r;
-              }
-            }
+            for (; flags != 0; flags &= flags - 1, ++r)
+              if (r >= r0 && r < r1) s_list[r - r0] = static_cast<uint16_t>(i0 + __ffs(flags) - 1);
             rank += __shfl_sync(0xffffffffu, x, 31);
           }
           kept_here = min(rank, r1) - r0;
           __syncwarp();
         }
-        if (lane == 0) {
-          const int qb = ui % p.q_bufs;
-          if (ui >= p.q_bufs) ok = mbar_wait(bars + L::kQEmpty + qb, (ui / p.q_bufs - 1) & 1, ab, kDecQEmpty);
-          if (ok) {
-            mbar_arrive_expect_tx(bars + L::kQFull + qb, KC * p.rows * 128);
-            for (int c = 0; c < KC; ++c)
-              tma_load_rows(sQ + qb * p.q_bytes + c * (p.rows_pad * 128), &tmQ, bars + L::kQFull + qb, c * 64, 0, hk * p.group, b, p.oq);
-          }
-          for (int i = 0; i < u.n && ok; ++i) {
-            const int jj = J + i, st = jj % ST;
-            const uint32_t par = ((jj / ST) & 1) ^ 1;
-            for (int kv = 0; kv < 2 && ok; ++kv) {
-              uint64_t* full = bars + (kv == 0 ? L::kKFull : L::kVFull) + st;
-              ok = mbar_wait(bars + (kv == 0 ? L::kKEmpty : L::kVEmpty) + st, par, ab, kv == 0 ? kDecKEmpty : kDecVEmpty);
-              if (!ok) break;
-              uint8_t* dst = (kv == 0 ? sK : sV) + st * L::kTileBytes;
-              const CUtensorMap* tm = kv == 0 ? &tmK : &tmV;
-              const CoordOrder& ord = kv == 0 ? p.ok : p.ov;
-              mbar_arrive_expect_tx(full, L::kTileBytes);
-              if (sparse) {
-                // slots past the last kept block repeat it: masked, but what lies there is multiplied by zero
-                for (int s = 0; s < bpt; ++s) {
-                  const int r = s_list[min(i * bpt + s, kept_here - 1)] * p.block;
-                  for (int c = 0; c < KC; ++c) tma_load_rows(dst + c * kChunk + s * p.block * 128, tm, full, c * 64, r, hk, b, ord);
-                }
-              } else {
-                for (int c = 0; c < KC; ++c) tma_load_rows(dst + c * kChunk, tm, full, c * 64, (u.t0 + i) * N, hk, b, ord);
-              }
+        // A tile's boxes are spread over the lanes: K's and V's bpt blocks of KC column chunks (at most 32 boxes; one lane
+        // issuing all of them, sixteen a tile with blocks of 32, took 3100 cycles a tile against 2400 for its bytes)
+        const int qb = ui % p.q_bufs;
+        if (ui >= p.q_bufs) ok = mbar_wait(bars + L::kQEmpty + qb, (ui / p.q_bufs - 1) & 1, ab, kDecQEmpty);
+        if (lane == 0 && ok && (kCounted || ui > 0)) load_q(qb, u.pair);
+        const int blk = lane / KC, chunk = lane - blk * KC;
+        for (int i = 0; i < u.n && ok; ++i) {
+          const int jj = J + i, st = jj % ST;
+          if (!kCounted && jj < n_early) continue;
+          const uint32_t par = ((jj / ST) & 1) ^ 1;
+          // slots past the last kept block repeat it: masked, but what lies there is multiplied by zero
+          const int r = sparse ? s_list[min(i * bpt + blk, kept_here - 1)] * p.block : (u.t0 + i) * N;
+          const int off = st * L::kTileBytes + chunk * kChunk + (sparse ? blk * p.block * 128 : 0);
+          for (int kv = 0; kv < 2 && ok; ++kv) {
+            uint64_t* full = bars + (kv == 0 ? L::kKFull : L::kVFull) + st;
+            ok = mbar_wait(bars + (kv == 0 ? L::kKEmpty : L::kVEmpty) + st, par, ab, kv == 0 ? kDecKEmpty : kDecVEmpty);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            if (lane == 0) mbar_arrive_expect_tx(full, L::kTileBytes);
+            __syncwarp();
+            if (blk < bpt) {
+              if (kv == 0) tma_load_rows(sK + off, &tmK, full, chunk * 64, r, hk, b, p.ok);
+              else tma_load_rows(sV + off, &tmV, full, chunk * 64, r, hk, b, p.ov);
             }
           }
         }
         J += u.n;
-        if (sparse) ok = __all_sync(0xffffffffu, ok);
+        ok = __all_sync(0xffffffffu, ok);
       }
     }
   } else if (warp == 9) {
@@ -462,14 +493,21 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       // a partial result: the pair's first share leaves it in the second slot of its CTA, the later ones in the first
       const long long slot = (2LL * blockIdx.x + (u.t0 == 0 ? 1 : 0)) * p.rows + row;
       uint16_t* orow = static_cast<uint16_t*>(p.o) + b * p.o_sb + qi * p.o_ss + h * p.o_sh;
-#pragma unroll
+      // not unrolled: it runs once or twice a call, and fetching 13 KB of code for it took 2700 cycles
+#pragma unroll 1
       for (int c = 0; c < D / 32; ++c) {
         float a0[32], a1[32];
         tmem_ld32f(tO + c * 32, a0);
         tmem_ld32f(tO + D + c * 32, a1);
         tmem_wait_ld();
+        if (has0 && has1) {   // an accumulator that the unit has not used holds anything
 #pragma unroll
-        for (int i = 0; i < 32; ++i) a0[i] = (has0 ? a0[i] * f0 : 0.0f) + (has1 ? a1[i] * f1 : 0.0f);
+          for (int i = 0; i < 32; ++i) a0[i] = fmaf(a0[i], f0, a1[i] * f1);
+        } else {
+          const float f = has0 ? f0 : f1;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) a0[i] = (has0 ? a0[i] : a1[i]) * f;
+        }
         if (row < p.rows) {
           if (whole) {
 #pragma unroll
@@ -513,50 +551,88 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // that one CTA held whole were written by it; a pair without a kept row gets what an empty softmax is (nan, -inf).
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p, int ctas, int counted) {
-  asm volatile("griddepcontrol.wait;" ::: "memory");   // the decode kernel's results are complete and visible
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int pairs = p.batch * p.heads_kv;
   if (w >= pairs * p.rows) return;
   const int pair = w / p.rows, row = w - pair * p.rows;
   const int per = (p.seq_kv + kDecTile - 1) / kDecTile;
-  const int total = counted ? p.cum[pairs] : pairs * per;
-  const int shares = min(ctas, total);
-  const int first = counted ? p.cum[pair] : pair * per, end = counted ? p.cum[pair + 1] : first + per;
-  const int c_lo = end > first ? dec_owner(first, shares, total) : 0, c_hi = end > first ? dec_owner(end - 1, shares, total) : -1;
-  if (c_lo == c_hi) return;
-  auto slot_of = [&](int c) { return (2LL * c + (c == c_lo ? 1 : 0)) * p.rows + row; };
-  float mx = -INFINITY;
-  for (int c = c_lo + lane; c <= c_hi; c += 32) mx = fmaxf(mx, p.part_lse[slot_of(c)]);
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-  float den = 0.0f;
-  for (int c = c_lo + lane; c <= c_hi; c += 32) den += __expf(p.part_lse[slot_of(c)] - mx);
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) den += __shfl_xor_sync(0xffffffffu, den, d);
-  constexpr int E = D / 32;
-  float acc[E];
-#pragma unroll
-  for (int e = 0; e < E; ++e) acc[e] = 0.0f;
-#pragma unroll 4
-  for (int c = c_lo; c <= c_hi; ++c) {
-    const long long slot = slot_of(c);
-    const float wgt = __expf(p.part_lse[slot] - mx);
-    const float* src = p.part_o + slot * D + lane * E;
-#pragma unroll
-    for (int e = 0; e < E; e += 2) {
-      const float2 x = *reinterpret_cast<const float2*>(src + e);
-      acc[e] = fmaf(wgt, x.x, acc[e]);
-      acc[e + 1] = fmaf(wgt, x.y, acc[e + 1]);
-    }
-  }
-  const float inv = 1.0f / den;   // no partial result at all: 0 * inf
   const int g = p.head_major ? row / p.seq_q : row % p.group, qi = p.head_major ? row % p.seq_q : row / p.group;
   const int b = pair / p.heads_kv, h = (pair - b * p.heads_kv) * p.group + g;
+  constexpr int E = D / 32;
   uint16_t* orow = static_cast<uint16_t*>(p.o) + b * p.o_sb + qi * p.o_ss + h * p.o_sh + lane * E;
+  // The blocks of this kernel stand ready while the decode kernel still runs.  A first pass over the same code, on scratch
+  // that is not written yet and without a store, fetches the instructions and page translations meanwhile: the pass that
+  // counts took 4 to 5 us without it, behind the decode kernel's end.  All reads pass L1 by, so nothing stale is kept there.
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool real = pass == 1;
+    if (real) asm volatile("griddepcontrol.wait;" ::: "memory");   // the decode kernel's results are complete and visible
+    int total = pairs * per, first = pair * per, end = first + per;
+    if (counted) {
+      total = __ldcg(p.cum + pairs);
+      first = __ldcg(p.cum + pair);
+      end = __ldcg(p.cum + pair + 1);
+    }
+    const int shares = min(ctas, total);
+    int c_lo = 0, c_hi = -1;
+    if (end > first && shares > 0) {
+      c_lo = dec_owner(first, shares, total);
+      c_hi = dec_owner(end - 1, shares, total);
+    }
+    if (!real) {   // what the counts say is not to be relied on yet: two slots that exist
+      c_lo = 0;
+      c_hi = min(1, ctas - 1);
+    } else if (c_lo == c_hi) {
+      return;
+    }
+    auto slot_of = [&](int c) { return (2LL * c + (c == c_lo ? 1 : 0)) * p.rows + row; };
+    // Four shares at a time, their statistics and rows loaded together (one after the other they are two round trips to
+    // memory), added up against a running maximum.
+    float mx = -INFINITY, den = 0.0f;
+    float acc[E];
 #pragma unroll
-  for (int e = 0; e < E; e += 2) *reinterpret_cast<uint32_t*>(orow + e) = pack2<kBf16>(acc[e] * inv, acc[e + 1] * inv);
-  if (lane == 0 && p.lse != nullptr)
-    p.lse[(static_cast<long long>(b) * p.heads + h) * p.seq_q + qi] = end > first ? mx + logf(den) : -INFINITY;
+    for (int e = 0; e < E; ++e) acc[e] = 0.0f;
+#pragma unroll 1
+    for (int c0 = c_lo; c0 <= c_hi; c0 += 4) {
+      float l[4], x[4][E];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool in = c0 + k <= c_hi;
+        const long long slot = slot_of(in ? c0 + k : c_hi);
+        const float* src = p.part_o + slot * D + lane * E;
+        l[k] = __ldcg(p.part_lse + slot);
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+          const float2 v = __ldcg(reinterpret_cast<const float2*>(src + e));
+          x[k][e] = v.x;
+          x[k][e + 1] = v.y;
+        }
+        if (!in) l[k] = -INFINITY;
+      }
+      const float m = fmaxf(mx, fmaxf(fmaxf(l[0], l[1]), fmaxf(l[2], l[3])));
+      const float old = __expf(mx - m);
+      den *= old;
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[e] *= old;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool in = c0 + k <= c_hi;
+        const float wgt = in ? __expf(l[k] - m) : 0.0f;
+        den += wgt;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] = in ? fmaf(wgt, x[k][e], acc[e]) : acc[e];
+      }
+      mx = m;
+    }
+    const float inv = 1.0f / den;   // no partial result at all: 0 * inf
+    const float lse = end > first ? mx + logf(den) : -INFINITY;
+#pragma unroll
+    for (int e = 0; e < E; e += 2) {
+      const uint32_t two = pack2<kBf16>(acc[e] * inv, acc[e + 1] * inv);
+      if (real) *reinterpret_cast<uint32_t*>(orow + e) = two;
+    }
+    if (real && lane == 0 && p.lse != nullptr) p.lse[(static_cast<long long>(b) * p.heads + h) * p.seq_q + qi] = lse;
+  }
 }
 
 struct DecodePlan {

@@ -86,6 +86,8 @@ def decode_engine(B, H, Hkv, Sq, S, D, block):
     (4, 32, 4, 1, 4096, 128, 64, True, True),
     (70, 8, 4, 1, 640, 64, 128, True, True),       # more pairs than SMs
     (6, 8, 2, 2, 2000, 128, 32, False, True),      # lengths only
+    (2, 4, 2, 1, 5120, 64, 8, True, True),         # 640 blocks: a row's list takes two steps of 512 flags
+    (2, 4, 2, 1, 4808, 128, 8, True, True),        # 601 blocks, byte by byte
     (2, 4, 2, 1, 960, 64, 48, True, True),         # a block that does not divide a tile: left to the forward kernel
     (2, 8, 1, 9, 640, 128, 32, True, True),        # 72 rows with a block mask: left to the forward kernel
 ])
@@ -112,6 +114,8 @@ def test_blocks_and_lengths(B, H, Hkv, Sq, S, D, block, masked, varlen):
     some = keep.any(-1).repeat_interleave(H // Hkv, 1)     # [B, H]
     assert torch.isnan(o.transpose(1, 2)[~some]).all() and (lse[~some] == -float("inf")).all()
     check((o.transpose(1, 2)[some], lse[some]), (want_o.transpose(1, 2)[some], want_lse[some]), dtype)
+    if masked:   # a mask that does not begin on a 16-byte boundary is read byte by byte
+        mask = torch.cat([mask.new_zeros(1), mask.flatten()])[1:].view(mask.shape)
     again = run(eng, q, k, v, block_mask=mask, cache_seqlens=lens)
     assert torch.equal(o.nan_to_num(7.0), again[0].nan_to_num(7.0)) and torch.equal(lse, again[1])
     assert lib.last_device_status() == 0
