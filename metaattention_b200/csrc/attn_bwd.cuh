@@ -188,6 +188,8 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const AbortState ab{abort_flag, p.status};
+  pdl_launch_dependents();
+  if constexpr (kBits) pdl_wait();   // the tile bitmaps are read right away
   const int nq = (p.seq_q + T - 1) / T, nk = (p.seq_kv + T - 1) / T;
   // The streamed tiles are those the band q_idx - left <= kv_idx <= q_idx + right lets the resident tile meet: KV tiles
   // [j0, j0 + n_iter) for a query tile; for a KV tile the query tiles [i0, i0 + per_head) of every query head of its
@@ -208,7 +210,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   const int n_iter = kRoleQ ? (walk_tiles ? n_kept : max(j1 - j0 + 1, 0)) : p.kv_group * per_head;
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
+    *abort_flag = 0;
     // the operand tiles use the 128-byte swizzle, whose pattern repeats every 1024 bytes of the shared window
     if ((smem_u32(smem) & 1023u) != 0) {
       *abort_flag = 1;
@@ -240,11 +242,14 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmDO);
+    pdl_wait();
+    if (*reinterpret_cast<volatile int*>(p.status) != 0) *abort_flag = 1;
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -657,8 +662,7 @@ int launch_attn_bwd(const BwdCall& a, cudaStream_t stream, int* status) {
   }
   const long long ctas = (static_cast<long long>(nk) * a.heads_kv + static_cast<long long>(nq) * a.heads) * a.batch;
   if (ctas > 0x7fffffffLL) return ATTN_B200_E_UNSUPPORTED;
-  kernel<<<static_cast<unsigned>(ctas), kBwdThreads, L::kBytes, stream>>>(tmQ, tmK, tmV, tmDO, p);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, dim3(static_cast<unsigned>(ctas)), dim3(kBwdThreads), L::kBytes, stream, tmQ, tmK, tmV, tmDO, p)) return ATTN_B200_E_LAUNCH;
   return ATTN_B200_OK;
 }
 

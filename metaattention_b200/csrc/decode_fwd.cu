@@ -168,7 +168,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int active_warps = (p.rows + 31) / 32;   // of each softmax group
   const bool sparse = kCounted && p.block_mask != nullptr;
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the merge kernel may be made ready
+  pdl_launch_dependents();   // the merge kernel may be made ready
 
   const int per_pair = (p.seq_kv + N - 1) / N;
   const int cta = static_cast<int>(blockIdx.x);
@@ -200,6 +200,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     }
     fence_barrier_init();
     if constexpr (!kCounted) {
+      pdl_wait();
       const int total = pairs * per_pair, shares = min(static_cast<int>(gridDim.x), total);
       if (cta < shares) {
         DecodeWalk u(nullptr, nullptr, pairs, per_pair, p.seq_kv, dec_share(total, cta, shares), dec_share(total, cta + 1, shares));
@@ -223,11 +224,12 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tma_prefetch_desc(&tmV);
     }
   }
-  if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
+  if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   // ---- how many KV rows of every pair take part, and the tiles in front of it ----
   const bool wide = sparse && (p.n_blocks & 15) == 0 && (reinterpret_cast<uintptr_t>(p.block_mask) & 15) == 0;
   if constexpr (kCounted) {
@@ -551,9 +553,10 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // that one CTA held whole were written by it; a pair without a kept row gets what an empty softmax is (nan, -inf).
 template <int D, bool kBf16>
 __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p, int ctas, int counted) {
+  pdl_launch_dependents();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int pairs = p.batch * p.heads_kv;
-  if (w >= pairs * p.rows) return;
+  if (w >= pairs * p.rows) return;   // (the block's first warp never does)
   const int pair = w / p.rows, row = w - pair * p.rows;
   const int per = (p.seq_kv + kDecTile - 1) / kDecTile;
   const int g = p.head_major ? row / p.seq_q : row % p.group, qi = p.head_major ? row % p.seq_q : row / p.group;
@@ -566,7 +569,7 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p,
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     const bool real = pass == 1;
-    if (real) asm volatile("griddepcontrol.wait;" ::: "memory");   // the decode kernel's results are complete and visible
+    if (real) pdl_wait();   // the decode kernel's results are complete and visible
     int total = pairs * per, first = pair * per, end = first + per;
     if (counted) {
       total = __ldcg(p.cum + pairs);
@@ -718,26 +721,12 @@ int launch_decode(const AttnB200DecodeArgs* a, const DecodePlan& d, cudaStream_t
     cudaGetLastError();
     return ATTN_B200_E_LAUNCH;
   }
-  kernel<<<d.ctas, kDecThreads, L::kBytes, stream>>>(tmQ, tmK, tmV, p);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, dim3(d.ctas), dim3(kDecThreads), L::kBytes, stream, tmQ, tmK, tmV, p)) return ATTN_B200_E_LAUNCH;
   const long long pairs = static_cast<long long>(a->batch) * a->heads_kv;
   // every share of a dense call is whole pairs: nothing to merge
   if (!d.counted && pairs % d.ctas == 0) return ATTN_B200_OK;
-  cudaLaunchConfig_t cfg;
-  std::memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(static_cast<unsigned>((pairs * d.rows + 3) / 4));
-  cfg.blockDim = dim3(128);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, decode_merge_kernel<D, kBf16>, p, d.ctas, d.counted ? 1 : 0) != cudaSuccess) {
-    cudaGetLastError();
-    return ATTN_B200_E_LAUNCH;
-  }
-  return ATTN_B200_OK;
+  const dim3 merge_grid(static_cast<unsigned>((pairs * d.rows + 3) / 4));
+  return launch_pdl(decode_merge_kernel<D, kBf16>, merge_grid, dim3(128), 0, stream, p, d.ctas, d.counted ? 1 : 0) ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
 }
 
 }  // namespace b200

@@ -169,7 +169,6 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int bh_q = b_idx * p.heads_q + h_idx / (p.heads / p.heads_q), bh_k = b_idx * p.heads_k + h_idx / (p.heads / p.heads_k);
 
   if (tid == 0) {
-    *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     mbar_init(q_full, 1);
     mbar_init(k_full, 1);
     mbar_init(v_full, 1);
@@ -196,6 +195,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
+  if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -796,6 +797,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (lane == 0) tma_store_wait_all();   // the staged rows of the last block are still being read
   }
 
+  pdl_launch_dependents();   // not at the start: 2 x 8 x 2000 training step 213.5 us so, 210.8 from here
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {
@@ -973,8 +975,7 @@ int launch_linear(const AttnB200LinearArgs* a, cudaStream_t stream, int* status)
     return ATTN_B200_E_LAUNCH;
   }
   dim3 grid(slices, static_cast<unsigned>(pair ? bh / 2 : bh), segments);
-  kernel<<<grid, kLinThreads, L::kBytes, stream>>>(tmQ, tmK, tmV, tmO, p);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, grid, dim3(kLinThreads), L::kBytes, stream, tmQ, tmK, tmV, tmO, p)) return ATTN_B200_E_LAUNCH;
   if (a->normalize) {
     const int blocks = static_cast<int>((rows * 32 + 255) / 256);
     if (f32_out) linear_norm_f32_kernel<<<blocks, 256, 0, stream>>>(p.o_f32, p.stats, rows, a->dim_v, a->norm_eps);

@@ -217,6 +217,8 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();       // 0 = score CTA, 1 = value CTA
+  pdl_launch_dependents();
+  pdl_wait();   // the units are read from memory right away
   const AbortState ab{abort_flag, p.status};
   // scheduled mode: blockIdx.y = head block * parts + part; uniform splits: blockIdx.y = head block * splits + split
   const int per_hb = p.sched != nullptr ? p.num_parts : p.num_splits;
@@ -754,9 +756,11 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
 // The partial rows of sequence b are rows [cum[b], cum[b+1]) of part_o / part_lse (scheduled mode; a sequence with one
 // row was written directly by the decode kernel and is skipped), or rows [b*num_splits, (b+1)*num_splits) (cum == null).
 template <int DV, bool kBf16>
-__global__ void __launch_bounds__(256) mla_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_lse,
-                                                        void* __restrict__ o, float* __restrict__ lse_out, int batch,
-                                                        int heads, int uniform_splits, const int* __restrict__ cum) {
+__global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, const float* part_lse,
+                                                        void* o, float* lse_out, int batch,
+                                                        int heads, int uniform_splits, const int* cum) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= batch * heads) return;
@@ -807,8 +811,10 @@ __global__ void __launch_bounds__(256) mla_combine_kernel(const float* __restric
 // remaining payload and then as many tiles of the next one as are left beyond the overhead.  Record of a part: first
 // sequence, first token, last sequence (inclusive), end token (exclusive), split index of its first unit, KV tiles.
 // cum[b] = partial-result rows in front of sequence b.  One warp; the walk itself is serial.
-__global__ void __launch_bounds__(32) mla_schedule_kernel(const int* __restrict__ seq_lens, int batch, int seq_kv, int parts,
-                                                        int* __restrict__ sched, int* __restrict__ cum) {
+__global__ void __launch_bounds__(32) mla_schedule_kernel(const int* seq_lens, int batch, int seq_kv, int parts,
+                                                        int* sched, int* cum) {
+  pdl_launch_dependents();
+  pdl_wait();
   auto tiles_of = [&](int b) {
     const int len = seq_lens != nullptr ? max(1, min(seq_lens[b], seq_kv)) : seq_kv;
     return (len + kMlaTileN - 1) / kMlaTileN;
@@ -977,8 +983,7 @@ int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
       p.sched = a->sched_meta;
       p.num_splits_cum = a->sched_num_splits;
     } else {
-      mla_schedule_kernel<<<1, 32, 0, stream>>>(a->seq_lens, s.batch, s.seq_kv, parts, sched, cum);
-      if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+      if (!launch_pdl(mla_schedule_kernel, dim3(1), dim3(32), 0, stream, a->seq_lens, s.batch, s.seq_kv, parts, sched, cum)) return ATTN_B200_E_LAUNCH;
       p.sched = sched;
       p.num_splits_cum = cum;
     }
@@ -996,14 +1001,13 @@ int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
     return ATTN_B200_E_LAUNCH;
   }
   if (grid.y > 65535) return ATTN_B200_E_UNSUPPORTED;
-  kernel<<<grid, kMlaThreads, kMlaSmemBytes, stream>>>(tmKV, tmKVr, tmV, tmQr, p);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, grid, dim3(kMlaThreads), kMlaSmemBytes, stream, tmKV, tmKVr, tmV, tmQr, p)) return ATTN_B200_E_LAUNCH;
   if (scheduled || splits > 1) {
     const long long warps = static_cast<long long>(s.batch) * s.heads_q;
     const int blocks = static_cast<int>((warps * 32 + 255) / 256);
-    mla_combine_kernel<DV, kBf16><<<blocks, 256, 0, stream>>>(p.part_o, p.part_lse, a->o, a->lse, s.batch, s.heads_q, splits,
-                                                             scheduled ? p.num_splits_cum : nullptr);
-    if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+    if (!launch_pdl(mla_combine_kernel<DV, kBf16>, dim3(blocks), dim3(256), 0, stream, p.part_o, p.part_lse, a->o, a->lse, s.batch, s.heads_q, splits,
+                    scheduled ? p.num_splits_cum : nullptr))
+      return ATTN_B200_E_LAUNCH;
   }
   return ATTN_B200_OK;
 }
@@ -1072,9 +1076,10 @@ int attn_b200_mla_metadata(const int32_t* cache_seqlens, int32_t batch, int32_t 
                            int32_t* tile_scheduler_metadata, int32_t* num_splits, void* cuda_stream) {
   if (tile_scheduler_metadata == nullptr || num_splits == nullptr || batch <= 0 || seq_kv <= 0 || num_parts <= 0)
     return ATTN_B200_E_INVALID_ARG;
-  b200::mla_schedule_kernel<<<1, 32, 0, static_cast<cudaStream_t>(cuda_stream)>>>(cache_seqlens, batch, seq_kv, num_parts,
-                                                                                 tile_scheduler_metadata, num_splits);
-  return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
+  return b200::launch_pdl(b200::mla_schedule_kernel, dim3(1), dim3(32), 0, static_cast<cudaStream_t>(cuda_stream), cache_seqlens, batch, seq_kv,
+                          num_parts, tile_scheduler_metadata, num_splits)
+             ? ATTN_B200_OK
+             : ATTN_B200_E_LAUNCH;
 }
 
 int64_t attn_b200_mla_workspace_bytes(const AttnB200MlaShape* shape, int32_t num_splits) {

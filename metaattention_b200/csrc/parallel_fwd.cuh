@@ -198,6 +198,8 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const AbortState ab{abort_flag, p.status};
+  pdl_launch_dependents();
+  if constexpr (kSparse) pdl_wait();   // the bitmaps are read right away
 
   // Every mask is a band kv_idx in [q_idx - left, q_idx + right]: none = open on both sides, causal = open
   // to the left with right = 0, sliding windows bound the left side as well.
@@ -307,6 +309,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(&o_done[t], 1);
     }
     fence_barrier_init();
+    pdl_wait();
     if (n_max > 0 && !kSparse) {
       // in the order of first use: query tile 0 and K so that its scores can start, then query tile 1, then V
       if (act0) load_q(0);
@@ -319,6 +322,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // round trip that the first loads do not wait for.  If it is set, nobody consumes those loads and the teardown
   // below gives them time to land.
   if (threadIdx.x == 0) {
+    pdl_wait();
     *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;
     // the operand tiles use the 128-byte swizzle, whose pattern repeats every 1024 bytes of the shared window
     if ((smem_u32(smem) & 1023u) != 0) {
@@ -330,6 +334,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
   }
+  pdl_wait();
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -712,10 +717,12 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 // of attn_decode_tl.py:158-206).  For the built-in softmax that is exp(lse_i - lse), lse = log sum_i exp(lse_i), and
 // the combined lse is written out as the call's final row scale.  One warp per (batch, head, query row).
 template <class F, int DV, bool kBf16>
-__global__ void __launch_bounds__(256) parallel_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_final,
-                                                             long long part_final_stride, void* __restrict__ o,
-                                                             float* __restrict__ final_out, int batch, int heads, int seq_q,
+__global__ void __launch_bounds__(256) parallel_combine_kernel(const float* part_o, const float* part_final,
+                                                             long long part_final_stride, void* o,
+                                                             float* final_out, int batch, int heads, int seq_q,
                                                              int splits, long long o_sb, long long o_ss, long long o_sh) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long row = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (row >= static_cast<long long>(batch) * heads * seq_q) return;

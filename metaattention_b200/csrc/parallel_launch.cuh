@@ -7,6 +7,7 @@
 #include <cstring>
 
 #include "../../include/attn_b200.h"
+#include "common_host.cuh"
 #include "parallel_fwd.cuh"
 
 namespace b200 {
@@ -181,15 +182,13 @@ int launch_parallel(const AttnB200ParallelArgs* a, cudaStream_t stream, int* dev
     return ATTN_B200_E_LAUNCH;
   }
   dim3 grid((a->seq_q + NT * L::kBM - 1) / (NT * L::kBM), a->heads, a->batch * splits);
-  kernel<<<grid, kParallelThreads<NT, kRowThreads<F>>, kSmem, stream>>>(tmQ, tmK, tmV, p);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, grid, dim3(kParallelThreads<NT, kRowThreads<F>>), kSmem, stream, tmQ, tmK, tmV, p)) return ATTN_B200_E_LAUNCH;
   if (splits > 1) {
     const long long rows = static_cast<long long>(a->batch) * a->heads * a->seq_q;
     const unsigned blocks = static_cast<unsigned>((rows * 32 + 255) / 256);
-    parallel_combine_kernel<F, DV, kBf16><<<blocks, 256, 0, stream>>>(p.part_o, p.part_final, p.part_final_stride, a->o,
-                                                                     a->final_rowscales[0], a->batch, a->heads, a->seq_q, splits,
-                                                                     p.o_sb, p.o_ss, p.o_sh);
-    if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+    if (!launch_pdl(parallel_combine_kernel<F, DV, kBf16>, dim3(blocks), dim3(256), 0, stream, p.part_o, p.part_final, p.part_final_stride, a->o,
+                    a->final_rowscales[0], a->batch, a->heads, a->seq_q, splits, p.o_sb, p.o_ss, p.o_sh))
+      return ATTN_B200_E_LAUNCH;
   }
   return ATTN_B200_OK;
 }

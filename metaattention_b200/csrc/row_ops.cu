@@ -6,12 +6,15 @@
 #include <cstdint>
 
 #include "../../include/attn_b200.h"
+#include "common_host.cuh"
 #include "sm100.cuh"
 
 namespace b200 {
 
-__global__ void __launch_bounds__(256) rows_copy16_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, long long rows,
+__global__ void __launch_bounds__(256) rows_copy16_kernel(const uint16_t* src, uint16_t* dst, long long rows,
                                                          int seq, int src_cols, int col0, int width, int reverse) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vpr = width / 8;   // 16-byte vectors per row
   const long long total = rows * vpr;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -27,8 +30,10 @@ __global__ void __launch_bounds__(256) rows_copy16_kernel(const uint16_t* __rest
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(256) rows_sum_cast_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                                                           uint16_t* __restrict__ dst, long long rows, int seq, int cols, int reverse) {
+__global__ void __launch_bounds__(256) rows_sum_cast_kernel(const float* a, const float* b,
+                                                           uint16_t* dst, long long rows, int seq, int cols, int reverse) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int vpr = cols / 8;
   const long long total = rows * vpr;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < total;
@@ -59,11 +64,13 @@ __global__ void __launch_bounds__(256) rows_sum_cast_kernel(const float* __restr
 // gradients and leaves the row's term; torch took six passes over [rows, cols] fp32 for the same (93 us of 2 x 8 x 2000 x
 // 128, now 16 with the scan below).  Bound by HBM.
 template <bool kBf16>
-__global__ void __launch_bounds__(256) decay_grad_rows_kernel(const uint16_t* __restrict__ q, const uint16_t* __restrict__ k,
-                                                             const float* __restrict__ dq_a, const float* __restrict__ dq_b,
-                                                             const float* __restrict__ dk_a, const float* __restrict__ dk_b,
-                                                             uint16_t* __restrict__ dq, uint16_t* __restrict__ dk,
-                                                             float* __restrict__ row_term, long long rows, int cols) {
+__global__ void __launch_bounds__(256) decay_grad_rows_kernel(const uint16_t* q, const uint16_t* k,
+                                                             const float* dq_a, const float* dq_b,
+                                                             const float* dk_a, const float* dk_b,
+                                                             uint16_t* dq, uint16_t* dk,
+                                                             float* row_term, long long rows, int cols) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long r = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -100,7 +107,9 @@ __global__ void __launch_bounds__(256) decay_grad_rows_kernel(const uint16_t* __
 
 // dg[t] = sum of row_term from t to the end: a CTA per sequence, from the last 1024 tokens to the first, the sum so far
 // carried along.
-__global__ void __launch_bounds__(1024) decay_grad_scan_kernel(const float* __restrict__ row_term, float* __restrict__ dg, int seq) {
+__global__ void __launch_bounds__(1024) decay_grad_scan_kernel(const float* row_term, float* dg, int seq) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float warp_sum[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* in = row_term + static_cast<long long>(blockIdx.x) * seq;
@@ -150,9 +159,11 @@ int attn_b200_rows_copy16(const void* src, void* dst, int64_t outer, int32_t seq
   if (width % 8 != 0 || col0 % 8 != 0 || src_cols % 8 != 0) return ATTN_B200_E_UNSUPPORTED;
   if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
   const long long rows = static_cast<long long>(outer) * seq;
-  b200::rows_copy16_kernel<<<b200::row_ops_grid(rows * (width / 8)), 256, 0, static_cast<cudaStream_t>(cuda_stream)>>>(
-      static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows, seq, src_cols, col0, width, reverse);
-  return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
+  return b200::launch_pdl(b200::rows_copy16_kernel, dim3(b200::row_ops_grid(rows * (width / 8))), dim3(256), 0,
+                          static_cast<cudaStream_t>(cuda_stream), static_cast<const uint16_t*>(src), static_cast<uint16_t*>(dst), rows, seq, src_cols,
+                          col0, width, reverse)
+             ? ATTN_B200_OK
+             : ATTN_B200_E_LAUNCH;
 }
 
 int attn_b200_linear_decay_grad(const void* q, const void* k, const float* dq_a, const float* dq_b, const float* dk_a,
@@ -172,11 +183,11 @@ int attn_b200_linear_decay_grad(const void* q, const void* k, const float* dq_a,
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
   const unsigned grid = b200::row_ops_grid(rows * 32);
   auto kernel = dtype == ATTN_B200_DTYPE_BF16 ? b200::decay_grad_rows_kernel<true> : b200::decay_grad_rows_kernel<false>;
-  kernel<<<grid, 256, 0, stream>>>(static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), dq_a, dq_b, dk_a, dk_b,
-                                   static_cast<uint16_t*>(dq), static_cast<uint16_t*>(dk), row_term, rows, cols);
-  if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
-  b200::decay_grad_scan_kernel<<<static_cast<unsigned>(outer), 1024, 0, stream>>>(row_term, dg, seq);
-  return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
+  if (!b200::launch_pdl(kernel, dim3(grid), dim3(256), 0, stream, static_cast<const uint16_t*>(q), static_cast<const uint16_t*>(k), dq_a, dq_b, dk_a,
+                        dk_b, static_cast<uint16_t*>(dq), static_cast<uint16_t*>(dk), row_term, rows, cols))
+    return ATTN_B200_E_LAUNCH;
+  return b200::launch_pdl(b200::decay_grad_scan_kernel, dim3(static_cast<unsigned>(outer)), dim3(1024), 0, stream, row_term, dg, seq) ? ATTN_B200_OK
+                                                                                                                                   : ATTN_B200_E_LAUNCH;
 }
 
 int attn_b200_rows_sum_cast(const float* a, const float* b, void* dst, int32_t dtype, int64_t outer, int32_t seq, int32_t cols,
@@ -189,11 +200,9 @@ int attn_b200_rows_sum_cast(const float* a, const float* b, void* dst, int32_t d
   const long long rows = static_cast<long long>(outer) * seq;
   const unsigned grid = b200::row_ops_grid(rows * (cols / 8));
   cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-  if (dtype == ATTN_B200_DTYPE_BF16)
-    b200::rows_sum_cast_kernel<true><<<grid, 256, 0, stream>>>(a, b, static_cast<uint16_t*>(dst), rows, seq, cols, reverse);
-  else
-    b200::rows_sum_cast_kernel<false><<<grid, 256, 0, stream>>>(a, b, static_cast<uint16_t*>(dst), rows, seq, cols, reverse);
-  return cudaGetLastError() == cudaSuccess ? ATTN_B200_OK : ATTN_B200_E_LAUNCH;
+  auto kernel = dtype == ATTN_B200_DTYPE_BF16 ? b200::rows_sum_cast_kernel<true> : b200::rows_sum_cast_kernel<false>;
+  return b200::launch_pdl(kernel, dim3(grid), dim3(256), 0, stream, a, b, static_cast<uint16_t*>(dst), rows, seq, cols, reverse) ? ATTN_B200_OK
+                                                                                                                                : ATTN_B200_E_LAUNCH;
 }
 
 }  // extern "C"

@@ -153,6 +153,14 @@ __device__ __forceinline__ bool named_sync_and(int id, int count, bool pred) {
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch: a kernel of this library is made ready (launched, barriers, tensor memory) while the
+// kernel in front of it in the stream still runs.  Every thread that touches memory another kernel writes or reads, and one
+// thread of every CTA at least, passes pdl_wait() first; pdl_launch_dependents() lets the next kernel begin its own set-up.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // thread-block clusters: distributed shared memory and cross-CTA barriers
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {

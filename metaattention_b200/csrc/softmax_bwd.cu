@@ -63,14 +63,16 @@ struct SoftmaxBwdFunctor {
 constexpr int kPrepTokens = 32, kPrepHeads = 8;
 
 template <bool kBf16, int D, bool kAligned>
-__global__ void __launch_bounds__(256) bwd_prepare_kernel(const void* __restrict__ o, const void* __restrict__ d_o,
-                                                        const float* __restrict__ lse, float* __restrict__ delta,
-                                                        float* __restrict__ lse2, int heads, int seq_q, int seq_q_pad, long long o_sb,
+__global__ void __launch_bounds__(256) bwd_prepare_kernel(const void* o, const void* d_o,
+                                                        const float* lse, float* delta,
+                                                        float* lse2, int heads, int seq_q, int seq_q_pad, long long o_sb,
                                                         long long o_ss, long long o_sh, long long do_sb, long long do_ss, long long do_sh) {
   constexpr int G = D / 8;             // lanes of a row
   constexpr int kGroups = 256 / G;     // rows a block reads at a time
   constexpr int kRows = kPrepTokens * kPrepHeads;
   __shared__ float acc_s[kPrepHeads][kPrepTokens + 1];
+  pdl_launch_dependents();
+  pdl_wait();
   const int s0 = blockIdx.x * kPrepTokens, h0 = blockIdx.y * kPrepHeads, b = blockIdx.z;
   const int grp = threadIdx.x / G, l = threadIdx.x % G;
   auto load = [&](const void* base, long long off) -> uint4 {
@@ -133,9 +135,9 @@ int launch_softmax_bwd(const AttnB200SoftmaxBwdArgs* a, const BwdCall& call_in, 
     for (int d = 0; d < 3; ++d) aligned = aligned && a->o_stride[d] % 8 == 0 && a->do_stride[d] % 8 == 0;
     const dim3 grid((seq_q_pad + kPrepTokens - 1) / kPrepTokens, (a->heads + kPrepHeads - 1) / kPrepHeads, a->batch);
     auto kernel = aligned ? bwd_prepare_kernel<kBf16, D, true> : bwd_prepare_kernel<kBf16, D, false>;
-    kernel<<<grid, 256, 0, stream>>>(a->o, a->d_o, a->lse, delta, lse2, a->heads, a->seq_q, seq_q_pad, a->o_stride[0], a->o_stride[1],
-                                     a->o_stride[2], a->do_stride[0], a->do_stride[1], a->do_stride[2]);
-    if (cudaGetLastError() != cudaSuccess) return ATTN_B200_E_LAUNCH;
+    if (!launch_pdl(kernel, grid, dim3(256), 0, stream, a->o, a->d_o, a->lse, delta, lse2, a->heads, a->seq_q, seq_q_pad, a->o_stride[0], a->o_stride[1],
+                    a->o_stride[2], a->do_stride[0], a->do_stride[1], a->do_stride[2]))
+      return ATTN_B200_E_LAUNCH;
   }
   BwdCall call = call_in;
   call.lse2 = lse2;

@@ -129,3 +129,65 @@ def test_refusals_of_the_library_arrive_as_its_error():
         with pytest.raises(lib.NativeError, match="invalid argument"):
             lib.softmax_bwd(q, k, v, o, torch.zeros(1, 2, 256, device="cuda"), o, 0.125, lib.MASK_NONE, mask_bits=bits)
     assert lib.last_device_status() == 0
+
+
+def _chains():
+    """Calls whose output is the next call's input, one per kernel family: name -> (start tensors, step)."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda").to(torch.bfloat16)
+    k, v = rnd(1, 700, 4, 64), rnd(1, 700, 4, 64)
+    prefill = programs.softmax_engine(1, 4, 700, 64, 64, is_causal=True)
+    decode = programs.gqa_engine(2, 8, 2, 1, 900, 128, 128)
+    dk, dv = rnd(2, 900, 2, 128), rnd(2, 900, 2, 128)
+    lin = programs.gla_engine(1, 4, 600, 128, 128)
+    lk, lv, lg = rnd(1, 4, 600, 128), rnd(1, 4, 600, 128), torch.full((1, 4, 600), -0.3, device="cuda")
+    kv = rnd(2, 500, 576)
+
+    def mla(q):
+        from attn_engine.mla import mla_decode_forward
+        o, _ = mla_decode_forward(q, kv, 512, 576 ** -0.5, num_splits=0)
+        return torch.cat([o, q[..., 512:]], -1)
+
+    def train(x):
+        x = x.detach().requires_grad_()
+        return torch.autograd.grad(prefill(x, k, v), x, torch.ones_like(x))[0] * 100 + k
+
+    def train_linear(x):
+        x = x.detach().requires_grad_()
+        g = lg.detach().requires_grad_()
+        dx, dg = torch.autograd.grad(lin(x, lk, lv, g), (x, g), lv)
+        return dx + dg[..., None].to(dx.dtype)
+    return {"prefill": (rnd(1, 700, 4, 64), lambda x: prefill(x, k, v)), "train": (rnd(1, 700, 4, 64), train),
+            "decode": (rnd(2, 1, 8, 128), lambda x: decode(x, dk, dv)), "linear": (rnd(1, 4, 600, 128), lambda x: lin(x, lk, lv, lg)),
+            "linear_train": (rnd(1, 4, 600, 128), train_linear), "mla": (rnd(2, 128, 576), mla)}
+
+
+@pytest.mark.parametrize("name", ["prefill", "train", "decode", "linear", "linear_train", "mla"])
+def test_calls_that_feed_one_another(name):
+    """A kernel is made ready while the one in front of it still runs: what it reads and overwrites must wait all the same,
+    the allocator handing scratch and outputs from one call to the next.  The same bits as with a wait behind every call."""
+    x0, step = _chains()[name]
+    want = x0
+    for _ in range(12):
+        want = step(want)
+        torch.cuda.synchronize()
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            for _ in range(5):
+                x = x0
+                for _ in range(12):
+                    x = step(x)
+                assert torch.equal(x, want)
+    if "train" not in name:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            x = x0
+            for _ in range(12):
+                x = step(x)
+        for _ in range(3):
+            graph.replay()
+            assert torch.equal(x, want)
+    assert lib.last_device_status() == 0
