@@ -17,7 +17,8 @@
 //   TMEM: Q[:, :512] as 16-bit pairs (256 columns) and    TMEM: O, 128 x 512 fp32 (512 columns)
 //         two 128-column score tiles
 //   smem: Q[:, 512:] tile, ring of 4 slots of three KV    smem: ring of five 32-row V stages, four
-//         chunks (128 rows x 64 columns) each                   64-row P slots
+//         chunks (128 rows x 64 columns) each, through          64-row P slots
+//         which Q[:, :512] comes as well
 //   warp 8: TMA, chunk by chunk                           warp 4: TMA
 //   warp 9: S = Q.KV^T over 128 KV rows: 36 MMAs with      warp 5: O += P.V per 64-row half tile
 //           N = 128 (full tensor rate; an MMA costs        warps 0-3: one head per thread: rescale O when
@@ -62,7 +63,8 @@ constexpr int kMlaThreads = 320;   // 10 warps
 constexpr int kMlaSmemBytes = 232448;  // the per-block maximum: the value CTA needs all of it
 
 struct MlaParams {
-  const void* q;        // first DV columns of q (read with 16-byte loads)
+  const void* q;        // first DV columns of q, where q_slots is 0 (then read with 16-byte loads)
+  int q_slots;          // 3: they come through the chunk ring ahead of a unit's KV tiles; 0: strides that a tensor map does not take
   long long q_sb, q_sh; // element strides (batch, head)
   void* o;              // [B, H, DV] 16-bit, written when num_splits == 1
   float* lse;           // [B, H] or null
@@ -192,7 +194,9 @@ struct MlaSmem {
 template <int D, int DV, bool kBf16>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kMlaThreads, 1)
 mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant__ CUtensorMap tmKVr,
-                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQr, const MlaParams p) {
+                 const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmQr,
+                 const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmOut,
+                 const __grid_constant__ CUtensorMap tmPart, const MlaParams p) {
   using L = MlaSmem;
   constexpr int N = kMlaTileN, M = kMlaHeads;
   static_assert(D == 576 && DV == 512, "tile bookkeeping below is written for 576/512");
@@ -255,32 +259,17 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
       while (count.next(u)) tiles += u.n;
       *part_tiles_s = tiles;
     }
-    for (int i = 0; i < 12; ++i) {
-      mbar_init(&bars[L::kSlotFull + i], 1);
-      mbar_init(&bars[L::kSlotEmpty + i], 1);
+  }
+  if (warp == 7) {   // two barriers a lane
+    for (int i = lane; i < L::kNumBars; i += 32) {
+      const bool rows256 = i == L::kSFree || i == L::kSFree + 1 || i == L::kRowMax || i == L::kRowMax + 1 || i == L::kQReady;
+      const bool rows128 = (i >= L::kPvGo && i < L::kPvGo + 4) || i == L::kFinalFull || i == L::kRowSum;
+      mbar_init(&bars[i], rows256 ? 256 : rows128 ? 128 : i == L::kStageFree || i == L::kFinalFree ? 4 : 1);
     }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&bars[L::kSFull + i], 1);
-      mbar_init(&bars[L::kSFree + i], 256);
-      mbar_init(&bars[L::kRowMax + i], 256);
-    }
-    for (int i = 0; i < 4; ++i) {
-      mbar_init(&bars[L::kPFull + i], 1);
-      mbar_init(&bars[L::kPFree + i], 1);
-      mbar_init(&bars[L::kPvGo + i], 128);
-      mbar_init(&bars[L::kPvDone + i], 1);
-    }
-    mbar_init(&bars[L::kStageFree], 4);
-    mbar_init(&bars[L::kFinalFree], 4);
-    mbar_init(&bars[L::kFinalFull], 128);
-    mbar_init(&bars[L::kQReady], 256);
-    mbar_init(&bars[L::kQrFull], 1);
-    mbar_init(&bars[L::kRowSum], 128);
     fence_barrier_init();
-    if (rank == 1) {
-      // every P slot expects its first half tile before the score CTA can send anything
-      for (int i = 0; i < 4; ++i) mbar_arrive_expect_tx(&bars[L::kPFull + i], (i & 1) ? kPTxOdd : kPTxEven);
-    }
+    // every P slot expects its first half tile before the score CTA can send anything
+    if (rank == 1 && lane >= L::kPFull && lane < L::kPFull + 4) mbar_arrive_expect_tx(&bars[lane], ((lane - L::kPFull) & 1) ? kPTxOdd : kPTxEven);
+    static_assert(L::kPFull + 4 <= 32, "a lane arms a barrier that it has set up");
   }
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -309,16 +298,26 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
         int J = 0;     // KV tiles of the units before this one: ring positions and barrier phases run on across units
         bool ok = true;
         for (int ui = 0; ok && walk.next(u); ++ui, J += u.n) {
-          if (ui > 0) {
-            // the rope tile of the previous unit is read by the MMAs of its last slot load
-            const int gl = 3 * J - 1;
-            ok = mbar_wait(&bars[L::kSlotEmpty + gl % L::kScoreSlots], (gl / L::kScoreSlots) & 1, ab, kMlaSlotEmpty);
+          const int R = 3 * J + p.q_slots * ui;   // slot loads before this unit's
+          for (int i = 0; i < p.q_slots && ok; ++i) {
+            // the query rows' first 512 columns, three chunks to a slot; the row threads move them on to tensor memory
+            const int slot = (R + i) % L::kScoreSlots, chunks = i < 2 ? 3 : 2;
+            ok = mbar_wait(&bars[L::kSlotEmpty + slot], (((R + i) / L::kScoreSlots) & 1) ^ 1, ab, kMlaSlotEmpty);
             if (!ok) break;
+            mbar_arrive_expect_tx(&bars[L::kSlotFull + slot], chunks * L::kChunkBytes);
+            for (int c = 0; c < chunks; ++c)
+              tma_load_3d(sChunk + slot * L::kSlotBytes + c * L::kChunkBytes, &tmQ, &bars[L::kSlotFull + slot], (i * 3 + c) * 64, head0, u.b);
           }
+          if (ok && ui > 0) {
+            // the rope tile of the previous unit is read by the MMAs of its last slot load
+            const int gl = R - 1;
+            ok = mbar_wait(&bars[L::kSlotEmpty + gl % L::kScoreSlots], (gl / L::kScoreSlots) & 1, ab, kMlaSlotEmpty);
+          }
+          if (!ok) break;
           mbar_arrive_expect_tx(&bars[L::kQrFull], L::kQrBytes);
           tma_load_3d(sQr, &tmQr, &bars[L::kQrFull], 0, head0, u.b);
           for (int g = 0; g < u.n * 3; ++g) {   // slot loads: three 64-column chunks of one 128-row tile each
-            const int gg = 3 * J + g;
+            const int gg = R + p.q_slots + g;
             const int j = g / 3, c0 = (g - j * 3) * 3, slot = gg % L::kScoreSlots;
             ok = mbar_wait(&bars[L::kSlotEmpty + slot], ((gg / L::kScoreSlots) & 1) ^ 1, ab, kMlaSlotEmpty);
             if (!ok) break;
@@ -358,12 +357,15 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
         bool ok = true;
         for (int ui = 0; ok && walk.next(unit); ++ui, J += unit.n) {
         ok = wait(&bars[L::kQReady], ui & 1, kMlaQReady) && wait(&bars[L::kQrFull], ui & 1, kMlaQrFull);
+        const int R = 3 * J + p.q_slots * ui;
+        if (ok && lane == 0)   // the query rows are in tensor memory: their slots are free
+          for (int i = 0; i < p.q_slots; ++i) mbar_arrive(&bars[L::kSlotEmpty + (R + i) % L::kScoreSlots]);
         for (int jl = 0; jl < unit.n && ok; ++jl) {
           const int j = J + jl;
           const int buf = j & 1;
           ok = wait(&bars[L::kSFree + buf], ((j >> 1) & 1) ^ 1, kMlaSFree);
           for (int u = 0; u < 3 && ok; ++u) {
-            const int g = j * 3 + u, slot = g % L::kScoreSlots;
+            const int g = R + p.q_slots + jl * 3 + u, slot = g % L::kScoreSlots;
             ok = wait(&bars[L::kSlotFull + slot], (g / L::kScoreSlots) & 1, kMlaSlotFull);
             if (!ok) break;
             tc_fence_after_sync();
@@ -405,11 +407,34 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
         const int b = unit.b, n = unit.n, seq_len = unit.seq_len, tile_begin = unit.t0;
         // ---- this head's query row, columns [256*wg, 256*wg+256) -> TMEM as 16-bit pairs (every score MMA of the
         //      previous unit has completed: this thread has seen its last score tile) ----
+        if (p.q_slots > 0) {
+          // They come as tiles through the chunk ring (a thread that reads its own row from memory touches 32 lines with
+          // every warp instruction: 11-16 k cycles a unit, 6-9 k of them now saved)
+          const int R = 3 * J + p.q_slots * ui;
+#pragma unroll 1
+          for (int cc = 0; cc < 4; ++cc) {
+            const int c = wg * 4 + cc, g = R + c / 3, slot = g % L::kScoreSlots;
+            ok = ok && mbar_wait(&bars[L::kSlotFull + slot], (g / L::kScoreSlots) & 1, ab, kMlaSlotFull);
+            if (!ok) break;
+            const uint32_t src = smem_u32(sChunk) + slot * L::kSlotBytes + (c % 3) * L::kChunkBytes + row * 128;
+            uint32_t w[32];
+#pragma unroll
+            for (int v = 0; v < 8; ++v) {
+              const uint4 x = ld_shared_v4(src + ((v ^ (row & 7)) << 4));
+              w[4 * v + 0] = x.x;
+              w[4 * v + 1] = x.y;
+              w[4 * v + 2] = x.z;
+              w[4 * v + 3] = x.w;
+            }
+            tmem_st32(tmem_base + lane_base + kColQ + c * 32, w);
+          }
+          if (!ok) break;
+        } else {
         const bool valid = head < p.heads;
         const uint4* qm = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.q) + b * p.q_sb +
                                                          static_cast<long long>(head) * p.q_sh + wg * 256);
-        // a thread reads its own row (rows are a kilobyte apart): the loads of half a row are issued together,
-        // so that the copy costs two memory round trips instead of one per 128 bytes
+        // a thread reads its own row: the loads of half a row are issued together, so that the copy costs two memory
+        // round trips instead of one per 128 bytes
 #pragma unroll 1
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t w[64];
@@ -428,6 +453,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
             for (int i = 0; i < 32; ++i) wc[i] = w[c * 32 + i];
             tmem_st32(tmem_base + lane_base + kColQ + wg * 128 + (hf * 2 + c) * 32, wc);
           }
+        }
         }
         tmem_wait_st();
         tc_fence_before_sync();
@@ -613,7 +639,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
       bool any_unit = false;
       for (int ui = 0; ok && walk.next(unit); ++ui, J += unit.n) {
       any_unit = true;
-      const int b = unit.b, n = unit.n, n_half = 2 * unit.n;
+      const int b = unit.b, n_half = 2 * unit.n;
       for (int hl = 0; hl < n_half && ok; ++hl) {
         const int h = 2 * J + hl;   // position in the cluster's whole run
         const int pslot = h & 3;
@@ -655,82 +681,65 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
           // the statistics are in registers: the score CTA may send the next unit's
           __syncwarp();
           if (lane == 0) mbar_arrive_cluster(peer_final_free);
-          // Rows leave through the V stages (all consumed by now), 1024 bytes of a row at a time: the whole 16-bit
-          // output row of a unit that is its whole sequence, or half of the fp32 row of a partial result (two
-          // passes).  Each warp stages the 32 rows it holds (16-byte pieces, piece index xor row: conflict-free) and
-          // then stores them as 512 contiguous bytes per instruction; a thread storing its own row scatters every
-          // warp instruction over 32 rows (and 16 bytes into each 32-byte sector).
-          static_assert(4 * 32 * 1024 <= L::kVStages * L::kVStageBytes && DV == 512, "row staging is laid out for 1 KB pieces of 512-wide rows");
-          const bool partial = unit.slot >= 0;
-          const uint32_t stage = smem_u32(sV) + warp * (32 * 1024);
-          const uint32_t mine = stage + lane * 1024;
-          uint8_t* gbase = partial
-              ? reinterpret_cast<uint8_t*>(p.part_o + (static_cast<long long>(unit.slot) * p.heads + head0 + warp * 32) * DV)
-              : reinterpret_cast<uint8_t*>(p.o) + 2 * ((static_cast<long long>(b) * p.heads + head0 + warp * 32) * DV);
-          const long long grow = partial ? DV * 4 : DV * 2;   // bytes between rows
-          for (int pass = 0; pass < (partial ? 2 : 1); ++pass) {
-            if (pass > 0) __syncwarp();   // the first half has been read back
-            if (!partial) {
-#pragma unroll 2
-              for (int c = 0; c < DV / 32; ++c) {
-                float o[32];
-                tmem_ld32f(tO + c * 32, o);
-                tmem_wait_ld();
-#pragma unroll
-                for (int v = 0; v < 4; ++v) {
-                  uint4 pk;
-                  pk.x = pack2<kBf16>(o[8 * v + 0] * inv, o[8 * v + 1] * inv);
-                  pk.y = pack2<kBf16>(o[8 * v + 2] * inv, o[8 * v + 3] * inv);
-                  pk.z = pack2<kBf16>(o[8 * v + 4] * inv, o[8 * v + 5] * inv);
-                  pk.w = pack2<kBf16>(o[8 * v + 6] * inv, o[8 * v + 7] * inv);
-                  st_shared_v4(mine + (((c * 4 + v) ^ (lane & 7)) << 4), pk);
-                }
-              }
-            } else {
-#pragma unroll 2
-              for (int c = 0; c < 8; ++c) {
-                float o[32];
-                tmem_ld32f(tO + (pass * 8 + c) * 32, o);
-                tmem_wait_ld();
-#pragma unroll
-                for (int v = 0; v < 8; ++v) {
-                  uint4 pk;
-                  pk.x = __float_as_uint(o[4 * v + 0] * inv);
-                  pk.y = __float_as_uint(o[4 * v + 1] * inv);
-                  pk.z = __float_as_uint(o[4 * v + 2] * inv);
-                  pk.w = __float_as_uint(o[4 * v + 3] * inv);
-                  st_shared_v4(mine + (((c * 8 + v) ^ (lane & 7)) << 4), pk);
-                }
-              }
+          // Rows leave through the V stages (all consumed by now) in tiles of 128 bytes of a warp's 32 rows, four tiles written
+          // while the four before them are stored by TMA.  (1 KB of a row at a time, read back and stored by the warp: 12 k
+          // cycles for a partial result, as long as bulk copies of a row each took to issue; a proxy fence costs ~400, so
+          // one for each tile took 10 k.)
+          constexpr int kOutBytes = 32 * 128, kOutBatch = 4, kOutSlots = 2 * kOutBatch;
+          static_assert(4 * kOutSlots * kOutBytes <= L::kVStages * L::kVStageBytes && DV == 512, "output tiles in the V stages");
+          const bool partial = unit.slot >= 0, rows_here = head0 + warp * 32 < p.heads;
+          uint8_t* const out = sV + warp * (kOutSlots * kOutBytes);
+          const int n_out = partial ? DV / 32 : DV / 64;
+          const int dc = partial ? 32 : 64;   // accumulator columns of a tile
+          float o[64];
+          auto fetch = [&](int c) {
+            tmem_ld32f(tO + c * dc, o);
+            if (!partial) tmem_ld32f(tO + c * dc + 32, o + 32);
+          };
+          fetch(0);
+          for (int c = 0; c < n_out; ++c) {
+            uint8_t* tile = out + (c % kOutSlots) * kOutBytes;
+            if (c >= kOutSlots && c % kOutBatch == 0) {   // the batch before the last one has been read
+              if (lane == 0) tma_store_wait_read_but<1>();
+              __syncwarp();
             }
-            __syncwarp();
-            uint8_t* obase = gbase + pass * 1024 + lane * 16;
-#pragma unroll 1
-            for (int r0 = 0; r0 < 32; r0 += 8) {
-              uint4 val[16];
+            const uint32_t mine = smem_u32(tile) + lane * 128;
+            uint32_t w[32];
+            tmem_wait_ld();
+            if (partial) {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const int r = r0 + i / 2, piece = (i % 2) * 32 + lane;
-                val[i] = ld_shared_v4(stage + r * 1024 + ((piece ^ (r & 7)) << 4));
-              }
+              for (int i = 0; i < 32; ++i) w[i] = __float_as_uint(o[i] * inv);
+            } else {
 #pragma unroll
-              for (int i = 0; i < 16; ++i) {
-                const int r = r0 + i / 2;
-                if (head0 + warp * 32 + r < p.heads)
-                  *reinterpret_cast<uint4*>(obase + static_cast<long long>(r) * grow + (i % 2) * 512) = val[i];
+              for (int i = 0; i < 32; ++i) w[i] = pack2<kBf16>(o[2 * i] * inv, o[2 * i + 1] * inv);
+            }
+            if (c + 1 < n_out) fetch(c + 1);   // under the stores of this tile
+#pragma unroll
+            for (int v = 0; v < 8; ++v)
+              st_shared_v4(mine + ((v ^ (lane & 7)) << 4), make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]));
+            if (c % kOutBatch == kOutBatch - 1) {
+              fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                for (int i = 0; rows_here && i < kOutBatch; ++i)
+                  tma_store_3d(partial ? &tmPart : &tmOut, tile - (kOutBatch - 1 - i) * kOutBytes, (c - (kOutBatch - 1 - i)) * dc,
+                               head0 + warp * 32, partial ? unit.slot : b);
+                tma_store_commit();
               }
             }
           }
+          if (lane == 0) tma_store_wait_read();
           if (in_range) {
             if (partial) p.part_lse[static_cast<long long>(unit.slot) * p.heads + head] = lse;
             else if (p.lse != nullptr) p.lse[static_cast<long long>(b) * p.heads + head] = lse;
           }
-          // the staged rows have been read back (or none were staged): the V stages may be refilled
+          // the staged rows have left: the V stages may be refilled
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars[L::kStageFree]);
         }
       }
       }
+      tma_store_wait_all();   // before the CTA's shared memory goes
       if (!any_unit && p.sched == nullptr && p.num_splits > 1 && head < p.heads && !*abort_flag) {
         // uniform splits: a split with no KV rows contributes nothing
         p.part_lse[(static_cast<long long>(blockIdx.z) * p.num_splits + part) * p.heads + head] = -INFINITY;
@@ -760,49 +769,80 @@ __global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, c
                                                         void* o, float* lse_out, int batch,
                                                         int heads, int uniform_splits, const int* cum) {
   pdl_launch_dependents();
-  pdl_wait();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= batch * heads) return;
+  if (warp >= batch * heads) return;   // (the block's first warp never does)
   const int b = warp / heads, h = warp % heads;
-  const int row0 = cum != nullptr ? cum[b] : b * uniform_splits;
-  const int num_splits = cum != nullptr ? cum[b + 1] - row0 : uniform_splits;
-  if (cum != nullptr && num_splits <= 1) return;
-  part_o += static_cast<long long>(row0) * heads * DV;
-  part_lse += static_cast<long long>(row0) * heads;
-  float mx = -INFINITY;
-  for (int i = 0; i < num_splits; ++i) mx = fmaxf(mx, part_lse[static_cast<long long>(i) * heads + h]);
-  float den = 0.f;
-  for (int i = 0; i < num_splits; ++i) den += __expf(part_lse[static_cast<long long>(i) * heads + h] - mx);
-  const float lse = mx + __logf(den);
   constexpr int V4 = DV / 128;  // float4 groups per lane
-  float4 acc[V4];
+  uint8_t* orow = reinterpret_cast<uint8_t*>(o) + 2 * (static_cast<long long>(b) * heads + h) * DV;
+  // A first pass on scratch that is not written yet, without a store, fetches the code while the decode kernel still runs;
+  // reads pass L1 by, so nothing stale is kept there.
+#pragma unroll 1
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool real = pass == 1;
+    if (real) pdl_wait();
+    int row0 = 0, num_splits = 1;
+    if (real) {
+      row0 = cum != nullptr ? __ldcg(cum + b) : b * uniform_splits;
+      num_splits = cum != nullptr ? __ldcg(cum + b + 1) - row0 : uniform_splits;
+      if (cum != nullptr && num_splits <= 1) return;
+    }
+    const float* po = part_o + static_cast<long long>(row0) * heads * DV;
+    const float* pl = part_lse + static_cast<long long>(row0) * heads + h;
+    // two parts at a time, their statistics and rows loaded together, against a running maximum
+    float mx = -INFINITY, den = 0.0f;
+    float4 acc[V4];
 #pragma unroll
-  for (int v = 0; v < V4; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int i = 0; i < num_splits; ++i) {
-    const long long row = static_cast<long long>(i) * heads + h;
-    const float li = part_lse[row];
-    if (li == -INFINITY) continue;
-    const float w = __expf(li - lse);
-    const float4* src = reinterpret_cast<const float4*>(part_o + row * DV);
+    for (int v = 0; v < V4; ++v) acc[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int i0 = 0; i0 < num_splits; i0 += 2) {
+      float l[2];
+      float4 x[2][V4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const long long row = static_cast<long long>(min(i0 + k, num_splits - 1)) * heads;
+        l[k] = __ldcg(pl + row);
+        const float4* src = reinterpret_cast<const float4*>(po + (row + h) * DV);
+#pragma unroll
+        for (int v = 0; v < V4; ++v) x[k][v] = __ldcg(src + v * 32 + lane);
+        if (i0 + k >= num_splits) l[k] = -INFINITY;
+      }
+      const float m = fmaxf(mx, fmaxf(l[0], l[1]));
+      if (m == -INFINITY) continue;   // only empty parts so far: their rows were never written
+      const float old = __expf(mx - m);
+      den *= old;
+#pragma unroll
+      for (int v = 0; v < V4; ++v) {
+        acc[v].x *= old;
+        acc[v].y *= old;
+        acc[v].z *= old;
+        acc[v].w *= old;
+      }
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (l[k] == -INFINITY) continue;
+        const float w = __expf(l[k] - m);
+        den += w;
+#pragma unroll
+        for (int v = 0; v < V4; ++v) {
+          acc[v].x += w * x[k][v].x;
+          acc[v].y += w * x[k][v].y;
+          acc[v].z += w * x[k][v].z;
+          acc[v].w += w * x[k][v].w;
+        }
+      }
+      mx = m;
+    }
+    const float inv = 1.0f / den, lse = mx + __logf(den);
 #pragma unroll
     for (int v = 0; v < V4; ++v) {
-      const float4 x = src[v * 32 + lane];
-      acc[v].x += w * x.x;
-      acc[v].y += w * x.y;
-      acc[v].z += w * x.z;
-      acc[v].w += w * x.w;
+      uint2 pk;
+      pk.x = pack2<kBf16>(acc[v].x * inv, acc[v].y * inv);
+      pk.y = pack2<kBf16>(acc[v].z * inv, acc[v].w * inv);
+      if (real) *reinterpret_cast<uint2*>(orow + (v * 32 + lane) * 8) = pk;
     }
+    if (real && lane == 0 && lse_out != nullptr) lse_out[static_cast<long long>(b) * heads + h] = lse;
   }
-  uint8_t* orow = reinterpret_cast<uint8_t*>(o) + 2 * (static_cast<long long>(b) * heads + h) * DV;
-#pragma unroll
-  for (int v = 0; v < V4; ++v) {
-    uint2 pk;
-    pk.x = pack2<kBf16>(acc[v].x, acc[v].y);
-    pk.y = pack2<kBf16>(acc[v].z, acc[v].w);
-    *reinterpret_cast<uint2*>(orow + (v * 32 + lane) * 8) = pk;
-  }
-  if (lane == 0 && lse_out != nullptr) lse_out[static_cast<long long>(b) * heads + h] = lse;
 }
 
 // Scheduler: cuts the KV tiles of all sequences (each sequence, and each part of a sequence, charged
@@ -888,20 +928,24 @@ struct MlaSchedLayout {
   }
 };
 
-// 3-D map over a 16-bit [batch][rows][cols] tensor view with element strides (batch, row), cols contiguous.
+// 3-D map over a [batch][rows][cols] tensor view with element strides (batch, row), cols contiguous; boxes of 128 bytes by
+// `box_rows` rows.  Types: the 16-bit ones, and ATTN_B200_DTYPE_FP32.
 inline int encode_3d(CUtensorMap* tm, const void* base, int dtype, uint64_t cols, uint64_t rows, uint64_t batch,
                      int64_t stride_batch, int64_t stride_row, uint32_t box_rows) {
   TensorMapEncodeTiledFn enc = tensor_map_encoder();
   if (enc == nullptr) return ATTN_B200_E_LAUNCH;
+  const int size = dtype == ATTN_B200_DTYPE_FP32 ? 4 : 2;
   if ((reinterpret_cast<uintptr_t>(base) & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
-  if (stride_row <= 0 || stride_row % 8 != 0) return ATTN_B200_E_UNSUPPORTED;
+  if (stride_row <= 0 || stride_row * size % 16 != 0) return ATTN_B200_E_UNSUPPORTED;
   if (batch <= 1) stride_batch = stride_row * static_cast<int64_t>(rows);
-  if (stride_batch <= 0 || stride_batch % 8 != 0) return ATTN_B200_E_UNSUPPORTED;
+  if (stride_batch <= 0 || stride_batch * size % 16 != 0) return ATTN_B200_E_UNSUPPORTED;
   cuuint64_t gdim[3] = {cols, rows, batch};
-  cuuint64_t gstride[2] = {static_cast<cuuint64_t>(stride_row) * 2, static_cast<cuuint64_t>(stride_batch) * 2};
-  cuuint32_t box[3] = {64, box_rows, 1};
+  cuuint64_t gstride[2] = {static_cast<cuuint64_t>(stride_row) * size, static_cast<cuuint64_t>(stride_batch) * size};
+  cuuint32_t box[3] = {static_cast<cuuint32_t>(128 / size), box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapDataType dt = dtype == ATTN_B200_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const CUtensorMapDataType dt = dtype == ATTN_B200_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                 : dtype == ATTN_B200_DTYPE_FP32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                                                 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const CUresult r = enc(tm, dt, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? ATTN_B200_OK : ATTN_B200_E_UNSUPPORTED;
@@ -919,14 +963,14 @@ template <bool kBf16>
 int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
   constexpr int D = 576, DV = 512;
   const AttnB200MlaShape& s = a->shape;
-  CUtensorMap tmKV, tmKVr, tmV, tmQr;
+  CUtensorMap tmKV, tmKVr, tmV, tmQr, tmQ, tmOut, tmPart;
   const int esz = 2;
   // rope columns: a separate tensor, or columns [DV, D) of the fused rows
   const void* q_rope = a->q_rope != nullptr ? a->q_rope : static_cast<const uint8_t*>(a->q) + DV * esz;
   const void* kv_rope = a->kv_rope != nullptr ? a->kv_rope : static_cast<const uint8_t*>(a->kv) + DV * esz;
   const int64_t* qr_st = a->q_rope != nullptr ? a->q_rope_stride : a->q_stride;
   const int64_t* kr_st = a->kv_rope != nullptr ? a->kv_rope_stride : a->kv_stride;
-  // the first DV columns of a q row are read with 16-byte loads straight into tensor memory
+  // the first DV columns of a q row come through a tensor map, or (strides it does not take) with 16-byte loads
   if ((reinterpret_cast<uintptr_t>(a->q) & 15) != 0) return ATTN_B200_E_UNSUPPORTED;
   for (int i = 0; i < 2; ++i)
     if (a->q_stride[i] % 8 != 0) return ATTN_B200_E_UNSUPPORTED;
@@ -949,6 +993,8 @@ int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
   MlaParams p;
   std::memset(&p, 0, sizeof(p));
   const int total_tiles = (s.seq_kv + kMlaTileN - 1) / kMlaTileN;
+  p.q_slots = encode_3d(&tmQ, a->q, a->dtype, DV, s.heads_q, s.batch, a->q_stride[0], a->q_stride[1], kMlaHeads) == ATTN_B200_OK ? 3 : 0;
+  if (p.q_slots == 0) tmQ = tmQr;
   p.q = a->q;
   p.q_sb = a->q_stride[0];
   p.q_sh = a->q_stride[1];
@@ -995,13 +1041,22 @@ int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
     p.part_o = static_cast<float*>(a->workspace);
     p.part_lse = p.part_o + static_cast<long long>(s.batch) * splits * s.heads_q * DV;
   }
+  const int64_t row_block = static_cast<int64_t>(s.heads_q) * DV;
+  rc = encode_3d(&tmOut, a->o, a->dtype, DV, s.heads_q, s.batch, row_block, DV, 32);
+  if (rc != ATTN_B200_OK) return rc;
+  tmPart = tmOut;
+  if (p.part_o != nullptr) {
+    const long long part_rows = scheduled ? static_cast<long long>(s.batch) + p.num_parts : static_cast<long long>(s.batch) * splits;
+    rc = encode_3d(&tmPart, p.part_o, ATTN_B200_DTYPE_FP32, DV, s.heads_q, part_rows, row_block, DV, 32);
+    if (rc != ATTN_B200_OK) return rc;
+  }
   auto kernel = mla_split_kernel<D, DV, kBf16>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMlaSmemBytes) != cudaSuccess) {
     cudaGetLastError();
     return ATTN_B200_E_LAUNCH;
   }
   if (grid.y > 65535) return ATTN_B200_E_UNSUPPORTED;
-  if (!launch_pdl(kernel, grid, dim3(kMlaThreads), kMlaSmemBytes, stream, tmKV, tmKVr, tmV, tmQr, p)) return ATTN_B200_E_LAUNCH;
+  if (!launch_pdl(kernel, grid, dim3(kMlaThreads), kMlaSmemBytes, stream, tmKV, tmKVr, tmV, tmQr, tmQ, tmOut, tmPart, p)) return ATTN_B200_E_LAUNCH;
   if (scheduled || splits > 1) {
     const long long warps = static_cast<long long>(s.batch) * s.heads_q;
     const int blocks = static_cast<int>((warps * 32 + 255) / 256);
