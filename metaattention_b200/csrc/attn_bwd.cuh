@@ -216,34 +216,46 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       *abort_flag = 1;
       atomicCAS(p.status, 0, kStatusTimeoutBase + kBwdSmemAlign);
     }
-    mbar_init(x_full, 1);
-    for (int i = 0; i < N1; ++i) {
-      mbar_init(y1_full + i, 1);
-      mbar_init(y1_empty + i, 1);
-    }
-    for (int i = 0; i < N2; ++i) {
-      mbar_init(y2_full + i, 1);
-      mbar_init(y2_empty + i, 1);
-    }
-    mbar_init(s_full, 1);
-    mbar_init(s_free, kRowWarps);
-    mbar_init(dp_full, 1);
-    mbar_init(dp_free, kRowWarps);
-    mbar_init(p_ready, kRowWarps);
-    mbar_init(p_free, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(ds_ready + i, kRowWarps);
-      mbar_init(ds_free + i, 1);
-    }
-    mbar_init(s_issued, 1);
-    mbar_init(acc_done, 1);
-    fence_barrier_init();
-    tma_prefetch_desc(&tmQ);
-    tma_prefetch_desc(&tmK);
-    tma_prefetch_desc(&tmV);
-    tma_prefetch_desc(&tmDO);
     pdl_wait();
     if (*reinterpret_cast<volatile int*>(p.status) != 0) *abort_flag = 1;
+  }
+  // Loads.  The loading warp sets the barriers up and sends the resident pair and the first streamed pair off at once, under
+  // the tensor-memory allocation and the CTA-wide sync.  (If the status word turns out set nobody takes them, and the
+  // teardown below gives them time to land.)
+  auto load_y1 = [&](int it, int ys, int hq) {   // streamed tile: row offset and head in the tensors it comes from
+    const int st = it % N1;
+    mbar_arrive_expect_tx(y1_full + st, L::kTileBytes + ((!kRoleQ && F::kUsesStats) ? L::kStatBytes : 0));
+    for (int c = 0; c < KC; ++c)
+      tma_load_rows(sY1 + st * L::kTileBytes + c * L::kChunkBytes, kRoleQ ? &tmK : &tmQ, y1_full + st, c * 64, ys * T, hq, b, kRoleQ ? p.ok : p.oq);
+    if constexpr (!kRoleQ && F::kUsesStats)
+      bulk_load(sLse + st * T, p.lse2 + (static_cast<long long>(b) * p.heads + hq) * p.seq_q_pad + ys * T, L::kStatBytes, y1_full + st);
+  };
+  auto load_y2 = [&](int it, int ys, int hq) {
+    const int st = it % N2;
+    mbar_arrive_expect_tx(y2_full + st, L::kTileBytes + ((!kRoleQ && F::kUsesStats) ? L::kStatBytes : 0));
+    for (int c = 0; c < KC; ++c)
+      tma_load_rows(sY2 + st * L::kTileBytes + c * L::kChunkBytes, kRoleQ ? &tmV : &tmDO, y2_full + st, c * 64, ys * T, hq, b, kRoleQ ? p.ov : p.odo);
+    if constexpr (!kRoleQ && F::kUsesStats)
+      bulk_load(sDelta + st * T, p.delta + (static_cast<long long>(b) * p.heads + hq) * p.seq_q_pad + ys * T, L::kStatBytes, y2_full + st);
+  };
+  KeptTiles load_walk(tiles_row, tiles_words);
+  if (warp == kRowWarps) {
+    static_assert(kNumBwdBarriers <= 32, "a barrier for each lane");
+    const bool rows = lane == kBarSFree || lane == kBarDpFree || lane == kBarPReady || lane == kBarDsReady || lane == kBarDsReady + 1;
+    if (lane < kNumBwdBarriers) mbar_init(bars + lane, rows ? kRowWarps : 1);
+    fence_barrier_init();
+    __syncwarp();
+    if (lane == 0 && n_iter > 0) {
+      pdl_wait();
+      mbar_arrive_expect_tx(x_full, 2 * L::kTileBytes);
+      for (int c = 0; c < KC; ++c) {
+        tma_load_rows(sX1 + c * L::kChunkBytes, kRoleQ ? &tmQ : &tmK, x_full, c * 64, tile * T, hx, b, kRoleQ ? p.oq : p.ok);
+        tma_load_rows(sX2 + c * L::kChunkBytes, kRoleQ ? &tmDO : &tmV, x_full, c * 64, tile * T, hx, b, kRoleQ ? p.odo : p.ov);
+      }
+      const int ys = walk_tiles ? load_walk.next() : (kRoleQ ? j0 : i0), hq = kRoleQ ? hx / p.kv_group : hx * p.kv_group;
+      load_y1(0, ys, hq);
+      load_y2(0, ys, hq);
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -259,46 +271,13 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   if (warp == kRowWarps) {
     // ======================= loading warp =======================
     if (lane == 0 && start_ok && n_iter > 0) {
-      mbar_arrive_expect_tx(x_full, 2 * L::kTileBytes);
-      for (int c = 0; c < KC; ++c) {
-        if constexpr (kRoleQ) {
-          tma_load_rows(sX1 + c * L::kChunkBytes, &tmQ, x_full, c * 64, tile * T, hx, b, p.oq);
-          tma_load_rows(sX2 + c * L::kChunkBytes, &tmDO, x_full, c * 64, tile * T, hx, b, p.odo);
-        } else {
-          tma_load_rows(sX1 + c * L::kChunkBytes, &tmK, x_full, c * 64, tile * T, hx, b, p.ok);
-          tma_load_rows(sX2 + c * L::kChunkBytes, &tmV, x_full, c * 64, tile * T, hx, b, p.ov);
-        }
-      }
-      KeptTiles kept(tiles_row, tiles_words);
-      for (int it = 0; it < n_iter; ++it) {
-        const int s1 = it % N1, s2 = it % N2;
-        const int ys = walk_tiles ? kept.next() : (kRoleQ ? j0 + it : i0 + it % max(per_head, 1));   // the streamed tile
-        uint8_t* y1 = sY1 + s1 * L::kTileBytes;
-        uint8_t* y2 = sY2 + s2 * L::kTileBytes;
-        // streamed tile: row offset and head in the tensors it comes from
-        const int hk = hx / p.kv_group;
-        const int hq = kRoleQ ? 0 : hx * p.kv_group + it / per_head, i = ys;
-        const long long stat_off = kRoleQ ? 0 : (static_cast<long long>(b) * p.heads + hq) * p.seq_q_pad + i * T;
-        if (!mbar_wait(y1_empty + s1, ((it / N1) & 1) ^ 1, ab, kBwdYEmpty)) break;
-        mbar_arrive_expect_tx(y1_full + s1, L::kTileBytes + ((!kRoleQ && F::kUsesStats) ? L::kStatBytes : 0));
-        for (int c = 0; c < KC; ++c) {
-          if constexpr (kRoleQ) {
-            tma_load_rows(y1 + c * L::kChunkBytes, &tmK, y1_full + s1, c * 64, ys * T, hk, b, p.ok);
-          } else {
-            tma_load_rows(y1 + c * L::kChunkBytes, &tmQ, y1_full + s1, c * 64, i * T, hq, b, p.oq);
-          }
-        }
-        if constexpr (!kRoleQ && F::kUsesStats) bulk_load(sLse + s1 * T, p.lse2 + stat_off, L::kStatBytes, y1_full + s1);
-        if (!mbar_wait(y2_empty + s2, ((it / N2) & 1) ^ 1, ab, kBwdYEmpty)) break;
-        mbar_arrive_expect_tx(y2_full + s2, L::kTileBytes + ((!kRoleQ && F::kUsesStats) ? L::kStatBytes : 0));
-        for (int c = 0; c < KC; ++c) {
-          if constexpr (kRoleQ) {
-            tma_load_rows(y2 + c * L::kChunkBytes, &tmV, y2_full + s2, c * 64, ys * T, hk, b, p.ov);
-          } else {
-            tma_load_rows(y2 + c * L::kChunkBytes, &tmDO, y2_full + s2, c * 64, i * T, hq, b, p.odo);
-          }
-        }
-        if constexpr (!kRoleQ && F::kUsesStats) bulk_load(sDelta + s2 * T, p.delta + stat_off, L::kStatBytes, y2_full + s2);
+      for (int it = 1; it < n_iter; ++it) {
+        const int ys = walk_tiles ? load_walk.next() : (kRoleQ ? j0 + it : i0 + it % max(per_head, 1));   // the streamed tile
+        const int hq = kRoleQ ? hx / p.kv_group : hx * p.kv_group + it / max(per_head, 1);
+        if (!mbar_wait(y1_empty + it % N1, ((it / N1) & 1) ^ 1, ab, kBwdYEmpty)) break;
+        load_y1(it, ys, hq);
+        if (!mbar_wait(y2_empty + it % N2, ((it / N2) & 1) ^ 1, ab, kBwdYEmpty)) break;
+        load_y2(it, ys, hq);
       }
     }
   } else if (warp > kRowWarps) {

@@ -182,23 +182,15 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       tma_load_rows(sQ + buf * p.q_bytes + c * (p.rows_pad * 128), &tmQ, bars + L::kQFull + buf, c * 64, 0, hk * p.group, b, p.oq);
   };
   int early = 0;   // tiles of the first unit on their way
-  if (warp == 8 && lane == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bars + L::kQFull + i, 1);
-      mbar_init(bars + L::kQEmpty + i, 1);
-      mbar_init(bars + L::kSFull + i, 1);
-      mbar_init(bars + L::kPReady + i, active_warps * 32);
-      mbar_init(bars + L::kODone + i, 1);
-    }
-    mbar_init(bars + L::kStats, active_warps * 32);
-    mbar_init(bars + L::kOFree, active_warps * 32);
-    for (int i = 0; i < ST; ++i) {
-      mbar_init(bars + L::kKFull + i, 1);
-      mbar_init(bars + L::kKEmpty + i, 1);
-      mbar_init(bars + L::kVFull + i, 1);
-      mbar_init(bars + L::kVEmpty + i, 1);
+  if (warp == 8) {   // two barriers a lane
+    for (int i = lane; i < L::kNumBars; i += 32) {
+      const bool rows = i == L::kPReady || i == L::kPReady + 1 || i == L::kStats || i == L::kOFree;
+      mbar_init(bars + i, rows ? active_warps * 32 : 1);
     }
     fence_barrier_init();
+    __syncwarp();
+  }
+  if (warp == 8 && lane == 0) {
     if constexpr (!kCounted) {
       pdl_wait();
       const int total = pairs * per_pair, shares = min(static_cast<int>(gridDim.x), total);

@@ -169,27 +169,16 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int bh_q = b_idx * p.heads_q + h_idx / (p.heads / p.heads_q), bh_k = b_idx * p.heads_k + h_idx / (p.heads / p.heads_k);
 
   if (tid == 0) {
-    mbar_init(q_full, 1);
-    mbar_init(k_full, 1);
-    mbar_init(v_full, 1);
-    mbar_init(s_bar, 1);
-    mbar_init(hi_ready, kLinRowThreads / 32);
-    mbar_init(pv_bar, 1);
-    mbar_init(st_bar, 1);
-    mbar_init(p_ready, kLinRowThreads / 32);
-    mbar_init(v_ready, kLinRowThreads / 32);
-    mbar_init(conv_done, kLinRowThreads / 32);
-    mbar_init(g_ready, 1);
-    for (int i = 0; i < 2; ++i) mbar_init(pre_k + i, 1);
-    for (int i = 0; i < 3; ++i) mbar_init(pre_v + i, 1);
-    mbar_init(pre_vready, kLinRowThreads / 32);
-    mbar_init(pre_h, kLinRowThreads / 32);
-    mbar_init(pre_st, 1);
-    fence_barrier_init();
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmO);
+  }
+  if (warp == 2) {   // one barrier a lane
+    static_assert(kNumLinBarriers <= 32, "a barrier for each lane");
+    const bool rows = lane == kBarHiReady || lane == kBarPReady || lane == kBarVReady || lane == kBarConvDone || lane == kBarPreVReady || lane == kBarPreH;
+    if (lane < kNumLinBarriers) mbar_init(bars + lane, rows ? kLinRowThreads / 32 : 1);
+    fence_barrier_init();
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);

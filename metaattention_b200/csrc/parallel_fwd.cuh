@@ -288,27 +288,19 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int c = 0; c < D / 64; ++c)
       tma_load_rows(sQ + t * L::kQBytes + c * (BM * 128), &tmQ, &q_full[t], c * 64, m0 + t * BM, h, b, p.oq);
   };
-  if (warp == kKWarp && lane == 0) {
+  if (warp == kVWarp && lane == 0) {
     tma_prefetch_desc(&tmQ);
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
-    mbar_init(&q_full[0], 1);
-    mbar_init(&q_full[1], 1);
-    for (int i = 0; i < ST; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-    }
-    for (int i = 0; i < STV; ++i) {
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
-    }
-    for (int t = 0; t < 2; ++t) {
-      mbar_init(&s_full[t], 1);
-      mbar_init(&s_free[t], 4 * RT);
-      mbar_init(&p_ready[t], 4 * RT);
-      mbar_init(&o_done[t], 1);
-    }
+  }
+  if (warp == kKWarp) {   // one barrier a lane
+    constexpr int kSFreeBar = 2 + 2 * ST + 2 * STV + 2;   // s_free and p_ready: an arrival from each functor warp of a tile
+    if (lane < L::kNumBars) mbar_init(bars + lane, lane >= kSFreeBar && lane < kSFreeBar + 4 ? 4 * RT : 1);
+    static_assert(L::kNumBars <= 32, "a barrier for each lane");
     fence_barrier_init();
+    __syncwarp();
+  }
+  if (warp == kKWarp && lane == 0) {
     pdl_wait();
     if (n_max > 0 && !kSparse) {
       // in the order of first use: query tile 0 and K so that its scores can start, then query tile 1, then V
@@ -525,16 +517,26 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // a tile needs element masking when it crosses an edge of the mask band or the end of the KV sequence
       const bool crosses = (banded && ((right < kNoBound && kv0 + BN - 1 > row0 + right) ||
                                        (left < kNoBound && kv0 < row0 + BM - 1 - left))) || (kv0 + BN > p.seq_kv);
-      if (crosses) {
-        if (F::kNegInfMask) {
-          const int kv_first = left < kNoBound ? q_idx - left : -kNoBound;
-          const int kv_last = right < kNoBound ? min(q_idx + right, p.seq_kv - 1) : p.seq_kv - 1;
+      if (F::kNegInfMask && crosses) {
+        // 32 columns at a time, those that a warp's 32 rows keep as a whole left alone, and a compare per element for an open
+        // side left out: two compares on every element took 1000 of 2960 cycles on a lone causal tile
+        const int q_w = row0 + (warp & 3) * 32;   // the warp's first row
+        const int kv_end = p.seq_kv - 1;
+        const int k0 = kv0 + half * TC;
+        const int first_max = left < kNoBound ? q_w + 31 - left : -kNoBound;
+        const int last_min = right < kNoBound ? min(q_w + right, kv_end) : kv_end;
+        const int hi = (right < kNoBound ? min(q_idx + right, kv_end) : kv_end) - k0;
 #pragma unroll
-          for (int i = 0; i < TC; ++i) {
-            const int kv = kv0 + half * TC + i;
-            const bool keep = (kv >= kv_first) && (kv <= kv_last);
-            s[i] = keep ? s[i] : -INFINITY;
+        for (int c = 0; c < TC; c += 32) {
+          if (k0 + c + 31 > last_min) {
+#pragma unroll
+            for (int i = c; i < c + 32; ++i) s[i] = i <= hi ? s[i] : -INFINITY;
           }
+        }
+        if (k0 < first_max) {
+          const int lo = q_idx - left - k0;
+#pragma unroll
+          for (int i = 0; i < TC; ++i) s[i] = i >= lo ? s[i] : -INFINITY;
         }
       }
       // P: 16-bit, two per column, in columns of its own
