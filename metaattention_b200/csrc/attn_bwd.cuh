@@ -74,6 +74,7 @@ struct BwdParams {
   float scale;
   long long dq_s[3], dk_s[3], dv_s[3];   // element strides (batch, seq, head)
   CoordOrder oq, ok, ov, odo;
+  int heads_at_once;   // of so many (query head, batch) pairs at a time the longest CTAs first; 0: of each
   int* status;
 };
 
@@ -565,12 +566,15 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int nq = (p.seq_q + kBwdT - 1) / kBwdT, nk = (p.seq_kv + kBwdT - 1) / kBwdT;
   const int n_kv_ctas = nk * p.heads_kv * p.batch;
   const int i = static_cast<int>(blockIdx.x);
+  // the longest first: a causal KV tile meets the more query tiles the earlier it lies, a query tile the fewer KV tiles
   if (i < n_kv_ctas) {
-    const int rest = i / nk;
-    attn_bwd_cta<F, false, kBf16, D, kBits>(tmQ, tmK, tmV, tmDO, p, i - rest * nk, rest % p.heads_kv, rest / p.heads_kv);
+    int tile, pair;
+    heavy_order(i, nk, p.heads_kv * p.batch, max(p.heads_at_once / p.kv_group, 1), tile, pair);
+    attn_bwd_cta<F, false, kBf16, D, kBits>(tmQ, tmK, tmV, tmDO, p, tile, pair % p.heads_kv, pair / p.heads_kv);
   } else {
-    const int j = i - n_kv_ctas, rest = j / nq;
-    attn_bwd_cta<F, true, kBf16, D, kBits>(tmQ, tmK, tmV, tmDO, p, j - rest * nq, rest % p.heads, rest / p.heads);
+    int tile, pair;
+    heavy_order(i - n_kv_ctas, nq, p.heads * p.batch, max(p.heads_at_once, 1), tile, pair);
+    attn_bwd_cta<F, true, kBf16, D, kBits>(tmQ, tmK, tmV, tmDO, p, nq - 1 - tile, pair % p.heads, pair / p.heads);
   }
 }
 
@@ -634,6 +638,8 @@ int launch_attn_bwd(const BwdCall& a, cudaStream_t stream, int* status) {
   for (int i = 0; i < ATTN_B200_MAX_CUSTOM; ++i) p.custom[i] = a.custom != nullptr ? a.custom[i] : nullptr;
   p.status = status;
   const bool with_bits = a.bits_q != nullptr;
+  if (a.mask_left >= ATTN_B200_MASK_OPEN && a.mask_right == 0)
+    p.heads_at_once = heavy_heads_at_once(static_cast<long long>(a.seq_q) * D * 4, static_cast<long long>(a.batch) * a.heads);
   auto kernel = with_bits ? attn_bwd_kernel<F, kBf16, D, true> : attn_bwd_kernel<F, kBf16, D, false>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes) != cudaSuccess) {
     cudaGetLastError();

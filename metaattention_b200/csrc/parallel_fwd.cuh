@@ -93,6 +93,7 @@ struct ParallelParams {
                                // [4]-word column mask per (sparse batch, sparse head, KV tile)
   int sparse_batch, sparse_heads, tile_words, elem_mask_rows;
   long long o_sb, o_ss, o_sh;  // element strides of o
+  int heads_at_once;           // causal: of so many (head, batch) pairs at a time the heaviest query tiles first; 0: of each
   int mask_kind;               // 0 none, 1 causal (keep q_idx >= kv_idx), 2 band
   int win_left, win_right;     // band: keep kv_idx in [q_idx - win_left, q_idx + win_right]; kNoBound = open side
   CoordOrder oq, ok, ov;
@@ -106,6 +107,14 @@ __device__ __forceinline__ void tma_load_rows(void* dst, const CUtensorMap* tm, 
   const int c2 = (o.pos_s == 2) ? s : (o.pos_h == 2) ? h : b;
   const int c3 = (o.pos_s == 3) ? s : (o.pos_h == 3) ? h : b;
   tma_load_4d(dst, tm, bar, c0, c1, c2, c3);
+}
+
+// The i-th CTA of `pairs` (head, batch) pairs with `tiles` tiles each, taken `at_once` pairs at a time, tile by tile.
+__device__ __forceinline__ void heavy_order(int i, int tiles, int pairs, int at_once, int& tile, int& pair) {
+  const int group = i / (tiles * at_once), first = group * at_once, n = min(at_once, pairs - first);
+  const int r = i - first * tiles;
+  tile = r / n;
+  pair = first + r - tile * n;
 }
 
 // wait-site ids reported through the device status word
@@ -208,10 +217,16 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int right = p.mask_kind == 0 ? kNoBound : (p.mask_kind == 1 ? 0 : p.win_right);
   const bool banded = p.mask_kind != 0;
   // heaviest query tiles (largest KV range under a causal mask) are launched first
-  const int m_pair = causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;
-  const int h = blockIdx.y;
-  const int b = p.kv_splits > 1 ? blockIdx.z / p.kv_splits : blockIdx.z;
-  const int split = p.kv_splits > 1 ? blockIdx.z % p.kv_splits : 0;
+  int m_of = blockIdx.x, h = blockIdx.y, z = blockIdx.z;
+  if (p.heads_at_once > 0) {
+    int pair;
+    heavy_order(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), gridDim.x, gridDim.y * gridDim.z, p.heads_at_once, m_of, pair);
+    z = pair / static_cast<int>(gridDim.y);
+    h = pair - z * static_cast<int>(gridDim.y);
+  }
+  const int m_pair = causal ? gridDim.x - 1 - m_of : m_of;
+  const int b = p.kv_splits > 1 ? z / p.kv_splits : z;
+  const int split = p.kv_splits > 1 ? z % p.kv_splits : 0;
   const int m0 = m_pair * NT * BM;
   const int n_kv_tiles = (p.seq_kv + BN - 1) / BN;
   // KV tiles [j_lo, j_hi) of each query tile; the CTA walks the union [j_min, j_max)

@@ -340,3 +340,22 @@ def test_elementwise_program_under_a_general_mask():
     check(o.detach(), ref.detach(), "o")
     for got, want, what in zip((qc.grad, kc.grad, vc.grad), (qf.grad, kf.grad, vf.grad), ("dq", "dk", "dv")):
         check(got, want, what)
+
+
+@pytest.mark.parametrize("B,H,Hkv,S,D", [(2, 12, 3, 900, 64), (1, 5, 5, 30000, 64)])
+def test_causal_backward_of_several_rounds(B, H, Hkv, S, D):
+    """More CTAs than SMs: the longest of several heads go first, with 30000 tokens of 5 heads in groups of heads.  dq has the
+    same bits as every query head by itself, dk and dv as every KV head with its group."""
+    from core.native import lib
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    q, d_o = (torch.randn(B, S, H, D, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, S, Hkv, D, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    G, scale = H // Hkv, D ** -0.5
+    o, lse = native_forward(q, k, v, True, scale)
+    dq, dk, dv = lib.softmax_bwd(q, k, v, o, lse, d_o, scale, lib.MASK_CAUSAL)
+    for b in range(B):
+        for g in range(Hkv):
+            qs, ks = (slice(b, b + 1), slice(None), slice(g * G, (g + 1) * G)), (slice(b, b + 1), slice(None), slice(g, g + 1))
+            part = lib.softmax_bwd(q[qs], k[ks], v[ks], o[qs], lse[b:b + 1, g * G:(g + 1) * G], d_o[qs], scale, lib.MASK_CAUSAL)
+            assert torch.equal(part[0], dq[qs]) and torch.equal(part[1], dk[ks]) and torch.equal(part[2], dv[ks])
+    assert lib.last_device_status() == 0

@@ -640,3 +640,24 @@ def _engine(B, H, Hkv, Sq, Skv, D, Dv, causal):
              meta_tensor(B, Hkv, Skv, Dv, dtype=torch.bfloat16))
     return AttentionEngine(metas, CustomIO({}), score_mod=score_mod, mask_mod=programs.causal if causal else None,
                            online_func=programs.NaturalSoftmax())
+
+
+@pytest.mark.parametrize("B,H,Hkv,S", [(1, 40, 8, 1100), (3, 16, 16, 1300), (1, 7, 7, 12000)])
+def test_causal_calls_of_several_rounds(B, H, Hkv, S):
+    """More CTAs than SMs: the longest of several heads go first, with 12000 tokens of 7 heads in two groups of heads.  The
+    same bits as every head by itself (one head's CTAs start at once, in the order of its tiles)."""
+    D = 128
+    gen = torch.Generator(device="cuda").manual_seed(S)
+    q = torch.randn(B, S, H, D, generator=gen, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn(B, S, Hkv, D, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2))
+    whole, one = _engine(B, H, Hkv, S, S, D, D, True), _engine(1, 1, 1, S, S, D, D, True)
+    o = whole(q, k, v)
+    lse = whole.last_final_rowscales["lse"]
+    for b in range(B):
+        for h in range(H):
+            g = h // (H // Hkv)
+            # one head's grid is small: without this its KV tiles would be split among CTAs
+            one.kv_splits = 1
+            part = one(q[b:b + 1, :, h:h + 1], k[b:b + 1, :, g:g + 1], v[b:b + 1, :, g:g + 1])
+            assert torch.equal(part[0, :, 0], o[b, :, h]) and torch.equal(one.last_final_rowscales["lse"][0, 0], lse[b, h])
+    assert native_lib.last_device_status() == 0
