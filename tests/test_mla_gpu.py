@@ -53,6 +53,20 @@ def test_shapes_and_splits(B, H, S, splits):
     assert (lse.cpu() - want_lse).abs().max().item() < 2e-3
 
 
+@pytest.mark.parametrize("H,splits", [(128, 1), (130, 2)])
+def test_query_rows_whose_strides_no_tensor_map_takes(H, splits):
+    """Every head reads the same query row (stride 0): the rows come with plain loads, as they come otherwise by TMA."""
+    B, S, D, Dv = 2, 300, 576, 512
+    q, kv = inputs.mla_inputs(B, H, S, D, Dv, 31)
+    q[..., :Dv] = q[:, :, :1, :Dv].clone()
+    nope, rope = q[:, 0, :1, :Dv].contiguous().cuda().expand(B, H, Dv), q[:, 0, :, Dv:].contiguous().cuda()
+    kvc = kv.cuda()
+    got = [mla_decode_forward(n, kvc[..., :Dv], Dv, D ** -0.5, q_rope=rope, kv_rope=kvc[..., Dv:], num_splits=splits)
+           for n in (nope, nope.contiguous())]
+    check(got[0][0], oracle(q, kv, Dv))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_split_invariance_property():
     """Size-independent property: the result does not depend on how the KV range is split."""
     B, H, S, D, Dv = 2, 128, 4096, 576, 512
