@@ -248,6 +248,9 @@ class AttentionEngine:
             self.functor_kind = "lowered"
             self._fparams = []
             fs = functor_lowering.emit_functor(tr, neg_inf_mask=neg_inf_mask, input_ctype=input_ctype)
+            if fs.row_epilogue and Dv > 128:
+                raise NotImplementedError(f"an online_fwd_epilogue that reduces over the accumulator row needs all of dim_v in one "
+                                          f"kernel, which takes up to 128 columns (got dim_v = {Dv})")
             self.functor_source = functor_lowering.translation_unit(fs, D, Dv, dtype == torch.bfloat16, sparse=self.sparse_walk)
             # compile now (works without a GPU); loading is deferred to the first call
             native_jit.build(self.functor_source)

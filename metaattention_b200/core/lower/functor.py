@@ -169,6 +169,7 @@ class _Lowerer:
     def __init__(self, body: _Body, leaves: dict):
         self.b = body
         self.memo: dict[int, object] = dict(leaves)
+        self.reduces = False   # whether a tile was reduced over its columns
 
     def alpha(self, t: Tile):
         return t.alpha if t.alpha is not None else Const(1.0)
@@ -275,6 +276,7 @@ class _Lowerer:
 
     def _reduce(self, x: Tile, combine: str, init: str | None) -> Row:
         """Four independent partial accumulators, combined at the end."""
+        self.reduces = True
         b = self.b
         base = b.fresh("a")
         e = b.elem(x)
@@ -405,6 +407,7 @@ class FunctorSource:
     final_names: list
     custom_names: list
     unit_o_scale: bool
+    row_epilogue: bool   # the epilogue reduces over the accumulator row: it needs all of dim_v at once
 
 
 def emit_functor(tr: TracedParallel, *, neg_inf_mask: bool, input_ctype: str, struct_name: str = "UserFunctor") -> FunctorSource:
@@ -490,6 +493,7 @@ def emit_functor(tr: TracedParallel, *, neg_inf_mask: bool, input_ctype: str, st
   static constexpr int kFinal = {len(final_names)};
   static constexpr bool kUnitOScale = {'true' if unit else 'false'};
   static constexpr bool kNegInfMask = {'true' if neg_inf_mask else 'false'};
+  static constexpr bool kRowEpilogue = {'true' if elow.reduces else 'false'};
   __device__ static void init(float* rs, const b200::RowCtx& c) {{
     {init_code}
   }}
@@ -512,7 +516,7 @@ def emit_functor(tr: TracedParallel, *, neg_inf_mask: bool, input_ctype: str, st
 }};
 """
     return FunctorSource(struct_name, code, len(rs_names), len(final_names), final_names,
-                         list(tr.custom.keys()), unit)
+                         list(tr.custom.keys()), unit, elow.reduces)
 
 
 def translation_unit(fs: FunctorSource, dim_qk: int, dim_v: int, bf16: bool, sparse: bool = False) -> str:

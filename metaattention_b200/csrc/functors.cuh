@@ -9,6 +9,7 @@
 //   init(rs, ctx)                  initial row-scale values
 //   tile<N>(s, rs, ctx) -> o_scale in-place score tile -> probabilities for one row
 //   kSplitSum, tile_pieces  instead of tile(): rows that several threads share, see SoftmaxFunctor
+//   kRowEpilogue epilogue() reduces over the columns it is given: it gets a whole row of dim_v
 //   epilogue<N>(o, rs, ctx)        in-place transform of N accumulator columns
 //   final_rowscale(i, rs, ctx)     i-th per-row output
 //   combine(i, n, fin, ...)        split-KV: weight of split i among n (OnlineFunc.combine), from all splits' final
@@ -38,6 +39,7 @@ struct SoftmaxFunctor {
   static constexpr int kFinal = 1;      // lse
   static constexpr bool kUnitOScale = false;
   static constexpr bool kNegInfMask = true;
+  static constexpr bool kRowEpilogue = false;
 
   __device__ static void init(float* rs, const RowCtx&) {
     rs[0] = -1.0e30f;  // stands for -inf; finite so that differences stay finite

@@ -51,13 +51,14 @@ struct FunctorArgs {
 };
 
 // Threads that share a row: two where the functor allows it (it keeps nothing per row, or its row values are a maximum
-// that the threads exchange and a sum that is added up at the end), so that four functor warps run on each scheduler.
+// that the threads exchange and a sum that is added up at the end; its epilogue works on each accumulator column by itself), so
+// that four functor warps run on each scheduler.
 template <class F, class = void>
 struct functor_split_sum : std::false_type {};
 template <class F>
 struct functor_split_sum<F, std::void_t<decltype(F::kSplitSum)>> : std::true_type {};
 template <class F>
-constexpr int kRowThreads = functor_split_sum<F>::value || (F::kRowScales == 0 && F::kUnitOScale) ? 2 : 1;
+constexpr int kRowThreads = functor_split_sum<F>::value || (F::kRowScales == 0 && F::kUnitOScale && !F::kRowEpilogue) ? 2 : 1;
 
 // What a functor knows about the row it is working on.
 struct RowCtx {

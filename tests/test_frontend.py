@@ -119,6 +119,30 @@ def test_emitted_functor_source_shape():
     assert "b200::fast_exp2(fmaf(s[i]" in e.functor_source and "kFinal = 2" in e.functor_source
 
 
+def _row_normalised(B, H, S, D, Dv, mask_mod=None):
+    """Elementwise exponentials whose accumulator row is divided by its own mean magnitude: no row scales, no rescale."""
+    class RowNorm(OnlineFunc):
+        def __init__(self):
+            super().__init__({}, {}, CustomIO())
+
+        @staticmethod
+        def online_fwd_epilogue(o, online_rowscales, b, h, q_idx):
+            return o * float(Dv) / o.get_reduce("abssum"), {}
+
+    def score_mod(score, custom, b, h, q_idx, kv_idx):
+        return (score * D ** -0.5).exp()
+    metas = [meta_tensor(B, H, S, d, dtype=torch.bfloat16) for d in (D, D, Dv)]
+    return AttentionEngine(metas, CustomIO({}), score_mod=score_mod, mask_mod=mask_mod, online_func=RowNorm())
+
+
+def test_epilogues_that_reduce_over_the_row_get_all_of_it():
+    """one thread per row, whose epilogue sees the whole of dim_v; refused where a kernel has a part of dim_v only"""
+    assert "kRowEpilogue = true" in _row_normalised(1, 1, 128, 64, 64).functor_source
+    assert "kRowEpilogue = false" in programs.relu_engine(1, 1, 128, 64, 64).functor_source
+    with pytest.raises(NotImplementedError, match="reduces over the accumulator row"):
+        _row_normalised(1, 1, 128, 128, 256)
+
+
 def test_engine_needs_cuda_tensors():
     e = programs.softmax_engine(1, 2, 128, 64, 64)
     q, k, v = inputs.attention_bshd(1, 2, 128, 64, 64, 1)

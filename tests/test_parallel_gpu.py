@@ -661,3 +661,18 @@ def test_causal_calls_of_several_rounds(B, H, Hkv, S):
             part = one(q[b:b + 1, :, h:h + 1], k[b:b + 1, :, g:g + 1], v[b:b + 1, :, g:g + 1])
             assert torch.equal(part[0, :, 0], o[b, :, h]) and torch.equal(one.last_final_rowscales["lse"][0, 0], lse[b, h])
     assert native_lib.last_device_status() == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("mask", ["none", "causal", "document"])
+def test_epilogue_that_reduces_over_the_accumulator_row(D, mask):
+    """o / mean(|o|) over all of dim_v, without row scales: dense and block-sparse, against fp32"""
+    from test_frontend import _row_normalised
+    B, H, S = 1, 3, 333
+    q, k, v = inputs.attention_bshd(B, H, S, D, D, 41)
+    masks = {"none": None, "causal": programs.causal, "document": lambda b, h, q_idx, kv_idx: (q_idx // 150 == kv_idx // 150) & (q_idx >= kv_idx)}
+    o = _row_normalised(B, H, S, D, D, masks[mask])(*cuda(q, k, v))
+    keep = torch.ones(S, S, dtype=torch.bool) if mask == "none" else masks[mask](0, 0, torch.arange(S)[:, None], torch.arange(S))
+    p = (torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * D ** -0.5).exp() * keep
+    acc = torch.einsum("bhqk,bkhd->bqhd", p, v.float())
+    check(o, acc / acc.abs().mean(-1, keepdim=True))
