@@ -380,8 +380,8 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       delta_r = p.delta[idx];
     }
     // P and g of one element.  KV role: lanes are KV rows, columns query rows; query role the other way round.  The
-    // band keeps, for this thread's row, the columns [col_lo, col_hi] of the tile (set per streamed tile; everything
-    // when no edge of the band crosses the pair); a functor whose P vanishes at a score of -inf (softmax) gets the mask
+    // band and the sequence's end keep, for this thread's row, the columns [col_lo, col_hi] of the tile (set per streamed
+    // tile; everything when neither crosses the pair); a functor whose P vanishes at a score of -inf (softmax) gets the mask
     // through the score
     int col_lo = 0, col_hi = T;   // counted from this thread's first column
     uint32_t keep_bits = 0;       // kBits: this thread's part of its row of the streamed tile
@@ -417,7 +417,12 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       // Pairs of tiles that an edge of the band crosses take a second copy of the row loops, with the mask: the row
       // phases sit on the kernel's serial chain, and two compares per element on every tile cost 15 %
       const int kv_minus_q = (kRoleQ ? ys - tile : tile - ys) * T;   // of the tiles' first rows
-      const bool edge = kBits || kv_minus_q + T - 1 > p.mask_right || kv_minus_q - (T - 1) < -p.mask_left;
+      // So does a tile that the sequence ends in, where its columns past the end would not come out as zeros: their score is 0
+      // (zero rows), and dS there is exp(-lse) times a finite value, which a row of strongly negative logits makes infinite --
+      // infinity times the zero rows of K is NaN for the whole row of dQ.  (Query rows past the end have lse = +inf.)
+      const int col_last = p.seq_kv - 1 - ys * T;
+      const bool tail = kRoleQ && col_last < T - 1;
+      const bool edge = kBits || tail || kv_minus_q + T - 1 > p.mask_right || kv_minus_q - (T - 1) < -p.mask_left;
       if constexpr (kBits) {
         const uint32_t* bits = kRoleQ ? p.bits_q : p.bits_kv;
         const long long pitch = 4LL * (kRoleQ ? nk : nq);   // words per row: four per streamed tile
@@ -428,7 +433,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         const long long lo = kRoleQ ? -static_cast<long long>(p.mask_left) - base : base - p.mask_right;
         const long long hi = kRoleQ ? static_cast<long long>(p.mask_right) - base : base + p.mask_left;
         col_lo = static_cast<int>(max(lo, 0LL)) - wg * C;
-        col_hi = static_cast<int>(min(hi, static_cast<long long>(T))) - wg * C;
+        col_hi = static_cast<int>(min(hi, static_cast<long long>(tail ? col_last : T))) - wg * C;
       }
       // this thread's columns of S or dP to registers, their buffer free behind them
       auto take = [&](uint32_t taddr, uint64_t* free_bar, float (&x)[C]) {

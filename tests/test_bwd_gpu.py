@@ -359,3 +359,27 @@ def test_causal_backward_of_several_rounds(B, H, Hkv, S, D):
             part = lib.softmax_bwd(q[qs], k[ks], v[ks], o[qs], lse[b:b + 1, g * G:(g + 1) * G], d_o[qs], scale, lib.MASK_CAUSAL)
             assert torch.equal(part[0], dq[qs]) and torch.equal(part[1], dk[ks]) and torch.equal(part[2], dv[ks])
     assert lib.last_device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,logit", [(torch.float16, -20.0), (torch.bfloat16, -100.0)])
+@pytest.mark.parametrize("Sq,Skv,D,kind", [(200, 333, 64, "none"), (333, 300, 128, "none"), (300, 130, 128, "causal"), (333, 333, 64, "window")])
+def test_strongly_negative_logits_beside_the_end_of_the_sequence(Sq, Skv, D, kind, dtype, logit):
+    """exp(-lse) is beyond the 16-bit type: the columns past the last key must not reach dq through their zero scores.  Against
+    autograd in 64 bits."""
+    from core.native import lib
+    gen = torch.Generator().manual_seed(Sq + Skv)
+    q, d_o = (torch.randn(1, Sq, 2, D, generator=gen) for _ in range(2))
+    k, v = (torch.randn(1, Skv, 2, D, generator=gen) for _ in range(2))
+    q[..., 0] = (-logit * D ** 0.5) ** 0.5
+    k[..., 0] = -q[0, 0, 0, 0]
+    q, k, v, d_o = (t.to(dtype) for t in (q, k, v, d_o))
+    scale, diff = D ** -0.5, torch.arange(Sq)[:, None] - torch.arange(Skv)
+    keep = {"none": diff == diff, "causal": diff >= 0, "window": diff.abs() < 90}[kind]
+    leaves = [t.double().requires_grad_() for t in (q, k, v)]
+    s = (torch.einsum("bqhd,bkhd->bhqk", leaves[0], leaves[1]) * scale).masked_fill(~keep, -float("inf"))
+    o = torch.einsum("bhqk,bkhd->bqhd", s.softmax(-1), leaves[2])
+    want = torch.autograd.grad(o, leaves, d_o.double())
+    args = [t.cuda() for t in (q, k, v, o.to(dtype), s.logsumexp(-1).float(), d_o)]
+    mask = {"none": (lib.MASK_NONE,), "causal": (lib.MASK_CAUSAL,), "window": (lib.MASK_BAND, (89, 89))}[kind]
+    for got, ref, what in zip(lib.softmax_bwd(*args, scale, *mask), want, ("dq", "dk", "dv")):
+        check(got, ref, what)
