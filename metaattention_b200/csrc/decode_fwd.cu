@@ -604,14 +604,16 @@ __global__ void __launch_bounds__(128) decode_merge_kernel(const DecodeParams p,
         }
         if (!in) l[k] = -INFINITY;
       }
+      // Shares whose scores are all -inf count nothing, in front of others as well as behind them (their rows are 0 / 0); NaN
+      // passes through: the maxima ignore it, its weight does not.
       const float m = fmaxf(mx, fmaxf(fmaxf(l[0], l[1]), fmaxf(l[2], l[3])));
-      const float old = __expf(mx - m);
+      const float old = mx == -INFINITY ? 0.0f : __expf(mx - m);
       den *= old;
 #pragma unroll
       for (int e = 0; e < E; ++e) acc[e] *= old;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const bool in = c0 + k <= c_hi;
+        const bool in = l[k] != -INFINITY;
         const float wgt = in ? __expf(l[k] - m) : 0.0f;
         den += wgt;
 #pragma unroll

@@ -807,9 +807,10 @@ __global__ void __launch_bounds__(256) mla_combine_kernel(const float* part_o, c
         for (int v = 0; v < V4; ++v) x[k][v] = __ldcg(src + v * 32 + lane);
         if (i0 + k >= num_splits) l[k] = -INFINITY;
       }
+      // parts without rows (-inf; their rows were never written) count nothing; NaN passes through: the maxima ignore it, its
+      // weight does not
       const float m = fmaxf(mx, fmaxf(l[0], l[1]));
-      if (m == -INFINITY) continue;   // only empty parts so far: their rows were never written
-      const float old = __expf(mx - m);
+      const float old = mx == -INFINITY ? 0.0f : __expf(mx - m);
       den *= old;
 #pragma unroll
       for (int v = 0; v < V4; ++v) {

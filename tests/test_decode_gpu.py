@@ -119,3 +119,23 @@ def test_blocks_and_lengths(B, H, Hkv, Sq, S, D, block, masked, varlen):
     again = run(eng, q, k, v, block_mask=mask, cache_seqlens=lens)
     assert torch.equal(o.nan_to_num(7.0), again[0].nan_to_num(7.0)) and torch.equal(lse, again[1])
     assert lib.last_device_status() == 0
+
+
+def test_shares_whose_scores_are_all_minus_infinity():
+    """One sequence cut into twenty shares, the keys of the first six tiles and of one in the middle -inf against every query
+    row: those shares count nothing wherever they stand, and NaN in one of them reaches the result."""
+    B, H, Hkv, S, D = 1, 4, 1, 20 * 128, 128
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    q, k, v = (rand(gen, B, n, h, D, dtype=torch.bfloat16) for n, h in ((1, H), (S, Hkv), (S, Hkv)))
+    q[..., 0] = 1.0
+    keep = torch.ones(B, Hkv, S, dtype=torch.bool, device="cuda")
+    keep[..., :6 * 128] = keep[..., 11 * 128:12 * 128] = False
+    k[0, ~keep[0, 0], 0, 0] = -float("inf")
+    eng = programs.gqa_engine(B, H, Hkv, 1, S, D, D)
+    kz = k.clone()
+    kz[0, ~keep[0, 0]] = 0
+    check(run(eng, q, k, v), reference(q, kz, v, D ** -0.5, keep), torch.bfloat16)
+    k[0, :8 * 128, 0, 1] = float("nan")
+    o, lse = run(eng, q, k, v)
+    assert torch.isnan(o).all() and torch.isnan(lse).all()
+    assert lib.last_device_status() == 0

@@ -293,3 +293,15 @@ def test_reference_call_with_scheduler_metadata():
     assert out.shape == (B, 1, H, Dv) and lse.shape == (B, H, 1)
     want = torch.cat([oracle(q[b:b + 1], kv[b:b + 1, :int(lens[b])], Dv) for b in range(B)])
     check(out, want)
+
+
+@pytest.mark.parametrize("splits", [4, 0])
+def test_nan_in_the_first_parts_reaches_the_result(splits):
+    """the combine adds parts up against a running maximum that ignores NaN; the NaN itself must not be lost"""
+    B, H, S, D, Dv = 2, 128, 8192, 576, 512
+    q, kv = inputs.mla_inputs(B, H, S, D, Dv, 77)
+    want = oracle(q[1:], kv[1:], Dv)
+    kv[0, :S // 2] = float("nan")
+    o, lse = mla_decode_forward(q.cuda(), kv.cuda(), Dv, D ** -0.5, num_splits=splits)
+    assert torch.isnan(o[0]).all() and torch.isnan(lse[0]).all()
+    check(o[1:], want)
