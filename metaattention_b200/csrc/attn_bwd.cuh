@@ -189,7 +189,6 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const AbortState ab{abort_flag, p.status};
-  pdl_launch_dependents();
   if constexpr (kBits) pdl_wait();   // the tile bitmaps are read right away
   const int nq = (p.seq_q + T - 1) / T, nk = (p.seq_kv + T - 1) / T;
   // The streamed tiles are those the band q_idx - left <= kv_idx <= q_idx + right lets the resident tile meet: KV tiles
@@ -261,6 +260,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   if (warp == 1) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
+    pdl_launch_dependents();   // behind the allocation: see sm100.cuh
   }
   pdl_wait();
   tc_fence_before_sync();

@@ -168,8 +168,6 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int active_warps = (p.rows + 31) / 32;   // of each softmax group
   const bool sparse = kCounted && p.block_mask != nullptr;
 
-  pdl_launch_dependents();   // the merge kernel may be made ready
-
   const int per_pair = (p.seq_kv + N - 1) / N;
   const int cta = static_cast<int>(blockIdx.x);
   // The loading lane sets the barriers up; without counts to wait for it sends the first loads off at once, under the
@@ -219,6 +217,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
+    pdl_launch_dependents();   // the merge kernel may be made ready; behind the allocation: see sm100.cuh
   }
   pdl_wait();
   if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;

@@ -221,7 +221,6 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();       // 0 = score CTA, 1 = value CTA
-  pdl_launch_dependents();
   pdl_wait();   // the units are read from memory right away
   const AbortState ab{abort_flag, p.status};
   // scheduled mode: blockIdx.y = head block * parts + part; uniform splits: blockIdx.y = head block * splits + split
@@ -274,6 +273,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
+    pdl_launch_dependents();   // behind the allocation: see sm100.cuh
   }
   if (warp == 8 && lane == 0) {
     tma_prefetch_desc(&tmKV);

@@ -208,7 +208,6 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const AbortState ab{abort_flag, p.status};
-  pdl_launch_dependents();
   if constexpr (kSparse) pdl_wait();   // the bitmaps are read right away
 
   // Every mask is a band kv_idx in [q_idx - left, q_idx + right]: none = open on both sides, causal = open
@@ -341,6 +340,7 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (warp == kQkWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
+    pdl_launch_dependents();   // behind the allocation: see sm100.cuh
   }
   pdl_wait();
   tc_fence_before_sync();

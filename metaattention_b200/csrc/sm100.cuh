@@ -156,6 +156,12 @@ __device__ __forceinline__ bool named_sync_and(int id, int count, bool pred) {
 // programmatic dependent launch: a kernel of this library is made ready (launched, barriers, tensor memory) while the
 // kernel in front of it in the stream still runs.  Every thread that touches memory another kernel writes or reads, and one
 // thread of every CTA at least, passes pdl_wait() first; pdl_launch_dependents() lets the next kernel begin its own set-up.
+// The exception: the merge kernels of split decodes read their scratch once before the wait, to fetch code and translations.
+// Such reads pass L1 by, go to slots that exist, and nothing comes of their values.
+// A kernel with tensor memory calls pdl_launch_dependents() behind its own allocation, by the allocating warp: a CTA of
+// the next kernel allocates before its wait, and on the same SM it would otherwise take all columns and wait for a kernel
+// that waits for columns (tcgen05.alloc has no bound).  Registers and shared memory keep today's kernels apart; functor
+// kernels are compiled at run time, with counts of their own.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

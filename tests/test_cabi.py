@@ -66,3 +66,19 @@ def test_version(native_lib):
 
 def test_null_args_rejected_without_gpu(native_lib):
     assert native_lib.attn_b200_parallel_fwd(None, None) == -1
+
+
+def test_kernels_let_the_next_one_start_behind_their_tensor_memory():
+    """A CTA of the next kernel allocates tensor memory while the one in front still runs: where both fit one SM it must find
+    that one's columns taken, or each would wait for the other."""
+    import glob
+    seen = 0
+    for path in glob.glob(os.path.join(lib.CSRC_DIR, "*.cu*")):
+        with open(path) as f:
+            code = re.sub(r"//[^\n]*", "", f.read())
+        for body in re.split(r"__global__|__device__ __forceinline__ void attn_bwd_cta", code)[1:]:
+            alloc, start = body.find("tmem_alloc("), body.find("pdl_launch_dependents()")
+            if alloc >= 0 and os.path.basename(path) != "sm100.cuh":
+                seen += 1
+                assert 0 <= alloc < start, path
+    assert seen >= 5
