@@ -403,10 +403,11 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       const float4 v4 = *reinterpret_cast<const float4*>(base + (k & ~3));
       return (k & 3) == 0 ? v4.x : (k & 3) == 1 ? v4.y : (k & 3) == 2 ? v4.z : v4.w;
     };
+    // a wait that a lane has given up is acted on where the warp votes: before it takes S or dP, and at the end
     bool ok = start_ok;
     KeptTiles kept(tiles_row, tiles_words);
     int next_i = 0, next_hq = kRoleQ ? hx : hx * p.kv_group;   // without a division per tile: rows are the serial chain
-    for (int it = 0; ok && it < n_iter; ++it) {
+    for (int it = 0; it < n_iter; ++it) {
       // the streamed tile index, its query head, and whether an edge of the band crosses this pair of tiles
       const int ys = walk_tiles ? kept.next() : (kRoleQ ? j0 : i0) + next_i;
       const int hq = next_hq;
@@ -455,7 +456,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         if (lane == 0) mbar_arrive(ready_bar);
       };
       static_assert(C == 32, "one tensor-memory load and one store of a row's part, one word of its keep bits");
-      ok = mbar_wait(s_full, it & 1, ab, kBwdSFull);
+      ok = warp_all(ok && mbar_wait(s_full, it & 1, ab, kBwdSFull));
       if (!ok) break;
       // the statistics of the query rows: this thread's own (query role) or those of its columns, which came with the tiles
       const float* st_lse = sLse + (it % N1) * T + wg * C;
@@ -479,13 +480,12 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       if constexpr (!kRoleQ) {
         if (it > 0) {   // dV of the last tile has read its P
           ok = mbar_wait(p_free, (it - 1) & 1, ab, kBwdPFree);
-          if (!ok) break;
           tc_fence_after_sync();
         }
         hand_over(tP, s, p_ready);
       }
       // ---- dP -> dS ----
-      ok = mbar_wait(dp_full, it & 1, ab, kBwdDpFull);
+      ok = warp_all(ok && mbar_wait(dp_full, it & 1, ab, kBwdDpFull));
       if (!ok) break;
       take(tDP, dp_free, s);
       if constexpr (F::kUsesStats) {
@@ -496,7 +496,6 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       }
       if (!kRoleQ && it > 0) {   // dK of the last tile has read its dS
         ok = mbar_wait(ds_free, (it - 1) & 1, ab, kBwdDsFree);
-        if (!ok) break;
         tc_fence_after_sync();
       }
       const int ds_buf = kRoleQ ? it & 1 : 0;
@@ -507,6 +506,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       ok = mbar_wait(acc_done, 0, ab, kBwdAccDone);
       tc_fence_after_sync();
     }
+    ok = warp_all(ok);
     if (ok) {
       const int r = tile * T + row;
       const int n_out = kRoleQ ? 1 : 2;

@@ -272,12 +272,12 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int T0 = cta < shares ? dec_share(total, cta, shares) : 0, T1 = cta < shares ? dec_share(total, cta + 1, shares) : 0;
   if (kCounted && blockIdx.x == 0)
     for (int i = tid; i <= pairs; i += kDecThreads) p.cum[i] = s_cum[i];
-  const bool run_cta = T1 > T0 && !*abort_flag;
+  const bool run_cta = warp_all(T1 > T0 && !*abort_flag);
   auto make_walk = [&]() { return DecodeWalk(kCounted ? s_cum : nullptr, s_valid, pairs, per_pair, p.seq_kv, T0, T1); };
 
   if (warp == 8) {
     // ======================= loading warp =======================
-    if (__all_sync(0xffffffffu, run_cta)) {
+    if (run_cta) {
       DecodeWalk u = make_walk();
       const int n_early = __shfl_sync(0xffffffffu, early, 0);
       bool ok = true;
@@ -316,7 +316,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         // A tile's boxes are spread over the lanes: K's and V's bpt blocks of KC column chunks (at most 32 boxes; one lane
         // issuing all of them, sixteen a tile with blocks of 32, took 3100 cycles a tile against 2400 for its bytes)
         const int qb = ui % p.q_bufs;
-        if (ui >= p.q_bufs) ok = mbar_wait(bars + L::kQEmpty + qb, (ui / p.q_bufs - 1) & 1, ab, kDecQEmpty);
+        if (ui >= p.q_bufs) ok = warp_all(mbar_wait(bars + L::kQEmpty + qb, (ui / p.q_bufs - 1) & 1, ab, kDecQEmpty));
         if (lane == 0 && ok && (kCounted || ui > 0)) load_q(qb, u.pair);
         const int blk = lane / KC, chunk = lane - blk * KC;
         for (int i = 0; i < u.n && ok; ++i) {
@@ -328,8 +328,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           const int off = st * L::kTileBytes + chunk * kChunk + (sparse ? blk * p.block * 128 : 0);
           for (int kv = 0; kv < 2 && ok; ++kv) {
             uint64_t* full = bars + (kv == 0 ? L::kKFull : L::kVFull) + st;
-            ok = mbar_wait(bars + (kv == 0 ? L::kKEmpty : L::kVEmpty) + st, par, ab, kv == 0 ? kDecKEmpty : kDecVEmpty);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_all(mbar_wait(bars + (kv == 0 ? L::kKEmpty : L::kVEmpty) + st, par, ab, kv == 0 ? kDecKEmpty : kDecVEmpty));
             if (!ok) break;
             if (lane == 0) mbar_arrive_expect_tx(full, L::kTileBytes);
             __syncwarp();
@@ -340,15 +339,14 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           }
         }
         J += u.n;
-        ok = __all_sync(0xffffffffu, ok);
       }
     }
   } else if (warp == 9) {
     // ======================= issuing warp (converged, one elected lane per batch) =======================
-    if (__all_sync(0xffffffffu, run_cta)) {
+    if (run_cta) {
       constexpr uint32_t idesc_qk = make_idesc_f16(128, N, kBf16, false, false);
       constexpr uint32_t idesc_pv = make_idesc_f16(128, D, kBf16, false, true);
-      auto wait = [&](uint64_t* bar, uint32_t parity, int site) -> bool { return __all_sync(0xffffffffu, mbar_wait_poll(bar, parity, ab, site)); };
+      auto wait = [&](uint64_t* bar, uint32_t parity, int site) -> bool { return warp_all(mbar_wait_poll(bar, parity, ab, site)); };
       const uint64_t k_desc0 = make_smem_desc(smem_u32(sK), 16, 1024);
       const uint64_t v_desc0 = make_smem_desc(smem_u32(sV), kChunk, 1024);
       DecodeWalk uq = make_walk();
@@ -420,7 +418,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       float rs[2];
       F::init(rs, ctx);
       for (int J = J0 + ((J0 ^ t) & 1); J < J0 + u.n && ok; J += 2) {
-        ok = mbar_wait(bars + L::kSFull + t, (J >> 1) & 1, ab, kDecSFull);
+        ok = warp_all(mbar_wait(bars + L::kSFull + t, (J >> 1) & 1, ab, kDecSFull));
         if (!ok) break;
         tc_fence_after_sync();
         float s[N];
@@ -441,7 +439,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tmem_st16(tS + c * W, pk);
         });
         if (J - J0 >= 2 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
-          ok = mbar_wait(bars + L::kODone + t, ((J >> 1) - 1) & 1, ab, kDecODone);
+          ok = warp_all(mbar_wait(bars + L::kODone + t, ((J >> 1) - 1) & 1, ab, kDecODone));
           if (ok) {
             tc_fence_after_sync();
 #pragma unroll
@@ -461,7 +459,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       if (!ok) break;
       if (t == 1) {
-        if (ui > 0) ok = mbar_wait(bars + L::kOFree, (ui - 1) & 1, ab, kDecOFree);   // group 0 has read the last unit's
+        if (ui > 0) ok = warp_all(mbar_wait(bars + L::kOFree, (ui - 1) & 1, ab, kDecOFree));   // group 0 has read the last unit's
         s_ml[row] = make_float2(rs[0], rs[1]);
         mbar_arrive(bars + L::kStats);
         continue;
@@ -472,6 +470,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       ok = mbar_wait(bars + L::kStats, ui & 1, ab, kDecStats);
       if (ok && has0) ok = mbar_wait(bars + L::kODone, (l0 >> 1) & 1, ab, kDecODone);
       if (ok && has1) ok = mbar_wait(bars + L::kODone + 1, (l1 >> 1) & 1, ab, kDecODone);
+      ok = warp_all(ok);
       if (!ok) break;
       tc_fence_after_sync();
       const float2 ml1 = s_ml[row];

@@ -190,7 +190,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const bool start_ok = !*abort_flag;
+  const bool start_ok = warp_all(!*abort_flag);
 
   if (warp == kLinRowThreads / 32) {
     // ======================= issuing warp: every TMA copy and every MMA =======================
@@ -391,7 +391,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       if (t > 0 && lane == 0)   // before the CTA's own blocks a table is read by the rescaling of V only
         ok = t <= t0 ? mbar_wait_poll(pre_vready, (t - 1) & 1, ab, kLinDecay) : mbar_wait_poll(p_ready, (t - 1 - t0) & 1, ab, kLinDecay);
-      ok = __all_sync(0xffffffffu, ok);
+      ok = warp_all(ok);
       if (!ok) break;
 #pragma unroll
       for (int n = 0; n < NH; ++n) {
@@ -507,16 +507,16 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
     bool ok = start_ok;
     // ---- the state alone, over the blocks before this CTA's own ----
-    for (int t = 0; kCut && ok && t < t0; ++t) {
+    for (int t = 0; kCut && t < t0; ++t) {
       const int b = (t0 - t) % 3;
       uint8_t* v_buf = b == 0 ? sV : smem + (b == 1 ? L::kOffPreV1 : L::kOffPreV2);
       const int tok = first_token(t) + row;
       const float vs = p.v_scale != nullptr && tok < p.seq ? p.v_scale[static_cast<long long>(bh + hv) * p.seq + tok] : 1.0f;
-      ok = mbar_wait_poll(g_ready, t & 1, ab, kLinDecay);
+      ok = mbar_wait_poll(g_ready, t & 1, ab, kLinDecay) && ok;
       const float* g = g_v(t);
       const float decay = fast_exp2(g_s(t)[kLast]);
       const float w = fast_exp2(g[kLast] - g[row]) * vs;
-      ok = mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok;
+      ok = warp_all(mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok);
       if (!ok) break;
       uint4* line = reinterpret_cast<uint4*>(v_buf + wg * (T * 128) + row * 128);
       rescale_row(line, line, w, vs, false);
@@ -539,7 +539,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       warp_arrive(pre_h);
     }
-    ok = ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay);
+    ok = warp_all(ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay));
     if (ok) {
       const bool mild_first = block_mild(t0);
       if (mild_first) ok = rescale_v(t0, true);
@@ -559,8 +559,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         warp_arrive(conv_done);
       }
     }
-    if (kCut && t0 > 0) ok = named_sync_and(1 + (warp & 3), 64, ok);   // the two warps of a lane quarter enter the loop together or not at all
-    for (int t = t0; ok && t < t_end; ++t) {
+    // the two warps of a lane quarter leave the loop where they meet in it, and nowhere else
+    for (int t = t0; t < t_end; ++t) {
       const bool last = (t + 1 == t_end);
       const uint32_t par = (t - t0) & 1;
       const float gi = g_v(t)[row];
@@ -576,7 +576,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const float g_last = g_v(t)[kLast];
       const bool mild = kPair ? block_mild(t) : g_last >= kMildLog2;
       if (!mild) {
-        ok = mbar_wait(s_bar, par, ab, kLinQh);   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
+        ok = mbar_wait(s_bar, par, ab, kLinQh) && ok;   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
         tc_fence_after_sync();
       }
       // ---- rows of V times their decay factors (mild decay: done in the previous block's tail) ----

@@ -287,7 +287,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   const int part_tiles = *part_tiles_s;
-  const bool run = (part_tiles > 0) && !*abort_flag && (*reinterpret_cast<volatile int*>(p.status) == 0);
+  const bool run = warp_all((part_tiles > 0) && !*abort_flag && (*reinterpret_cast<volatile int*>(p.status) == 0));
 
   if (rank == 0) {
     // ===================================== score CTA =====================================
@@ -414,7 +414,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
 #pragma unroll 1
           for (int cc = 0; cc < 4; ++cc) {
             const int c = wg * 4 + cc, g = R + c / 3, slot = g % L::kScoreSlots;
-            ok = ok && mbar_wait(&bars[L::kSlotFull + slot], (g / L::kScoreSlots) & 1, ab, kMlaSlotFull);
+            ok = warp_all(mbar_wait(&bars[L::kSlotFull + slot], (g / L::kScoreSlots) & 1, ab, kMlaSlotFull));
             if (!ok) break;
             const uint32_t src = smem_u32(sChunk) + slot * L::kSlotBytes + (c % 3) * L::kChunkBytes + row * 128;
             uint32_t w[32];
@@ -470,7 +470,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
           const int j = J + jl;   // position in the cluster's whole run: rings, buffers and phases
           const int buf = j & 1;
           const int pslot = (2 * j + wg) & 3;
-          ok = mbar_wait(&bars[L::kSFull + buf], (j >> 1) & 1, ab, kMlaSFull);
+          ok = warp_all(mbar_wait(&bars[L::kSFull + buf], (j >> 1) & 1, ab, kMlaSFull));
           if (!ok) break;
           tc_fence_after_sync();
           float s[64];
@@ -493,8 +493,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
           // the row maximum needs the other half too: post mine, wait for both
           s_rowmax[(buf * 2 + wg) * M + row] = fmaxf(mx0, mx1);
           mbar_arrive(&bars[L::kRowMax + buf]);
-          ok = mbar_wait(&bars[L::kRowMax + buf], (j >> 1) & 1, ab, kMlaRowMax);
-          if (!ok) break;
+          ok = mbar_wait(&bars[L::kRowMax + buf], (j >> 1) & 1, ab, kMlaRowMax);   // given up: left at the vote below
           const float mx = fmaxf(s_rowmax[(buf * 2) * M + row], s_rowmax[(buf * 2 + 1) * M + row]);
           float o_scale = 1.0f;
           if ((mx - m_ref) * c2 > 8.0f) {   // both halves take the same decision from the same numbers
@@ -516,7 +515,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
           r_sum += a0 + a1;
           // P half tile (128-byte row, swizzled like a TMA-written K-major tile) and, with half 0, the rescale
           // factor go to the value CTA; every byte is counted on its p_full barrier
-          ok = mbar_wait_cluster(&bars[L::kPFree + pslot], ((j >> 1) & 1) ^ 1, ab, kMlaPFree);
+          ok = warp_all(ok && mbar_wait_cluster(&bars[L::kPFree + pslot], ((j >> 1) & 1) ^ 1, ab, kMlaPFree));
           if (!ok) break;
           const uint32_t dst = peer_p + pslot * L::kPBytes;
           const uint32_t bar = peer_pfull + pslot * 8;
@@ -554,6 +553,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
               mbar_arrive_cluster(map_to_cta(smem_u32(&bars[L::kFinalFull]), 1));
             }
           }
+          ok = warp_all(ok);
         }
       }
     }
@@ -643,14 +643,14 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
       for (int hl = 0; hl < n_half && ok; ++hl) {
         const int h = 2 * J + hl;   // position in the cluster's whole run
         const int pslot = h & 3;
-        ok = mbar_wait_cluster(&bars[L::kPFull + pslot], (h >> 2) & 1, ab, kMlaPFull);
+        ok = warp_all(mbar_wait_cluster(&bars[L::kPFull + pslot], (h >> 2) & 1, ab, kMlaPFull));
         if (!ok) break;
         const float o_scale = (h & 1) ? 1.0f : s_scale[((h >> 1) & 1) * M + row];
         if (hl > 0 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
           // O must hold everything up to half tile h-1.  A parity wait is only unambiguous if the barrier
           // cannot be two phases away: these threads run far ahead of the MMAs, so they wait on the ring of
           // per-slot barriers (slot (h-1)&3 was last completed for half tile h-5, which p_full(h) implies).
-          ok = mbar_wait(&bars[L::kPvDone + ((h - 1) & 3)], ((h - 1) >> 2) & 1, ab, kMlaODone);
+          ok = warp_all(mbar_wait(&bars[L::kPvDone + ((h - 1) & 3)], ((h - 1) >> 2) & 1, ab, kMlaODone));
           if (ok) {
             tc_fence_after_sync();
 #pragma unroll 4
@@ -673,6 +673,7 @@ mla_split_kernel(const __grid_constant__ CUtensorMap tmKV, const __grid_constant
         const int h_last = 2 * J + n_half - 1;
         ok = mbar_wait_cluster(&bars[L::kFinalFull], ui & 1, ab, kMlaFinal) &&
              mbar_wait(&bars[L::kPvDone + (h_last & 3)], (h_last >> 2) & 1, ab, kMlaOFinal);
+        ok = warp_all(ok);
         if (ok) {
           tc_fence_after_sync();
           const bool in_range = head < p.heads;

@@ -137,6 +137,10 @@ __device__ __forceinline__ bool mbar_wait_poll(uint64_t* bar, uint32_t parity, c
   return true;
 }
 
+// What a warp's lanes have made of their waits, as one answer.  Lanes that give a wait up may see the abort at different polls;
+// a warp whose lanes load and store tensor memory or meet at barriers together goes on, or leaves, together.
+__device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
+
 // Named CTA barriers for a subset of the warps (`count` threads, a multiple of 32; id 1..15, 0 is __syncthreads).
 __device__ __forceinline__ void named_sync(int id, int count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");

@@ -1,5 +1,6 @@
 """The native host side of a call (csrc/host_ops.cpp) on the GPU: what surrounds the launches."""
 
+import ctypes
 import gc
 import threading
 import time
@@ -190,4 +191,44 @@ def test_calls_that_feed_one_another(name):
         for _ in range(3):
             graph.replay()
             assert torch.equal(x, want)
+    assert lib.last_device_status() == 0
+
+
+def _more_families():
+    gen = torch.Generator(device="cuda").manual_seed(4)
+
+    def rnd(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda").to(torch.bfloat16)
+    k, v, bias = rnd(1, 300, 2, 64), rnd(1, 300, 2, 64), torch.tensor([-3.0], device="cuda")
+    masked, sigmoid = programs.masked_softmax_engine(1, 2, 300, 64, 64, document), programs.sigmoid_engine(1, 2, 300, 64, 64)
+    other = programs.softmax_engine_noprobe(1, 2, 300, 64, 64, is_causal=True)
+
+    def train(engine, *custom):
+        def step(x):
+            x = x.detach().requires_grad_()
+            return torch.autograd.grad(engine(x, k, v, *custom), x, v)[0]
+        return rnd(1, 300, 2, 64), step
+    return {"sparse": train(masked), "elementwise": train(sigmoid, bias), "rows": (rnd(1, 300, 2, 64), lambda x: other(x, k, v))}
+
+
+class _Word:
+    """The device status word as an array that torch can write."""
+
+    def __init__(self):
+        ptr = ctypes.c_void_p()
+        lib.check(lib.load_library().attn_b200_device_status_word(0, ctypes.byref(ptr)), "attn_b200_device_status_word")
+        self.__cuda_array_interface__ = {"shape": (1,), "typestr": "<i4", "data": (ptr.value, False), "version": 3}
+
+
+@pytest.mark.parametrize("name", ["prefill", "train", "decode", "linear", "linear_train", "mla", "sparse", "elementwise", "rows"])
+def test_calls_behind_a_recorded_failure_leave(name):
+    """The status word says that a wait ran out: every kernel of a call leaves, its warps together, with copies under way or
+    not; once the word has been read the same call is right again."""
+    x0, step = {**_chains(), **_more_families()}[name]
+    want = step(x0)
+    assert lib.last_device_status() == 0
+    torch.as_tensor(_Word(), device="cuda").fill_(177)
+    step(x0)
+    assert lib.last_device_status() == 177
+    assert torch.equal(step(x0), want)
     assert lib.last_device_status() == 0
