@@ -267,7 +267,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const bool start_ok = !*abort_flag;
+  const bool start_ok = warp_all(!*abort_flag);
 
   if (warp == kRowWarps) {
     // ======================= loading warp =======================
@@ -403,11 +403,9 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       const float4 v4 = *reinterpret_cast<const float4*>(base + (k & ~3));
       return (k & 3) == 0 ? v4.x : (k & 3) == 1 ? v4.y : (k & 3) == 2 ? v4.z : v4.w;
     };
-    // a wait that a lane has given up is acted on where the warp votes: before it takes S or dP, and at the end
-    bool ok = start_ok;
     KeptTiles kept(tiles_row, tiles_words);
     int next_i = 0, next_hq = kRoleQ ? hx : hx * p.kv_group;   // without a division per tile: rows are the serial chain
-    for (int it = 0; it < n_iter; ++it) {
+    for (int it = 0; start_ok && it < n_iter; ++it) {
       // the streamed tile index, its query head, and whether an edge of the band crosses this pair of tiles
       const int ys = walk_tiles ? kept.next() : (kRoleQ ? j0 : i0) + next_i;
       const int hq = next_hq;
@@ -456,8 +454,7 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         if (lane == 0) mbar_arrive(ready_bar);
       };
       static_assert(C == 32, "one tensor-memory load and one store of a row's part, one word of its keep bits");
-      ok = warp_all(ok && mbar_wait(s_full, it & 1, ab, kBwdSFull));
-      if (!ok) break;
+      mbar_wait_rows(s_full, it & 1, ab, kBwdSFull);
       // the statistics of the query rows: this thread's own (query role) or those of its columns, which came with the tiles
       const float* st_lse = sLse + (it % N1) * T + wg * C;
       const float* st_delta = sDelta + (it % N2) * T + wg * C;
@@ -479,14 +476,13 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       }
       if constexpr (!kRoleQ) {
         if (it > 0) {   // dV of the last tile has read its P
-          ok = mbar_wait(p_free, (it - 1) & 1, ab, kBwdPFree);
+          mbar_wait_rows(p_free, (it - 1) & 1, ab, kBwdPFree);
           tc_fence_after_sync();
         }
         hand_over(tP, s, p_ready);
       }
       // ---- dP -> dS ----
-      ok = warp_all(ok && mbar_wait(dp_full, it & 1, ab, kBwdDpFull));
-      if (!ok) break;
+      mbar_wait_rows(dp_full, it & 1, ab, kBwdDpFull);
       take(tDP, dp_free, s);
       if constexpr (F::kUsesStats) {
         F::template grad_row<C, !kRoleQ>(g, s, kRoleQ ? &delta_r : st_delta);
@@ -495,19 +491,18 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
         for (int k = 0; k < C; ++k) s[k] = F::grad(g[k], s[k], fctx);
       }
       if (!kRoleQ && it > 0) {   // dK of the last tile has read its dS
-        ok = mbar_wait(ds_free, (it - 1) & 1, ab, kBwdDsFree);
+        mbar_wait_rows(ds_free, (it - 1) & 1, ab, kBwdDsFree);
         tc_fence_after_sync();
       }
       const int ds_buf = kRoleQ ? it & 1 : 0;
       hand_over(tDS + ds_buf * 64, s, ds_ready + ds_buf);
     }
     // ---- epilogue: the accumulators as 16-bit rows (dK and dQ times the functor's constant factor) ----
-    if (ok && n_iter > 0) {
-      ok = mbar_wait(acc_done, 0, ab, kBwdAccDone);
+    if (n_iter > 0) {
+      mbar_wait_rows(acc_done, 0, ab, kBwdAccDone);
       tc_fence_after_sync();
     }
-    ok = warp_all(ok);
-    if (ok) {
+    if (warp_all(!*abort_flag)) {
       const int r = tile * T + row;
       const int n_out = kRoleQ ? 1 : 2;
       for (int a = 0; a < n_out; ++a) {

@@ -412,14 +412,12 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const int qi = p.head_major ? row % p.seq_q : row / p.group;
     RowCtx ctx{0, 0, qi, 0, p.seq_q, p.seq_kv, &p.fa};
     DecodeWalk u = make_walk();
-    bool ok = true;
     int J0 = 0;   // tiles of the units before this one
-    for (int ui = 0; ok && u.next(); ++ui, J0 += u.n) {
+    for (int ui = 0; u.next(); ++ui, J0 += u.n) {
       float rs[2];
       F::init(rs, ctx);
-      for (int J = J0 + ((J0 ^ t) & 1); J < J0 + u.n && ok; J += 2) {
-        ok = warp_all(mbar_wait(bars + L::kSFull + t, (J >> 1) & 1, ab, kDecSFull));
-        if (!ok) break;
+      for (int J = J0 + ((J0 ^ t) & 1); J < J0 + u.n; J += 2) {
+        mbar_wait_rows(bars + L::kSFull + t, (J >> 1) & 1, ab, kDecSFull);
         tc_fence_after_sync();
         float s[N];
 #pragma unroll
@@ -439,27 +437,24 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tmem_st16(tS + c * W, pk);
         });
         if (J - J0 >= 2 && __any_sync(0xffffffffu, o_scale != 1.0f)) {
-          ok = warp_all(mbar_wait(bars + L::kODone + t, ((J >> 1) - 1) & 1, ab, kDecODone));
-          if (ok) {
-            tc_fence_after_sync();
+          mbar_wait_rows(bars + L::kODone + t, ((J >> 1) - 1) & 1, ab, kDecODone);
+          tc_fence_after_sync();
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
-              float o[32];
-              tmem_ld32f(tO + c * 32, o);
-              tmem_wait_ld();
+          for (int c = 0; c < D / 32; ++c) {
+            float o[32];
+            tmem_ld32f(tO + c * 32, o);
+            tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] *= o_scale;
-              tmem_st32f(tO + c * 32, o);
-            }
+            for (int i = 0; i < 32; ++i) o[i] *= o_scale;
+            tmem_st32f(tO + c * 32, o);
           }
         }
         tmem_wait_st();
         tc_fence_before_sync();
         mbar_arrive(bars + L::kPReady + t);
       }
-      if (!ok) break;
       if (t == 1) {
-        if (ui > 0) ok = warp_all(mbar_wait(bars + L::kOFree, (ui - 1) & 1, ab, kDecOFree));   // group 0 has read the last unit's
+        if (ui > 0) mbar_wait_rows(bars + L::kOFree, (ui - 1) & 1, ab, kDecOFree);   // group 0 has read the last unit's
         s_ml[row] = make_float2(rs[0], rs[1]);
         mbar_arrive(bars + L::kStats);
         continue;
@@ -467,11 +462,10 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       // ---- end of a unit (group 0): both accumulators of the row, weighted ----
       const int Jl = J0 + u.n - 1, l0 = (Jl & 1) == 0 ? Jl : Jl - 1, l1 = (Jl & 1) == 1 ? Jl : Jl - 1;
       const bool has0 = l0 >= J0, has1 = l1 >= J0;
-      ok = mbar_wait(bars + L::kStats, ui & 1, ab, kDecStats);
-      if (ok && has0) ok = mbar_wait(bars + L::kODone, (l0 >> 1) & 1, ab, kDecODone);
-      if (ok && has1) ok = mbar_wait(bars + L::kODone + 1, (l1 >> 1) & 1, ab, kDecODone);
-      ok = warp_all(ok);
-      if (!ok) break;
+      mbar_wait_rows(bars + L::kStats, ui & 1, ab, kDecStats);
+      if (has0) mbar_wait_rows(bars + L::kODone, (l0 >> 1) & 1, ab, kDecODone);
+      if (has1) mbar_wait_rows(bars + L::kODone + 1, (l1 >> 1) & 1, ab, kDecODone);
+      if (!warp_all(!*abort_flag)) break;
       tc_fence_after_sync();
       const float2 ml1 = s_ml[row];
       const float c2 = p.fa.f[0] * 1.4426950408889634f;

@@ -505,6 +505,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       return v_ok;
     };
 
+    // A wait that has run out is carried along: the lanes of a warp, and the two warps of a lane quarter, leave where those two
+    // meet in the loop, and nowhere else.  (A vote in front of the loop cost retention of 8 x 8 x 4096 tokens 3 %.)
     bool ok = start_ok;
     // ---- the state alone, over the blocks before this CTA's own ----
     for (int t = 0; kCut && t < t0; ++t) {
@@ -516,8 +518,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const float* g = g_v(t);
       const float decay = fast_exp2(g_s(t)[kLast]);
       const float w = fast_exp2(g[kLast] - g[row]) * vs;
-      ok = warp_all(mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok);
-      if (!ok) break;
+      ok = mbar_wait_poll(pre_v + b, (t / 3) & 1, ab, kLinPreFull) && ok;
       uint4* line = reinterpret_cast<uint4*>(v_buf + wg * (T * 128) + row * 128);
       rescale_row(line, line, w, vs, false);
       fence_proxy_async_smem();
@@ -539,8 +540,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       warp_arrive(pre_h);
     }
-    ok = warp_all(ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay));
-    if (ok) {
+    ok = ok && mbar_wait(g_ready, t0 & 1, ab, kLinDecay);
+    {
       const bool mild_first = block_mild(t0);
       if (mild_first) ok = rescale_v(t0, true);
       if (kCut && t0 > 0) {
@@ -559,7 +560,6 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         warp_arrive(conv_done);
       }
     }
-    // the two warps of a lane quarter leave the loop where they meet in it, and nowhere else
     for (int t = t0; t < t_end; ++t) {
       const bool last = (t + 1 == t_end);
       const uint32_t par = (t - t0) & 1;
@@ -576,7 +576,7 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const float g_last = g_v(t)[kLast];
       const bool mild = kPair ? block_mild(t) : g_last >= kMildLog2;
       if (!mild) {
-        ok = mbar_wait(s_bar, par, ab, kLinQh) && ok;   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
+        ok = mbar_wait(s_bar, par, ab, kLinQh);   // Q h has run: O may be rescaled, the copy's upper chunks overwritten
         tc_fence_after_sync();
       }
       // ---- rows of V times their decay factors (mild decay: done in the previous block's tail) ----

@@ -137,8 +137,31 @@ __device__ __forceinline__ bool mbar_wait_poll(uint64_t* bar, uint32_t parity, c
   return true;
 }
 
-// What a warp's lanes have made of their waits, as one answer.  Lanes that give a wait up may see the abort at different polls;
-// a warp whose lanes load and store tensor memory or meet at barriers together goes on, or leaves, together.
+// The wait of row threads, whose lanes load and store tensor memory and meet at barriers together.  Lanes that give a wait up
+// may see the abort at different polls, so it returns all the same, and the next waits of an aborted CTA return soon: the
+// warps run through their loops and look at the CTA's flag behind them (warp_all).  Leaving where a wait has failed takes a
+// vote per wait, and carrying the answer along a branch: 3 % of the backward, whose row phases are its serial chain.
+__device__ __forceinline__ void mbar_wait_rows(uint64_t* bar, uint32_t parity, const AbortState& ab, int site) {
+  if (mbar_try_wait(bar, parity)) return;
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if (*ab.cta_flag) return;
+    if ((++spins & 0xff) == 0) {
+      if (*reinterpret_cast<volatile int*>(ab.device_status) != 0) {
+        *ab.cta_flag = 1;
+        return;
+      }
+      if (clock64() - t0 > kWaitCycleLimit) {
+        *ab.cta_flag = 1;
+        atomicCAS(ab.device_status, 0, kStatusTimeoutBase + site);
+        return;
+      }
+    }
+  }
+}
+
+// One answer for a warp that goes on, or leaves, together.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok) != 0; }
 
 // Named CTA barriers for a subset of the warps (`count` threads, a multiple of 32; id 1..15, 0 is __syncthreads).
