@@ -168,6 +168,11 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   const int active_warps = (p.rows + 31) / 32;   // of each softmax group
   const bool sparse = kCounted && p.block_mask != nullptr;
 
+  // The merge kernel may be made ready, ahead of this kernel's own allocation (behind it a dense call of 1 x 32 x 13172 x 64 took
+  // 34.2 us, so 32.8): the rule of sm100.cuh is kept by shared memory, of which no kernel with tensor memory takes less than 64 KB.
+  static_assert(L::kBytes + 65536 > 233472, "a CTA with tensor memory could share the SM");
+  pdl_launch_dependents();
+
   const int per_pair = (p.seq_kv + N - 1) / N;
   const int cta = static_cast<int>(blockIdx.x);
   // The loading lane sets the barriers up; without counts to wait for it sends the first loads off at once, under the
@@ -217,7 +222,6 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   if (warp == 9) {
     tmem_alloc(tmem_slot, kTmemCols);
     tmem_relinquish();
-    pdl_launch_dependents();   // the merge kernel may be made ready; behind the allocation: see sm100.cuh
   }
   pdl_wait();
   if (tid == 0) *abort_flag = (*reinterpret_cast<volatile int*>(p.status) != 0) ? 1 : 0;

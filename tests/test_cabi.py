@@ -70,7 +70,7 @@ def test_null_args_rejected_without_gpu(native_lib):
 
 def test_kernels_let_the_next_one_start_behind_their_tensor_memory():
     """A CTA of the next kernel allocates tensor memory while the one in front still runs: where both fit one SM it must find
-    that one's columns taken, or each would wait for the other."""
+    that one's columns taken, or each would wait for the other.  (Or a kernel asserts that its shared memory leaves none room.)"""
     import glob
     seen = 0
     for path in glob.glob(os.path.join(lib.CSRC_DIR, "*.cu*")):
@@ -80,5 +80,5 @@ def test_kernels_let_the_next_one_start_behind_their_tensor_memory():
             alloc, start = body.find("tmem_alloc("), body.find("pdl_launch_dependents()")
             if alloc >= 0 and os.path.basename(path) != "sm100.cuh":
                 seen += 1
-                assert 0 <= alloc < start, path
+                assert alloc < start or start < 0 or "a CTA with tensor memory could share the SM" in body, path
     assert seen >= 5
