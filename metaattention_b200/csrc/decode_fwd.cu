@@ -412,9 +412,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t tS = tmem_base + lane_base + kColS + t * N;
     const uint32_t tO = tmem_base + lane_base + kColO + t * D;
-    const int g = p.head_major ? row / p.seq_q : row % p.group;
-    const int qi = p.head_major ? row % p.seq_q : row / p.group;
-    RowCtx ctx{0, 0, qi, 0, p.seq_q, p.seq_kv, &p.fa};
+    const RowCtx ctx{0, 0, 0, 0, p.seq_q, p.seq_kv, &p.fa};   // softmax asks for the scale only
     DecodeWalk u = make_walk();
     int J0 = 0;   // tiles of the units before this one
     for (int ui = 0; u.next(); ++ui, J0 += u.n) {
@@ -432,7 +430,7 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
           for (int i = 0; i < N; ++i) s[i] = i < left ? s[i] : -INFINITY;
         }
-        const float o_scale = F::template tile_pieces<N, 4>(s, rs, ctx, [](float mx) { return mx; }, [&](int c) {
+        const float o_scale = F::template tile_pieces<N, 4, false>(s, rs, ctx, [](float mx) { return mx; }, [&](int c) {
           constexpr int W = N / 4 / 2;
           uint32_t pk[W];
 #pragma unroll
@@ -478,6 +476,8 @@ decode_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       const float sum = rs[1] * w0 + ml1.y * w1;
       const float inv = 1.0f / sum, f0 = has0 ? w0 * inv : 0.0f, f1 = has1 ? w1 * inv : 0.0f;
       const float lse = logf(sum) + m * p.fa.f[0];
+      const int g = p.head_major ? row / p.seq_q : row % p.group;
+      const int qi = p.head_major ? row % p.seq_q : row / p.group;
       const int b = u.pair / p.heads_kv, h = (u.pair - b * p.heads_kv) * p.group + g;
       const bool whole = u.n == u.total;
       // a partial result: the pair's first share leaves it in the second slot of its CTA, the later ones in the first

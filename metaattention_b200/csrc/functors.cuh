@@ -52,9 +52,11 @@ struct SoftmaxFunctor {
   // is on its way to tensor memory while the next piece's exponentials run.  Multiply-adds and sums go two elements to
   // an instruction and the maximum three: with two or four warps to a scheduler this stage is bound by the
   // special-function unit (16 exponentials a cycle) and, in long calls, by the power it draws; prefill of
-  // 8 x 32 x 4096 x 128 causal 1203 -> 1165 us against one element to an instruction, with the same bits.
+  // 8 x 32 x 4096 x 128 causal 1203 -> 1165 us against one element to an instruction, with the same bits.  kPacked false: one
+  // element to an instruction.  A thread with a whole row of 128 columns (the decode kernel, bound by memory) has no room
+  // for the aligned register pairs: 20 to 96 bytes of spills in its instances, none without.
   static constexpr int kSplitSum = 1;
-  template <int N, int kPieces, class RowMax, class StorePiece>
+  template <int N, int kPieces, bool kPacked = true, class RowMax, class StorePiece>
   __device__ static float tile_pieces(float (&s)[N], float* rs, const RowCtx& c, RowMax&& row_max, StorePiece&& store_piece) {
     static_assert(N % (4 * kPieces) == 0 && N % 8 == 0, "pieces of whole groups");
     const float c2 = c.fa->f[0] * 1.4426950408889634f;
@@ -83,14 +85,26 @@ struct SoftmaxFunctor {
     for (int hf = 0; hf < kPieces; ++hf) {
 #pragma unroll
       for (int i = hf * (N / kPieces); i < (hf + 1) * (N / kPieces); i += 4) {
-        fma_x2(s[i], s[i + 1], c2, c2, neg, neg);
-        fma_x2(s[i + 2], s[i + 3], c2, c2, neg, neg);
+        if constexpr (kPacked) {
+          fma_x2(s[i], s[i + 1], c2, c2, neg, neg);
+          fma_x2(s[i + 2], s[i + 3], c2, c2, neg, neg);
+        } else {
+#pragma unroll
+          for (int k = i; k < i + 4; ++k) s[k] = fmaf(s[k], c2, neg);
+        }
         s[i] = fast_exp2(s[i]);
         s[i + 1] = fast_exp2(s[i + 1]);
         s[i + 2] = fast_exp2(s[i + 2]);
         s[i + 3] = fast_exp2(s[i + 3]);
-        add_x2(a0, a1, s[i], s[i + 1]);
-        add_x2(a2, a3, s[i + 2], s[i + 3]);
+        if constexpr (kPacked) {
+          add_x2(a0, a1, s[i], s[i + 1]);
+          add_x2(a2, a3, s[i + 2], s[i + 3]);
+        } else {
+          a0 += s[i];
+          a1 += s[i + 1];
+          a2 += s[i + 2];
+          a3 += s[i + 3];
+        }
       }
       store_piece(hf);
     }
