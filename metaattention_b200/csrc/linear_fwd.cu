@@ -794,7 +794,11 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     if (lane == 0) tma_store_wait_all();   // the staged rows of the last block are still being read
   }
 
-  pdl_launch_dependents();   // not at the start: 2 x 8 x 2000 training step 213.5 us so, 210.8 from here
+  // No pdl_launch_dependents(): the next kernel starts when this one's CTAs have left, its launch prepared.  Made ready
+  // earlier its CTAs went to whatever SMs were idle or first free, and calls that do not fill the chip lost more than the set-up
+  // costs: gated retention 5 x 8 x 1300 x 256 / 256, 80 CTAs, 74.4 us so, 64.0-67.6 now (65.7
+  // to 69.9 without early launches); gradients of 5 x 8 x 1000 x 256 / 256 with the forward 311 -> 279-286.  Called by the row
+  // warps at their end: 63.5, but 214 instead of 199 for the training step of 2 x 8 x 2000 x 128 / 256.
   tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag) {
