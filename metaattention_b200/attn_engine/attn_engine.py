@@ -24,7 +24,7 @@ import torch
 from core.lower import functor as functor_lowering
 from core.lower import sparse as sparse_lowering
 from core.lower import derivative
-from core.lower.trace import probe_softmax_scale, trace_parallel
+from core.lower.trace import mergeable, probe_softmax_scale, trace_parallel
 from core.native import jit as native_jit
 from core.native import lib as native
 from core.transform.core import CustomIO, SymbolicArray, SymbolScalar, Var, _eval_mask_2d, \
@@ -300,6 +300,7 @@ class AttentionEngine:
         self._plan = native.host().make_plan({
             "builtin": self.functor_kind == "builtin_softmax", "fn": fn, "fparams": self._fparams, "n_final": len(self.final_names),
             "mask_kind": self.mask_kind, "left": self.mask_band[0], "right": self.mask_band[1], "may_decode": self._may_decode,
+            "may_split": self.functor_kind == "builtin_softmax" or (self.mask_kind == native.MASK_NONE and mergeable(self.traced)),
             "decode_block": self._decode_block or 0, "has_mask_walk": walk,
             "mask_extents": (*self._mask_lengths, self._sparse_host["batch"] * self._sparse_host["heads"]) if walk else (0, 0, 1),
             "backward": 1 if self.functor_kind == "builtin_softmax" else 2, "load_mask": load_mask, "load_backward": load_backward,

@@ -120,6 +120,31 @@ def trace_parallel(score_mod, online_func, custom_fwd_inputs: CustomIO | None) -
     return tr
 
 
+def mergeable(tr: TracedParallel) -> bool:
+    """Whether results over parts of the KV sequence merge into the result over all of it: through the program's own
+    ``OnlineFunc.combine``, or, without one, by adding them up.  The latter needs a program without row scales or a rescale
+    of the accumulator, and an epilogue that is linear in the accumulator."""
+    if tr.combine_out is not None:
+        return True
+    if tr.rowscale_in or tr.o_scale is not None:
+        return False
+    linear: dict[int, bool | None] = {id(tr.o_in): True}     # None: does not depend on the accumulator
+
+    def kind(sym):
+        key = id(sym)
+        if key not in linear:
+            a = [kind(p) for p in sym.prev]
+            t = sym.code.type
+            if all(x is None for x in a):
+                linear[key] = None
+            elif t in ("Neg", "ReduceSum") or (t in ("Add", "Sub") and a == [True, True]):
+                linear[key] = all(a)
+            else:
+                linear[key] = (t == "Mul" and set(a) == {True, None}) or (t == "Div" and a == [True, None])
+        return linear[key]
+    return kind(tr.o_out) is True
+
+
 # --------------------------------------------------------------------------
 # torch interpreter
 # --------------------------------------------------------------------------

@@ -133,6 +133,7 @@ struct Plan {
   int n_final = 0;
   int mask_kind = 0, left = 0, right = 0;
   bool may_decode = false;     // attn_b200_decode_fwd computes this program
+  bool may_split = false;      // results over parts of the KV sequence merge into the whole one
   int decode_block = 0;        // > 0: block_mask / cache_seqlens arrive with the call
   bool has_mask_walk = false;  // a general mask_mod, evaluated for mask_q x mask_kv positions of mask_bh (batch, head) pairs
   int64_t mask_q = 0, mask_kv = 0, mask_bh = 1;
@@ -318,11 +319,12 @@ Forward forward(const Plan& plan, const std::shared_ptr<const Sparse>& mask, con
     a.final_rowscales[i] = r.finals.back().data_ptr<float>();
   }
   // split-KV when the launch would leave most SMs idle; the split results are added up with the weights of the functor's
-  // combine (lowered functors: the user's, which needs every split to be non-empty, i.e. no mask)
+  // combine (lowered functors: the user's, which needs every split to be non-empty, i.e. no mask).  A program without one
+  // whose results do not add up is split on demand only
   int splits = 1;
   Tensor ws;
   if (a.tile_keep == nullptr && Dv <= 128 && D <= 128 && (plan.builtin || plan.mask_kind == ATTN_B200_MASK_NONE)) {
-    splits = forced_splits >= 0 ? forced_splits : kv_splits_for(B, H, Sq, Skv, q.device().index());
+    splits = forced_splits >= 0 ? forced_splits : plan.may_split ? kv_splits_for(B, H, Sq, Skv, q.device().index()) : 1;
     if (splits > 1 && !plan.builtin) {
       const int64_t nt = (Skv + 127) / 128, per = (nt + std::min<int64_t>(splits, nt) - 1) / std::min<int64_t>(splits, nt);
       splits = (nt + per - 1) / per;   // no split without KV tiles
@@ -609,6 +611,7 @@ std::shared_ptr<Plan> make_plan(const py::dict& d) {
   p->left = py::cast<int>(d["left"]);
   p->right = py::cast<int>(d["right"]);
   p->may_decode = py::cast<bool>(d["may_decode"]);
+  p->may_split = py::cast<bool>(d["may_split"]);
   p->decode_block = py::cast<int>(d["decode_block"]);
   p->has_mask_walk = py::cast<bool>(d["has_mask_walk"]);
   std::tie(p->mask_q, p->mask_kv, p->mask_bh) = py::cast<std::tuple<int64_t, int64_t, int64_t>>(d["mask_extents"]);

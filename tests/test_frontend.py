@@ -145,6 +145,28 @@ def test_epilogues_that_reduce_over_the_row_get_all_of_it():
         _row_normalised(1, 1, 128, 128, 256)
 
 
+def test_programs_whose_split_results_merge():
+    from core.lower.trace import mergeable
+    assert not mergeable(_row_normalised(1, 1, 128, 64, 64).traced)                       # not linear in the accumulator
+    assert not mergeable(programs.softmax_engine_noprobe(1, 2, 128, 64, 64).traced)       # row scales and no combine
+    assert mergeable(programs.relu_engine(1, 1, 128, 64, 64).traced)
+    assert mergeable(programs.split_decode_engine(1, 2, 1, 256, 64, 64).traced)
+
+    class Scaled(OnlineFunc):
+        def __init__(self):
+            super().__init__({}, {}, CustomIO())
+
+        @staticmethod
+        def online_fwd_epilogue(o, online_rowscales, b, h, q_idx):
+            return (o * 2.0 - o / 4.0) / (h + 1.0), {}
+
+    class Shifted(Scaled):
+        @staticmethod
+        def online_fwd_epilogue(o, online_rowscales, b, h, q_idx):
+            return o + 1.0, {}
+    assert mergeable(trace_parallel(None, Scaled(), None)) and not mergeable(trace_parallel(None, Shifted(), None))
+
+
 def test_engine_needs_cuda_tensors():
     e = programs.softmax_engine(1, 2, 128, 64, 64)
     q, k, v = inputs.attention_bshd(1, 2, 128, 64, 64, 1)

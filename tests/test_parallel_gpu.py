@@ -676,3 +676,17 @@ def test_epilogue_that_reduces_over_the_accumulator_row(D, mask):
     p = (torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * D ** -0.5).exp() * keep
     acc = torch.einsum("bhqk,bkhd->bqhd", p, v.float())
     check(o, acc / (4 * acc.abs().mean(-1, keepdim=True)))
+
+
+def test_programs_whose_split_results_do_not_merge_are_not_split():
+    """One head against 2048 keys leaves most of the chip idle: a program with a combine, or whose results add up, is split; a
+    softmax without a combine and an epilogue that is not linear are not."""
+    from test_frontend import _row_normalised
+    B, H, S, D = 1, 1, 2048, 64
+    q, k, v = inputs.attention_bshd(B, H, S, D, D, 43)
+    o = _row_normalised(B, H, S, D, D)(*cuda(q, k, v))
+    acc = torch.einsum("bhqk,bkhd->bqhd", (torch.einsum("bqhd,bkhd->bhqk", q.float(), k.float()) * D ** -0.5).exp(), v.float())
+    check(o, acc / (4 * acc.abs().mean(-1, keepdim=True)))
+    e = programs.softmax_engine_noprobe(B, H, S, D, D, is_causal=False)
+    check(e(*cuda(q, k, v)), rm.softmax_attention(q, k, v, False))
+    assert (e.last_final_rowscales["lse"].cpu() - rm.softmax_lse(q, k, False)).abs().max().item() < 1e-3
