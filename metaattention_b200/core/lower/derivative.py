@@ -17,8 +17,10 @@ from __future__ import annotations
 
 import math
 
+import torch
+
 from core.lower.functor import _f, custom_kind
-from core.lower.trace import TracedParallel, init_value
+from core.lower.trace import TracedParallel, evaluate, init_value
 
 LOG2E = 1.4426950408889634
 LN2 = 0.6931471805599453
@@ -30,6 +32,21 @@ def elementwise_program(tr: TracedParallel) -> bool:
     if tr.rowscale_in or tr.rowscale_out or tr.final or tr.o_scale is not None or tr.o_out is not tr.o_in:
         return False
     return all(custom_kind(sym) == "scalar" for sym in tr.custom.values())
+
+
+def _finite_at_zero(tr: TracedParallel) -> bool:
+    """Whether P and its derivative are finite at a score of 0, which is that of the zero rows past the ends of the sequences.
+    Custom inputs and positions are tried at a few values."""
+    for value in (0.0, 0.7, -3.0):
+        score = torch.zeros(2, 4, requires_grad=True)
+        env = {id(tr.scores_in): score}
+        env.update({id(sym): torch.full_like(score, abs(value)) for sym in tr.index_leaves.values()})
+        env.update({id(sym): torch.full_like(score, value) for sym in tr.custom.values()})
+        p = torch.as_tensor(evaluate([tr.scores_out], env)[0], dtype=torch.float32)
+        d = torch.autograd.grad(p.sum(), score, allow_unused=True)[0] if p.requires_grad else None
+        if not torch.isfinite(p).all() or (d is not None and not torch.isfinite(d).all()):
+            return False
+    return True
 
 
 class _Dual:
@@ -135,6 +152,7 @@ def emit_backward_functor(tr: TracedParallel, struct_name: str = "UserBwdFunctor
     return f"""struct {struct_name} {{
   static constexpr bool kUsesStats = false;
   static constexpr bool kNegInfMask = false;
+  static constexpr bool kFiniteTail = {'true' if _finite_at_zero(tr) else 'false'};
   struct Ctx {{
     float cu[{n}];
   }};

@@ -24,7 +24,9 @@ import hashlib
 import math
 from dataclasses import dataclass
 
-from core.lower.trace import TracedParallel, custom_axes
+import torch
+
+from core.lower.trace import TracedParallel, custom_axes, evaluate
 
 LOG2E = 1.4426950408889634
 LN2 = 0.6931471805599453
@@ -410,6 +412,21 @@ class FunctorSource:
     row_epilogue: bool   # the epilogue reduces over the accumulator row: it needs all of dim_v at once
 
 
+def finite_tail(tr: TracedParallel, neg_inf_mask: bool) -> bool:
+    """Whether an elementwise program (no row scales) makes a finite weight of the score that stands for keys past the end of
+    the sequence: -inf, or 0 with another mask value.  Custom inputs and positions are tried at a few values."""
+    if tr.rowscale_in or tr.o_scale is not None:
+        return True
+    score = torch.full((2, 4), -math.inf if neg_inf_mask else 0.0)
+    for value in (0.0, 0.7, -3.0):
+        env = {id(tr.scores_in): score}
+        env.update({id(sym): torch.full_like(score, abs(value)) for sym in tr.index_leaves.values()})
+        env.update({id(sym): torch.full_like(score, value) for sym in tr.custom.values()})
+        if not torch.isfinite(torch.as_tensor(evaluate([tr.scores_out], env)[0], dtype=torch.float32)).all():
+            return False
+    return True
+
+
 def emit_functor(tr: TracedParallel, *, neg_inf_mask: bool, input_ctype: str, struct_name: str = "UserFunctor") -> FunctorSource:
     rs_names = list(tr.rowscale_in.keys())
     # ---------------- tile() ----------------
@@ -494,6 +511,7 @@ def emit_functor(tr: TracedParallel, *, neg_inf_mask: bool, input_ctype: str, st
   static constexpr bool kUnitOScale = {'true' if unit else 'false'};
   static constexpr bool kNegInfMask = {'true' if neg_inf_mask else 'false'};
   static constexpr bool kRowEpilogue = {'true' if elow.reduces else 'false'};
+  static constexpr bool kFiniteTail = {'true' if finite_tail(tr, neg_inf_mask) else 'false'};
   __device__ static void init(float* rs, const b200::RowCtx& c) {{
     {init_code}
   }}

@@ -12,6 +12,7 @@
 // With the KV role the lanes are KV rows and the columns query rows (S^T, dP^T), so that P^T and dS^T are the A
 // operands as they stand.  The functor F supplies
 //   F::kUsesStats            per-query-row statistics (softmax: lse and delta) travel with the query tiles
+//   F::kFiniteTail           without statistics: P and g are finite at a score of 0, so zero rows need no mask
 //   F::kNegInfMask           P and dS vanish at a score of -inf: masked pairs are given that score
 //   F::Ctx F::make(params)   per-thread constants
 //   F::score(s, lse2, ctx, b, h, q_idx, kv_idx, p_out, g_out)   P, and the factor g that turns dP into dS
@@ -418,9 +419,10 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
       const int kv_minus_q = (kRoleQ ? ys - tile : tile - ys) * T;   // of the tiles' first rows
       // So does a tile that the sequence ends in, where its columns past the end would not come out as zeros: their score is 0
       // (zero rows), and dS there is exp(-lse) times a finite value, which a row of strongly negative logits makes infinite --
-      // infinity times the zero rows of K is NaN for the whole row of dQ.  (Query rows past the end have lse = +inf.)
-      const int col_last = p.seq_kv - 1 - ys * T;
-      const bool tail = kRoleQ && col_last < T - 1;
+      // infinity times the zero rows of K is NaN for the whole row of dQ.  (Query rows past the end have lse = +inf; without
+      // statistics theirs are such columns too, where P or its derivative may be anything at a score of 0.)
+      const int col_last = (kRoleQ ? p.seq_kv : p.seq_q) - 1 - ys * T;
+      const bool tail = (F::kUsesStats ? kRoleQ : !F::kFiniteTail) && col_last < T - 1;
       const bool edge = kBits || tail || kv_minus_q + T - 1 > p.mask_right || kv_minus_q - (T - 1) < -p.mask_left;
       if constexpr (kBits) {
         const uint32_t* bits = kRoleQ ? p.bits_q : p.bits_kv;

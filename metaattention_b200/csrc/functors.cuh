@@ -10,6 +10,7 @@
 //   tile<N>(s, rs, ctx) -> o_scale in-place score tile -> probabilities for one row
 //   kSplitSum, tile_pieces  instead of tile(): rows that several threads share, see SoftmaxFunctor
 //   kRowEpilogue epilogue() reduces over the columns it is given: it gets a whole row of dim_v
+//   kFiniteTail  with kUnitOScale: tile() makes finite values of what stands for keys past the end of the sequence
 //   epilogue<N>(o, rs, ctx)        in-place transform of N accumulator columns
 //   final_rowscale(i, rs, ctx)     i-th per-row output
 //   combine(i, n, fin, ...)        split-KV: weight of split i among n (OnlineFunc.combine), from all splits' final

@@ -593,6 +593,14 @@ parallel_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int c = 0; c < TC / 32; ++c) {
           ctx.kv0 = kv0 + half * TC + c * 32;
           F::template tile<32>(reinterpret_cast<float(&)[32]>(s[c * 32]), rs, ctx);
+          // keys past the end of the sequence weigh nothing: a weight that is not finite, times their zero rows of V, would be
+          // NaN.  (On functors that need none of it these lines cost 9 % of sigmoid 7 x 8 x 3544 x 64.)
+          if constexpr (!F::kFiniteTail) {
+            if (kv0 + BN > p.seq_kv) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i) s[c * 32 + i] = ctx.kv0 + i < p.seq_kv ? s[c * 32 + i] : 0.0f;
+            }
+          }
           uint32_t pk[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = pack2<kBf16>(s[c * 32 + 2 * i], s[c * 32 + 2 * i + 1]);

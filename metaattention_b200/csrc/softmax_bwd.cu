@@ -19,7 +19,7 @@ namespace b200 {
 // The built-in softmax: P = exp2(s * scale * log2e - lse2), dS = P (dP - delta) * scale; the scale is left to the
 // finished dK and dQ rows.
 struct SoftmaxBwdFunctor {
-  static constexpr bool kUsesStats = true;
+  static constexpr bool kUsesStats = true, kFiniteTail = false;
   static constexpr bool kNegInfMask = true;
   struct Ctx {
     float c2, scale;

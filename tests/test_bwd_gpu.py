@@ -384,3 +384,26 @@ def test_strongly_negative_logits_beside_the_end_of_the_sequence(Sq, Skv, D, kin
     mask = {"none": (lib.MASK_NONE,), "causal": (lib.MASK_CAUSAL,), "window": (lib.MASK_BAND, (89, 89))}[kind]
     for got, ref, what in zip(lib.softmax_bwd(*args, scale, *mask), want, ("dq", "dk", "dv")):
         check(got, ref, what)
+
+
+@pytest.mark.parametrize("S,D", [(333, 64), (200, 128)])
+def test_elementwise_program_that_is_infinite_or_undefined_outside_the_sequence(S, D):
+    """P = |score| as exp(log(score^2) / 2): infinite at the -inf of a masked score, its derivative undefined at the 0 of a zero
+    row.  Neither reaches the result or a gradient from the rows that the last tiles have past the ends."""
+    from attn_engine import AttentionEngine
+    from core import CustomIO, meta_tensor
+
+    def score_mod(score, custom, b, h, q_idx, kv_idx):
+        x = score * (4.0 / (S * D ** 0.5))
+        return ((x * x).log() * 0.5).exp()
+    meta = meta_tensor(1, 2, S, D, dtype=torch.bfloat16)
+    eng = AttentionEngine((meta, meta, meta), CustomIO({}), score_mod=score_mod, mask_mod=None, online_func=None)
+    gen = torch.Generator().manual_seed(S)
+    q, k, v, d_o = (torch.randn(1, S, 2, D, generator=gen).to(torch.bfloat16) for _ in range(4))
+    leaves = [t.double().requires_grad_() for t in (q, k, v)]
+    o = torch.einsum("bhqk,bkhd->bqhd", (torch.einsum("bqhd,bkhd->bhqk", *leaves[:2]) * (4.0 / (S * D ** 0.5))).abs(), leaves[2])
+    got = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o2 = eng(*got)
+    check(o2.detach(), o.detach(), "o")
+    for g, w, what in zip(torch.autograd.grad(o2, got, d_o.cuda()), torch.autograd.grad(o, leaves, d_o.double()), ("dq", "dk", "dv")):
+        check(g, w, what)
