@@ -98,8 +98,8 @@ def mla_decode_forward(q, kv, dim_v: int, scale: float, q_rope=None, kv_rope=Non
     to be faster for equal lengths.
     Returns (o [B,H,dim_v] in the input dtype, lse [B,H] fp32)."""
     global last_plan
-    r = native.host().mla_decode(q, kv, dim_v, scale, q_rope, kv_rope, num_splits, workspace, cache_seqlens, block_table, max_seqlen,
-                                 tile_scheduler_metadata, num_splits_cum)
+    r = native.host().mla_decode(q, kv, dim_v, float(scale), q_rope, kv_rope, num_splits, workspace, cache_seqlens, block_table,
+                                 None if max_seqlen is None else int(max_seqlen), tile_scheduler_metadata, num_splits_cum)
     if isinstance(r, int):
         _refuse(r, q, kv, q_rope, kv_rope, dim_v)
     o, lse, splits, parts = r

@@ -181,3 +181,13 @@ def test_refusals_of_linear_and_mla_calls_keep_their_errors():
         mla_decode_forward(torch.zeros(2, 2, 128, 576), torch.zeros(2, 64, 576), 512, 1.0)
     with pytest.raises(ValueError, match="kv: expected .batch, rows, cols. with contiguous columns"):
         mla_decode_forward(torch.zeros(2, 128, 576), torch.zeros(2, 576, 64).transpose(1, 2), 512, 1.0)
+
+
+def test_mla_lengths_may_be_any_number():
+    """max_seqlen and scale as what a program computes them as; the call is refused for its CPU tensors, not for their type"""
+    from attn_engine.mla import mla_decode_forward
+    from core.native.lib import NativeError
+    table = torch.zeros(2, 1, dtype=torch.int32)
+    for length in (64, 64.0, torch.tensor(64), torch.tensor(64.0)):
+        with pytest.raises(NativeError, match="needs CUDA tensors"):
+            mla_decode_forward(torch.zeros(2, 128, 576), torch.zeros(2, 64, 576), 512, torch.tensor(0.5), block_table=table, max_seqlen=length)
