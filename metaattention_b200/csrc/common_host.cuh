@@ -12,6 +12,16 @@ namespace b200 {
 // attn_b200_last_device_status() has read (and thereby cleared) it.
 int* device_status_word(int device);
 
+// SMs of the current device, 0 if it cannot be asked.
+inline int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return sms;
+}
+
 // Launches a kernel that passes pdl_wait() before it touches memory (sm100.cuh has the rules): it may be made ready while the
 // one in front of it in the stream still runs (behind anything but a kernel that calls pdl_launch_dependents() it starts as
 // usual).  Two calls of 1 x 16 / 4 x 333 x 64 one after the other: 10.4 us each without, 8.2 with; the launches inside a

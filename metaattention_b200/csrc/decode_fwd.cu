@@ -659,15 +659,6 @@ inline int plan_decode(const AttnB200DecodeArgs* a, int sms, DecodePlan* d) {
   return ATTN_B200_OK;
 }
 
-inline int device_sms() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return sms;
-}
-
 template <int D, bool kBf16, bool kCounted>
 int launch_decode(const AttnB200DecodeArgs* a, const DecodePlan& d, cudaStream_t stream, int* status) {
   using L = DecodeSmem<D, kCounted>;

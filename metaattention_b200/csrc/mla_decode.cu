@@ -908,15 +908,6 @@ inline int mla_num_parts(int heads_q, int sm_count) {
   return std::max(1, sm_count / 2 / head_blocks);
 }
 
-inline int current_sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return sms;
-}
-
 // Scheduled mode: layout of the workspace -- scheduler records, cumulative split counts, then the partial rows.
 struct MlaSchedLayout {
   int parts;
@@ -1020,7 +1011,7 @@ int launch_mla(const AttnB200MlaArgs* a, cudaStream_t stream, int* status) {
   dim3 grid(2, splits * p.head_blocks, s.batch);  // x = the two CTAs of a cluster
   if (scheduled) {
     // one cluster per SM pair and head block runs the units the scheduler gives it
-    const int parts = a->sched_meta != nullptr ? a->sched_parts : mla_num_parts(s.heads_q, current_sm_count());
+    const int parts = a->sched_meta != nullptr ? a->sched_parts : mla_num_parts(s.heads_q, device_sms());
     if (parts <= 0) return ATTN_B200_E_INVALID_ARG;
     const MlaSchedLayout lay(s, parts);
     uint8_t* ws = static_cast<uint8_t*>(a->workspace);
@@ -1142,7 +1133,7 @@ int attn_b200_mla_metadata(const int32_t* cache_seqlens, int32_t batch, int32_t 
 int64_t attn_b200_mla_workspace_bytes(const AttnB200MlaShape* shape, int32_t num_splits) {
   if (b200::validate_mla_shape(shape) != ATTN_B200_OK || num_splits < 0) return -1;
   if (num_splits == 0) {   // scheduled mode on the current device
-    const int sms = b200::current_sm_count();
+    const int sms = b200::device_sms();
     if (sms <= 0) return -1;
     return b200::MlaSchedLayout(*shape, b200::mla_num_parts(shape->heads_q, sms)).bytes;
   }

@@ -191,8 +191,8 @@ int launch_parallel(const AttnB200ParallelArgs* a, cudaStream_t stream, int* dev
     return ATTN_B200_E_LAUNCH;
   }
   dim3 grid((a->seq_q + NT * L::kBM - 1) / (NT * L::kBM), a->heads, a->batch * splits);
-  const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z;   // up to one an SM (148) all start at once, in any order
-  if (a->mask_kind == ATTN_B200_MASK_CAUSAL && ctas > 148 && ctas < 0x7fffffffLL)
+  const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z;   // up to one an SM all start at once, in any order
+  if (a->mask_kind == ATTN_B200_MASK_CAUSAL && ctas > device_sms() && ctas < 0x7fffffffLL)
     p.heads_at_once = heavy_heads_at_once(static_cast<long long>(a->seq_kv) * (D + DV) * 2 / p.kv_group, static_cast<long long>(grid.y) * grid.z);
   if (!launch_pdl(kernel, grid, dim3(kParallelThreads<NT, kRowThreads<F>>), kSmem, stream, tmQ, tmK, tmV, p)) return ATTN_B200_E_LAUNCH;
   if (splits > 1) {
