@@ -133,36 +133,36 @@ def test_refusals_of_the_library_arrive_as_its_error():
 
 
 def _chains():
-    """Calls whose output is the next call's input, one per kernel family: name -> (start tensors, step)."""
+    """Calls whose output is the next call's input as it stands, one per kernel family: name -> (start tensor, step).  No torch
+    kernel runs between two calls: it would end before the next of the library's kernels is made ready."""
+    from attn_engine.mla import mla_decode_forward
     gen = torch.Generator(device="cuda").manual_seed(3)
 
     def rnd(*shape):
         return torch.randn(*shape, generator=gen, device="cuda").to(torch.bfloat16)
-    k, v = rnd(1, 700, 4, 64), rnd(1, 700, 4, 64)
+    k, v, ones = rnd(1, 700, 4, 64), rnd(1, 700, 4, 64), torch.ones(1, 700, 4, 64, device="cuda", dtype=torch.bfloat16)
     prefill = programs.softmax_engine(1, 4, 700, 64, 64, is_causal=True)
     decode = programs.gqa_engine(2, 8, 2, 1, 900, 128, 128)
     dk, dv = rnd(2, 900, 2, 128), rnd(2, 900, 2, 128)
     lin = programs.gla_engine(1, 4, 600, 128, 128)
-    lk, lv, lg = rnd(1, 4, 600, 128), rnd(1, 4, 600, 128), torch.full((1, 4, 600), -0.3, device="cuda")
-    kv = rnd(2, 500, 576)
+    lk, lv, lg, ld = rnd(1, 4, 600, 128), rnd(1, 4, 600, 128), torch.full((1, 4, 600), -0.3, device="cuda"), rnd(1, 4, 600, 128) * 0.1
+    lk.requires_grad_()
+    lg_leaf = lg.clone().requires_grad_()
+    kv, q_rope = rnd(2, 500, 576), rnd(2, 128, 64)
 
-    def mla(q):
-        from attn_engine.mla import mla_decode_forward
-        o, _ = mla_decode_forward(q, kv, 512, 576 ** -0.5, num_splits=0)
-        return torch.cat([o, q[..., 512:]], -1)
+    def mla(q):   # the output's 512 columns are the next call's
+        return mla_decode_forward(q, kv[..., :512], 512, 576 ** -0.5, q_rope=q_rope, kv_rope=kv[..., 512:], num_splits=0)[0]
 
     def train(x):
         x = x.detach().requires_grad_()
-        return torch.autograd.grad(prefill(x, k, v), x, torch.ones_like(x))[0] * 100 + k
+        return torch.autograd.grad(prefill(x, k, v), x, ones)[0]
 
-    def train_linear(x):
-        x = x.detach().requires_grad_()
-        g = lg.detach().requires_grad_()
-        dx, dg = torch.autograd.grad(lin(x, lk, lv, g), (x, g), lv)
-        return dx + dg[..., None].to(dx.dtype)
+    def train_linear(x):   # dk depends on q (dq would not), and is the next call's q
+        return torch.autograd.grad(lin(x, lk, lv, lg_leaf), (lk, lg_leaf), ld)[0]
     return {"prefill": (rnd(1, 700, 4, 64), lambda x: prefill(x, k, v)), "train": (rnd(1, 700, 4, 64), train),
-            "decode": (rnd(2, 1, 8, 128), lambda x: decode(x, dk, dv)), "linear": (rnd(1, 4, 600, 128), lambda x: lin(x, lk, lv, lg)),
-            "linear_train": (rnd(1, 4, 600, 128), train_linear), "mla": (rnd(2, 128, 576), mla)}
+            "decode": (rnd(2, 1, 8, 128), lambda x: decode(x, dk, dv)),
+            "linear": (rnd(1, 4, 600, 128), lambda x: lin(x, lk.detach(), lv, lg)),
+            "linear_train": (rnd(1, 4, 600, 128), train_linear), "mla": (rnd(2, 128, 512), mla)}
 
 
 @pytest.mark.parametrize("name", ["prefill", "train", "decode", "linear", "linear_train", "mla"])
