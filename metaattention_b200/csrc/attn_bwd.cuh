@@ -5,7 +5,7 @@
 //
 // One kernel template in two roles.  A CTA keeps one 128-row tile pair resident (X: K_j, V_j or Q_i, dO_i) and streams
 // the other (Y1: Q_i or K_j through a three-stage TMA ring, Y2: dO_i or V_j through a two-stage one).  Per streamed tile:
-//   S  = X1 Y1^T, dP = X2 Y2^T           tcgen05 SS, fp32 in tensor memory (columns [0,128) and [128,256))
+//   S  = X1 Y1^T, dP = X2 Y2^T           tcgen05 SS, fp32 in tensor memory (attn_bwd_cta has the columns)
 //   row threads (thread = TMEM lane x column half): P and dS as 16-bit pairs
 //   acc1 += P  Y2   (dV; KV role only)    tcgen05 TS, A from tensor memory, B = the streamed tile MN-major
 //   acc2 += dS Y1   (dK or dQ)
@@ -315,7 +315,9 @@ __device__ __forceinline__ void attn_bwd_cta(const CUtensorMap& tmQ, const CUten
           if (!wait(y1_full + s1, (it / N1) & 1, kBwdYFull)) break;
           // the buffer's last contents are in the row threads' registers.  The row threads learn from s_full and dp_full
           // what else they need for a tile (every barrier that they look at costs them 50-200 cycles behind their
-          // exponentials): the statistics came with the tiles waited for here; query role: dS's buffer has been read
+          // exponentials): query role: dS's buffer has been read; KV role: the statistics have arrived.  They came by bulk
+          // copies on the tiles' barriers, which this warp waits for and the row threads do not: that the row threads see them
+          // rests on this wait, the commit behind it and their own wait for that commit.
           if (it > 0 && !(kShared ? wait(dp_free, (it - 1) & 1, kBwdDpFree) : wait(s_free, (it - 1) & 1, kBwdSFree))) break;
           issue_xy(kColS, x1_desc, sY1 + s1 * L::kTileBytes, s_full, nullptr);
           if (kShared && it > 0 && lane == 0) mbar_arrive(s_issued);

@@ -17,8 +17,8 @@
 //     unit through tensor memory (both accumulators of a row are in the lane of its thread).  With one group the warp that
 //     holds the only used rows is the bound: ~1600 cycles a tile, against 1480 for the bytes of a 64-wide tile;
 //   * K and V each have a ring of 96 KB: ~190 KB in flight per SM, three times what latency times bandwidth asks for.
-// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 94 us = 5.7 TB/s of K and V, x 4312
-// tokens 23.7 (25.2 before the first loads went ahead of the CTA's set-up and the merge kernel fetched its code early); 8
+// Measured (calls back to back, bf16, D = 128): 1 sequence x 32 heads x 32768 tokens 93-103 us from box to box = 5.2-5.8 TB/s of
+// K and V, x 4312 tokens 23.7-28 (25.2 before the first loads went ahead of the CTA's set-up and the merge kernel fetched its code early); 8
 // sequences x 32 heads on 8 KV heads, up to 8192 tokens, 30 % of the 32-token blocks kept 38 -> 30: of its 26 us in the
 // kernel 8 went to counting the mask at four flags a load, 2 to a list of kept blocks made the same way, 2 to boxes issued
 // by one lane.  8 such sequences of 16384 tokens, dense: 5.8 TB/s.

@@ -452,7 +452,8 @@ linear_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
     };
 
     // (Products of the row phases go two elements to an instruction: the phases are the block's serial chain.  Training step of
-    // gated retention 2 x 8 x 2000 211 -> 198 us, gated retention 2 x 16 x 1573 x 256 58.8 -> 54.8, retention 8 x 8 x 4096 331 -> 323.)
+    // gated retention 2 x 8 x 2000 211 -> 198 us, gated retention 2 x 16 x 1573 x 256 58.8 -> 54.8, 8 x 8 x 2000 x 256 / 512 209 -> 198,
+    // retention 8 x 8 x 4096 338 -> 331 on one box.)
     // Rows of V times their decay factors, the A operand of the state update: token `row` of block tb's V (chunk `wg`)
     // is multiplied by exp(g_last - g_row).  Every 16-byte piece of the row gets the same factor, so neither the
     // swizzle nor the order matters: lanes start at different pieces to stay off each other's banks (rows are 128
